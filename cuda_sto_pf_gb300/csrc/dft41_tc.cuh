@@ -298,7 +298,7 @@ k_y246tc(Grid3 g, const float2 *tw_g, const float4 *btab, AxisIO<float, 6, 6> io
     if (warp == 0) tc41::tmem_alloc(&tbase, tc41::TMEM_COLS);
     if (threadIdx.x == 0) tc41::mbar_init(&mbar);
     const int k0 = blockIdx.x * TC, i = blockIdx.y;
-    const int kcnt = min(TC, g.NzC - k0);
+    const int kcnt = min(TC, g.NzK - k0);
     const long long base = (long long)i * N * g.NzC + k0;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
@@ -307,11 +307,12 @@ k_y246tc(Grid3 g, const float2 *tw_g, const float4 *btab, AxisIO<float, 6, 6> io
             const int t = 2 * tp;
             float2 *dst = buf + y * PS + s * TC + t;
             const float2 *src = io.in[s] + base + (long long)y * g.NzC + t;
-            if (t + 1 < kcnt) {
+            const bool keep = DIR < 0 || !g.cut_row(y);
+            if (keep && t + 1 < kcnt) {
                 const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src));
             } else {
-                dst[0] = t < kcnt ? src[0] : make_float2(0.f, 0.f);
+                dst[0] = keep && t < kcnt ? src[0] : make_float2(0.f, 0.f);
                 dst[1] = make_float2(0.f, 0.f);
             }
         }
@@ -337,6 +338,7 @@ k_y246tc(Grid3 g, const float2 *tw_g, const float4 *btab, AxisIO<float, 6, 6> io
         for (int e = threadIdx.x; e < N * TP; e += blockDim.x) {
             const int tp = e % TP, y = e / TP;
             const int t = 2 * tp;
+            if (DIR < 0 && g.cut_row(y)) continue;
             const float2 *srcs = buf + y * PS + s * TC + t;
             float2 *dst = io.out[s] + base + (long long)y * g.NzC + t;
             if (t + 1 < kcnt) *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(srcs);

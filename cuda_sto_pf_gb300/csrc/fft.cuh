@@ -437,10 +437,29 @@ __device__ __forceinline__ void load_tw(cplx_t<T> *s, const cplx_t<T> *g, int n)
     for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = g[i];
 }
 
-// 3D grid description passed to every pass kernel
+// 3D grid description passed to every pass kernel.  A solver's grid carries
+// the 2/3 dealias rule as the box of modes it keeps: kz < NzK and ky rows
+// outside [jc0, jc1).  Every x pass of the solver masks its result with that
+// rule, so the passes around it move and transform only what the box holds:
+// a z pass reads and writes the columns kz < NzK, a forward y pass writes and
+// an inverse y pass reads the kept rows (the others count as zero), and an x
+// pass runs over kept columns and rows alone.  What lies outside the box is
+// never read.  That is 4/9 of an x pass and 2/3 of the columns elsewhere, with
+// bitwise the results of the full passes.  Plain transforms keep everything
+// (NzK = NzC, jc0 = jc1 = Ny).
 struct Grid3 {
     int Nx, Ny, Nz, NzC;
     long long N, Nk;
+    int NzK, jc0, jc1;
+    __host__ void keep_all() { NzK = NzC; jc0 = jc1 = Ny; }
+    __host__ __device__ int kept_rows() const { return Ny - (jc1 - jc0); }
+    // spectral points of one array that a z pass (all rows) and an x pass
+    // (kept rows) move
+    __host__ double cols() const { return (double)Nx * Ny * NzK; }
+    __host__ double kept() const { return (double)Nx * kept_rows() * NzK; }
+    // the b-th kept ky row
+    __device__ __forceinline__ int kept_row(int b) const { return b < jc0 ? b : b + (jc1 - jc0); }
+    __device__ __forceinline__ bool cut_row(int j) const { return j >= jc0 && j < jc1; }
 };
 
 // ---------------------------------------------------------------------------
@@ -477,19 +496,22 @@ k_axis_pass(Grid3 g, int axis, AxisPlan plan, const cplx_t<T> *tw_g, int TK,
     constexpr bool INPL = Op::kInplace;   // identity op: outputs are the inputs
 
     const int k0 = blockIdx.x * TK;
-    const int slab = blockIdx.y;       // i for the y pass, j for the x pass
+    const int slab = axis == 1 ? blockIdx.y : g.kept_row(blockIdx.y);   // i for the y pass, j for the x pass
     long long base, es;
     if (axis == 1) { base = (long long)slab * g.Ny * g.NzC + k0; es = g.NzC; }
     else { base = (long long)slab * g.NzC + k0; es = (long long)g.Ny * g.NzC; }
-    const int kcnt = min(TK, g.NzC - k0);
+    const int kcnt = min(TK, g.NzK - k0);
     const int lgTK = __ffs(TK) - 1;    // TK is a power of two
+    // rows cut by the dealias rule: zero into an inverse y pass, not written
+    // by a forward one
+    const int z0 = axis == 1 ? g.jc0 : n, z1 = axis == 1 ? g.jc1 : n;
 
     if (DIN != 0 || DOUT != 0) load_tw<T>(tw, tw_g, n);
 #pragma unroll
     for (int a = 0; a < NIN; ++a) {
         for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
             const int q = e >> lgTK, l = e & (TK - 1);
-            const bool ok = l < kcnt;
+            const bool ok = l < kcnt && !(DIN > 0 && q >= z0 && q < z1);
             cp_async_elem(&A[q * SPI + a * TK + l], io.in[a] + (ok ? base + q * es + l : base), ok);
         }
     }
@@ -527,7 +549,7 @@ k_axis_pass(Grid3 g, int axis, AxisPlan plan, const cplx_t<T> *tw_g, int TK,
     for (int a = 0; a < NOUT; ++a) {
         for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
             const int q = e >> lgTK, l = e & (TK - 1);
-            if (l < kcnt) io.out[a][base + q * es + l] = cur[q * SP + a * TK + l];
+            if (l < kcnt && !(DIN < 0 && q >= z0 && q < z1)) io.out[a][base + q * es + l] = cur[q * SP + a * TK + l];
         }
     }
 }
@@ -619,7 +641,7 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
         for (int e = threadIdx.x; e < R * nc; e += blockDim.x) {
             const int rr = e / nc, k = e - rr * nc;
             T2 v[NFI > 0 ? NFI : 1];
-            if (rr < rcnt) op.load_spec(row0 + rr, k, v);
+            if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
             else {
 #pragma unroll
                 for (int f = 0; f < NFI; ++f) v[f] = mk2<T2>(T(0), T(0));
@@ -639,12 +661,12 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
             const int ra = la / (NFI > 0 ? NFI : 1), fa = la - ra * (NFI > 0 ? NFI : 1);
             const int rb = lb / (NFI > 0 ? NFI : 1), fb = lb - rb * (NFI > 0 ? NFI : 1);
             T2 v[NFI > 0 ? NFI : 1];
-            if (ra < rcnt) {
+            if (ra < rcnt && k < g.NzK) {
                 op.load_spec(row0 + ra, k, v);
                 A = v[fa];
                 if (rb == ra) B = v[fb];
             }
-            if (rb != ra && rb < rcnt) {
+            if (rb != ra && rb < rcnt && k < g.NzK) {
                 op.load_spec(row0 + rb, k, v);
                 B = v[fb];
             }
@@ -726,8 +748,9 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
         T2 *r = fft_lines<T, -1>(outA, outB, plan, tw, PO_, 1, n, true);
         if (r != outA) { outB = outA; outA = r; }
         // unpack and store: per (row, kz) gather all NFO fields
-        for (int e = threadIdx.x; e < rcnt * nc; e += blockDim.x) {
-            const int rr = e / nc, k = e - rr * nc;
+        const int nk = g.NzK;
+        for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
+            const int rr = e / nk, k = e - rr * nk;
             T2 v[NFO > 0 ? NFO : 1];
 #pragma unroll
             for (int f = 0; f < NFO; ++f) {

@@ -147,7 +147,7 @@ k_y246(Grid3 g, const float2 *tw_g, AxisIO<float, 6, 6> io, const double *skip) 
     float2 *tw = reinterpret_cast<float2 *>(smem_raw);
     float2 *buf = tw + N;
     const int k0 = blockIdx.x * YC, i = blockIdx.y, h = blockIdx.z;
-    const int kcnt = min(YC, g.NzC - k0);
+    const int kcnt = min(YC, g.NzK - k0);
     const long long base = (long long)i * N * g.NzC + k0;   // (i, y = 0, k0)
     // 16-byte copies: (spectrum, y, column pair); the spectrum loop is
     // unrolled and the half picked by a select, so that every io.in index is
@@ -160,11 +160,12 @@ k_y246(Grid3 g, const float2 *tw_g, AxisIO<float, 6, 6> io, const double *skip) 
             const int t = 2 * tp;
             float2 *dst = buf + y * PSTR + s * YC + t;
             const float2 *src = in + (long long)y * g.NzC + t;
-            if (t + 1 < kcnt) {
+            const bool keep = DIR < 0 || !g.cut_row(y);
+            if (keep && t + 1 < kcnt) {
                 const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src));
             } else {
-                dst[0] = t < kcnt ? src[0] : make_float2(0.f, 0.f);
+                dst[0] = keep && t < kcnt ? src[0] : make_float2(0.f, 0.f);
                 dst[1] = make_float2(0.f, 0.f);
             }
         }
@@ -181,6 +182,7 @@ k_y246(Grid3 g, const float2 *tw_g, AxisIO<float, 6, 6> io, const double *skip) 
         for (int e = threadIdx.x; e < N * TP; e += blockDim.x) {
             const int tp = e % TP, y = e / TP;
             const int t = 2 * tp;
+            if (DIR < 0 && g.cut_row(y)) continue;
             const float2 *srcs = buf + y * PSTR + s * YC + t;
             float2 *dst = out + (long long)y * g.NzC + t;
             if (t + 1 < kcnt) *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(srcs);
@@ -213,8 +215,9 @@ k_axis246(Grid3 g, int axis, const float2 *tw_g, AxisIO<float, NIN, NOUT> io, Op
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *tw = reinterpret_cast<float2 *>(smem_raw);
     float2 *buf = tw + N;
-    const int k0 = blockIdx.x * TCW, slab = blockIdx.y;
-    const int kcnt = min(TCW, g.NzC - k0);
+    const int k0 = blockIdx.x * TCW, slab = axis == 1 ? blockIdx.y : g.kept_row(blockIdx.y);
+    const int kcnt = min(TCW, g.NzK - k0);
+    const int z0 = axis == 1 ? g.jc0 : N, z1 = axis == 1 ? g.jc1 : N;   // cut rows of a y pass
     long long base, es;
     if (axis == 1) { base = (long long)slab * N * g.NzC + k0; es = g.NzC; }
     else { base = (long long)slab * g.NzC + k0; es = (long long)g.Ny * g.NzC; }
@@ -225,11 +228,12 @@ k_axis246(Grid3 g, int axis, const float2 *tw_g, AxisIO<float, NIN, NOUT> io, Op
             const int t = 2 * tp;
             float2 *dst = buf + q * PSTR + s * TCW + t;
             const float2 *src = io.in[s] + base + (long long)q * es + t;
-            if (t + 1 < kcnt) {
+            const bool keep = DIN <= 0 || q < z0 || q >= z1;
+            if (keep && t + 1 < kcnt) {
                 const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src));
             } else {
-                dst[0] = t < kcnt ? src[0] : make_float2(0.f, 0.f);
+                dst[0] = keep && t < kcnt ? src[0] : make_float2(0.f, 0.f);
                 dst[1] = make_float2(0.f, 0.f);
             }
         }
@@ -259,6 +263,7 @@ k_axis246(Grid3 g, int axis, const float2 *tw_g, AxisIO<float, NIN, NOUT> io, Op
         for (int e = threadIdx.x; e < N * TPW; e += blockDim.x) {
             const int tp = e % TPW, q = e / TPW;
             const int t = 2 * tp;
+            if (DIN < 0 && q >= z0 && q < z1) continue;
             const float2 *srcs = buf + q * PSTR + s * TCW + t;
             float2 *dst = io.out[s] + base + (long long)q * es + t;
             if (t + 1 < kcnt) *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(srcs);

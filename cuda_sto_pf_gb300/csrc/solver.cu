@@ -385,7 +385,7 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
     auto kern = k_axis_pass<T, NIN, NOUT, DIN, DOUT, Op>;
     int dev = 0;
     cudaGetDevice(&dev);
-    const int gy = axis == 1 ? c->g.Nx : c->g.Ny;
+    const int gy = axis == 1 ? c->g.Nx : c->g.kept_rows();
     const TileKey key{dev, (const void *)kern, pl.n, c->g.NzC, gy};
     {
         std::lock_guard<std::mutex> lk(g_tile_mu);
@@ -405,10 +405,10 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
                 for (int b = 0; b < NOUT; ++b) io[i].out[b] = (T2 *)ts.sc[i]->p[NIN + b];
             }
             for (int tk = 1; tk <= 32; tk <<= 1) {
-                if (tk > 1 && tk / 2 >= c->g.NzC) break;
+                if (tk > 1 && tk / 2 >= c->g.NzK) break;
                 const size_t smem = bytes(tk);
                 if (smem > kSmemWide || allow_smem(kern, smem) != cudaSuccess) break;
-                const dim3 grid((c->g.NzC + tk - 1) / tk, gy);
+                const dim3 grid((c->g.NzK + tk - 1) / tk, gy);
                 const T2 *tw = twp<T>(c, axis == 1 ? 1 : 0);
                 const float t = time_launch(ts.ss, [&](int i) {
                     kern<<<grid, 256, smem, ts.ss[i]>>>(c->g, axis, pl, tw, tk, io[i], op, nullptr);
@@ -474,6 +474,15 @@ static int tuned_r(pfgb_ctx *c, int rule, size_t (*bytes)(int, int), const char 
     return g_tiles.emplace(key, rec).first->second.tile;
 }
 
+// algorithmic bytes of an x pass (kept rows both ways) or a y pass (all rows
+// on its real-y side, kept rows on its spectral side)
+template <typename T2>
+static double axis_bytes(const pfgb_ctx *c, int axis, int nin, int nout, int din) {
+    const double kept = c->g.kept(), cols = c->g.cols();
+    const double in = axis == 1 && din < 0 ? cols : kept, out = axis == 1 && din > 0 ? cols : kept;
+    return (nin * in + nout * out) * sizeof(T2);
+}
+
 template <typename T, int NIN, int NOUT, int DIN, int DOUT, class Op>
 static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, Op op, const char *tag) {
     using T2 = cplx_t<T>;
@@ -486,8 +495,8 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
             const size_t smem = f246::axis_smem_bytes();
             auto kern = k_axis246<NIN, NOUT, DIN, DOUT, Op>;
             PFGB_CUDA_TRY(allow_smem(kern, smem));
-            dim3 grid((c->g.NzC + TCW - 1) / TCW, axis == 1 ? c->g.Nx : c->g.Ny);
-            ProfScope ps(c, {tag, (double)(NIN + NOUT) * (double)c->g.Nk * sizeof(T2)});
+            dim3 grid((c->g.NzK + TCW - 1) / TCW, axis == 1 ? c->g.Nx : c->g.kept_rows());
+            ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
             kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, axis, (const float2 *)twp<T>(c, axis == 1 ? 1 : 0),
                                                          io, op, c->skip);
             PFGB_CUDA_TRY(cudaGetLastError());
@@ -499,13 +508,13 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
     int TK = 16;
     while (TK > 1 && bytes(TK) > kSmemBudget) TK >>= 1;
     if (TK < 4 && sizeof(T) == 4 && bytes(4) <= kSmemWide) TK = 4;
-    while (TK > 1 && TK / 2 >= c->g.NzC) TK >>= 1;
+    while (TK > 1 && TK / 2 >= c->g.NzK) TK >>= 1;
     if (c->p.fft_autotune & 1) TK = tuned_tk<T, NIN, NOUT, DIN, DOUT, Op>(c, axis, pl, op, TK, tag);
     const size_t smem = bytes(TK);
     auto kern = k_axis_pass<T, NIN, NOUT, DIN, DOUT, Op>;
     PFGB_CUDA_TRY(allow_smem(kern, smem));
-    dim3 grid((c->g.NzC + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.Ny);
-    ProfScope ps(c, {tag, (double)(NIN + NOUT) * (double)c->g.Nk * sizeof(T2)});
+    dim3 grid((c->g.NzK + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.kept_rows());
+    ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
     kern<<<grid, 256, smem, c->stream>>>(c->g, axis, pl, twp<T>(c, axis == 1 ? 1 : 0), TK, io, op, c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
@@ -540,7 +549,7 @@ k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
         for (int e = threadIdx.x; e < R * NC; e += blockDim.x) {
             const int rr = e / NC, k = e - rr * NC;
             float2 v[NFI];
-            if (rr < rcnt) op.load_spec(row0 + rr, k, v);
+            if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
             else {
 #pragma unroll
                 for (int f = 0; f < NFI; ++f) v[f] = make_float2(0.f, 0.f);
@@ -601,8 +610,9 @@ k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
     if constexpr (NFO > 0) {
         __syncthreads();
         lines<-1, 1, N>(buf, tw);
-        for (int e = threadIdx.x; e < rcnt * NC; e += blockDim.x) {
-            const int rr = e / NC, k = e - rr * NC;
+        const int nk = g.NzK;
+        for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
+            const int rr = e / nk, k = e - rr * nk;
             float2 v[NFO];
 #pragma unroll
             for (int f = 0; f < LO; ++f) {
@@ -631,7 +641,7 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
             PFGB_CUDA_TRY(allow_smem(kern, smem));
             const long long rows = (long long)c->g.Nx * c->g.Ny;
             const int nb = (int)((rows + R - 1) / R);
-            ProfScope ps(c, {tag, (double)(NFI + NFO) * (double)c->g.Nk * sizeof(T2) + extra_bytes});
+            ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
             kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)twp<T>(c, 2), op, c->skip);
             PFGB_CUDA_TRY(cudaGetLastError());
             if (nblocks) *nblocks = nb;
@@ -648,7 +658,7 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     auto kern = k_zpass<T, NFI, NFO, Op>;
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     const int nb = (int)((rows + R - 1) / R);
-    ProfScope ps(c, {tag, (double)(NFI + NFO) * (double)c->g.Nk * sizeof(T2) + extra_bytes});
+    ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
     kern<<<nb, 256, smem, c->stream>>>(c->g, c->plz, twp<T>(c, 2), R, op, c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     if (nblocks) *nblocks = nb;
@@ -2109,10 +2119,10 @@ k_x_green(GreenArgs<TE> A, AxisPlan plan, int TK) {
     const int n = plan.n, SP = 6 * TK + 1;   // six components interleaved per row
     T2 *tw = sm;
     T2 *X = sm + n, *Yb = X + n * SP;
-    const int k0 = blockIdx.x * TK, j = blockIdx.y;
+    const int k0 = blockIdx.x * TK, j = A.g.kept_row(blockIdx.y);
     const long long base = (long long)j * A.g.NzC + k0;
     const long long es = (long long)A.g.Ny * A.g.NzC;
-    const int kcnt = min(TK, A.g.NzC - k0);
+    const int kcnt = min(TK, A.g.NzK - k0);
     const int lgTK = __ffs(TK) - 1;
 #pragma unroll
     for (int cmp = 0; cmp < 6; ++cmp) {
@@ -2253,7 +2263,7 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
     int TK = 16;
     while (TK > 1 && bytes(TK) > kSmemBudget) TK >>= 1;
     if (TK < 4 && sizeof(TE) == 4 && bytes(4) <= kSmemWide) TK = 4;
-    while (TK > 1 && TK / 2 >= c->g.NzC) TK >>= 1;
+    while (TK > 1 && TK / 2 >= c->g.NzK) TK >>= 1;
     const size_t smem = bytes(TK);
     GreenArgs<TE> A;
     A.g = c->g;
@@ -2272,10 +2282,10 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
     A.tc_err = c->tc_err;
     A.resid = resid;
     A.mode = mode;
-    dim3 grid((c->g.NzC + TK - 1) / TK, c->g.Ny);
+    dim3 grid((c->g.NzK + TK - 1) / TK, c->g.kept_rows());
     // reads 6 source spectra (+3 old u for the residual), writes 3 u + 6 strain spectra
     ProfScope ps(c, {eigen ? "x_green_eigen" : "x_green_hij",
-                     (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * (double)c->g.Nk * sizeof(T2)});
+                     (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(T2)});
     if (eigen) {
         auto kern = k_x_green<TE, true>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
@@ -2312,8 +2322,8 @@ k_x_green246(GreenArgs<float> A) {
     float2 *tw = reinterpret_cast<float2 *>(smem_raw + (TCS ? 2 * tc41::B_BYTES : 0));
     float2 *buf = tw + N;
     if constexpr (TCS) tc41::begin(&tc_tbase, &tc_mbar, bt, A.btab);
-    const int k0 = blockIdx.x * TC, j = blockIdx.y;
-    const int kcnt = min(TC, A.g.NzC - k0);
+    const int k0 = blockIdx.x * TC, j = A.g.kept_row(blockIdx.y);
+    const int kcnt = min(TC, A.g.NzK - k0);
     const long long base = (long long)j * A.g.NzC + k0;
     const long long es = (long long)A.g.Ny * A.g.NzC;   // stride of x
     for (int e = threadIdx.x; e < 6 * N * TP; e += blockDim.x) {
@@ -2440,7 +2450,7 @@ k_zpass246(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float4 
     for (int e = threadIdx.x; e < R * NC; e += blockDim.x) {
         const int rr = e / NC, k = e - rr * NC;
         float2 v[6];
-        if (rr < rcnt) op.load_spec(row0 + rr, k, v);
+        if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
         else {
 #pragma unroll
             for (int f = 0; f < 6; ++f) v[f] = make_float2(0.f, 0.f);
@@ -2485,8 +2495,9 @@ k_zpass246(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float4 
     __syncthreads();
     if constexpr (TCS) tc41::lines<-1, 1, N>(buf, tw, tcx);
     else lines<-1, 1, N>(buf, tw);
-    for (int e = threadIdx.x; e < rcnt * NC; e += blockDim.x) {
-        const int rr = e / NC, k = e - rr * NC;
+    const int nk = g.NzK;
+    for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
+        const int rr = e / nk, k = e - rr * nk;
         float2 v[6];
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
@@ -2509,8 +2520,8 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
         PFGB_CUDA_TRY(allow_smem(kern, smem));
         AxisIO<float, 6, 6> io;
         for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
-        dim3 grid((c->g.NzC + f246::TC - 1) / f246::TC, c->g.Nx);
-        ProfScope ps(c, {tag, 12.0 * (double)c->g.Nk * sizeof(float2)});
+        dim3 grid((c->g.NzK + f246::TC - 1) / f246::TC, c->g.Nx);
+        ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
         kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], (const float4 *)c->tc_btab,
                                                        io, c->skip, c->tc_err);
         PFGB_CUDA_TRY(cudaGetLastError());
@@ -2521,8 +2532,8 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     AxisIO<float, 6, 6> io;
     for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
-    dim3 grid((c->g.NzC + f246::YC - 1) / f246::YC, c->g.Nx, 6 / f246::YS);
-    ProfScope ps(c, {tag, 12.0 * (double)c->g.Nk * sizeof(float2)});
+    dim3 grid((c->g.NzK + f246::YC - 1) / f246::YC, c->g.Nx, 6 / f246::YS);
+    ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
     kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], io, c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
@@ -2548,9 +2559,9 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     A.tc_err = c->tc_err;
     A.resid = resid;
     A.mode = mode;
-    dim3 grid((c->g.NzC + f246::TC - 1) / f246::TC, c->g.Ny);
+    dim3 grid((c->g.NzK + f246::TC - 1) / f246::TC, c->g.kept_rows());
     ProfScope ps(c, {eigen ? "x_green_eigen" : "x_green_hij",
-                     (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * (double)c->g.Nk * sizeof(float2)});
+                     (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(float2)});
     auto go = [&](auto kern, size_t sm) -> pfgb_status {
         PFGB_CUDA_TRY(allow_smem(kern, sm));
         kern<<<grid, f246::THREADS, sm, c->stream>>>(A);
@@ -2572,7 +2583,7 @@ static pfgb_status launch_z246(pfgb_ctx *c, Op op, const char *tag, double extra
     const size_t smem = f246::z_smem_bytes();
     const long long rows = (long long)c->g.Nx * c->g.Ny;
     const int nb = (int)((rows + f246::ZR - 1) / f246::ZR);
-    ProfScope ps(c, {tag, 12.0 * (double)c->g.Nk * sizeof(float2) + extra_bytes});
+    ProfScope ps(c, {tag, 12.0 * c->g.cols() * sizeof(float2) + extra_bytes});
     if (c->tc_z) {   // the 41-point stages on the tensor cores
         auto kern = k_zpass246<Op, true>;
         const size_t smem_tc = 2 * tc41::B_BYTES + smem;
@@ -2636,14 +2647,36 @@ static pfgb_status sync_read(pfgb_ctx *c, int first, int count) {
     return PFGB_OK;
 }
 
+// the kept modes (Grid3) one by one: a warp's lanes walk the columns of one
+// (i, kept j) row, the warps of the grid (blockDim = 32 x 8) the rows
+template <typename F>
+__device__ __forceinline__ void for_kept(const Grid3 &g, F &&f) {
+    const int nj = g.kept_rows();
+    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < g.Nx * nj; r += gridDim.x * blockDim.y) {
+        const int i = r / nj, j = g.kept_row(r - i * nj);
+        const long long o = ((long long)i * g.Ny + j) * g.NzC;
+        for (int k = threadIdx.x; k < g.NzK; k += 32) f(o + k);
+    }
+}
+
 template <typename TE>
-__global__ void k_add_increment(cplx_t<TE> *u0, cplx_t<TE> *u1, cplx_t<TE> *u2, const cplx_t<TE> *d0,
-                                const cplx_t<TE> *d1, const cplx_t<TE> *d2, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256)
+k_add_increment(Grid3 g, cplx_t<TE> *u0, cplx_t<TE> *u1, cplx_t<TE> *u2, const cplx_t<TE> *d0,
+                const cplx_t<TE> *d1, const cplx_t<TE> *d2) {
+    for_kept(g, [&](long long i) {
         u0[i] = cadd(u0[i], d0[i]);
         u1[i] = cadd(u1[i], d1[i]);
         u2[i] = cadd(u2[i], d2[i]);
+    });
+}
+
+// zero outside the kept modes (a restored displacement)
+template <typename TE>
+__global__ void k_zero_cut(Grid3 g, cplx_t<TE> *u0, cplx_t<TE> *u1, cplx_t<TE> *u2) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < g.Nk;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int k = (int)(i % g.NzC), j = (int)((i / g.NzC) % g.Ny);
+        if (k >= g.NzK || g.cut_row(j)) u0[i] = u1[i] = u2[i] = mk2<cplx_t<TE>>(TE(0), TE(0));
     }
 }
 
@@ -2660,9 +2693,9 @@ __global__ void k_add_increment(cplx_t<TE> *u0, cplx_t<TE> *u1, cplx_t<TE> *u2, 
 template <typename TE>
 struct ExtrapArgs { cplx_t<TE> *u[3], *h[5][3], *slot[3]; };
 template <typename TE>
-__global__ void k_extrapolate_u(ExtrapArgs<TE> a, long long n, int m) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256)
+k_extrapolate_u(Grid3 g, ExtrapArgs<TE> a, int m) {
+    for_kept(g, [&](long long i) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             cplx_t<TE> d[6];
@@ -2685,7 +2718,7 @@ __global__ void k_extrapolate_u(ExtrapArgs<TE> a, long long n, int m) {
                 a.u[c][i] = sum;
             }
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -2793,9 +2826,9 @@ static pfgb_status model_start(pfgb_ctx *c) {
     TRY((launch_axis<TE, 3, 3, -1, 0>(c, 1, io, OpCopy<TE, 3>{}, "y_fwd3")));
     TRY((launch_axis<TE, 3, 3, -1, 0>(c, 2, io, OpCutU3<TE>{KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz}},
                                       "x_fwd3")));
-    ProfScope ps(c, {"add_increment", 9.0 * (double)c->g.Nk * sizeof(T2e)});
-    k_add_increment<TE><<<1216, 256, 0, c->stream>>>((T2e *)c->U[0], (T2e *)c->U[1], (T2e *)c->U[2], E0, E1, E2,
-                                                     c->g.Nk);
+    ProfScope ps(c, {"add_increment", 9.0 * c->g.kept() * sizeof(T2e)});
+    k_add_increment<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, (T2e *)c->U[0], (T2e *)c->U[1], (T2e *)c->U[2],
+                                                             E0, E1, E2);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
 }
@@ -2860,14 +2893,14 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
             // level, which the pointer rotation below makes u^{n-1}
             const int nh = P.elastic_warm_start_extrapolate;
             const int m = std::min(nh, c->warm_count - 1);
-            ProfScope ps(c, {"extrapolate_u", (3.0 + (double)std::max(m, 0)) * 3.0 * (double)c->g.Nk * sizeof(T2e)});
+            ProfScope ps(c, {"extrapolate_u", (3.0 + (double)std::max(m, 0)) * 3.0 * c->g.kept() * sizeof(T2e)});
             ExtrapArgs<TE> a;
             for (int i = 0; i < 3; ++i) {
                 a.u[i] = (T2e *)c->U[i];
                 for (int l = 0; l < 5; ++l) a.h[l][i] = (T2e *)c->Uhist[l][i];
                 a.slot[i] = (T2e *)c->Uhist[nh - 1][i];
             }
-            k_extrapolate_u<TE><<<1216, 256, 0, c->stream>>>(a, c->g.Nk, std::max(m, 0));
+            k_extrapolate_u<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, a, std::max(m, 0));
             PFGB_CUDA_TRY(cudaGetLastError());
             for (int i = 0; i < 3; ++i) {
                 void *oldest = c->Uhist[nh - 1][i];
@@ -2989,10 +3022,10 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
     if (inc) {
         // u = u0 + delta, and the strain of u for the final pass
         {
-            ProfScope ps(c, {"add_increment", 9.0 * (double)c->g.Nk * sizeof(T2e)});
-            k_add_increment<TE><<<1216, 256, 0, c->stream>>>((T2e *)c->U[0], (T2e *)c->U[1], (T2e *)c->U[2],
-                                                             (const T2e *)c->Dk[0], (const T2e *)c->Dk[1],
-                                                             (const T2e *)c->Dk[2], c->g.Nk);
+            ProfScope ps(c, {"add_increment", 9.0 * c->g.kept() * sizeof(T2e)});
+            k_add_increment<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, (T2e *)c->U[0], (T2e *)c->U[1],
+                                                                     (T2e *)c->U[2], (const T2e *)c->Dk[0],
+                                                                     (const T2e *)c->Dk[1], (const T2e *)c->Dk[2]);
             PFGB_CUDA_TRY(cudaGetLastError());
         }
         AxisIO<TE, 3, 6> io;
@@ -4149,6 +4182,12 @@ static pfgb_status make_ktab(pfgb_ctx *c) {
     for (int i = 0; i < P.Nx; ++i) { kx[i] = wrap(i, P.Nx, P.dx); mx[i] = cut(kx[i], P.dx); }
     for (int j = 0; j < P.Ny; ++j) { ky[j] = wrap(j, P.Ny, P.dy); my[j] = cut(ky[j], P.dy); }
     for (int k = 0; k < c->g.NzC; ++k) { kz[k] = 2.0 * PFGB_PI * k / (P.dz * P.Nz); mz[k] = cut(kz[k], P.dz); }
+    // the box of kept modes: |k| grows with k, and with j up to Ny / 2, so the
+    // cut columns are the last ones and the cut rows one run in the middle
+    c->g.NzK = (int)(std::find(mz.begin(), mz.end(), 1) - mz.begin());
+    c->g.jc0 = (int)(std::find(my.begin(), my.end(), 1) - my.begin());
+    c->g.jc1 = P.Ny - (int)(std::find(my.rbegin(), my.rend(), 1) - my.rbegin());
+    if (c->g.jc0 == P.Ny) c->g.jc1 = P.Ny;
     TRY(dalloc(c, (void **)&c->kx, sizeof(double) * P.Nx));
     TRY(dalloc(c, (void **)&c->ky, sizeof(double) * P.Ny));
     TRY(dalloc(c, (void **)&c->kz, sizeof(double) * c->g.NzC));
@@ -4618,6 +4657,7 @@ pfgb_status pfgb_create(const pfgb_params *pin, int device, pfgb_ctx **out) {
     c->g.Nx = pin->Nx; c->g.Ny = pin->Ny; c->g.Nz = pin->Nz; c->g.NzC = pin->Nz / 2 + 1;
     c->g.N = (long long)pin->Nx * pin->Ny * pin->Nz;
     c->g.Nk = (long long)pin->Nx * pin->Ny * c->g.NzC;
+    c->g.keep_all();   // make_ktab sets the dealias box
     pfgb_make_plan(pin->Nx, &c->plx);
     pfgb_make_plan(pin->Ny, &c->ply);
     pfgb_make_plan(pin->Nz, &c->plz);
@@ -4701,6 +4741,12 @@ pfgb_status pfgb_create(const pfgb_params *pin, int device, pfgb_ctx **out) {
     }
     if (s == PFGB_OK && !c->pc.gp) {
         cudaError_t e = cudaMemset(c->eta[0], 0, rs * N);
+        if (e != cudaSuccess) { pfgb_set_error("cudaMemset", e, __FILE__, __LINE__); s = PFGB_ERR_CUDA; }
+    }
+    // the x passes write the kept modes of the displacement alone (Grid3): the
+    // others are zero from here on
+    for (int i = 0; i < 3 && s == PFGB_OK && c->U[0]; ++i) {
+        cudaError_t e = cudaMemset(c->U[i], 0, sizeof(float2) * Nk);
         if (e != cudaSuccess) { pfgb_set_error("cudaMemset", e, __FILE__, __LINE__); s = PFGB_ERR_CUDA; }
     }
     // the table uploads and the memset above run on the legacy default
@@ -5120,6 +5166,8 @@ pfgb_status pfgb_checkpoint_restore(pfgb_ctx *c, const char *path, const char *i
         for (int a = 0; a < 3; ++a)
             PFGB_CUDA_TRY(cudaMemcpyAsync(c->U[a], u.data() + 2 * a * Nk, sizeof(float2) * Nk,
                                           cudaMemcpyHostToDevice, c->stream));
+        k_zero_cut<float><<<1216, 256, 0, c->stream>>>(c->g, (float2 *)c->U[0], (float2 *)c->U[1], (float2 *)c->U[2]);
+        PFGB_CUDA_TRY(cudaGetLastError());
     }
     for (int i = 0; i < 6; ++i) PFGB_CUDA_TRY(cudaMemsetAsync(c->eps[i], 0, sizeof(float) * N, c->stream));
     PFGB_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -5266,6 +5314,7 @@ static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *strea
     c->g.Nx = Nx; c->g.Ny = Ny; c->g.Nz = Nz; c->g.NzC = Nz / 2 + 1;
     c->g.N = (long long)Nx * Ny * Nz;
     c->g.Nk = (long long)Nx * Ny * c->g.NzC;
+    c->g.keep_all();
     pfgb_make_plan(Nx, &c->plx);
     pfgb_make_plan(Ny, &c->ply);
     pfgb_make_plan(Nz, &c->plz);
@@ -5352,6 +5401,7 @@ pfgb_status pfgb_fft_y246x6(int tensor_cores, int dir, int Nx, int NzC, void *sp
     pfgb_status s = fft_ctx_init(&c, Nx, f246::N, 2 * (NzC - 1), stream);
     c.g.NzC = NzC;
     c.g.Nk = (long long)Nx * f246::N * NzC;
+    c.g.keep_all();
     const size_t per = sizeof(float2) * (size_t)c.g.Nk;
     for (int i = 0; i < 6; ++i) c.E[i] = (unsigned char *)spec6 + i * per;
     if (s == PFGB_OK && tensor_cores) {
@@ -5461,6 +5511,7 @@ static pfgb_status fft_r2c_noalloc(int Nx, int Ny, int Nz, const T *in, cplx_t<T
     c.g.Nx = Nx; c.g.Ny = Ny; c.g.Nz = Nz; c.g.NzC = Nz / 2 + 1;
     c.g.N = (long long)Nx * Ny * Nz;
     c.g.Nk = (long long)Nx * Ny * c.g.NzC;
+    c.g.keep_all();
     pfgb_make_plan(Nx, &c.plx);
     pfgb_make_plan(Ny, &c.ply);
     pfgb_make_plan(Nz, &c.plz);
