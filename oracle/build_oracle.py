@@ -76,18 +76,17 @@ def build_ref(force: bool = False) -> str | None:
     otherwise.  The shim (ref_pin.c) defines away the CUDA qualifiers and
     includes the headers from the reference tree by absolute path.
     """
-    if not os.path.isdir(REFERENCE_TREE):
+    hdrs = [os.path.join(REFERENCE_TREE, "thermo_utils.h"),
+            os.path.join(REFERENCE_TREE, "phase_functions.h")]
+    if not all(os.path.exists(h) for h in hdrs):
         return None
     os.makedirs(REF_OUT, exist_ok=True)
     shim = os.path.join(HERE, "ref_pin.c")
-    hdrs = [os.path.join(REFERENCE_TREE, "thermo_utils.h"),
-            os.path.join(REFERENCE_TREE, "phase_functions.h")]
     if force or _stale(REF_LIB, [shim]):
         tmp = REF_LIB + ".tmp"
         subprocess.run(["gcc", "-O2", "-fPIC", "-shared", "-ffp-contract=off",
                         "-I", REFERENCE_TREE, "-o", tmp, shim, "-lm"], check=True)
         os.replace(tmp, REF_LIB)
-    del hdrs
     return REF_LIB
 
 
