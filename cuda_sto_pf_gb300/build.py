@@ -35,7 +35,12 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE,
               "--expt-relaxed-constexpr"] + ARCH
 
-CU_SOURCES = ["solver.cu", "params.cu", "paramfile.cpp", "batch.cpp", "fno.cu", "checkpoint.cpp", "init.cu"]
+# (source, extra flags, object suffix): solver.cu is three translation units,
+# its entry points and the kernels of each field precision, compiled at once
+CU_SOURCES = [("solver.cu", [], ""), ("solver.cu", ["-DPFGB_FIELDS=float"], ".f32"),
+              ("solver.cu", ["-DPFGB_FIELDS=double"], ".f64")]
+CU_SOURCES = [(s, f + ["--split-compile", "4"], x) for s, f, x in CU_SOURCES]
+CU_SOURCES += [(s, [], "") for s in ("params.cu", "paramfile.cpp", "batch.cpp", "fno.cu", "checkpoint.cpp", "init.cu")]
 HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41_tc.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
 
 
@@ -46,20 +51,19 @@ def _newer(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
-def _compile(src: str, force: bool) -> str:
-    obj = os.path.join(BUILD, os.path.basename(src) + ".o")
+def _compile(src: str, flags: list[str], suffix: str, force: bool) -> str:
+    obj = os.path.join(BUILD, os.path.basename(src) + suffix + ".o")
     deps = [src] + [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "pfgb.h")]
     if force or _newer(obj, deps):
-        subprocess.run([NVCC, *NVCC_FLAGS, "-c", src, "-o", obj + ".tmp"], check=True)
+        subprocess.run([NVCC, *NVCC_FLAGS, *flags, "-c", src, "-o", obj + ".tmp"], check=True)
         os.replace(obj + ".tmp", obj)
     return obj
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    srcs = [os.path.join(CSRC, s) for s in CU_SOURCES]
-    with cf.ThreadPoolExecutor(max_workers=len(srcs)) as ex:
-        objs = list(ex.map(lambda s: _compile(s, force), srcs))
+    with cf.ThreadPoolExecutor(max_workers=len(CU_SOURCES)) as ex:
+        objs = list(ex.map(lambda s: _compile(os.path.join(CSRC, s[0]), s[1], s[2], force), CU_SOURCES))
     if force or _newer(LIB, objs):
         subprocess.run([NVCC, *ARCH, "-shared", "-cudart", "shared", "-o", LIB + ".tmp", *objs],
                        check=True)

@@ -203,8 +203,8 @@ static int smem_optin_max() {
     }
     return m;
 }
-static std::mutex g_smem_mu;
-static std::map<std::pair<int, const void *>, int> g_smem_limit;   // (device, kernel) -> dynamic limit
+inline std::mutex g_smem_mu;
+inline std::map<std::pair<int, const void *>, int> g_smem_limit;   // (device, kernel) -> dynamic limit
 
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -256,8 +256,8 @@ struct TileKey {
     }
 };
 struct TileRec { int tile, rule; float t_ms, t_rule_ms; std::string tag; long long a, b, c; };
-static std::mutex g_tile_mu;
-static std::map<TileKey, TileRec> g_tiles;
+inline std::mutex g_tile_mu;
+inline std::map<TileKey, TileRec> g_tiles;
 
 // zeroed scratch arrays of `bytes` each, stream-ordered (no device-wide
 // synchronisation while other contexts run), freed with the object
@@ -284,7 +284,7 @@ struct TuneScratch {
 // the number of copies of a candidate timed together: the concurrency of
 // the caller's cases (pfgb_batch_minimize sets it while it tunes), so the
 // choice is the one with the best throughput on a device the cases share
-static std::atomic<int> g_tune_copies(1);
+inline std::atomic<int> g_tune_copies(1);
 
 // one warm-up round, then the best of three (ms per round); a round is one
 // launch on each of the given streams, forked from and joined to the
@@ -1493,7 +1493,7 @@ static ConsArgs cons_args(const pfgb_ctx *c) {
 }
 
 // initialize_conservative_storage_kernel (:3123-3132), from the loaded fields
-__global__ void k_cons_load(const double *phi, const double *xB, double *cst, long long N, int ctot, double vB) {
+static __global__ void k_cons_load(const double *phi, const double *xB, double *cst, long long N, int ctot, double vB) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
         const double h = pf_h(clamp01(phi[i]));
         const double q = (1.0 - h) * clamp01(xB[i]);
@@ -2209,7 +2209,7 @@ k_x_green(GreenArgs<TE> A, AxisPlan plan, int TK) {
 }
 
 // residual finalize: rel = sqrt(diff / max(ref, floor))
-__global__ void k_resid_final(double *dscal, double floor_) {
+static __global__ void k_resid_final(double *dscal, double floor_) {
     const double d = dscal[DS_RES_DIFF], r = dscal[DS_RES_REF];
     dscal[3] = sqrt(d / fmax(r, floor_));
 }
@@ -2219,7 +2219,7 @@ __global__ void k_resid_final(double *dscal, double floor_) {
 // max(ref, floor)); stop when iter >= iter_min and rel <= tol, at iter_max,
 // or on a non-finite / negative residual sum.  Slots DS_EL + 0..3: done,
 // updates taken, non-finite, converged.  Nothing changes once done is set.
-__global__ void k_resid_step(double *dscal, double floor_, double tol, int iter_min, int iter_max) {
+static __global__ void k_resid_step(double *dscal, double floor_, double tol, int iter_min, int iter_max) {
     double *st = dscal + DS_EL;
     if (st[0] != 0.0) return;
     const double d = dscal[DS_RES_DIFF], r = dscal[DS_RES_REF];
@@ -2240,7 +2240,7 @@ __global__ void k_resid_step(double *dscal, double floor_, double tol, int iter_
     }
 }
 
-__global__ void k_el_status_reset(double *dscal) {
+static __global__ void k_el_status_reset(double *dscal) {
     if (threadIdx.x < 4) dscal[DS_EL + threadIdx.x] = 0.0;
 }
 
@@ -3571,7 +3571,7 @@ static pfgb_status y_update(pfgb_ctx *c, const DevState<T, TE> &d, pfgb_step_sta
 }
 
 template <typename T, typename TE>
-static pfgb_status step_once(pfgb_ctx *c, pfgb_step_stats *st) {
+pfgb_status step_once(pfgb_ctx *c, pfgb_step_stats *st) {
     using T2 = cplx_t<T>;
     const pfgb_params &P = c->p;
     const PhysCT<T> pc = phys_as<T>(c->pc);
@@ -3896,7 +3896,7 @@ static pfgb_status min_reduce(pfgb_ctx *c, const char *tag, double bytes, int sl
 }
 
 template <typename T, typename TE>
-static pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
+pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     const pfgb_params &P = c->p;
     const double Nf = (double)c->g.N;
     const long long N = c->g.N;
@@ -4063,6 +4063,49 @@ static pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     }
     return PFGB_OK;
 }
+
+// training pair: cold solve with u_hom kept, then the model inputs and the
+// real-space correction (U - U_hom) / N
+template <typename T>
+pfgb_status training_pair(pfgb_ctx *c, float *in8, float *tgt3, pfgb_step_stats *st) {
+    using T2e = float2;
+    c->Yc_prev = c->Yc;
+    c->pair_mode = 1;
+    pfgb_status s = elastic_solve<T, float>(c, st);
+    c->pair_mode = 0;
+    TRY(s);
+    T2e *E0 = (T2e *)c->E[0], *E1 = (T2e *)c->E[1], *E2 = (T2e *)c->E[2];
+    {
+        ProfScope ps(c, {"pair_difference", 9.0 * (double)c->g.Nk * sizeof(T2e)});
+        k_sub3<float><<<1216, 256, 0, c->stream>>>(E0, E1, E2, (const T2e *)c->U[0], (const T2e *)c->U[1],
+                                                   (const T2e *)c->U[2], (const T2e *)c->Uhom[0],
+                                                   (const T2e *)c->Uhom[1], (const T2e *)c->Uhom[2], c->g.Nk);
+        PFGB_CUDA_TRY(cudaGetLastError());
+    }
+    AxisIO<float, 3, 3> io;
+    for (int i = 0; i < 3; ++i) { io.in[i] = (const T2e *)c->E[i]; io.out[i] = (T2e *)c->E[i]; }
+    TRY((launch_axis<float, 3, 3, +1, 0>(c, 2, io, OpCopy<float, 3>{}, "x_inv3")));
+    TRY((launch_axis<float, 3, 3, +1, 0>(c, 1, io, OpCopy<float, 3>{}, "y_inv3")));
+    TRY((launch_z<float, 3, 0>(c, OpReal3Out<float>{E0, E1, E2, tgt3, c->g.N, c->g.NzC, (float)(1.0 / (double)c->g.N)},
+                               "z_pair_c2r", 3.0 * (double)c->g.N * sizeof(float))));
+    return launch_fno_inputs<T, float>(c, in8);
+}
+
+// The file is compiled three times, at the same time (build.py): as it is,
+// with the entry points, and once for each field precision with PFGB_FIELDS
+// (float or double), for the step, the minimize iteration and the training
+// pair of that precision with every kernel that they launch.
+#ifdef PFGB_FIELDS
+template pfgb_status step_once<PFGB_FIELDS, float>(pfgb_ctx *, pfgb_step_stats *);
+template pfgb_status minimize_once<PFGB_FIELDS, float>(pfgb_ctx *, pfgb_min_stats *);
+template pfgb_status training_pair<PFGB_FIELDS>(pfgb_ctx *, float *, float *, pfgb_step_stats *);
+#else
+extern template pfgb_status step_once<float, float>(pfgb_ctx *, pfgb_step_stats *);
+extern template pfgb_status step_once<double, float>(pfgb_ctx *, pfgb_step_stats *);
+extern template pfgb_status minimize_once<float, float>(pfgb_ctx *, pfgb_min_stats *);
+extern template pfgb_status minimize_once<double, float>(pfgb_ctx *, pfgb_min_stats *);
+extern template pfgb_status training_pair<float>(pfgb_ctx *, float *, float *, pfgb_step_stats *);
+extern template pfgb_status training_pair<double>(pfgb_ctx *, float *, float *, pfgb_step_stats *);
 
 // ---------------------------------------------------------------------------
 // construction
@@ -4985,33 +5028,6 @@ pfgb_status pfgb_read_elastic(pfgb_ctx *c, float *sigma6, float *strain6) {
 
 }  // extern "C"
 
-// training pair: cold solve with u_hom kept, then the model inputs and the
-// real-space correction (U - U_hom) / N
-template <typename T>
-static pfgb_status training_pair(pfgb_ctx *c, float *in8, float *tgt3, pfgb_step_stats *st) {
-    using T2e = float2;
-    c->Yc_prev = c->Yc;
-    c->pair_mode = 1;
-    pfgb_status s = elastic_solve<T, float>(c, st);
-    c->pair_mode = 0;
-    TRY(s);
-    T2e *E0 = (T2e *)c->E[0], *E1 = (T2e *)c->E[1], *E2 = (T2e *)c->E[2];
-    {
-        ProfScope ps(c, {"pair_difference", 9.0 * (double)c->g.Nk * sizeof(T2e)});
-        k_sub3<float><<<1216, 256, 0, c->stream>>>(E0, E1, E2, (const T2e *)c->U[0], (const T2e *)c->U[1],
-                                                   (const T2e *)c->U[2], (const T2e *)c->Uhom[0],
-                                                   (const T2e *)c->Uhom[1], (const T2e *)c->Uhom[2], c->g.Nk);
-        PFGB_CUDA_TRY(cudaGetLastError());
-    }
-    AxisIO<float, 3, 3> io;
-    for (int i = 0; i < 3; ++i) { io.in[i] = (const T2e *)c->E[i]; io.out[i] = (T2e *)c->E[i]; }
-    TRY((launch_axis<float, 3, 3, +1, 0>(c, 2, io, OpCopy<float, 3>{}, "x_inv3")));
-    TRY((launch_axis<float, 3, 3, +1, 0>(c, 1, io, OpCopy<float, 3>{}, "y_inv3")));
-    TRY((launch_z<float, 3, 0>(c, OpReal3Out<float>{E0, E1, E2, tgt3, c->g.N, c->g.NzC, (float)(1.0 / (double)c->g.N)},
-                               "z_pair_c2r", 3.0 * (double)c->g.N * sizeof(float))));
-    return launch_fno_inputs<T, float>(c, in8);
-}
-
 extern "C" {
 
 pfgb_status pfgb_set_warm_start_model(pfgb_ctx *c, pfgb_fno *f) {
@@ -5585,3 +5601,5 @@ int pfgb_profile_read(pfgb_ctx *c, const char **names, double *ms, double *bytes
 }
 
 }  // extern "C"
+
+#endif   // PFGB_FIELDS
