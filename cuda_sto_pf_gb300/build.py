@@ -39,9 +39,8 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INC
 # its entry points and the kernels of each field precision, compiled at once
 CU_SOURCES = [("solver.cu", [], ""), ("solver.cu", ["-DPFGB_FIELDS=float"], ".f32"),
               ("solver.cu", ["-DPFGB_FIELDS=double"], ".f64")]
-CU_SOURCES = [(s, f + ["--split-compile", "4"], x) for s, f, x in CU_SOURCES]
 CU_SOURCES += [(s, [], "") for s in ("params.cu", "paramfile.cpp", "batch.cpp", "fno.cu", "checkpoint.cpp", "init.cu")]
-HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41_tc.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
+HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41.cuh", "dft41_tc.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

@@ -330,7 +330,7 @@ k_y246tc(Grid3 g, const float2 *tw_g, const float4 *btab, AxisIO<float, 6, 6> io
     __syncthreads();
     tc41::fence_after();
     tc41::Ctx c{tbase, &mbar, 0u, tc41::smem_u32(bt), tc41::smem_u32(bt) + tc41::B_BYTES, err};
-    stage_a<DIR, PS, 1>(buf, tw);
+    stage_a<NL, DIR, PS, 1>(buf, tw);
     __syncthreads();
     tc41::stage_c<DIR, PS, 1>(buf, c);
 #pragma unroll
@@ -381,7 +381,7 @@ __device__ __forceinline__ void end(uint32_t tmem) {
 // cores, the 41-point stage on the tensor cores
 template <int DIR, int PS, int LS>
 __device__ __forceinline__ void lines(float2 *buf, const float2 *tw, Ctx &c) {
-    f246::stage_a<DIR, PS, LS>(buf, tw);
+    f246::stage_a<f246::NL, DIR, PS, LS>(buf, tw);
     __syncthreads();
     stage_c<DIR, PS, LS>(buf, c);
 }

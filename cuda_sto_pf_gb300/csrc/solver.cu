@@ -493,14 +493,15 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
     if constexpr (std::is_same<T, float>::value && f246_axis_fits<NIN, NOUT>()) {
         // 246-long FP32 axes with an even half-spectrum row: the 6 x 41 engine
         if (n == f246::N && c->g.NzC % 2 == 0) {
-            constexpr int TCW = f246::NL / axis_width<NIN, NOUT>();
-            const size_t smem = f246::axis_smem_bytes();
+            using E = f246::Eng<f246_axis_lines(axis_width<NIN, NOUT>())>;
+            constexpr int TCW = E::NL / axis_width<NIN, NOUT>();
+            const size_t smem = E::SMEM;
             auto kern = k_axis246<NIN, NOUT, DIN, DOUT, Op>;
             PFGB_CUDA_TRY(allow_smem(kern, smem));
             dim3 grid((c->g.NzK + TCW - 1) / TCW, axis == 1 ? c->g.Nx : c->g.kept_rows());
             ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-            kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, axis, (const float2 *)twp<T>(c, axis == 1 ? 1 : 0),
-                                                         io, op, c->skip);
+            kern<<<grid, E::THREADS, smem, c->stream>>>(c->g, axis, (const float2 *)twp<T>(c, axis == 1 ? 1 : 0), io,
+                                                      op, c->skip);
             PFGB_CUDA_TRY(cudaGetLastError());
             return PFGB_OK;
         }
@@ -525,21 +526,22 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
 // generic z pass on the 246-point engine: NFI half spectra per row in
 // (Hermitian-packed two per complex line), C2R, the op's pointwise stage,
 // R2C, NFO half spectra out.  A row takes LW = max(ceil(NFI/2), ceil(NFO/2))
-// lines, a block NL / LW rows.
+// lines, a block NL / LW rows: four blocks of 20 or 21 lines per SM.
 template <int NFI, int NFO>
-constexpr bool f246_z_fits() {
-    constexpr int LI = (NFI + 1) / 2, LO = (NFO + 1) / 2, LW = LI > LO ? LI : LO;
-    return LW >= 1 && LW <= 3;
-}
+constexpr int f246_z_width() { return (NFI + 1) / 2 > (NFO + 1) / 2 ? (NFI + 1) / 2 : (NFO + 1) / 2; }
+template <int NFI, int NFO>
+constexpr bool f246_z_fits() { return f246_z_width<NFI, NFO>() >= 1 && f246_z_width<NFI, NFO>() <= 3; }
+constexpr int f246_z_lines(int LW) { return LW == 2 ? 20 : 21; }
 
 template <int NFI, int NFO, class Op>
-__global__ void __launch_bounds__(f246::THREADS, f246::BLOCKS_PER_SM)
+__global__ void __launch_bounds__(f246::Eng<f246_z_lines(f246_z_width<NFI, NFO>())>::THREADS,
+                                  f246::Eng<f246_z_lines(f246_z_width<NFI, NFO>())>::BLOCKS)
 k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
     if (skip && *skip != 0.0) return;
     using namespace f246;
-    constexpr int LI = (NFI + 1) / 2, LO = (NFO + 1) / 2, LW = LI > LO ? LI : LO;
-    constexpr int R = NL / LW, NC = N / 2 + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int LO = (NFO + 1) / 2, LW = f246_z_width<NFI, NFO>();
+    constexpr int NLT = f246_z_lines(LW), R = NLT / LW;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     float2 *tw = reinterpret_cast<float2 *>(smem_raw);
     float2 *buf = tw + N;
     const long long row0 = (long long)blockIdx.x * R;
@@ -547,27 +549,9 @@ k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
     const int rcnt = (int)min((long long)R, nrows - row0);
     load_twiddles(tw, tw_g);
     if constexpr (NFI > 0) {
-#pragma unroll 2
-        for (int e = threadIdx.x; e < R * NC; e += blockDim.x) {
-            const int rr = e / NC, k = e - rr * NC;
-            float2 v[NFI];
-            if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
-            else {
-#pragma unroll
-                for (int f = 0; f < NFI; ++f) v[f] = make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int f = 0; f < LI; ++f) {
-                float2 Av = v[2 * f], Bv = 2 * f + 1 < NFI ? v[2 * f + 1] : make_float2(0.f, 0.f);
-                if (k == 0 || 2 * k == N) { Av.y = 0.f; Bv.y = 0.f; }
-                float2 *line = buf + (rr * LW + f) * N;
-                // Z_k = A_k + i B_k ; Z_(n-k) = conj(A_k) + i conj(B_k)
-                line[k] = make_float2(Av.x - Bv.y, Av.y + Bv.x);
-                if (k > 0 && 2 * k != N) line[N - k] = make_float2(Av.x + Bv.y, Bv.x - Av.y);
-            }
-        }
+        rows_in<NFI, LW>(buf, op, row0, R, rcnt, g.NzK);
         __syncthreads();
-        lines<+1, 1, N>(buf, tw);
+        lines<NLT, +1, 1, N>(buf, tw);
     } else {
         __syncthreads();   // twiddles
     }
@@ -611,21 +595,8 @@ k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
     }
     if constexpr (NFO > 0) {
         __syncthreads();
-        lines<-1, 1, N>(buf, tw);
-        const int nk = g.NzK;
-        for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
-            const int rr = e / nk, k = e - rr * nk;
-            float2 v[NFO];
-#pragma unroll
-            for (int f = 0; f < LO; ++f) {
-                const float2 *line = buf + (rr * LW + f) * N;
-                const float2 Zk = line[k], Zm = line[k == 0 ? 0 : N - k];
-                // A_k = (Z_k + conj Z_-k) / 2 ; B_k = (Z_k - conj Z_-k) / (2 i)
-                v[2 * f] = make_float2(0.5f * (Zk.x + Zm.x), 0.5f * (Zk.y - Zm.y));
-                if (2 * f + 1 < NFO) v[2 * f + 1] = make_float2(0.5f * (Zk.y + Zm.y), 0.5f * (Zm.x - Zk.x));
-            }
-            op.store_spec(row0 + rr, k, v);
-        }
+        lines<NLT, -1, 1, N>(buf, tw);
+        rows_out<NFO, LW>(buf, op, row0, rcnt, g.NzK);
     }
 }
 
@@ -636,15 +607,16 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     const int n = c->g.Nz;
     if constexpr (std::is_same<T, float>::value && f246_z_fits<NFI, NFO>()) {
         if (n == f246::N) {   // 246-long FP32 rows: the 6 x 41 engine
-            constexpr int LW = ((NFI + 1) / 2 > (NFO + 1) / 2) ? (NFI + 1) / 2 : (NFO + 1) / 2;
-            constexpr int R = f246::NL / LW;
-            const size_t smem = f246::z_smem_bytes();
+            constexpr int LW = f246_z_width<NFI, NFO>();
+            using E = f246::Eng<f246_z_lines(LW)>;
+            constexpr int R = E::NL / LW;
+            const size_t smem = E::SMEM;
             auto kern = k_zpass246g<NFI, NFO, Op>;
             PFGB_CUDA_TRY(allow_smem(kern, smem));
             const long long rows = (long long)c->g.Nx * c->g.Ny;
             const int nb = (int)((rows + R - 1) / R);
             ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-            kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)twp<T>(c, 2), op, c->skip);
+            kern<<<nb, E::THREADS, smem, c->stream>>>(c->g, (const float2 *)twp<T>(c, 2), op, c->skip);
             PFGB_CUDA_TRY(cudaGetLastError());
             if (nblocks) *nblocks = nb;
             return PFGB_OK;
@@ -2305,18 +2277,18 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
 // ---------------------------------------------------------------------------
 // elastic-iteration passes on 246-long axes (FP32, fft246.cuh engine): the
 // same operations as k_x_green / k_zpass<OpHijZ> / the y OpCopy pass, with
-// f246::NL lines per block in one in-place shared buffer
+// the lines of a block in one in-place shared buffer (x: 7 columns of the six
+// components, or 8 with the tensor-core stage)
 // ---------------------------------------------------------------------------
 // TCS: the 41-point stages on the tensor cores (dft41_tc.cuh): shared memory
 // B table | twiddles | line buffer without row padding
 template <bool EIGEN, bool TCS>
-__global__ void __launch_bounds__(f246::THREADS, f246::BLOCKS_PER_SM)
+__global__ void __launch_bounds__(f246::Eng<TCS ? 48 : 42>::THREADS, 2)
 k_x_green246(GreenArgs<float> A) {
     if (A.skip && *A.skip != 0.0) return;
     using namespace f246;
     using T2 = float2;
-    constexpr int TP = TC / 2;
-    constexpr int PSX = TCS ? NL : PSTR;
+    constexpr int PSX = TCS ? 48 : 42, TC = PSX / 6;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t tc_mbar;
     __shared__ uint32_t tc_tbase;
@@ -2328,20 +2300,8 @@ k_x_green246(GreenArgs<float> A) {
     const int kcnt = min(TC, A.g.NzK - k0);
     const long long base = (long long)j * A.g.NzC + k0;
     const long long es = (long long)A.g.Ny * A.g.NzC;   // stride of x
-    for (int e = threadIdx.x; e < 6 * N * TP; e += blockDim.x) {
-        const int tp = e % TP, r = e / TP;
-        const int q = r % N, s = r / N;
-        const int t = 2 * tp;
-        float2 *dst = buf + q * PSX + s * TC + t;
-        const float2 *src = A.E[s] + base + q * es + t;
-        if (t + 1 < kcnt) {
-            const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src));
-        } else {
-            dst[0] = t < kcnt ? src[0] : make_float2(0.f, 0.f);
-            dst[1] = make_float2(0.f, 0.f);
-        }
-    }
+#pragma unroll
+    for (int s = 0; s < 6; ++s) tile_in<TC, PSX>(buf + s * TC, A.E[s] + base, es, kcnt, N, N);
     cp_async_commit();
     load_twiddles(tw, A.tw);
     cp_async_wait_all();
@@ -2351,7 +2311,7 @@ k_x_green246(GreenArgs<float> A) {
         tc41::lines<-1, PSX, 1>(buf, tw, tcx);
     } else {
         __syncthreads();
-        lines<-1, PSX, 1>(buf, tw);
+        lines<PSX, -1, PSX, 1>(buf, tw);
     }
     float rd = 0.f, rr = 0.f;
     // mode 2 (every iteration after the first of a step): the k-point's
@@ -2410,72 +2370,38 @@ k_x_green246(GreenArgs<float> A) {
     }
     __syncthreads();
     if constexpr (TCS) tc41::lines<+1, PSX, 1>(buf, tw, tcx);
-    else lines<+1, PSX, 1>(buf, tw);
-    for (int e = threadIdx.x; e < 6 * N * TP; e += blockDim.x) {
-        const int tp = e % TP, r = e / TP;
-        const int q = r % N, s = r / N;
-        const int t = 2 * tp;
-        const float2 *srcs = buf + q * PSX + s * TC + t;
-        float2 *dst = A.E[s] + base + q * es + t;
-        if (t + 1 < kcnt) *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(srcs);
-        else if (t < kcnt) dst[0] = srcs[0];
-    }
+    else lines<PSX, +1, PSX, 1>(buf, tw);
+#pragma unroll
+    for (int s = 0; s < 6; ++s) tile_out<TC, PSX>(buf + s * TC, A.E[s] + base, es, kcnt, N, N);
     if constexpr (TCS) tc41::end(tcx.tmem);
 }
 
-// z pass with six fields in and six out (C2R -> op.point -> R2C), ZR rows
-// per block: the rows' three field pairs are the block's NL complex lines
-// TCS: the 41-point stages on the tensor cores (dft41_tc.cuh); shared
-// memory B table | twiddles | lines
-template <class Op, bool TCS>
+// z pass with six fields in and six out (C2R -> op.point -> R2C) with the
+// 41-point stages on the tensor cores (dft41_tc.cuh), ZR rows per block: the
+// rows' three field pairs are the block's NL complex lines; shared memory B
+// table | twiddles | lines
+template <class Op>
 __global__ void __launch_bounds__(f246::THREADS, f246::BLOCKS_PER_SM)
-k_zpass246(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float4 *btab, int *tc_err) {
+k_zpass246tc(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float4 *btab, int *tc_err) {
     if (skip && *skip != 0.0) return;
     using namespace f246;
-    constexpr int R = ZR, NC = N / 2 + 1;
+    constexpr int R = ZR;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t tc_mbar;
     __shared__ uint32_t tc_tbase;
     float4 *bt = reinterpret_cast<float4 *>(smem_raw);
-    float2 *tw = reinterpret_cast<float2 *>(smem_raw + (TCS ? 2 * tc41::B_BYTES : 0));
+    float2 *tw = reinterpret_cast<float2 *>(smem_raw + 2 * tc41::B_BYTES);
     float2 *buf = tw + N;
     const long long row0 = (long long)blockIdx.x * R;
     const long long nrows = (long long)g.Nx * g.Ny;
     const int rcnt = (int)min((long long)R, nrows - row0);
-    if constexpr (TCS) {
-        tc41::begin(&tc_tbase, &tc_mbar, bt, btab);
-        cp_async_commit();
-    }
+    tc41::begin(&tc_tbase, &tc_mbar, bt, btab);
+    cp_async_commit();
     load_twiddles(tw, tw_g);
-    // unrolled by two: two trips' spectral loads in flight together
-#pragma unroll 2
-    for (int e = threadIdx.x; e < R * NC; e += blockDim.x) {
-        const int rr = e / NC, k = e - rr * NC;
-        float2 v[6];
-        if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
-        else {
-#pragma unroll
-            for (int f = 0; f < 6; ++f) v[f] = make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            float2 Av = v[2 * f], Bv = v[2 * f + 1];
-            if (k == 0 || 2 * k == N) { Av.y = 0.f; Bv.y = 0.f; }
-            float2 *line = buf + (rr * 3 + f) * N;
-            // Z_k = A_k + i B_k ; Z_(n-k) = conj(A_k) + i conj(B_k)
-            line[k] = make_float2(Av.x - Bv.y, Av.y + Bv.x);
-            if (k > 0 && 2 * k != N) line[N - k] = make_float2(Av.x + Bv.y, Bv.x - Av.y);
-        }
-    }
-    tc41::Ctx tcx{};
-    if constexpr (TCS) {
-        cp_async_wait_all();
-        tcx = tc41::ready(&tc_tbase, &tc_mbar, bt, tc_err);
-        tc41::lines<+1, 1, N>(buf, tw, tcx);
-    } else {
-        __syncthreads();
-        lines<+1, 1, N>(buf, tw);
-    }
+    rows_in<6, 3>(buf, op, row0, R, rcnt, g.NzK);
+    cp_async_wait_all();
+    tc41::Ctx tcx = tc41::ready(&tc_tbase, &tc_mbar, bt, tc_err);
+    tc41::lines<+1, 1, N>(buf, tw, tcx);
     typename Op::Acc acc = Op::Acc::identity();
     for (int e = threadIdx.x; e < rcnt * N; e += blockDim.x) {
         const int r = e / N, z = e - r * N;
@@ -2495,23 +2421,9 @@ k_zpass246(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float4 
         if (threadIdx.x == 0) op.finish(blockIdx.x, acc);
     }
     __syncthreads();
-    if constexpr (TCS) tc41::lines<-1, 1, N>(buf, tw, tcx);
-    else lines<-1, 1, N>(buf, tw);
-    const int nk = g.NzK;
-    for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
-        const int rr = e / nk, k = e - rr * nk;
-        float2 v[6];
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            const float2 *line = buf + (rr * 3 + f) * N;
-            const float2 Zk = line[k], Zm = line[k == 0 ? 0 : N - k];
-            // A_k = (Z_k + conj Z_-k) / 2 ; B_k = (Z_k - conj Z_-k) / (2 i)
-            v[2 * f] = make_float2(0.5f * (Zk.x + Zm.x), 0.5f * (Zk.y - Zm.y));
-            v[2 * f + 1] = make_float2(0.5f * (Zk.y + Zm.y), 0.5f * (Zm.x - Zk.x));
-        }
-        op.store_spec(row0 + rr, k, v);
-    }
-    if constexpr (TCS) tc41::end(tcx.tmem);
+    tc41::lines<-1, 1, N>(buf, tw, tcx);
+    rows_out<6, 3>(buf, op, row0, rcnt, g.NzK);
+    tc41::end(tcx.tmem);
 }
 
 template <int DIR>
@@ -2529,20 +2441,21 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
         PFGB_CUDA_TRY(cudaGetLastError());
         return PFGB_OK;
     }
-    const size_t smem = f246::axis_smem_bytes();
+    using E = f246::Eng<f246::Y_NL>;
+    const size_t smem = E::SMEM;
     auto kern = k_y246<DIR>;
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     AxisIO<float, 6, 6> io;
     for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
-    dim3 grid((c->g.NzK + f246::YC - 1) / f246::YC, c->g.Nx, 6 / f246::YS);
+    dim3 grid((c->g.NzK + E::NL - 1) / E::NL, c->g.Nx, 6);
     ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
-    kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], io, c->skip);
+    kern<<<grid, E::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], io, c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
 }
 
 static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblocks, int mode = 0) {
-    const size_t smem = f246::axis_smem_bytes();
+    using E = f246::Eng<42>;
     GreenArgs<float> A;
     A.g = c->g;
     A.kt = KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz};
@@ -2561,19 +2474,20 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     A.tc_err = c->tc_err;
     A.resid = resid;
     A.mode = mode;
-    dim3 grid((c->g.NzK + f246::TC - 1) / f246::TC, c->g.kept_rows());
+    const int TC = c->tc_x ? f246::TC : E::NL / 6, threads = c->tc_x ? f246::THREADS : E::THREADS;
+    dim3 grid((c->g.NzK + TC - 1) / TC, c->g.kept_rows());
     ProfScope ps(c, {eigen ? "x_green_eigen" : "x_green_hij",
                      (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(float2)});
     auto go = [&](auto kern, size_t sm) -> pfgb_status {
         PFGB_CUDA_TRY(allow_smem(kern, sm));
-        kern<<<grid, f246::THREADS, sm, c->stream>>>(A);
+        kern<<<grid, threads, sm, c->stream>>>(A);
         return PFGB_OK;
     };
     if (c->tc_x) {   // the 41-point stages on the tensor cores
         const size_t smem_tc = tc41::y_smem_bytes();
         TRY(eigen ? go(k_x_green246<true, true>, smem_tc) : go(k_x_green246<false, true>, smem_tc));
     } else {
-        TRY(eigen ? go(k_x_green246<true, false>, smem) : go(k_x_green246<false, false>, smem));
+        TRY(eigen ? go(k_x_green246<true, false>, E::SMEM) : go(k_x_green246<false, false>, E::SMEM));
     }
     PFGB_CUDA_TRY(cudaGetLastError());
     *nblocks = grid.x * grid.y;
@@ -2581,23 +2495,15 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
 }
 
 template <class Op>
-static pfgb_status launch_z246(pfgb_ctx *c, Op op, const char *tag, double extra_bytes) {
-    const size_t smem = f246::z_smem_bytes();
+static pfgb_status launch_z246tc(pfgb_ctx *c, Op op, const char *tag, double extra_bytes) {
     const long long rows = (long long)c->g.Nx * c->g.Ny;
     const int nb = (int)((rows + f246::ZR - 1) / f246::ZR);
     ProfScope ps(c, {tag, 12.0 * c->g.cols() * sizeof(float2) + extra_bytes});
-    if (c->tc_z) {   // the 41-point stages on the tensor cores
-        auto kern = k_zpass246<Op, true>;
-        const size_t smem_tc = 2 * tc41::B_BYTES + smem;
-        PFGB_CUDA_TRY(allow_smem(kern, smem_tc));
-        kern<<<nb, f246::THREADS, smem_tc, c->stream>>>(c->g, (const float2 *)c->tw[1][2], op, c->skip,
-                                                         (const float4 *)c->tc_btab, c->tc_err);
-    } else {
-        auto kern = k_zpass246<Op, false>;
-        PFGB_CUDA_TRY(allow_smem(kern, smem));
-        kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][2], op, c->skip, nullptr,
-                                                     nullptr);
-    }
+    auto kern = k_zpass246tc<Op>;
+    const size_t smem = 2 * tc41::B_BYTES + (size_t)(f246::N + f246::NL * f246::N) * sizeof(float2);
+    PFGB_CUDA_TRY(allow_smem(kern, smem));
+    kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][2], op, c->skip,
+                                                  (const float4 *)c->tc_btab, c->tc_err);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
 }
@@ -2868,7 +2774,7 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
     auto hij = [&](int lin) -> pfgb_status {
         const double extra = lin ? 2.0 * Nf * sizeof(T) : (2.0 + pc.gp) * Nf * sizeof(T);
         if constexpr (std::is_same<TE, float>::value) {
-            if (c->f246[2]) return launch_z246(c, OpHijZ<T, TE>{d, pc, ec, lin}, "z_hij", extra);
+            if (c->tc_z) return launch_z246tc(c, OpHijZ<T, TE>{d, pc, ec, lin}, "z_hij", extra);
         }
         return launch_z<TE, 6, 6>(c, OpHijZ<T, TE>{d, pc, ec, lin}, "z_hij", extra);
     };

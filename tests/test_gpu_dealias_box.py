@@ -10,9 +10,10 @@ pytestmark = pytest.mark.gpu
 
 # axes of length 1 and 2 (one kept mode), 3 (the cut starts at the last mode),
 # odd and even ones, a z axis whose kept columns end inside, at and past a
-# tile of columns, and the 246-point engine on one axis at a time
+# tile of columns, and the 246-point engine on one axis at a time, its last tile
+# of columns full, with a pair and with an odd column left over
 SHAPES = [(4, 1, 2), (1, 3, 6), (3, 2, 5), (7, 9, 8), (12, 10, 47), (9, 12, 48), (5, 6, 49), (246, 4, 6), (4, 246, 9),
-          (3, 4, 246)]
+          (3, 4, 246), (246, 5, 126), (4, 246, 130), (246, 3, 134)]
 
 
 @pytest.mark.parametrize("prec,tol", [(0, 1e-6), (1, 1e-5)])
