@@ -35,10 +35,15 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE,
               "--expt-relaxed-constexpr"] + ARCH
 
-# (source, extra flags, object suffix): solver.cu is three translation units,
-# its entry points and the kernels of each field precision, compiled at once
-CU_SOURCES = [("solver.cu", [], ""), ("solver.cu", ["-DPFGB_FIELDS=float"], ".f32"),
-              ("solver.cu", ["-DPFGB_FIELDS=double"], ".f64")]
+RDC = "-rdc=true"   # the pass kernels call the line transforms of fftline.cu
+# (source, extra flags, object suffix): solver.cu is four translation units
+# (its entry points, the kernels of each field precision, the tensor-core
+# kernels), fftline.cu one per precision and direction; 80 registers in FP32,
+# 128 in FP64, as in the kernels that call it.  All are compiled at once.
+CU_SOURCES = [("solver.cu", [RDC], ""), ("solver.cu", [RDC, "-DPFGB_FIELDS=float"], ".f32"),
+              ("solver.cu", [RDC, "-DPFGB_FIELDS=double"], ".f64"), ("solver.cu", ["-DPFGB_TENSOR"], ".tc")]
+CU_SOURCES += [("fftline.cu", [RDC, f"-DPFGB_LINE_T={t}", f"-DPFGB_LINE_DIR={d}", f"-maxrregcount={r}"], f".{t[0]}{d + 1}")
+               for t, r in (("float", 80), ("double", 128)) for d in (-1, 1)]
 CU_SOURCES += [(s, [], "") for s in ("params.cu", "paramfile.cpp", "batch.cpp", "fno.cu", "checkpoint.cpp", "init.cu")]
 HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41.cuh", "dft41_tc.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
 

@@ -5,12 +5,11 @@
 //   z pass : real rows (contiguous, length Nz) <-> half spectra (NzC = Nz/2+1)
 //   y pass : complex lines of length Ny, element stride NzC
 //   x pass : complex lines of length Nx, element stride Ny*NzC
-// Each pass stages a tile of lines in shared memory and runs a Stockham
-// autosort FFT there (radices 8,4,2,3,5 coded, any other prime factor as a
-// direct DFT stage).  The passes take functors, so pointwise physics (RHS,
-// flux, eigenstrain/h_ij, stress) runs inside the z pass, and the spectral
-// updates (semi-implicit filters, gradients, Green's contraction) run inside
-// the x pass between the forward and the inverse x transform.
+// Each pass stages a tile of lines in shared memory and transforms them there
+// in place (fft_lines below).  The passes take functors, so pointwise physics
+// (RHS, flux, eigenstrain/h_ij, stress) runs inside the z pass, and the
+// spectral updates (semi-implicit filters, gradients, Green's contraction) run
+// inside the x pass between the forward and the inverse x transform.
 //
 // Real-data trick: two real lines a, b are transformed as one complex line
 // z = a + i b;  A_k = (Z_k + conj Z_{N-k})/2, B_k = (Z_k - conj Z_{N-k})/(2i).
@@ -19,7 +18,10 @@
 // of the reference.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
+#include <utility>
+#include <vector>
 
 #include "common.cuh"
 #include "rader41.cuh"
@@ -47,9 +49,32 @@ struct FastDiv {
     }
 };
 
+// A thread's walk over rows of d elements, blockDim elements at a time: (q, l)
+// advances by additions, with one division at the start.
+struct Walk {
+    int q, l, dq, dl, d;
+    __device__ __forceinline__ explicit Walk(const FastDiv &f) {
+        d = (int)f.d;
+        q = (int)f.div(threadIdx.x);
+        l = (int)threadIdx.x - q * d;
+        dq = (int)f.div(blockDim.x);
+        dl = (int)blockDim.x - dq * d;
+    }
+    __device__ __forceinline__ void step() {
+        q += dq;
+        l += dl;
+        if (l >= d) { l -= d; ++q; }
+    }
+};
+
+// One stage of a line transform of n points (decimation in frequency, in
+// place): blocks of B points, B = R * m.  It takes the R points j' + r m of a
+// block (j' < m), does their DFT, multiplies output r by W_B^(r j') and writes
+// the outputs to the same R places.  The last stage (m = 1) writes them to
+// their natural positions instead.
 struct StagePlan {
-    int R, Ns, nb, m;          // radix, span so far, butterflies per line, twiddle stride
-    FastDiv fNs, fnb;
+    int R, B, m, kind;         // kind: 0 butterfly in registers, 1 Rader 41, 2 direct sums
+    FastDiv fm, fR;
 };
 
 struct AxisPlan {
@@ -58,30 +83,54 @@ struct AxisPlan {
     StagePlan st[PFGB_MAX_STAGES];
 };
 
-// host: factor n into stages.  A radix-41 factor goes first (its Rader stage
-// then needs no input twiddles), then 8, 6, 4, 2, 3, 5, 7, other primes.
+// host: the smooth part's radices, at most 16 each: as few stages as there
+// can be, the largest radix as small as it can be
+static inline void pfgb_best_radices(int q, int lim, std::vector<int> &cur, std::vector<int> &best) {
+    if (q == 1) {
+        if (best.empty() || cur.size() < best.size() ||
+            (cur.size() == best.size() && *std::max_element(cur.begin(), cur.end()) <
+                                              *std::max_element(best.begin(), best.end())))
+            best = cur;
+        return;
+    }
+    for (int r = std::min(lim, q); r >= 2; --r) {
+        if (q % r) continue;
+        cur.push_back(r);
+        pfgb_best_radices(q / r, r, cur, best);
+        cur.pop_back();
+    }
+}
+
+// host: the stages of an n-point line.  A factor 41 goes first (Rader's
+// convolution), then the other primes above 13 as direct sums, then the
+// smooth part with radices up to 16, the largest first.
 static inline void pfgb_make_plan(int n, AxisPlan *p) {
     p->n = n;
     p->nst = 0;
-    int rad[PFGB_MAX_STAGES], nr = 0;
-    int m = n;
-    while (m % 41 == 0 && m > 1) { rad[nr++] = 41; m /= 41; }
-    while (m % 8 == 0 && m > 1) { rad[nr++] = 8; m /= 8; }
-    while (m % 6 == 0 && m > 1) { rad[nr++] = 6; m /= 6; }
-    while (m % 4 == 0 && m > 1) { rad[nr++] = 4; m /= 4; }
-    while (m % 2 == 0 && m > 1) { rad[nr++] = 2; m /= 2; }
-    for (int f = 3; m > 1; f += 2)
-        while (m % f == 0) { rad[nr++] = f; m /= f; }
-    int Ns = 1;
-    for (int s = 0; s < nr; ++s) {
+    std::vector<std::pair<int, int>> rad;   // radix, kind
+    int q = n;
+    if (q % 41 == 0) { rad.push_back({41, 1}); q /= 41; }
+    for (int f = 17; f <= q; ++f)
+        while (q % f == 0) {
+            bool prime = true;
+            for (int d = 2; d * d <= f; ++d) prime = prime && f % d;
+            if (!prime) break;
+            rad.push_back({f, 2});
+            q /= f;
+        }
+    std::vector<int> cur, best;
+    if (q > 1) pfgb_best_radices(q, 16, cur, best);
+    for (int r : best) rad.push_back({r, 0});
+    int B = n;
+    for (auto &rk : rad) {
         StagePlan &st = p->st[p->nst++];
-        st.R = rad[s];
-        st.Ns = Ns;
-        st.nb = n / rad[s];
-        st.m = n / (Ns * rad[s]);
-        st.fNs.init((unsigned)Ns);
-        st.fnb.init((unsigned)st.nb);
-        Ns *= rad[s];
+        st.R = rk.first;
+        st.kind = rk.second;
+        st.B = B;
+        st.m = B / rk.first;
+        st.fm.init((unsigned)st.m);
+        st.fR.init((unsigned)st.R);
+        B = st.m;
     }
 }
 
@@ -179,7 +228,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // twiddle w = W_n^e (table holds the forward roots); inverse uses conj
 template <int DIR, typename T2>
 __device__ __forceinline__ T2 twmul(T2 a, T2 w) {
-    return DIR < 0 ? cmul(a, w) : cmulconj(a, w);
+    // the fused form written out, the same rounding wherever it is inlined
+    const decltype(T2::x) wy = DIR < 0 ? w.y : -w.y;
+    return mk2<T2>(fma(a.x, w.x, -(a.y * wy)), fma(a.y, w.x, a.x * wy));
 }
 
 template <typename T, int DIR>
@@ -200,240 +251,75 @@ __device__ __forceinline__ void bfly6(cplx_t<T> *v) {
 }
 
 // ---------------------------------------------------------------------------
-// Radix-41 stage by Rader's algorithm, 8 lanes per 41-point DFT.
-//   X_0 = sum x ;  X_{7^q} = x_0 + (a (*) b)_q,  a_p = x_{6^p}  (mod 41)
-// The length-40 cyclic convolution is IFFT40(FFT40(a) . B) with
-// B = FFT40(b)/40 (rader41.cuh).  FFT40 = 5 x 8: lane t (0..7) owns
-// a[t + 8m], m = 0..4, does the 5-point DFTs in registers, the W40^{t k1}
-// twiddles, and the 8-point DFTs run across the 8 lanes with shuffles
-// (decimation in frequency forward -> bit-reversed lanes, decimation in time
-// inverse -> natural lanes).  Index maps: 6^(t+8m) = 6^t 10^m, 7^(t+8m) =
-// 7^t 37^m (mod 41).
+// Line transforms in shared memory, in place.  L lines of n points; element
+// (line l, position p) at buf[p * PS + l * LS] (PS = L, LS = 1 for strided
+// axes; PS = 1, LS odd for z rows).  The lanes of a warp walk the lines, so
+// every access is contiguous in l (or has the odd stride LS): no bank
+// conflicts at any stage, and the index arithmetic is per butterfly of up to
+// 16 points.  A line makes one trip through shared memory per stage: two
+// stages up to 256 points, three up to 1024.
+//
+// The transform is a device function of its own translation unit
+// (fftline.cu), one per precision and direction: every pass kernel calls the
+// same code, which is compiled once.  It takes shared-memory addresses, so
+// that its accesses stay shared-memory instructions.
 // ---------------------------------------------------------------------------
-template <typename T> struct RaderTab;
-template <> struct RaderTab<float> {
-    static __device__ __forceinline__ float2 B(int dir, int k) { return dir < 0 ? c_rader41_BF_f[k] : c_rader41_BI_f[k]; }
+// the tile of a transform: shared addresses of the lines and of the twiddle
+// table, the strides in bytes, the line count
+struct LineTile {
+    uint32_t buf, tw;
+    int PS, LS;
+    FastDiv fL;                // by the line count
 };
-template <> struct RaderTab<double> {
-    static __device__ __forceinline__ double2 B(int dir, int k) { return dir < 0 ? c_rader41_BF_d[k] : c_rader41_BI_d[k]; }
-};
 
-template <typename T2>
-__device__ __forceinline__ T2 shfl_x(T2 v, int m, unsigned mask) {
-    v.x = __shfl_xor_sync(mask, v.x, m, 8);
-    v.y = __shfl_xor_sync(mask, v.y, m, 8);
-    return v;
-}
+template <typename T, int DIR> __device__ void fft_lines_at(LineTile t, const AxisPlan *plan);
+template <> __device__ void fft_lines_at<float, -1>(LineTile, const AxisPlan *);
+template <> __device__ void fft_lines_at<float, +1>(LineTile, const AxisPlan *);
+template <> __device__ void fft_lines_at<double, -1>(LineTile, const AxisPlan *);
+template <> __device__ void fft_lines_at<double, +1>(LineTile, const AxisPlan *);
 
+// the whole transform of a tile's lines; all threads of the block call it,
+// ends with __syncthreads()
 template <typename T, int DIR>
-__device__ void stage_rader41(const cplx_t<T> *src, cplx_t<T> *dst, const StagePlan &st,
-                              const cplx_t<T> *tw, int nl, int sp, int sl, bool lineFast, const FastDiv &fnl) {
+__device__ __forceinline__ void fft_lines(const cplx_t<T> *buf, const cplx_t<T> *tw, const AxisPlan &p,
+                                          const FastDiv &fL, int PS, int LS) {
     using T2 = cplx_t<T>;
-    const int nb = st.nb, Ns = st.Ns, m = st.m;
-    const FastDiv fnb = st.fnb, fNs = st.fNs;     // register copies
-    const int t = threadIdx.x & 7;
-    const int group = threadIdx.x >> 3, ngroups = blockDim.x >> 3;
-    const unsigned gmask = 0xffu << (threadIdx.x & 24);
-    const int brt = ((t & 1) << 2) | (t & 2) | ((t & 4) >> 2);
-    // per-lane constants: W40^{t k1}, B[k1 + 5 br(t)], butterfly signs/twiddles,
-    // and the shared-memory offsets of the lane's 5 inputs and 5 outputs
-    T2 W[5], Bk[5];
-#pragma unroll
-    for (int k1 = 0; k1 < 5; ++k1) {
-        T sn, cs;
-        if constexpr (sizeof(T) == 4) sincospif(-2.0f * (float)(t * k1) / 40.0f, &sn, &cs);
-        else sincospi(-2.0 * (double)(t * k1) / 40.0, &sn, &cs);
-        W[k1] = mk2<T2>(cs, sn);
-        Bk[k1] = RaderTab<T>::B(DIR, k1 + 5 * brt);
-    }
-    const T r = T(0.70710678118654752440084436210485);
-    const int p4 = t & 3, p2 = t & 1;
-    // forward twiddles of the lane's DIF butterflies (W8^{p4}, W4^{p2}); the
-    // lower lane of a pair uses 1 and sign +1, the upper one f and sign -1
-    const T2 one = mk2<T2>(T(1), T(0));
-    const T2 f4 = p4 == 0 ? one : p4 == 1 ? mk2<T2>(r, -r) : p4 == 2 ? mk2<T2>(T(0), T(-1)) : mk2<T2>(-r, -r);
-    const T2 f2 = p2 == 0 ? one : mk2<T2>(T(0), T(-1));
-    const T s4 = (t & 4) ? T(-1) : T(1), s2 = (t & 2) ? T(-1) : T(1), s1 = (t & 1) ? T(-1) : T(1);
-    const T2 w4 = (t & 4) ? f4 : one, w2 = (t & 2) ? f2 : one;
-    // inverse (DIT) twiddles W8^{+p4}, W4^{+p2} applied by the upper lane
-    const T2 c4 = mk2<T2>(f4.x, -f4.y), c2 = mk2<T2>(f2.x, -f2.y);
-    int inoff[5], nidx[5], outoff[5];
-    {
-        int n = 1, o = 1;
-        for (int i = 0; i < t; ++i) { n = (n * 6) % 41; o = (o * 7) % 41; }
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            nidx[q] = n;
-            inoff[q] = n * nb * sp;
-            outoff[q] = o * Ns * sp;
-            n = (n * 10) % 41;
-            o = (o * 37) % 41;
-        }
-    }
-    const int items = nl * nb;
-    for (int it = group; it < items; it += ngroups) {
-        int j, l;
-        if (lineFast) { l = (int)fnb.div((unsigned)it); j = it - l * nb; }
-        else { j = (int)fnl.div((unsigned)it); l = it - j * nl; }
-        const int jq = (int)fNs.div((unsigned)j);
-        const int k = j - jq * Ns;
-        const T2 *sb = src + l * sl + j * sp;
-        T2 v[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            T2 x = sb[inoff[q]];
-            if (Ns > 1) x = twmul<DIR>(x, tw[nidx[q] * k * m]);
-            v[q] = x;
-        }
-        const T2 x0 = sb[0];
-        // X_0 = x_0 + sum over the 40 permuted inputs
-        T2 s = cadd(cadd(cadd(v[0], v[1]), cadd(v[2], v[3])), v[4]);
-        s = cadd(s, shfl_x(s, 1, gmask));
-        s = cadd(s, shfl_x(s, 2, gmask));
-        s = cadd(s, shfl_x(s, 4, gmask));
-        // forward FFT40 of a: in-lane DFT5, twiddle, cross-lane DFT8 (DIF)
-        bfly5<T, -1>(v);
-#pragma unroll
-        for (int q = 1; q < 5; ++q) v[q] = cmul(v[q], W[q]);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            // DIF: lower a + b, upper (a - b) w  ==  (partner + sign * own) * w_lane
-            T2 u = shfl_x(v[q], 4, gmask);
-            v[q] = cmul(mk2<T2>(u.x + s4 * v[q].x, u.y + s4 * v[q].y), w4);
-            u = shfl_x(v[q], 2, gmask);
-            v[q] = cmul(mk2<T2>(u.x + s2 * v[q].x, u.y + s2 * v[q].y), w2);
-            u = shfl_x(v[q], 1, gmask);
-            v[q] = mk2<T2>(u.x + s1 * v[q].x, u.y + s1 * v[q].y);
-            v[q] = cmul(v[q], Bk[q]);
-            // inverse DIT (bit-reversed in, natural out): the upper lane sends
-            // w b; lower: a + (w b), upper: a - (w b)
-            T2 sv = v[q];                                  // span 1: w = 1
-            u = shfl_x(sv, 1, gmask);
-            v[q] = (t & 1) ? csub(u, sv) : cadd(v[q], u);
-            sv = (t & 2) ? cmul(v[q], c2) : v[q];
-            u = shfl_x(sv, 2, gmask);
-            v[q] = (t & 2) ? csub(u, sv) : cadd(v[q], u);
-            sv = (t & 4) ? cmul(v[q], c4) : v[q];
-            u = shfl_x(sv, 4, gmask);
-            v[q] = (t & 4) ? csub(u, sv) : cadd(v[q], u);
-        }
-#pragma unroll
-        for (int q = 1; q < 5; ++q) v[q] = cmulconj(v[q], W[q]);
-        bfly5<T, +1>(v);
-        // outputs X[7^(t+8m)] = x0 + c[t+8m]
-        T2 *db = dst + l * sl + (jq * Ns * 41 + k) * sp;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) db[outoff[q]] = cadd(x0, v[q]);
-        if (t == 0) db[0] = cadd(x0, s);
-    }
+    LineTile t;
+    t.buf = (uint32_t)__cvta_generic_to_shared(buf);
+    t.tw = (uint32_t)__cvta_generic_to_shared(tw);
+    t.PS = PS * (int)sizeof(T2);
+    t.LS = LS * (int)sizeof(T2);
+    t.fL = fL;
+    fft_lines_at<T, DIR>(t, &p);
 }
 
-// one Stockham stage of compile-time radix R: each work item is one
-// butterfly (R inputs twiddled, R-point DFT in registers, R outputs)
-template <typename T, int DIR, int R>
-__device__ __forceinline__ void stage_bfly(const cplx_t<T> *src, cplx_t<T> *dst, const StagePlan &st,
-                                           const cplx_t<T> *tw, int nl, int sp, int sl, bool lineFast,
-                                           const FastDiv &fnl) {
-    using T2 = cplx_t<T>;
-    const int nb = st.nb, Ns = st.Ns, m = st.m;
-    const FastDiv fnb = st.fnb, fNs = st.fNs;     // register copies
-    const int work = nl * nb;
-    for (int w = threadIdx.x; w < work; w += blockDim.x) {
-        int j, l;
-        if (lineFast) { l = (int)fnb.div((unsigned)w); j = w - l * nb; }
-        else { j = (int)fnl.div((unsigned)w); l = w - j * nl; }
-        const int jq = (int)fNs.div((unsigned)j);
-        const int k = j - jq * Ns;
-        T2 v[R];
-        const T2 *sb = src + l * sl;
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = sb[(j + r * nb) * sp];
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = twmul<DIR>(v[r], tw[r * k * m]);
-        }
-        if constexpr (R == 2) bfly2<T, DIR>(v);
-        else if constexpr (R == 3) bfly3<T, DIR>(v);
-        else if constexpr (R == 4) bfly4<T, DIR>(v);
-        else if constexpr (R == 5) bfly5<T, DIR>(v);
-        else if constexpr (R == 6) bfly6<T, DIR>(v);
-        else bfly8<T, DIR>(v);
-        T2 *db = dst + l * sl;
-        const int base = jq * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) db[(base + r * Ns) * sp] = v[r];
-    }
-}
-
-// direct DFT stage for any other radix: one output per work item,
-// out_q = sum_r x_r W_n^{r (k m + q n/R)}  (exponent mod n)
-template <typename T, int DIR>
-__device__ void stage_direct(const cplx_t<T> *src, cplx_t<T> *dst, const StagePlan &st, int n,
-                             const cplx_t<T> *tw, int nl, int sp, int sl, bool lineFast, const FastDiv &fnl) {
-    using T2 = cplx_t<T>;
-    const int R = st.R, nb = st.nb, Ns = st.Ns, m = st.m;
-    const FastDiv fnb = st.fnb, fNs = st.fNs;
-    const int work = nl * n;
-    for (int w = threadIdx.x; w < work; w += blockDim.x) {
-        int o, l;
-        if (lineFast) { l = w / n; o = w - l * n; } else { o = (int)fnl.div((unsigned)w); l = w - o * nl; }
-        const int q = (int)fnb.div((unsigned)o);
-        const int j = o - q * nb;
-        const int jq = (int)fNs.div((unsigned)j);
-        const int k = j - jq * Ns;
-        int e = k * m + q * nb;
-        if (e >= n) e -= n;
-        const T2 *sb = src + l * sl;
-        T ar = 0, ai = 0;
-        int idx = 0;
-        for (int r = 0; r < R; ++r) {
-            T2 x = sb[(j + r * nb) * sp];
-            T2 t = tw[idx];
-            if (DIR < 0) { ar += x.x * t.x - x.y * t.y; ai += x.x * t.y + x.y * t.x; }
-            else { ar += x.x * t.x + x.y * t.y; ai += x.y * t.x - x.x * t.y; }
-            idx += e;
-            if (idx >= n) idx -= n;
-        }
-        dst[l * sl + (jq * Ns * R + k + q * Ns) * sp] = mk2<T2>(ar, ai);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// fft_lines: transform nl lines of length p.n held in shared memory.
-// Element (line l, position q) lives at buf[q*sp + l*sl].  Stockham stages
-// alternate between `a` and `b`; returns the buffer holding the result.
-// lineFast: consecutive threads walk butterflies of one line (sp == 1);
-// otherwise consecutive threads walk lines (sl == 1).
-// Must be called by all threads of the block; ends with __syncthreads().
-// ---------------------------------------------------------------------------
-template <typename T, int DIR>
-__device__ __forceinline__ cplx_t<T> *fft_lines(cplx_t<T> *a, cplx_t<T> *b, const AxisPlan &p,
-                                                const cplx_t<T> *tw, int nl, int sp, int sl, bool lineFast) {
-    using T2 = cplx_t<T>;
-    FastDiv fnl;
-    fnl.init((unsigned)nl);
-    T2 *src = a, *dst = b;
+// threads of a block whose tile has L lines: one trip of every stage where 256
+// threads hold it, else equal trips (a second trip of a few butterflies would
+// leave the block's other warps waiting).  The last stage has one butterfly per
+// thread in registers, a direct stage eight sums, and both take whole lines.
+static inline int pfgb_line_threads(const AxisPlan &p, int L) {
+    int t = 64, least = 64;
     for (int s = 0; s < p.nst; ++s) {
-        const StagePlan st = p.st[s];
-        switch (st.R) {
-            case 2: stage_bfly<T, DIR, 2>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 3: stage_bfly<T, DIR, 3>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 4: stage_bfly<T, DIR, 4>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 5: stage_bfly<T, DIR, 5>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 6: stage_bfly<T, DIR, 6>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 8: stage_bfly<T, DIR, 8>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            case 41: stage_rader41<T, DIR>(src, dst, st, tw, nl, sp, sl, lineFast, fnl); break;
-            default: stage_direct<T, DIR>(src, dst, st, p.n, tw, nl, sp, sl, lineFast, fnl); break;
-        }
-        __syncthreads();
-        T2 *t = src; src = dst; dst = t;
+        const int R = p.st[s].R, nb = p.n / R;
+        int per = 1;                                   // work items of a thread and trip
+        long long items = (long long)L * nb;
+        if (p.st[s].kind == 1) items *= 8;             // eight lanes per butterfly
+        else if (p.st[s].kind == 2) { items = (long long)L * p.n; per = 8; least = std::max(least, (p.n + 7) / 8); }
+        else if (s == p.nst - 1) least = std::max(least, nb);
+        const long long trips = (items + 256 * per - 1) / (256 * per);
+        t = std::max(t, (int)((items + trips * per - 1) / (trips * per)));
     }
-    return src;
+    return std::min(256, (std::max(t, least) + 31) / 32 * 32);
 }
+
+// blocks per SM that the pass kernels' registers allow for (80 or 128 per
+// thread at 256 threads)
+template <typename T> constexpr int pass_blocks() { return sizeof(T) == 4 ? 3 : 2; }
 
 // load the twiddle table of length n into shared memory
 template <typename T>
 __device__ __forceinline__ void load_tw(cplx_t<T> *s, const cplx_t<T> *g, int n) {
+#pragma unroll 1
     for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = g[i];
 }
 
@@ -466,10 +352,12 @@ struct Grid3 {
 // Strided axis pass (y or x).  A block owns TK consecutive kz columns of one
 // (i) slab (y pass) or one (j) slab (x pass): lines of length n, element
 // stride `es`.  All NIN arrays of the tile sit interleaved in one shared
-// buffer (row q holds NIN*TK values, array-major, padded by one) and are
-// transformed together by a single batched FFT with direction DIN (0 =
-// none); op.apply(i, j, k, vin, vout) combines them point by point; the NOUT
-// outputs are transformed together with DOUT (0 = none) and stored.
+// buffer (row q holds max(NIN, NOUT) x TK values, array-major) and are
+// transformed together with direction DIN (0 = none); op.apply(i, j, k, vin,
+// vout) combines them point by point in place; the NOUT outputs are
+// transformed together with DOUT (0 = none) and stored.  A pass with an
+// identity op transforms each array by itself: one array per block
+// (blockIdx.z), with as many more columns.
 // ---------------------------------------------------------------------------
 template <typename T, int NIN, int NOUT>
 struct AxisIO {
@@ -479,77 +367,92 @@ struct AxisIO {
 
 template <int NIN, int NOUT> constexpr int axis_width() { return NIN > NOUT ? NIN : NOUT; }
 
+// divisors of an axis pass's loops: the columns of a tile, the lines that it
+// transforms forward and back
+struct TileDiv {
+    FastDiv tk, in, out;
+};
+
+// arrays that share a block's tile
+template <int NIN, int NOUT, class Op> constexpr int axis_tile_arrays() {
+    return Op::kInplace ? 1 : axis_width<NIN, NOUT>();
+}
+
 template <typename T, int NIN, int NOUT, int DIN, int DOUT, class Op>
-__global__ void __launch_bounds__(256)
-k_axis_pass(Grid3 g, int axis, AxisPlan plan, const cplx_t<T> *tw_g, int TK,
+__global__ void __launch_bounds__(256, pass_blocks<T>())
+k_axis_pass(Grid3 g, int axis, const __grid_constant__ AxisPlan plan, const cplx_t<T> *tw_g, TileDiv td,
             AxisIO<T, NIN, NOUT> io, Op op, const double *skip) {
     if (skip && *skip != 0.0) return;   // a finished elastic iteration: launched ahead, nothing to do
     using T2 = cplx_t<T>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     T2 *sm = reinterpret_cast<T2 *>(smem_raw);
-    constexpr int NW = axis_width<NIN, NOUT>();
-    const int n = plan.n;
-    const int SPI = NIN * TK + 1, SPO = NOUT * TK + 1;   // padded row strides
-    const int buf = n * (NW * TK + 1);
-    T2 *tw = sm;
-    T2 *A = sm + n, *B = A + buf;
     constexpr bool INPL = Op::kInplace;   // identity op: outputs are the inputs
+    constexpr int NW = axis_tile_arrays<NIN, NOUT, Op>();
+    constexpr int NI = INPL ? 1 : NIN, NO = INPL ? 1 : NOUT;
+    const FastDiv fTK = td.tk;
+    const int n = plan.n, TK = (int)fTK.d, SP = NW * TK;
+    T2 *tw = sm, *A = sm + n;
 
     const int k0 = blockIdx.x * TK;
     const int slab = axis == 1 ? blockIdx.y : g.kept_row(blockIdx.y);   // i for the y pass, j for the x pass
-    long long base, es;
+    long long base;
+    int es;
     if (axis == 1) { base = (long long)slab * g.Ny * g.NzC + k0; es = g.NzC; }
-    else { base = (long long)slab * g.NzC + k0; es = (long long)g.Ny * g.NzC; }
+    else { base = (long long)slab * g.NzC + k0; es = g.Ny * g.NzC; }
     const int kcnt = min(TK, g.NzK - k0);
-    const int lgTK = __ffs(TK) - 1;    // TK is a power of two
     // rows cut by the dealias rule: zero into an inverse y pass, not written
     // by a forward one
     const int z0 = axis == 1 ? g.jc0 : n, z1 = axis == 1 ? g.jc1 : n;
+    // the arrays of this block (selects: a run-time index of io would put it
+    // in local memory)
+    const T2 *in[NI > 0 ? NI : 1];
+    T2 *out[NO > 0 ? NO : 1];
+#pragma unroll
+    for (int a = 0; a < NI; ++a) in[a] = io.in[a] + base;
+#pragma unroll
+    for (int a = 0; a < NO; ++a) out[a] = io.out[a] + base;
+    if constexpr (INPL) {
+#pragma unroll
+        for (int a = 1; a < NIN; ++a)
+            if ((int)blockIdx.z == a) { in[0] = io.in[a] + base; out[0] = io.out[a] + base; }
+    }
 
     if (DIN != 0 || DOUT != 0) load_tw<T>(tw, tw_g, n);
+    // (loops kept rolled here and below: a small grid runs each instruction
+    // once or twice per block, and fetching unrolled code is what it waits for)
+#pragma unroll 1
+    for (Walk w(fTK); w.q < n; w.step()) {
+        const bool ok = w.l < kcnt && !(DIN > 0 && w.q >= z0 && w.q < z1);
+        const int o = ok ? w.q * es + w.l : 0;
 #pragma unroll
-    for (int a = 0; a < NIN; ++a) {
-        for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-            const int q = e >> lgTK, l = e & (TK - 1);
-            const bool ok = l < kcnt && !(DIN > 0 && q >= z0 && q < z1);
-            cp_async_elem(&A[q * SPI + a * TK + l], io.in[a] + (ok ? base + q * es + l : base), ok);
-        }
+        for (int a = 0; a < NI; ++a) cp_async_elem(&A[w.q * SP + a * TK + w.l], in[a] + o, ok);
     }
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    T2 *cur = A, *oth = B;
-    if (DIN != 0) {
-        T2 *r = fft_lines<T, DIN>(cur, oth, plan, tw, NIN * TK, SPI, 1, false);
-        if (r != cur) { oth = cur; cur = r; }
-    }
-    int SP = SPI;
+    if (DIN != 0) fft_lines<T, DIN>(A, tw, plan, td.in, SP, 1);
     if constexpr (!INPL) {
-        for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-            const int q = e >> lgTK, l = e & (TK - 1);
-            const int k = k0 + l;
+#pragma unroll 1
+        for (Walk w(fTK); w.q < n; w.step()) {
+            const int q = w.q, l = w.l;
+            const int k = min(k0 + l, g.NzC - 1);
             const int i = (axis == 1) ? slab : q;
             const int j = (axis == 1) ? q : slab;
-            T2 vin[NIN > 0 ? NIN : 1], vout[NOUT > 0 ? NOUT : 1];
+            T2 vin[NI > 0 ? NI : 1], vout[NO > 0 ? NO : 1];
 #pragma unroll
-            for (int a = 0; a < NIN; ++a) vin[a] = cur[q * SPI + a * TK + l];
+            for (int a = 0; a < NI; ++a) vin[a] = A[q * SP + a * TK + l];
             op.apply(i, j, k, vin, vout);
 #pragma unroll
-            for (int a = 0; a < NOUT; ++a) oth[q * SPO + a * TK + l] = vout[a];
+            for (int a = 0; a < NO; ++a) A[q * SP + a * TK + l] = vout[a];
         }
         __syncthreads();
-        T2 *t = cur; cur = oth; oth = t;
-        SP = SPO;
     }
-    if (DOUT != 0) {
-        T2 *r = fft_lines<T, DOUT>(cur, oth, plan, tw, NOUT * TK, SP, 1, false);
-        if (r != cur) { oth = cur; cur = r; }
-    }
+    if (DOUT != 0) fft_lines<T, DOUT>(A, tw, plan, td.out, SP, 1);
+#pragma unroll 1
+    for (Walk w(fTK); w.q < n; w.step()) {
+        if (w.l < kcnt && !(DIN < 0 && w.q >= z0 && w.q < z1)) {
 #pragma unroll
-    for (int a = 0; a < NOUT; ++a) {
-        for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-            const int q = e >> lgTK, l = e & (TK - 1);
-            if (l < kcnt && !(DIN < 0 && q >= z0 && q < z1)) io.out[a][base + q * es + l] = cur[q * SP + a * TK + l];
+            for (int a = 0; a < NO; ++a) out[a][w.q * es + w.l] = A[w.q * SP + a * TK + w.l];
         }
     }
 }
@@ -607,23 +510,28 @@ __device__ void block_reduce_acc(Acc &a) {
     }
 }
 
+// divisors of the z pass's loops: Nz, NzC, the kept columns, the lines in and out
+struct ZDiv {
+    FastDiv n, nc, nk, in, out;
+};
+
 template <typename T, int NFI, int NFO, class Op>
-__global__ void __launch_bounds__(256)
-k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const double *skip) {
+__global__ void __launch_bounds__(256, 2)
+k_zpass(Grid3 g, const __grid_constant__ AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, ZDiv zd,
+        const double *skip) {
     if (skip && *skip != 0.0) return;
     using T2 = cplx_t<T>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     T2 *sm = reinterpret_cast<T2 *>(smem_raw);
-    const int n = g.Nz, nc = g.NzC;
+    const int n = g.Nz, nc = g.NzC, LS = n | 1;   // odd line stride: no bank conflicts across lines
     T2 *tw = sm;
     T2 *ws = sm + n;
     const int PI_ = (NFI > 0) ? (R * NFI + 1) / 2 : 0;
     const int PO_ = (NFO > 0) ? (R * NFO + 1) / 2 : 0;
     // NFI == NFO: the pointwise stage runs in place on the C2R result (same
-    // line layout), so two buffers suffice
+    // line layout)
     constexpr bool SAME = (NFI == NFO);
-    T2 *inA = ws, *inB = ws + PI_ * n;
-    T2 *outA = SAME ? nullptr : ws + 2 * PI_ * n, *outB = SAME ? nullptr : outA + PO_ * n;
+    T2 *inA = ws, *outA = SAME ? ws : ws + PI_ * LS;
     const long long row0 = (long long)blockIdx.x * R;
     const long long nrows = (long long)g.Nx * g.Ny;
     const int rcnt = (int)min((long long)R, nrows - row0);
@@ -632,14 +540,14 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
     auto pack = [&](int p, int k, T2 A, T2 B) {
         if (k == 0 || 2 * k == n) { A.y = T(0); B.y = T(0); }
         // Z_k = A_k + i B_k ; Z_{n-k} = conj(A_k) + i conj(B_k)
-        inA[p * n + k] = mk2<T2>(A.x - B.y, A.y + B.x);
-        if (k > 0 && 2 * k != n) inA[p * n + (n - k)] = mk2<T2>(A.x + B.y, B.x - A.y);
+        inA[p * LS + k] = mk2<T2>(A.x - B.y, A.y + B.x);
+        if (k > 0 && 2 * k != n) inA[p * LS + (n - k)] = mk2<T2>(A.x + B.y, B.x - A.y);
     };
     if (NFI > 0 && (NFI % 2) == 0) {
         // even field count: the pairs of a row are (f0,f1), (f2,f3), ...;
         // each (row, k) is loaded once
-        for (int e = threadIdx.x; e < R * nc; e += blockDim.x) {
-            const int rr = e / nc, k = e - rr * nc;
+        for (Walk w(zd.nc); w.q < R; w.step()) {
+            const int rr = w.q, k = w.l;
             T2 v[NFI > 0 ? NFI : 1];
             if (rr < rcnt && k < g.NzK) op.load_spec(row0 + rr, k, v);
             else {
@@ -650,12 +558,11 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
             for (int f = 0; f < NFI / 2; ++f) pack(rr * (NFI / 2) + f, k, v[2 * f], v[2 * f + 1]);
         }
         __syncthreads();
-        T2 *r = fft_lines<T, +1>(inA, inB, plan, tw, PI_, 1, n, true);
-        if (r != inA) { inB = inA; inA = r; }
+        fft_lines<T, +1>(inA, tw, plan, zd.in, 1, LS);
     } else if (NFI > 0) {
         // pack pairs of half spectra into full complex spectra
-        for (int e = threadIdx.x; e < PI_ * nc; e += blockDim.x) {
-            const int p = e / nc, k = e - p * nc;
+        for (Walk w(zd.nc); w.q < PI_; w.step()) {
+            const int p = w.q, k = w.l;
             T2 A = mk2<T2>(T(0), T(0)), B = mk2<T2>(T(0), T(0));
             const int la = 2 * p, lb = 2 * p + 1;
             const int ra = la / (NFI > 0 ? NFI : 1), fa = la - ra * (NFI > 0 ? NFI : 1);
@@ -673,20 +580,17 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
             pack(p, k, A, B);
         }
         __syncthreads();
-        T2 *r = fft_lines<T, +1>(inA, inB, plan, tw, PI_, 1, n, true);
-        if (r != inA) { inB = inA; inA = r; }
+        fft_lines<T, +1>(inA, tw, plan, zd.in, 1, LS);
     }
-    if constexpr (SAME) { outA = inA; outB = inB; }
     // pointwise stage
     typename Op::Acc acc = Op::Acc::identity();
-    auto cell_step = [&](int e, auto &&pointf) {
-        const int r = e / n, z = e - r * n;
+    auto cell_step = [&](int r, int z, auto &&pointf) {
         if (r >= rcnt) {
             if (NFO > 0) {
 #pragma unroll
                 for (int f = 0; f < NFO; ++f) {
                     const int l = r * NFO + f;
-                    T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * n + z]);
+                    T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * LS + z]);
                     dst[l & 1] = T(0);
                 }
             }
@@ -696,14 +600,14 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
 #pragma unroll
         for (int f = 0; f < NFI; ++f) {
             const int l = r * NFI + f;
-            const T *src = reinterpret_cast<const T *>(&inA[(l >> 1) * n + z]);
+            const T *src = reinterpret_cast<const T *>(&inA[(l >> 1) * LS + z]);
             vi[f] = src[l & 1];
         }
         pointf((row0 + r) * n + z, vi, vo);
 #pragma unroll
         for (int f = 0; f < NFO; ++f) {
             const int l = r * NFO + f;
-            T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * n + z]);
+            T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * LS + z]);
             dst[l & 1] = vo[f];
         }
     };
@@ -712,24 +616,25 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
         // the op's global reads of B cells go out together before any of
         // their stores (an op that reads and writes the same field cannot
         // have them reordered by the compiler)
-        for (int e0 = threadIdx.x; e0 < R * n; e0 += B * blockDim.x) {
+        for (Walk w(zd.n); w.q < R;) {
             typename Op::Pre pre[B];
+            int r[B], z[B];
 #pragma unroll
             for (int b = 0; b < B; ++b) {
-                const int e = e0 + b * blockDim.x;
-                const int r = e / n;
-                if (e < R * n && r < rcnt) op.fetch((row0 + r) * n + (e - r * n), pre[b]);
+                r[b] = w.q;
+                z[b] = w.l;
+                if (w.q < rcnt) op.fetch((row0 + w.q) * n + w.l, pre[b]);
+                w.step();
             }
 #pragma unroll
-            for (int b = 0; b < B; ++b) {
-                const int e = e0 + b * blockDim.x;
-                if (e < R * n)
-                    cell_step(e, [&](long long cell, const T *vi, T *vo) { op.point_with(cell, pre[b], vi, vo, acc); });
-            }
+            for (int b = 0; b < B; ++b)
+                if (r[b] < R)
+                    cell_step(r[b], z[b],
+                              [&](long long cell, const T *vi, T *vo) { op.point_with(cell, pre[b], vi, vo, acc); });
         }
     } else {
-        for (int e = threadIdx.x; e < R * n; e += blockDim.x)
-            cell_step(e, [&](long long cell, const T *vi, T *vo) { op.point(cell, vi, vo, acc); });
+        for (Walk w(zd.n); w.q < R; w.step())
+            cell_step(w.q, w.l, [&](long long cell, const T *vi, T *vo) { op.point(cell, vi, vo, acc); });
     }
     if constexpr (Op::Acc::kActive) {
         block_reduce_acc(acc);
@@ -740,23 +645,21 @@ k_zpass(Grid3 g, AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, const doubl
         if ((R * NFO) & 1) {
             const int l = R * NFO;
             for (int z = threadIdx.x; z < n; z += blockDim.x) {
-                T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * n + z]);
+                T *dst = reinterpret_cast<T *>(&outA[(l >> 1) * LS + z]);
                 dst[1] = T(0);
             }
         }
         __syncthreads();
-        T2 *r = fft_lines<T, -1>(outA, outB, plan, tw, PO_, 1, n, true);
-        if (r != outA) { outB = outA; outA = r; }
+        fft_lines<T, -1>(outA, tw, plan, zd.out, 1, LS);
         // unpack and store: per (row, kz) gather all NFO fields
-        const int nk = g.NzK;
-        for (int e = threadIdx.x; e < rcnt * nk; e += blockDim.x) {
-            const int rr = e / nk, k = e - rr * nk;
+        for (Walk w(zd.nk); w.q < rcnt; w.step()) {
+            const int rr = w.q, k = w.l;
             T2 v[NFO > 0 ? NFO : 1];
 #pragma unroll
             for (int f = 0; f < NFO; ++f) {
                 const int l = rr * NFO + f, p = l >> 1;
-                const T2 Zk = outA[p * n + k];
-                const T2 Zm = outA[p * n + (k == 0 ? 0 : n - k)];
+                const T2 Zk = outA[p * LS + k];
+                const T2 Zm = outA[p * LS + (k == 0 ? 0 : n - k)];
                 // A_k = (Z_k + conj Z_-k)/2 ; B_k = (Z_k - conj Z_-k)/(2i)
                 if ((l & 1) == 0) v[f] = mk2<T2>(T(0.5) * (Zk.x + Zm.x), T(0.5) * (Zk.y - Zm.y));
                 else v[f] = mk2<T2>(T(0.5) * (Zk.y + Zm.y), T(0.5) * (Zm.x - Zk.x));

@@ -70,7 +70,7 @@ def main():
     for prec, typ, mk in (("d", "double2", "make_double2"), ("f", "float2", "make_float2")):
         for key, nm in (("fwd", "BF"), ("inv", "BI")):
             body = ",\n    ".join(f"{{{v.real:.17e}, {v.imag:.17e}}}" for v in tables[key])
-            lines.append(f"__constant__ {typ} c_rader41_{nm}_{prec}[40] = {{\n    {body}}};")
+            lines.append(f"static __constant__ {typ} c_rader41_{nm}_{prec}[40] = {{\n    {body}}};")
     with open(os.path.join(HERE, "rader41.cuh"), "w") as f:
         f.write("\n".join(lines) + "\n")
     # self-check of the construction in double precision

@@ -38,8 +38,23 @@ const char *pfgb_error_buffer(void);
 // ---------------------------------------------------------------------------
 struct KTab {
     const double *kx, *ky, *kz;
+    const float *fx, *fy, *fz;           // the same rounded to float
     const unsigned char *mx, *my, *mz;   // 1 = removed by the 2/3 rule
     __device__ __forceinline__ bool cut(int i, int j, int k) const { return (mx[i] | my[j] | mz[k]) != 0; }
+    // the wave numbers in the type of a pass (a conversion from double per point
+    // would run on the FP64 pipe)
+    template <typename T> __device__ __forceinline__ T x(int i) const {
+        if constexpr (sizeof(T) == 4) return fx[i];
+        else return kx[i];
+    }
+    template <typename T> __device__ __forceinline__ T y(int j) const {
+        if constexpr (sizeof(T) == 4) return fy[j];
+        else return ky[j];
+    }
+    template <typename T> __device__ __forceinline__ T z(int k) const {
+        if constexpr (sizeof(T) == 4) return fz[k];
+        else return kz[k];
+    }
     __device__ __forceinline__ double k2(int i, int j, int k) const {
         double a = kx[i], b = ky[j], c = kz[k];
         return a * a + b * b + c * c;
@@ -82,6 +97,7 @@ struct pfgb_ctx {
     AxisPlan plx, ply, plz;
     void *tw[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};  // [fp64|fp32][x,y,z]
     double *kx = nullptr, *ky = nullptr, *kz = nullptr;
+    float *kf = nullptr;      // the wave numbers of the three axes in float, one after another
     unsigned char *mx = nullptr, *my = nullptr, *mz = nullptr;
     void *phi[2] = {nullptr, nullptr}, *eta[2] = {nullptr, nullptr}, *Y = nullptr, *dYdt = nullptr;
     void *Yprev = nullptr;   // Y_f of the last step's start, for the stress export
@@ -149,6 +165,10 @@ struct pfgb_ctx {
     bool tc_y = false, tc_x = false, tc_z = false;   // passes that use it
 };
 
+static KTab ktab(const pfgb_ctx *c) {
+    return KTab{c->kx, c->ky, c->kz, c->kf, c->kf + c->g.Nx, c->kf + c->g.Nx + c->g.Ny, c->mx, c->my, c->mz};
+}
+
 // tag + algorithmic bytes of the next launch (set by the op-level wrappers)
 struct LaunchTag { const char *tag; double bytes; };
 
@@ -181,11 +201,35 @@ struct ProfScope {
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
-static const size_t kSmemBudget = 112 * 1024;
-// strided-axis tiles narrower than 4 columns (8 bytes each) leave half of
-// every 32-byte DRAM sector unused; long axes take 4 columns at one block
-// per SM instead, up to this budget
+// A tile of the generic engine: at most 72 KiB, three blocks per SM.  Tiles
+// narrower than 32 bytes of columns leave part of every DRAM sector unused:
+// long axes take that width at up to kSmemWide instead.
+static const size_t kSmemBudget = 72 * 1024;
 static const size_t kSmemWide = 220 * 1024;
+
+// columns per block of a generic x or y pass: as many as the budget holds,
+// fewer where the grid would leave SMs without a second block, and then the
+// least that needs as many blocks (no nearly empty last one)
+template <typename T2>
+static size_t axis_tile_bytes(int n, int arrays, int tk) { return (size_t)n * (1 + (size_t)arrays * tk) * sizeof(T2); }
+static TileDiv tile_div(int tk, int nin, int nout) {
+    TileDiv t;
+    t.tk.init((unsigned)tk);
+    t.in.init((unsigned)(tk * std::max(nin, 1)));
+    t.out.init((unsigned)(tk * std::max(nout, 1)));
+    return t;
+}
+template <typename T2>
+static int axis_tile(int n, int arrays, int slabs, int ncol) {
+    const int least = std::min(ncol, 32 / (int)sizeof(T2) > 1 ? 32 / (int)sizeof(T2) : 1);
+    int tk = std::min(ncol, 64);
+    while (tk > least && axis_tile_bytes<T2>(n, arrays, tk) > kSmemBudget) --tk;
+    while (tk > 1 && axis_tile_bytes<T2>(n, arrays, tk) > kSmemWide) --tk;
+    int nblk = (ncol + tk - 1) / tk;
+    if ((long long)slabs * nblk < 304)
+        nblk = std::max(nblk, std::min((304 + slabs - 1) / slabs, (ncol + least - 1) / least));
+    return (ncol + nblk - 1) / nblk;
+}
 
 // The dynamic shared-memory limit is an attribute of the kernel function,
 // shared by every context in the process: it is raised to the device's
@@ -394,9 +438,8 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
         auto it = g_tiles.find(key);
         if (it != g_tiles.end()) return it->second.tile;
     }
-    constexpr int NW = axis_width<NIN, NOUT>();
-    const int n = pl.n;
-    auto bytes = [&](int tk) { return ((size_t)n + 2 * (size_t)n * (NW * tk + 1)) * sizeof(T2); };
+    constexpr int NW = axis_tile_arrays<NIN, NOUT, Op>();
+    const int n = pl.n, nz = Op::kInplace ? NIN : 1;
     TileRec rec{rule, rule, INFINITY, INFINITY, tag, n, c->g.NzC, gy};
     {
         TuneStreams ts(c->stream, NIN + NOUT, (size_t)c->g.Nk * sizeof(T2));
@@ -408,12 +451,14 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
             }
             for (int tk = 1; tk <= 32; tk <<= 1) {
                 if (tk > 1 && tk / 2 >= c->g.NzK) break;
-                const size_t smem = bytes(tk);
+                const size_t smem = axis_tile_bytes<T2>(n, NW, tk);
                 if (smem > kSmemWide || allow_smem(kern, smem) != cudaSuccess) break;
-                const dim3 grid((c->g.NzK + tk - 1) / tk, gy);
+                const dim3 grid((c->g.NzK + tk - 1) / tk, gy, nz);
                 const T2 *tw = twp<T>(c, axis == 1 ? 1 : 0);
+                const TileDiv ft = tile_div(tk, Op::kInplace ? 1 : NIN, Op::kInplace ? 1 : NOUT);
+                const int nt = pfgb_line_threads(pl, NW * tk);
                 const float t = time_launch(ts.ss, [&](int i) {
-                    kern<<<grid, 256, smem, ts.ss[i]>>>(c->g, axis, pl, tw, tk, io[i], op, nullptr);
+                    kern<<<grid, nt, smem, ts.ss[i]>>>(c->g, axis, pl, tw, ft, io[i], op, nullptr);
                 });
                 if (tk == rule) rec.t_rule_ms = t;
                 if (t < rec.t_ms) { rec.t_ms = t; rec.tile = tk; }
@@ -425,12 +470,26 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
     return g_tiles.emplace(key, rec).first->second.tile;   // the first thread's choice stands
 }
 
+// lines of a generic z pass of R rows, and its loops' divisors
+template <int NFI, int NFO>
+static int zpass_lines(int R) { return (R * std::max(NFI, NFO) + 1) / 2; }
+template <int NFI, int NFO>
+static ZDiv zdiv(const Grid3 &g, int R) {
+    ZDiv z;
+    z.in.init((unsigned)std::max(1, (R * NFI + 1) / 2));
+    z.out.init((unsigned)std::max(1, (R * NFO + 1) / 2));
+    z.n.init((unsigned)g.Nz);
+    z.nc.init((unsigned)g.NzC);
+    z.nk.init((unsigned)g.NzK);
+    return z;
+}
+
 // shared memory of a generic z pass of R rows of length n
 template <typename T, int NFI, int NFO>
 static size_t zpass_bytes(int R, int n) {
     int PI_ = NFI > 0 ? (R * NFI + 1) / 2 : 0, PO_ = NFO > 0 ? (R * NFO + 1) / 2 : 0;
     if (NFI == NFO) PO_ = 0;   // in-place pointwise stage
-    return ((size_t)n + 2 * (size_t)PI_ * n + 2 * (size_t)PO_ * n) * sizeof(cplx_t<T>);
+    return ((size_t)n + (size_t)(PI_ + PO_) * (n | 1)) * sizeof(cplx_t<T>);
 }
 
 template <typename T, int NFI, int NFO>
@@ -463,8 +522,9 @@ static int tuned_r(pfgb_ctx *c, int rule, size_t (*bytes)(int, int), const char 
                 if (smem > kSmemWide || allow_smem(kern, smem) != cudaSuccess) break;
                 const int nb = (int)((rows + r - 1) / r);
                 const T2 *tw = twp<T>(c, 2);
+                const int nt = pfgb_line_threads(c->plz, zpass_lines<NFI, NFO>(r));
                 const float t = time_launch(ts.ss, [&](int i) {
-                    kern<<<nb, 256, smem, ts.ss[i]>>>(c->g, c->plz, tw, r, op[i], nullptr);
+                    kern<<<nb, nt, smem, ts.ss[i]>>>(c->g, c->plz, tw, r, op[i], zdiv<NFI, NFO>(c->g, r), nullptr);
                 });
                 if (r == rule) rec.t_rule_ms = t;
                 if (t < rec.t_ms) { rec.t_ms = t; rec.tile = r; }
@@ -506,19 +566,18 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
             return PFGB_OK;
         }
     }
-    constexpr int NW = axis_width<NIN, NOUT>();
-    auto bytes = [&](int tk) { return ((size_t)n + 2 * (size_t)n * (NW * tk + 1)) * sizeof(T2); };
-    int TK = 16;
-    while (TK > 1 && bytes(TK) > kSmemBudget) TK >>= 1;
-    if (TK < 4 && sizeof(T) == 4 && bytes(4) <= kSmemWide) TK = 4;
-    while (TK > 1 && TK / 2 >= c->g.NzK) TK >>= 1;
+    constexpr int NW = axis_tile_arrays<NIN, NOUT, Op>();
+    const int slabs = (axis == 1 ? c->g.Nx : c->g.kept_rows()) * (Op::kInplace ? NIN : 1);
+    int TK = axis_tile<T2>(n, NW, slabs, c->g.NzK);
     if (c->p.fft_autotune & 1) TK = tuned_tk<T, NIN, NOUT, DIN, DOUT, Op>(c, axis, pl, op, TK, tag);
-    const size_t smem = bytes(TK);
+    const size_t smem = axis_tile_bytes<T2>(n, NW, TK);
     auto kern = k_axis_pass<T, NIN, NOUT, DIN, DOUT, Op>;
     PFGB_CUDA_TRY(allow_smem(kern, smem));
-    dim3 grid((c->g.NzK + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.kept_rows());
+    dim3 grid((c->g.NzK + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.kept_rows(), Op::kInplace ? NIN : 1);
+    const TileDiv ft = tile_div(TK, Op::kInplace ? 1 : NIN, Op::kInplace ? 1 : NOUT);
     ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-    kern<<<grid, 256, smem, c->stream>>>(c->g, axis, pl, twp<T>(c, axis == 1 ? 1 : 0), TK, io, op, c->skip);
+    kern<<<grid, pfgb_line_threads(pl, NW * TK), smem, c->stream>>>(c->g, axis, pl, twp<T>(c, axis == 1 ? 1 : 0), ft,
+                                                                    io, op, c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
 }
@@ -626,6 +685,7 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     int R = 64;
     while (R > 2 && bytes(R) > kSmemBudget) R >>= 1;
     const long long rows = (long long)c->g.Nx * c->g.Ny;
+    while (R > 4 && (rows + R - 1) / R < 304) R >>= 1;   // two blocks for every SM
     while (R > 2 && R / 2 >= rows) R >>= 1;
     if (c->p.fft_autotune & 2) R = tuned_r<T, NFI, NFO>(c, R, &zpass_bytes<T, NFI, NFO>, tag);
     const size_t smem = bytes(R);
@@ -633,7 +693,8 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     const int nb = (int)((rows + R - 1) / R);
     ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-    kern<<<nb, 256, smem, c->stream>>>(c->g, c->plz, twp<T>(c, 2), R, op, c->skip);
+    kern<<<nb, pfgb_line_threads(c->plz, zpass_lines<NFI, NFO>(R)), smem, c->stream>>>(c->g, c->plz, twp<T>(c, 2), R,
+                                                                                       op, zdiv<NFI, NFO>(c->g, R), c->skip);
     PFGB_CUDA_TRY(cudaGetLastError());
     if (nblocks) *nblocks = nb;
     return PFGB_OK;
@@ -887,9 +948,9 @@ struct OpGradX {
         using T2 = cplx_t<T>;
         if (kt.cut(i, j, k)) { out[0] = out[1] = out[2] = mk2<T2>(T(0), T(0)); return; }
         const T2 m = cscale(in[0], T(invN));
-        out[0] = cmul_is(m, T(kt.kx[i]));
-        out[1] = cmul_is(m, T(kt.ky[j]));
-        out[2] = cmul_is(m, T(kt.kz[k]));
+        out[0] = cmul_is(m, kt.template x<T>(i));
+        out[1] = cmul_is(m, kt.template y<T>(j));
+        out[2] = cmul_is(m, kt.template z<T>(k));
     }
 };
 
@@ -993,7 +1054,7 @@ struct OpFluxZ {
     double md[6] = {0, 0, 0, 0, 0, 0};
     __device__ void store_spec(long long row, int k, const cplx_t<T> *v) const {
         const long long o = row * d.g.NzC + k;
-        const T kz = T(d.kt.kz[k]);
+        const T kz = d.kt.template z<T>(k);
         d.S[0][o] = v[0];
         d.S[1][o] = v[1];
         d.S[2][o] = no_src ? cmul_is(v[2], kz) : csub(cmul_is(v[2], kz), v[3]);
@@ -1008,7 +1069,7 @@ struct OpYCombY {
     KTab kt;
     __device__ void apply(int, int j, int, const cplx_t<T> *in, cplx_t<T> *out) const {
         out[0] = in[0];
-        out[1] = cadd(cmul_is(in[1], T(kt.ky[j])), in[2]);
+        out[1] = cadd(cmul_is(in[1], kt.template y<T>(j)), in[2]);
         out[2] = in[3];
     }
 };
@@ -1025,7 +1086,7 @@ struct OpYUpdX {
         if (kt.cut(i, j, k)) { out[0] = mk2<T2>(T(0), T(0)); return; }
         const double den = 1.0 + dt * (*meanDY) * kt.k2(i, j, k);
         const T a = T(dt / den);
-        const T2 div = cadd(cmul_is(in[0], T(kt.kx[i])), in[1]);
+        const T2 div = cadd(cmul_is(in[0], kt.template x<T>(i)), in[1]);
         out[0] = cscale(cadd(in[2], cscale(div, a)), T(invN));
     }
 };
@@ -1038,7 +1099,7 @@ struct OpDivX {
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         using T2 = cplx_t<T>;
         if (kt.cut(i, j, k)) { out[0] = mk2<T2>(T(0), T(0)); return; }
-        out[0] = cscale(cadd(cmul_is(in[0], T(kt.kx[i])), in[1]), T(invN));
+        out[0] = cscale(cadd(cmul_is(in[0], kt.template x<T>(i)), in[1]), T(invN));
     }
 };
 
@@ -1901,7 +1962,7 @@ struct OpStrainFromUX {   // warm start: strain of the stored u, then inverse x
     static constexpr bool kInplace = false;
     KTab kt;
     __device__ void apply(int i, int j, int k, const cplx_t<TE> *u, cplx_t<TE> *out) const {
-        const TE kx = TE(kt.kx[i]), ky = TE(kt.ky[j]), kz = TE(kt.kz[k]);
+        const TE kx = kt.template x<TE>(i), ky = kt.template y<TE>(j), kz = kt.template z<TE>(k);
         const bool m = kt.cut(i, j, k);
 #pragma unroll
         for (int cmp = 0; cmp < 6; ++cmp)
@@ -2071,7 +2132,8 @@ __device__ __forceinline__ void green_u(const TE *S, TE kx, TE ky, TE kz, const 
     const TE c22 = K[0][0] * K[1][1] - K[0][1] * K[0][1];
     const TE det = K[0][0] * c00 + K[0][1] * c01 + K[0][2] * c02;
     using T2 = cplx_t<TE>;
-    if (fabs((double)det) < 1e-30) { u[0] = u[1] = u[2] = mk2<T2>(TE(0), TE(0)); return; }
+    // TE(1e-30) in float is the first value not below 1e-30: the same test
+    if (fabs(det) < TE(1e-30)) { u[0] = u[1] = u[2] = mk2<T2>(TE(0), TE(0)); return; }
     const TE id = TE(1) / det;
     const TE G[3][3] = {{c00 * id, c01 * id, c02 * id}, {c01 * id, c11 * id, c12 * id}, {c02 * id, c12 * id, c22 * id}};
 #pragma unroll
@@ -2084,49 +2146,46 @@ __device__ __forceinline__ void green_u(const TE *S, TE kx, TE ky, TE kz, const 
 }
 
 template <typename TE, bool EIGEN>
-__global__ void __launch_bounds__(256)
-k_x_green(GreenArgs<TE> A, AxisPlan plan, int TK) {
+__global__ void __launch_bounds__(256, pass_blocks<TE>())
+k_x_green(const __grid_constant__ GreenArgs<TE> A, const __grid_constant__ AxisPlan plan, TileDiv td) {
     if (A.skip && *A.skip != 0.0) return;
     using T2 = cplx_t<TE>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     T2 *sm = reinterpret_cast<T2 *>(smem_raw);
-    const int n = plan.n, SP = 6 * TK + 1;   // six components interleaved per row
-    T2 *tw = sm;
-    T2 *X = sm + n, *Yb = X + n * SP;
+    const FastDiv fTK = td.tk;
+    const int n = plan.n, TK = (int)fTK.d, SP = 6 * TK;   // six components interleaved per row
+    T2 *tw = sm, *X = sm + n;
     const int k0 = blockIdx.x * TK, j = A.g.kept_row(blockIdx.y);
     const long long base = (long long)j * A.g.NzC + k0;
     const long long es = (long long)A.g.Ny * A.g.NzC;
     const int kcnt = min(TK, A.g.NzK - k0);
-    const int lgTK = __ffs(TK) - 1;
+#pragma unroll 1
+    for (Walk w(fTK); w.q < n; w.step()) {
+        const bool ok = w.l < kcnt;
+        const long long o = base + (ok ? w.q * es + w.l : 0);
 #pragma unroll
-    for (int cmp = 0; cmp < 6; ++cmp) {
-        for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-            const int q = e >> lgTK, l = e & (TK - 1);
-            const bool ok = l < kcnt;
-            cp_async_elem(&X[q * SP + cmp * TK + l], A.E[cmp] + (ok ? base + q * es + l : base), ok);
-        }
+        for (int cmp = 0; cmp < 6; ++cmp) cp_async_elem(&X[w.q * SP + cmp * TK + w.l], A.E[cmp] + o, ok);
     }
     cp_async_commit();
     load_tw<TE>(tw, A.tw, n);
     cp_async_wait_all();
     __syncthreads();
-    T2 *cur = fft_lines<TE, -1>(X, Yb, plan, tw, 6 * TK, SP, 1, false);
-    T2 *oth = (cur == X) ? Yb : X;
+    fft_lines<TE, -1>(X, tw, plan, td.in, SP, 1);
     // per point: t_i = k_j tau_ij, u = -i G t (masked), residual, u stored,
-    // then the six strain components of u into the other buffer
+    // then the six strain components of u in place
     // residual sums: per element in elastic precision, per-thread partials
     // (a handful of elements) in elastic precision, block / grid sums in FP64
     TE rd = 0, rr = 0;
     const bool pre = A.mode == 2;   // increment update: its state loaded as one batch first
-    for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-        const int q = e >> lgTK, l = e & (TK - 1), k = k0 + l;
+    for (Walk wk(fTK); wk.q < n; wk.step()) {
+        const int q = wk.q, l = wk.l, k = k0 + l;
         GreenIn<TE> gin;
         if (pre && l < kcnt) green_fetch<TE>(A, base + q * es + l, gin);
         const int kk = min(k, A.g.NzC - 1);
-        const TE kv[3] = {TE(A.kt.kx[q]), TE(A.kt.ky[j]), TE(A.kt.kz[kk])};
+        const TE kv[3] = {A.kt.template x<TE>(q), A.kt.template y<TE>(j), A.kt.template z<TE>(kk)};
         T2 x[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) x[c] = cur[q * SP + c * TK + l];
+        for (int c = 0; c < 6; ++c) x[c] = X[q * SP + c * TK + l];
         T2 t[3];
         if (EIGEN) {
             // tau_ij = C_ij,ab eps0_ab: component c enters with weight 1
@@ -2163,7 +2222,7 @@ k_x_green(GreenArgs<TE> A, AxisPlan plan, int TK) {
             else green_update<TE>(A, o, u, w, rd, rr, v);
         }
 #pragma unroll
-        for (int c = 0; c < 6; ++c) oth[q * SP + c * TK + l] = strain_comp<TE>(c, kv[0], kv[1], kv[2], v);
+        for (int c = 0; c < 6; ++c) X[q * SP + c * TK + l] = strain_comp<TE>(c, kv[0], kv[1], kv[2], v);
     }
     if (A.resid) {
         AccSum2 s{double(rd), double(rr)};
@@ -2172,12 +2231,12 @@ k_x_green(GreenArgs<TE> A, AxisPlan plan, int TK) {
             reinterpret_cast<AccSum2 *>(A.partials)[blockIdx.y * gridDim.x + blockIdx.x] = s;
     }
     __syncthreads();
-    T2 *r = fft_lines<TE, +1>(oth, cur, plan, tw, 6 * TK, SP, 1, false);
+    fft_lines<TE, +1>(X, tw, plan, td.out, SP, 1);
+#pragma unroll 1
+    for (Walk w(fTK); w.q < n; w.step()) {
+        if (w.l < kcnt) {
 #pragma unroll
-    for (int cmp = 0; cmp < 6; ++cmp) {
-        for (int e = threadIdx.x; e < n * TK; e += blockDim.x) {
-            const int q = e >> lgTK, l = e & (TK - 1);
-            if (l < kcnt) A.E[cmp][base + q * es + l] = r[q * SP + cmp * TK + l];
+            for (int cmp = 0; cmp < 6; ++cmp) A.E[cmp][base + w.q * es + w.l] = X[w.q * SP + cmp * TK + w.l];
         }
     }
 }
@@ -2233,15 +2292,12 @@ template <typename TE>
 static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks, int mode = 0) {
     using T2 = cplx_t<TE>;
     const int n = c->plx.n;
-    auto bytes = [&](int tk) { return ((size_t)n + 2 * (size_t)n * (6 * tk + 1)) * sizeof(T2); };
-    int TK = 16;
-    while (TK > 1 && bytes(TK) > kSmemBudget) TK >>= 1;
-    if (TK < 4 && sizeof(TE) == 4 && bytes(4) <= kSmemWide) TK = 4;
-    while (TK > 1 && TK / 2 >= c->g.NzK) TK >>= 1;
-    const size_t smem = bytes(TK);
+    const int TK = axis_tile<T2>(n, 6, c->g.kept_rows(), c->g.NzK);
+    const size_t smem = axis_tile_bytes<T2>(n, 6, TK);
+    const TileDiv ft = tile_div(TK, 6, 6);
     GreenArgs<TE> A;
     A.g = c->g;
-    A.kt = KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz};
+    A.kt = ktab(c);
     for (int i = 0; i < 21; ++i) { A.ec.S[i] = (TE)c->p.S[i]; A.ec.Sp[i] = (TE)c->p.S_p[i]; }
     A.tw = (const T2 *)c->tw[sizeof(TE) == 8 ? 0 : 1][0];
     for (int i = 0; i < 6; ++i) A.E[i] = (T2 *)c->E[i];
@@ -2263,11 +2319,11 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
     if (eigen) {
         auto kern = k_x_green<TE, true>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        kern<<<grid, 256, smem, c->stream>>>(A, c->plx, TK);
+        kern<<<grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream>>>(A, c->plx, ft);
     } else {
         auto kern = k_x_green<TE, false>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        kern<<<grid, 256, smem, c->stream>>>(A, c->plx, TK);
+        kern<<<grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream>>>(A, c->plx, ft);
     }
     PFGB_CUDA_TRY(cudaGetLastError());
     *nblocks = grid.x * grid.y;
@@ -2322,7 +2378,7 @@ k_x_green246(GreenArgs<float> A) {
         GreenIn<float> cur;
         if (pre && l < kcnt) green_fetch<float>(A, base + q * es + l, cur);
         const int kk = min(k, A.g.NzC - 1);
-        const float kv[3] = {float(A.kt.kx[q]), float(A.kt.ky[j]), float(A.kt.kz[kk])};
+        const float kv[3] = {A.kt.fx[q], A.kt.fy[j], A.kt.fz[kk]};
         float2 *pt = buf + q * PSX + l;
         T2 x[6];
 #pragma unroll
@@ -2426,21 +2482,65 @@ k_zpass246tc(Grid3 g, const float2 *tw_g, Op op, const double *skip, const float
     tc41::end(tcx.tmem);
 }
 
+// the tensor-core forms' launches: their kernels sit in a translation unit
+// without relocatable device code (PFGB_TENSOR; linked as relocatable code
+// they gave wrong values)
+template <int DIR>
+pfgb_status launch_y246tc(pfgb_ctx *c, const char *tag) {
+    const size_t smem = tc41::y_smem_bytes();
+    auto kern = k_y246tc<DIR>;
+    PFGB_CUDA_TRY(allow_smem(kern, smem));
+    AxisIO<float, 6, 6> io;
+    for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
+    dim3 grid((c->g.NzK + f246::TC - 1) / f246::TC, c->g.Nx);
+    ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
+    kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], (const float4 *)c->tc_btab, io,
+                                                   c->skip, c->tc_err);
+    PFGB_CUDA_TRY(cudaGetLastError());
+    return PFGB_OK;
+}
+template <bool EIGEN>
+pfgb_status launch_green246tc(pfgb_ctx *c, const GreenArgs<float> &A, dim3 grid) {
+    auto kern = k_x_green246<EIGEN, true>;
+    const size_t smem = tc41::y_smem_bytes();
+    PFGB_CUDA_TRY(allow_smem(kern, smem));
+    kern<<<grid, f246::THREADS, smem, c->stream>>>(A);
+    return PFGB_OK;
+}
+template <class Op>
+pfgb_status launch_z246tc(pfgb_ctx *c, Op op, const char *tag, double extra_bytes) {
+    const long long rows = (long long)c->g.Nx * c->g.Ny;
+    const int nb = (int)((rows + f246::ZR - 1) / f246::ZR);
+    ProfScope ps(c, {tag, 12.0 * c->g.cols() * sizeof(float2) + extra_bytes});
+    auto kern = k_zpass246tc<Op>;
+    const size_t smem = 2 * tc41::B_BYTES + (size_t)(f246::N + f246::NL * f246::N) * sizeof(float2);
+    PFGB_CUDA_TRY(allow_smem(kern, smem));
+    kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][2], op, c->skip,
+                                                  (const float4 *)c->tc_btab, c->tc_err);
+    PFGB_CUDA_TRY(cudaGetLastError());
+    return PFGB_OK;
+}
+#ifndef PFGB_TENSOR
+extern template pfgb_status launch_y246tc<-1>(pfgb_ctx *, const char *);
+extern template pfgb_status launch_y246tc<+1>(pfgb_ctx *, const char *);
+extern template pfgb_status launch_green246tc<false>(pfgb_ctx *, const GreenArgs<float> &, dim3);
+extern template pfgb_status launch_green246tc<true>(pfgb_ctx *, const GreenArgs<float> &, dim3);
+extern template pfgb_status launch_z246tc(pfgb_ctx *, OpHijZ<float, float>, const char *, double);
+extern template pfgb_status launch_z246tc(pfgb_ctx *, OpHijZ<double, float>, const char *, double);
+#else
+template pfgb_status launch_y246tc<-1>(pfgb_ctx *, const char *);
+template pfgb_status launch_y246tc<+1>(pfgb_ctx *, const char *);
+template pfgb_status launch_green246tc<false>(pfgb_ctx *, const GreenArgs<float> &, dim3);
+template pfgb_status launch_green246tc<true>(pfgb_ctx *, const GreenArgs<float> &, dim3);
+template pfgb_status launch_z246tc(pfgb_ctx *, OpHijZ<float, float>, const char *, double);
+template pfgb_status launch_z246tc(pfgb_ctx *, OpHijZ<double, float>, const char *, double);
+#endif
+
+#ifndef PFGB_TENSOR
+
 template <int DIR>
 static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
-    if (c->tc_y) {   // the 41-point stage on the tensor cores
-        const size_t smem = tc41::y_smem_bytes();
-        auto kern = k_y246tc<DIR>;
-        PFGB_CUDA_TRY(allow_smem(kern, smem));
-        AxisIO<float, 6, 6> io;
-        for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
-        dim3 grid((c->g.NzK + f246::TC - 1) / f246::TC, c->g.Nx);
-        ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
-        kern<<<grid, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], (const float4 *)c->tc_btab,
-                                                       io, c->skip, c->tc_err);
-        PFGB_CUDA_TRY(cudaGetLastError());
-        return PFGB_OK;
-    }
+    if (c->tc_y) return launch_y246tc<DIR>(c, tag);   // the 41-point stage on the tensor cores
     using E = f246::Eng<f246::Y_NL>;
     const size_t smem = E::SMEM;
     auto kern = k_y246<DIR>;
@@ -2458,7 +2558,7 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     using E = f246::Eng<42>;
     GreenArgs<float> A;
     A.g = c->g;
-    A.kt = KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz};
+    A.kt = ktab(c);
     for (int i = 0; i < 21; ++i) { A.ec.S[i] = (float)c->p.S[i]; A.ec.Sp[i] = (float)c->p.S_p[i]; }
     A.tw = (const float2 *)c->tw[1][0];
     for (int i = 0; i < 6; ++i) A.E[i] = (float2 *)c->E[i];
@@ -2474,37 +2574,21 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     A.tc_err = c->tc_err;
     A.resid = resid;
     A.mode = mode;
-    const int TC = c->tc_x ? f246::TC : E::NL / 6, threads = c->tc_x ? f246::THREADS : E::THREADS;
+    const int TC = c->tc_x ? f246::TC : E::NL / 6;
     dim3 grid((c->g.NzK + TC - 1) / TC, c->g.kept_rows());
     ProfScope ps(c, {eigen ? "x_green_eigen" : "x_green_hij",
                      (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(float2)});
     auto go = [&](auto kern, size_t sm) -> pfgb_status {
         PFGB_CUDA_TRY(allow_smem(kern, sm));
-        kern<<<grid, threads, sm, c->stream>>>(A);
+        kern<<<grid, E::THREADS, sm, c->stream>>>(A);
         return PFGB_OK;
     };
-    if (c->tc_x) {   // the 41-point stages on the tensor cores
-        const size_t smem_tc = tc41::y_smem_bytes();
-        TRY(eigen ? go(k_x_green246<true, true>, smem_tc) : go(k_x_green246<false, true>, smem_tc));
-    } else {
+    if (c->tc_x)   // the 41-point stages on the tensor cores
+        TRY(eigen ? launch_green246tc<true>(c, A, grid) : launch_green246tc<false>(c, A, grid));
+    else
         TRY(eigen ? go(k_x_green246<true, false>, E::SMEM) : go(k_x_green246<false, false>, E::SMEM));
-    }
     PFGB_CUDA_TRY(cudaGetLastError());
     *nblocks = grid.x * grid.y;
-    return PFGB_OK;
-}
-
-template <class Op>
-static pfgb_status launch_z246tc(pfgb_ctx *c, Op op, const char *tag, double extra_bytes) {
-    const long long rows = (long long)c->g.Nx * c->g.Ny;
-    const int nb = (int)((rows + f246::ZR - 1) / f246::ZR);
-    ProfScope ps(c, {tag, 12.0 * c->g.cols() * sizeof(float2) + extra_bytes});
-    auto kern = k_zpass246tc<Op>;
-    const size_t smem = 2 * tc41::B_BYTES + (size_t)(f246::N + f246::NL * f246::N) * sizeof(float2);
-    PFGB_CUDA_TRY(allow_smem(kern, smem));
-    kern<<<nb, f246::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][2], op, c->skip,
-                                                  (const float4 *)c->tc_btab, c->tc_err);
-    PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
 }
 
@@ -2515,7 +2599,7 @@ template <typename T, typename TE>
 static DevState<T, TE> dev_state(pfgb_ctx *c) {
     DevState<T, TE> d;
     d.g = c->g;
-    d.kt = KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz};
+    d.kt = ktab(c);
     d.phi_old = (T *)c->phi[c->cur];
     d.phi_new = (T *)c->phi[1 - c->cur];
     d.eta_old = (T *)c->eta[c->ecur];
@@ -2732,7 +2816,7 @@ static pfgb_status model_start(pfgb_ctx *c) {
     AxisIO<TE, 3, 3> io;
     for (int i = 0; i < 3; ++i) { io.in[i] = (const T2e *)c->E[i]; io.out[i] = (T2e *)c->E[i]; }
     TRY((launch_axis<TE, 3, 3, -1, 0>(c, 1, io, OpCopy<TE, 3>{}, "y_fwd3")));
-    TRY((launch_axis<TE, 3, 3, -1, 0>(c, 2, io, OpCutU3<TE>{KTab{c->kx, c->ky, c->kz, c->mx, c->my, c->mz}},
+    TRY((launch_axis<TE, 3, 3, -1, 0>(c, 2, io, OpCutU3<TE>{ktab(c)},
                                       "x_fwd3")));
     ProfScope ps(c, {"add_increment", 9.0 * c->g.kept() * sizeof(T2e)});
     k_add_increment<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, (T2e *)c->U[0], (T2e *)c->U[1], (T2e *)c->U[2],
@@ -3999,10 +4083,11 @@ pfgb_status training_pair(pfgb_ctx *c, float *in8, float *tgt3, pfgb_step_stats 
     return launch_fno_inputs<T, float>(c, in8);
 }
 
-// The file is compiled three times, at the same time (build.py): as it is,
-// with the entry points, and once for each field precision with PFGB_FIELDS
+// The file is compiled four times, at the same time (build.py): as it is,
+// with the entry points; once for each field precision with PFGB_FIELDS
 // (float or double), for the step, the minimize iteration and the training
-// pair of that precision with every kernel that they launch.
+// pair of that precision with every kernel that they launch; and once with
+// PFGB_TENSOR for the tensor-core kernels.
 #ifdef PFGB_FIELDS
 template pfgb_status step_once<PFGB_FIELDS, float>(pfgb_ctx *, pfgb_step_stats *);
 template pfgb_status minimize_once<PFGB_FIELDS, float>(pfgb_ctx *, pfgb_min_stats *);
@@ -4148,6 +4233,11 @@ static pfgb_status make_ktab(pfgb_ctx *c) {
     PFGB_CUDA_TRY(cudaMemcpy(c->kx, kx.data(), sizeof(double) * P.Nx, cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->ky, ky.data(), sizeof(double) * P.Ny, cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->kz, kz.data(), sizeof(double) * c->g.NzC, cudaMemcpyHostToDevice));
+    std::vector<float> kf(kx.begin(), kx.end());
+    kf.insert(kf.end(), ky.begin(), ky.end());
+    kf.insert(kf.end(), kz.begin(), kz.end());
+    TRY(dalloc(c, (void **)&c->kf, sizeof(float) * kf.size()));
+    PFGB_CUDA_TRY(cudaMemcpy(c->kf, kf.data(), sizeof(float) * kf.size(), cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->mx, mx.data(), P.Nx, cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->my, my.data(), P.Ny, cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->mz, mz.data(), c->g.NzC, cudaMemcpyHostToDevice));
@@ -4368,7 +4458,7 @@ static void ctx_free(pfgb_ctx *c) {
     for (int a = 0; a < 2; ++a) for (int b = 0; b < 3; ++b) f(c->tw[a][b]);
     f(c->tc_btab);
     f(c->tc_err);
-    f(c->kx); f(c->ky); f(c->kz); f(c->mx); f(c->my); f(c->mz);
+    f(c->kx); f(c->ky); f(c->kz); f(c->kf); f(c->mx); f(c->my); f(c->mz);
     for (int i = 0; i < 2; ++i) f(c->phi[i]);
     f(c->eta[0]);
     if (c->eta[1] != c->eta[0]) f(c->eta[1]);
@@ -5511,3 +5601,4 @@ int pfgb_profile_read(pfgb_ctx *c, const char **names, double *ms, double *bytes
 }  // extern "C"
 
 #endif   // PFGB_FIELDS
+#endif   // PFGB_TENSOR
