@@ -133,6 +133,12 @@ template <> struct GammaEval<double> {
     static PFGB_HD double dmu_diff(const TC &c, double xc) {
         double dx = 1e-5;
         double xp = clamp_eps(xc + dx, 1e-12), xm = clamp_eps(xc - dx, 1e-12);
+        // the quotient in one logarithm: the compound constants cancel, the
+        // four logarithms are log[xp (1 - xm) / (xm (1 - xp))], and the
+        // quadratic terms' quotient is -2 L exactly (a double logarithm takes
+        // tens of instructions on the FP64 pipe)
+        if (!(c.convex && xp > PFGB_XC_CONVEX))
+            return double(c.RT_s) * log((xp * (1.0 - xm)) / (xm * (1.0 - xp))) / (xp - xm) - 2.0 * double(c.L_s);
         double aP, bP, aM, bM;
         thermo_mu<double>(c, xp, aP, bP);
         thermo_mu<double>(c, xm, aM, bM);
@@ -189,6 +195,25 @@ PFGB_HD T sigmoid_raw(T Y) {
     T e = exp(Y);
     return e / (T(1) + e);
 }
+// sigmoid(Y) and log(1 + e^-|Y|) of it from one exponential; in FP64 they give
+// log x = min(Y, 0) - ld and log(1 - x) = min(-Y, 0) - ld, one logarithm in
+// place of two (LogisticT<float> carries x alone: its logarithms are cheap)
+template <typename T>
+struct LogisticT { T Y, x, ld; };
+template <typename T>
+__device__ __forceinline__ LogisticT<T> logistic(T Y) {
+    LogisticT<T> g;
+    g.Y = Y;
+    if constexpr (sizeof(T) == 8) {
+        const T E = exp(-fabs(Y)), d = T(1) + E;
+        g.x = (Y >= T(0) ? T(1) : E) / d;
+        g.ld = log(d);
+    } else {
+        g.x = sigmoid_raw(Y);
+        g.ld = T(0);
+    }
+    return g;
+}
 template <typename T>
 PFGB_HD T sigmoid_clip(T Y, T Yc, T eps) {
     if (Y > Yc) Y = Yc;
@@ -198,6 +223,26 @@ PFGB_HD T sigmoid_clip(T Y, T Yc, T eps) {
     const T hi = one_minus_eps(eps);
     if (x > hi) x = hi;
     return x;
+}
+// sigmoid_clip of the same Y
+template <typename T>
+__device__ __forceinline__ T logistic_clip(const LogisticT<T> &g, T Yc, T eps) {
+    if (g.Y > Yc || g.Y < -Yc) return sigmoid_clip(g.Y, Yc, eps);
+    const T hi = one_minus_eps(eps);
+    return g.x < eps ? eps : (g.x > hi ? hi : g.x);
+}
+// thermo_mu_off at x, which is sigmoid(g.Y) up to the clips
+template <typename T, typename TC>
+__device__ __forceinline__ void thermo_mu_off_at(const TC &c, T x, const LogisticT<T> &g, T &offA, T &offB) {
+    if constexpr (sizeof(T) == 8) {
+        if (x == g.x && x > T(1e-12) && x < T(1) - T(1e-12) && !(c.convex && x > T(PFGB_XC_CONVEX))) {
+            const T omx = T(1) - x, lx = fmin(g.Y, T(0)) - g.ld, l1 = fmin(-g.Y, T(0)) - g.ld;
+            offA = T(c.RT_s) * l1 + T(c.L_s) * x * x;
+            offB = T(c.RT_s) * lx + T(c.L_s) * omx * omx;
+            return;
+        }
+    }
+    thermo_mu_off<T>(c, x, offA, offB);
 }
 template <typename T>
 PFGB_HD T logit_clip(T xB, T eps, T Yc) {

@@ -51,6 +51,11 @@ struct PhysCT {
     // has clamped xB; above 1 = inactive)
     R xbcap;
     R dx, dy, dz;
+    R e00f[6];         // e00 rounded to float (as the elastic solve holds it)
+    R cbc;             // 1 / Vm_alpha_0
+    unsigned spmask;   // bit v: Sp[v] is not zero
+    int cbconst;       // the molar volume does not depend on x or h: c_xB_phi is cbc
+    int e0same;        // the driving force's eigenstrain is the stress's: no GP elasticity, no cap
     ThermoConstT<R> tc;
 };
 using PhysC = PhysCT<double>;
@@ -75,6 +80,12 @@ PhysCT<R> phys_as(const PhysC &c) {
     o.disable_gamma = c.disable_gamma; o.xb_raw = c.xb_raw;
     o.gpy = c.gpy; o.haeps = R(c.haeps);
     o.xbcap = R(c.xbcap); o.dx = R(c.dx); o.dy = R(c.dy); o.dz = R(c.dz);
+    o.spmask = 0;
+    for (int i = 0; i < 21; ++i) o.spmask |= (c.Sp[i] != 0.0 ? 1u : 0u) << i;
+    for (int i = 0; i < 6; ++i) o.e00f[i] = R((float)c.e00[i]);
+    o.cbc = R(1.0 / c.Vm0);
+    o.cbconst = sizeof(R) == 8 && c.dVm == 0.0 && c.Vmc == c.Vm0 && fabs(c.Vm0) >= 1e-12;
+    o.e0same = sizeof(R) == 8 && !c.gp_el && c.xbcap > 1.0;
     o.tc = thermo_as<R>(c.tc);
     return o;
 }
@@ -94,6 +105,12 @@ struct ElasC {
     TE invN;
 };
 
+// the same from its logistic
+template <typename T, typename PC>
+__device__ __forceinline__ T xB_of(const PC &c, const LogisticT<T> &g) {
+    return c.xb_raw ? g.x : logistic_clip(g, T(c.Yclip), T(c.xBeps));
+}
+
 // xB from the logit Y: clipped form (sigmoid_from_logit) unless the zero mode
 // owns the composition, which uses the unclipped logistic
 // (apply_pf_Y_zero_mode_shift_kernel, cuda_kernels.cu:3434-3442).
@@ -112,18 +129,38 @@ __device__ __forceinline__ void eigenstrain(const PC &c, const ElasC<TE> &ec, T 
         T epsc = xBc * T(c.eiv);
         T omh = T(1) - h;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) e0[a] = (TE)(omh * epsc + h * T(ec.e00[a]));
+        for (int a = 0; a < 3; ++a) e0[a] = (TE)(omh * epsc + h * T(c.e00f[a]));
 #pragma unroll
-        for (int a = 3; a < 6; ++a) e0[a] = (TE)(h * T(ec.e00[a]));
+        for (int a = 3; a < 6; ++a) e0[a] = (TE)(h * T(c.e00f[a]));
         return;
     }
     T hb = pf_h(phi), he = pf_h(eta);
     T hg = (T(1) - hb) * he, ha = (T(1) - hb) * (T(1) - he);
     T ea = xBc * T(c.eiv);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) e0[a] = (TE)(ha * ea + hg * T(c.gpeiso) + hb * T(ec.e00[a]));
+    for (int a = 0; a < 3; ++a) e0[a] = (TE)(ha * ea + hg * T(c.gpeiso) + hb * T(c.e00f[a]));
 #pragma unroll
-    for (int a = 3; a < 6; ++a) e0[a] = (TE)(hb * T(ec.e00[a]));
+    for (int a = 3; a < 6; ++a) e0[a] = (TE)(hb * T(c.e00f[a]));
+}
+
+// FP64 fields: a value of [-1, 2] (h) as two floats, so that its products with
+// the float stiffness contrast run on the FP32 pipe: fma(hi, s, lo * s) rounds
+// like the double product (once, up to 2^-48)
+template <typename T, typename TE>
+__device__ __forceinline__ void split_hl(T h, TE &hi, TE &lo) {
+    hi = (TE)h;
+    if constexpr (sizeof(T) > sizeof(TE)) lo = (TE)(h - T(hi));
+    else lo = TE(0);
+}
+template <typename TE>
+__device__ __forceinline__ TE hl_mul(TE hi, TE lo, TE s) { return fma(hi, s, lo * s); }
+
+// c_xB_phi where the molar volume may be constant (no division then)
+template <typename T, typename PC>
+__device__ __forceinline__ T c_xB_of(const PC &c, T xB, T h) {
+    if constexpr (sizeof(T) == 8)
+        if (c.cbconst) return T(c.cbc);
+    return c_xB_phi<T>(xB, T(c.Vm0), T(c.dVm), T(c.Vmc), h);
 }
 
 // Hooke's law with C_eff = C0 + h dC on the elastic strain eps - eps0,
@@ -131,20 +168,25 @@ __device__ __forceinline__ void eigenstrain(const PC &c, const ElasC<TE> &ec, T 
 // cuda_kernels.cu:7381-7480).
 template <typename T, typename TE, typename PC>
 __device__ __forceinline__ void stress_at(const PC &c, const ElasC<TE> &ec, T phi, T eta, T xB,
-                                          const TE eps[6], TE sig[6]) {
+                                          const TE eps[6], TE sig[6], TE *e0_out = nullptr) {
     TE e0[6];
     eigenstrain<T, TE>(c, ec, phi, eta, xB_el(c, xB), c.gp_el != 0, e0);
     TE el[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) el[a] = eps[a] - e0[a];
-    const T h = pf_h(phi);
+    if (e0_out) {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) e0_out[a] = e0[a];
+    }
+    TE hh, hl;
+    split_hl<T, TE>(pf_h(phi), hh, hl);
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
         TE acc = 0;
 #pragma unroll
         for (int b = 0; b < 6; ++b) {
             const int v = vidx(a, b);
-            TE ce = ec.S[v] + (TE)(h * T(ec.Sp[v]));
+            TE ce = ec.S[v] + hl_mul(hh, hl, ec.Sp[v]);
             acc += (b >= 3 ? TE(2) * ce : ce) * el[b];
         }
         sig[a] = acc;
@@ -152,15 +194,20 @@ __device__ __forceinline__ void stress_at(const PC &c, const ElasC<TE> &ec, T ph
 }
 
 // e^T dC e with engineering shear (compute_Q_voigt, cuda_kernels.cu:162-181)
-template <typename T, typename SP>
-__device__ __forceinline__ T q_voigt(const SP *Sp, const T el[6]) {
+// (FP64: terms whose coefficient is zero are passed over, a uniform branch
+// against two instructions of the FP64 pipe)
+template <typename T, typename PC>
+__device__ __forceinline__ T q_voigt(const PC &c, const T el[6]) {
     T e[6] = {el[0], el[1], el[2], T(2) * el[3], T(2) * el[4], T(2) * el[5]};
     T q = 0;
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
-        q += T(Sp[vidx(a, a)]) * e[a] * e[a];
 #pragma unroll
-        for (int b = a + 1; b < 6; ++b) q += T(2) * T(Sp[vidx(a, b)]) * e[a] * e[b];
+        for (int b = a; b < 6; ++b) {
+            const int v = vidx(a, b);
+            if (sizeof(T) == 8 && !((c.spmask >> v) & 1u)) continue;
+            q += (a == b ? T(c.Sp[v]) : T(2) * T(c.Sp[v])) * e[a] * e[b];
+        }
     }
     return q;
 }
@@ -170,15 +217,16 @@ __device__ __forceinline__ T q_voigt(const SP *Sp, const T el[6]) {
 // stress given (the reference reads its stored sigma arrays)
 template <typename T, typename TE, typename PC>
 __device__ __forceinline__ T phi_rhs_sig(const PC &c, const ElasC<TE> &ec, T phi, T eta_raw, T xBraw,
-                                         const TE *eps, const TE *sg_) {
+                                         const LogisticT<T> &lg, const TE *eps, const TE *sg_,
+                                         const TE *e0_ = nullptr) {
     const T hp = pf_hp(phi), gp = pf_gp(phi), h = pf_h(phi);
     const T eta = clamp01(eta_raw);
     const T xB = clamp01(xBraw);
     T f = T(c.W) * gp;
     T offA, offB;
-    thermo_mu_off<T>(c.tc, xB, offA, offB);
+    thermo_mu_off_at<T>(c.tc, xB, lg, offA, offB);
     const T dmu = T(c.Cdmu) - T(c.vA) * offA - T(c.vB) * offB;
-    const T cb = c_xB_phi<T>(xB, T(c.Vm0), T(c.dVm), T(c.Vmc), h);
+    const T cb = c_xB_of<T>(c, xB, h);
     const T muA = T(c.tc.GA_s) + offA, muB = T(c.tc.GB_s) + offB;
     const T mt = (T(1) - h) * (muA * (T(1) - xB) + muB * xB) + h * T(c.mu0);
     const T Vma = T(c.Vm0) + T(c.dVm) * xB;
@@ -190,11 +238,16 @@ __device__ __forceinline__ T phi_rhs_sig(const PC &c, const ElasC<TE> &ec, T phi
         for (int a = 0; a < 6; ++a) sg[a] = T(sg_[a]);
         // eps0 of the two-phase form with float eps00 (as the reference)
         TE e0[6];
-        eigenstrain<T, TE>(c, ec, phi, eta, xB, false, e0);
+        if (e0_) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a) e0[a] = e0_[a];
+        } else {
+            eigenstrain<T, TE>(c, ec, phi, eta, xB, false, e0);
+        }
         T el[6];
 #pragma unroll
         for (int a = 0; a < 6; ++a) el[a] = T(eps[a]) - T(e0[a]);
-        const T Q = q_voigt<T>(c.Sp, el);
+        const T Q = q_voigt<T>(c, el);
         T part;
         const T eps_alpha = xB * T(c.eiv);
         const T diag = -eps_alpha + T(c.eiv) * (xB - T(c.vB));
@@ -245,7 +298,7 @@ __device__ __forceinline__ T phi_rhs_phi_only(const PC &c, const ElasC<TE> &ec, 
         T el[6];
 #pragma unroll
         for (int a = 0; a < 6; ++a) el[a] = T(eps[a]) - T(e0[a]);
-        f += dg + T(0.5) * hp * q_voigt<T>(c.Sp, el);
+        f += dg + T(0.5) * hp * q_voigt<T>(c, el);
     }
     return f;
 }
@@ -254,23 +307,23 @@ __device__ __forceinline__ T phi_rhs_phi_only(const PC &c, const ElasC<TE> &ec, 
 // where the stored stress of the reference is that of the current fields
 template <typename T, typename TE, typename PC>
 __device__ __forceinline__ T phi_rhs(const PC &c, const ElasC<TE> &ec, T phi, T eta_raw, T xBraw,
-                                     const TE *eps) {
-    TE sg[6];
-    if (c.coupling) stress_at<T, TE>(c, ec, phi, eta_raw, xBraw, eps, sg);
-    return phi_rhs_sig<T, TE>(c, ec, phi, eta_raw, xBraw, eps, sg);
+                                     const LogisticT<T> &lg, const TE *eps) {
+    TE sg[6], e0[6];
+    if (c.coupling) stress_at<T, TE>(c, ec, phi, eta_raw, xBraw, eps, sg, e0);
+    return phi_rhs_sig<T, TE>(c, ec, phi, eta_raw, xBraw, lg, eps, sg, c.coupling && c.e0same ? e0 : nullptr);
 }
 
 // GP-zone Allen-Cahn driving force of eta (compute_eta_rhs_kernel,
 // non-raw-drive branch, cuda_kernels.cu:845-946)
 template <typename T, typename TE, typename PC>
 __device__ __forceinline__ T eta_rhs(const PC &c, const ElasC<TE> &ec, T eta_raw, T phi_raw,
-                                     T xBraw, T sig_hydro) {
+                                     T xBraw, const LogisticT<T> &lg, T sig_hydro) {
     const T eta = clamp01(eta_raw), phi = clamp01(phi_raw);
     const T xa = clamp_eps(xBraw, T(1e-12));
     const T hphi = pf_h(phi), hpe = pf_hp(eta), gpe = pf_gp(eta);
-    const T cref = T(1) / (T(c.Vm0) + T(c.dVm) * xa);
+    const T cref = sizeof(T) == 8 && c.cbconst ? T(c.cbc) : T(1) / (T(c.Vm0) + T(c.dVm) * xa);
     T offA, offB;
-    thermo_mu_off<T>(c.tc, xa, offA, offB);
+    thermo_mu_off_at<T>(c.tc, xa, lg, offA, offB);
     // g_gp - g_alpha without cancelling the compound constants
     const T dgg = T(c.dG) * (T(c.gpxB) - xa) + T(c.gp_Cg) - (offA * (T(1) - xa) + offB * xa);
     const T d = cref * (T(1) - hphi) * hpe * dgg;
@@ -284,6 +337,14 @@ __device__ __forceinline__ T eta_rhs(const PC &c, const ElasC<TE> &ec, T eta_raw
     return d + T(c.gpW) * gpe + el;
 }
 
+// gamma_thermo with the constants of PC
+template <typename T, typename PC>
+__device__ __forceinline__ T gamma_of(const PC &c, T xB, T h) {
+    T xc = xB;
+    if (c.tc.convex && xc > T(0.08)) xc = T(0.08);
+    return c_xB_of<T>(c, xc, h) * GammaEval<T>::dmu_diff(c.tc, xc);
+}
+
 // transport mobility (compute_flux_single_component_kernel :1985 and the
 // GP variant :2039)
 template <typename T, typename PC>
@@ -291,12 +352,12 @@ __device__ __forceinline__ T mobility(const PC &c, T phiY, T etaN, T xBp) {
     if (!c.gp) {
         const T h = pf_h(phiY);
         const T Dm = (T(1) - h) * T(c.Da) + h * T(c.Dc);
-        const T G = gamma_thermo<T>(c.tc, xBp, h, T(c.Vm0), T(c.dVm), T(c.Vmc));
+        const T G = gamma_of<T>(c, xBp, h);
         return stabilized_meff<T>(Dm, G);
     }
     const T hb = pf_h(phiY), he = pf_h(etaN);
     const T hg = (T(1) - hb) * he, ha = (T(1) - hb) * (T(1) - he);
-    const T Ga = gamma_thermo<T>(c.tc, xBp, T(0), T(c.Vm0), T(c.dVm), T(c.Vmc));
+    const T Ga = gamma_of<T>(c, xBp, T(0));
     const T Ma = stabilized_meff<T>(T(c.Da), Ga);
     return ha * Ma + hg * T(c.gpMGP) + hb * T(c.gpMb);
 }

@@ -803,8 +803,8 @@ struct OpPhiR2C {   // z pass producer: phi - L dt rhs_phi
         point_with(cell, p, in, out, acc);
     }
     __device__ void point_with(long long, const Pre &p, const T *, T *out, Acc &) const {
-        const T xB = xB_of_Y<T>(c, p.Y + T(d.Yc));
-        const T r = phi_rhs<T, TE>(c, ec, p.phi, p.eta, xB, p.e);
+        const LogisticT<T> lg = logistic(p.Y + T(d.Yc));
+        const T r = phi_rhs<T, TE>(c, ec, p.phi, p.eta, xB_of(c, lg), lg, p.e);
         out[0] = p.phi - T(c.Ldt) * r;
     }
     __device__ void load_spec(long long, int, cplx_t<T> *) const {}
@@ -820,7 +820,8 @@ struct OpEtaR2C {   // z pass producer: eta - L_eta dt rhs_eta (phi = updated ph
     __device__ void point(long long cell, const T *, T *out, Acc &) const {
         const T eta = d.eta_old[cell];
         const T phi = d.phi_new[cell];
-        const T xB = xB_of_Y<T>(c, d.Y[cell] + T(d.Yc));
+        const LogisticT<T> lg = logistic(d.Y[cell] + T(d.Yc));
+        const T xB = xB_of(c, lg);
         T sh = 0;
         if (c.gp_el && c.act_eta && c.elastic) {
             TE e[6], s[6];
@@ -829,7 +830,7 @@ struct OpEtaR2C {   // z pass producer: eta - L_eta dt rhs_eta (phi = updated ph
             stress_at<T, TE>(c, ec, d.phi_old[cell], eta, xB, e, s);
             sh = T(s[0]) + T(s[1]) + T(s[2]);
         }
-        const T r = eta_rhs<T, TE>(c, ec, eta, phi, xB, sh);
+        const T r = eta_rhs<T, TE>(c, ec, eta, phi, xB, lg, sh);
         out[0] = eta - T(c.gpLdt) * r;
     }
     __device__ void load_spec(long long, int, cplx_t<T> *) const {}
@@ -895,16 +896,17 @@ struct OpMuR2C {
     __device__ void point_with(long long cell, const Pre &p, const T *, T *out, Acc &acc) const {
         const T Yv = p.Y + T(d.Yc);
         const T phiY = p.pn;
-        const T xB = sigmoid_clip(Yv, T(c.Yclip), T(c.xBeps));
+        const LogisticT<T> lg = logistic(Yv);
+        const T xB = logistic_clip(lg, T(c.Yclip), T(c.xBeps));
         T offA, offB;
-        thermo_mu_off<T>(c.tc, xB, offA, offB);
+        thermo_mu_off_at<T>(c.tc, xB, lg, offA, offB);
         T mu;
         if (c.gp) {
-            const T cref = T(1) / (T(c.Vm0) + T(c.dVm) * xB);
+            const T cref = sizeof(T) == 8 && c.cbconst ? T(c.cbc) : T(1) / (T(c.Vm0) + T(c.dVm) * xB);
             mu = cref * (T(c.dG) + offB - offA);
         } else {
             const T h = pf_h(phiY);
-            const T cb = c_xB_phi<T>(xB, T(c.Vm0), T(c.dVm), T(c.Vmc), h);
+            const T cb = c_xB_of<T>(c, xB, h);
             const T muA = T(c.tc.GA_s) + offA, muB = T(c.tc.GB_s) + offB;
             const T mt = (T(1) - h) * (muA * (T(1) - xB) + muB * xB) + h * T(c.mu0);
             mu = cb * ((T(c.dG) + offB - offA) - cb * mt * T(c.dVm));
@@ -912,8 +914,7 @@ struct OpMuR2C {
         if (c.elastic) {
             // stress of the elastic solve of this step: phi, eta, xB at step start
             TE s[6];
-            const T xB0 = xB_of_Y<T>(c, Yv);
-            stress_at<T, TE>(c, ec, p.po, p.eta, xB0, p.e, s);
+            stress_at<T, TE>(c, ec, p.po, p.eta, xB_of(c, lg), p.e, s);
             mu += -T(c.eiv) * (T(s[0]) + T(s[1]) + T(s[2]));
         }
         out[0] = mu;
@@ -927,7 +928,7 @@ struct OpMuR2C {
         }
         const T h = pf_h(phiY);
         const T Dm = (T(1) - h) * T(c.Da) + h * T(c.Dc);
-        T x = sigmoid_raw(Yv);
+        T x = lg.x;
         if (x < T(1e-12)) x = T(1e-12);
         if (x > T(1) - T(1e-12)) x = T(1) - T(1e-12);
         acc.s += double(Dm * x * (T(1) - x));
@@ -988,7 +989,8 @@ struct OpFluxZ {
         const T Yv = Yf + T(d.Yc);
         const T pn = p.pn, pp = p.pp;
         const T phiY = (c.zm || c.prev_level) ? pn : pp;
-        const T xBp = sigmoid_clip(Yv, T(c.Yclip), T(c.xBeps));
+        const T xraw = sigmoid_raw(Yv);
+        const T xBp = logistic_clip(LogisticT<T>{Yv, xraw, T(0)}, T(c.Yclip), T(c.xBeps));
         // q split: the matrix channel alone, (1 - h) M_alpha with G_alpha at
         // h = 0 (compute_flux_single_component_q_kernel, cuda_kernels.cu:2014-2037)
         T M;
@@ -1003,14 +1005,13 @@ struct OpFluxZ {
             M = T((1.0 - hb) * (1.0 - he) * Ma + (1.0 - hb) * he * md[4] + hb * md[5]);
         } else {
             M = qmob ? (T(1) - pf_h(clamp01(phiY))) *
-                           stabilized_meff<T>(T(c.Da), gamma_thermo<T>(c.tc, xBp, T(0), T(c.Vm0), T(c.dVm),
-                                                                        T(c.Vmc)))
+                           stabilized_meff<T>(T(c.Da), gamma_of<T>(c, xBp, T(0)))
                      : mobility<T>(c, phiY, p.eta, xBp);
         }
         out[0] = M * g[0];
         out[1] = M * g[1];
         out[2] = M * g[2];
-        T x = sigmoid_raw(Yv);
+        T x = xraw;
         if (x < T(1e-12)) x = T(1e-12);
         if (x > T(1) - T(1e-12)) x = T(1) - T(1e-12);
         const T ld = x * (T(1) - x);
@@ -1883,7 +1884,8 @@ struct OpHijZ {
 #pragma unroll
         for (int a = 0; a < 6; ++a) e[a] = in[a] * ec.invN;
         const T phi = d.phi_old[cell];
-        const T h = pf_h(phi);
+        TE hh, hl;
+        split_hl<T, TE>(pf_h(phi), hh, hl);
         TE tv[6];
         if (lin) {
 #pragma unroll
@@ -1901,7 +1903,7 @@ struct OpHijZ {
             for (int b = 0; b < 6; ++b) {
                 const int v = vidx(a, b);
                 const TE c0 = ec.S[v];
-                const TE ce = c0 + (TE)(h * T(ec.Sp[v]));
+                const TE ce = c0 + hl_mul(hh, hl, ec.Sp[v]);
                 const TE f = b >= 3 ? TE(2) : TE(1);
                 acc += f * (c0 * e[b] - ce * tv[b]);
             }
@@ -3641,8 +3643,8 @@ struct OpMinGradZ {
         if (phi_only) {
             d.mge[cell] = phi_rhs_phi_only<T, TE>(c, ec, p, e, sg);
         } else {
-            const T xB = xB_of_Y<T>(c, d.Y[cell] + T(d.Yc));
-            d.mge[cell] = phi_rhs_sig<T, TE>(c, ec, p, c.gp ? d.eta_old[cell] : T(0), xB, e, sg);
+            const LogisticT<T> lg = logistic(d.Y[cell] + T(d.Yc));
+            d.mge[cell] = phi_rhs_sig<T, TE>(c, ec, p, c.gp ? d.eta_old[cell] : T(0), xB_of(c, lg), lg, e, sg);
         }
         out[0] = p;
     }
@@ -4148,6 +4150,7 @@ static void build_physc(pfgb_ctx *c) {
         thermo_mu_off<double>(k.tc, xg, oA, oB);
         k.gp_Cg = oA * (1.0 - xg) + oB * xg - P.gp_delta_g0;
     }
+    k = phys_as<double>(PhysC(k));   // the fields that it derives
 }
 
 static pfgb_status dalloc(pfgb_ctx *c, void **p, size_t bytes) {
