@@ -45,7 +45,7 @@ CU_SOURCES = [("solver.cu", [RDC], ""), ("solver.cu", [RDC, "-DPFGB_FIELDS=float
 CU_SOURCES += [("fftline.cu", [RDC, f"-DPFGB_LINE_T={t}", f"-DPFGB_LINE_DIR={d}", f"-maxrregcount={r}"], f".{t[0]}{d + 1}")
                for t, r in (("float", 80), ("double", 128)) for d in (-1, 1)]
 CU_SOURCES += [(s, [], "") for s in ("params.cu", "paramfile.cpp", "batch.cpp", "fno.cu", "checkpoint.cpp", "init.cu")]
-HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41.cuh", "dft41_tc.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
+HEADERS = ["common.cuh", "dfexp.cuh", "dfloat.cuh", "dft41.cuh", "dft41_tc.cuh", "f32x2.cuh", "fft.cuh", "fft246.cuh", "physics.cuh", "rader41.cuh"]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "rader41.cuh"
 
 namespace d41 {
@@ -56,33 +57,7 @@ __host__ __device__ constexpr double cval(int which, int b) {
                           : 0.5 * (-h2 + R2 * (h1 + h3));
 }
 
-using P = unsigned long long;   // a packed pair of floats (f32x2)
-__device__ __forceinline__ P pk(float2 v) {
-    P r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
-    return r;
-}
-__device__ __forceinline__ float2 un(P v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ P add(P a, P b) {
-    P r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ P mul(P a, P b) {
-    P r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ P fma(P a, P b, P c) {
-    P r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ P both(float k) { return pk(make_float2(k, k)); }
+using namespace f2x;
 __device__ __forceinline__ P sub(P a, P b) { return fma(b, both(-1.f), a); }
 template <int W, int B, bool NEG = false> __device__ __forceinline__ P kc() {
     constexpr float k = (float)(NEG ? -cval(W, B) : cval(W, B));

@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 
 namespace {
 
@@ -97,95 +98,177 @@ __global__ void __launch_bounds__(256) k_lift(const float *__restrict__ a, const
 
 // ---------------------------------------------------------------------------
 // z: dst[L][k] = w_k sum_z src[L][z] e^{-2 pi i k z / Z}, k < Mz
-// (w_0 = w0, w_k = w1 for k > 0).  LB lines per block staged in shared
-// memory (row stride Z + 1) with the DFT matrix F[z][k] (k padded to even).
-// A thread computes 2 wavenumbers of one line: per z one line value and one
-// float4 table read feed 4 FMAs.
+// (w_0 = w0, w_k = w1 for k > 0).  A thread sums 2 wavenumbers of 4 lines: per z
+// one 16-byte read of the lines (staged transposed, kZC positions at a time)
+// and one of the DFT matrix F[z][k] (k padded to even) feed 16 multiply-adds,
+// eight packed ones.  Bound by issue: 128^3 x 32 lines, 12 modes, 300 us with
+// one line per thread (two shared reads for four multiply-adds).
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int pad2(int m) { return (m + 1) & ~1; }
+constexpr int kZC = 64;                // positions staged at a time
+// lines per block: about 256 tasks (4 lines x 2 wavenumbers each)
+__host__ __device__ constexpr int dft_z_lines(int Mz) {
+    const int kg = pad2(Mz) / 2, g = 256 / kg;
+    return 4 * (g > 42 ? 42 : (g < 1 ? 1 : g));
+}
+// row stride of the staged lines: an odd number of 16-byte words (conflict-free
+// 16-byte stores by consecutive positions)
+__host__ __device__ constexpr int dft_z_stride(int LB) { return (LB / 4) % 2 ? LB : LB + 4; }
 
 __global__ void __launch_bounds__(256) k_dft_z(const float *__restrict__ src, float2 *__restrict__ dst,
                                                const float4 *__restrict__ fz, long long nlines, int Z, int Mz,
                                                int LB, float w0, float w1) {
     extern __shared__ __align__(16) float smz[];
-    const int M2 = pad2(Mz), KG = M2 / 2, ZP = Z + 1;
-    float4 *F4s = reinterpret_cast<float4 *>(smz);
-    float *lines = smz + 2 * Z * M2;
-    for (int e = threadIdx.x; e < Z * KG; e += blockDim.x) F4s[e] = fz[e];
+    const int M2 = pad2(Mz), KG = M2 / 2, LS = dft_z_stride(LB), G4 = LB / 4;
+    float4 *F4 = reinterpret_cast<float4 *>(smz);                // [kZC][KG]
+    float *T = smz + 2 * kZC * M2;                               // [kZC][LS]
     const long long L0 = (long long)blockIdx.x * LB;
     const int nl = (int)min((long long)LB, nlines - L0);
     const float *s = src + L0 * Z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int l = warp; l < nl; l += nw)
-        for (int z = lane; z < Z; z += 32) lines[l * ZP + z] = s[(long long)l * Z + z];
-    __syncthreads();
-    const float4 *F4 = F4s;
-    for (int task = threadIdx.x; task < nl * KG; task += blockDim.x) {
-        const int l = task / KG, q = task - l * KG;
-        const float *ln = lines + l * ZP;
-        float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-#pragma unroll 8
-        for (int z = 0; z < Z; ++z) {
-            const float a = ln[z];
-            const float4 f = F4[z * KG + q];
-            c0 = fmaf(a, f.x, c0); c1 = fmaf(a, f.y, c1);
-            c2 = fmaf(a, f.z, c2); c3 = fmaf(a, f.w, c3);
+    const int ntask = ((nl + 3) / 4) * KG;
+    const int g = threadIdx.x / KG, q = threadIdx.x - g * KG;
+    const bool act = (int)threadIdx.x < ntask;
+    f2x::P acc[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = f2x::both(0.f);
+    for (int zb = 0; zb < Z; zb += kZC) {
+        const int nz = min(kZC, Z - zb);
+        __syncthreads();
+        for (int e = threadIdx.x; e < nz * KG; e += blockDim.x) F4[e] = fz[(long long)zb * KG + e];
+        for (int e = threadIdx.x; e < kZC * G4; e += blockDim.x) {
+            const int gg = e / kZC, z = e - gg * kZC;
+            if (z < nz && 4 * gg < nl) {
+                const float *p = s + (long long)(4 * gg) * Z + zb + z;
+                float4 v;
+                v.x = p[0];
+                v.y = 4 * gg + 1 < nl ? p[Z] : 0.f;
+                v.z = 4 * gg + 2 < nl ? p[2 * Z] : 0.f;
+                v.w = 4 * gg + 3 < nl ? p[3 * Z] : 0.f;
+                *reinterpret_cast<float4 *>(T + z * LS + 4 * gg) = v;
+            }
         }
-        float2 *d = dst + (L0 + l) * Mz;
-        const int k = 2 * q;
-        d[k] = make_float2(c0 * (k == 0 ? w0 : w1), c1 * (k == 0 ? w0 : w1));
-        if (k + 1 < Mz) d[k + 1] = make_float2(c2 * w1, c3 * w1);
+        __syncthreads();
+        if (act) {
+            const float *t = T + 4 * g;
+#pragma unroll 4
+            for (int z = 0; z < nz; ++z) {
+                const float4 a = *reinterpret_cast<const float4 *>(t + z * LS);
+                const float4 f = F4[z * KG + q];
+                const f2x::P f0 = f2x::pk(make_float2(f.x, f.y)), f1 = f2x::pk(make_float2(f.z, f.w));
+                const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const f2x::P b = f2x::both(av[i]);
+                    acc[i][0] = f2x::fma(b, f0, acc[i][0]);
+                    acc[i][1] = f2x::fma(b, f1, acc[i][1]);
+                }
+            }
+        }
+    }
+    if (!act) return;
+    const int k = 2 * q;
+    const float wk = k == 0 ? w0 : w1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (4 * g + i >= nl) break;
+        float2 *d = dst + (L0 + 4 * g + i) * Mz;
+        const float2 c0 = f2x::un(acc[i][0]), c1 = f2x::un(acc[i][1]);
+        d[k] = make_float2(c0.x * wk, c0.y * wk);
+        if (k + 1 < Mz) d[k + 1] = make_float2(c1.x * w1, c1.y * w1);
     }
 }
 
-// y forward (e^{-}) onto the corner blocks: one block per (channel, x) slab
+// y forward (e^{-}) onto the corner blocks: kYJ retained ky per thread share
+// each slab value, NS slabs (channel, x) per block
 // dst[r][jy][kz] = sum_y src[r][y][kz] e^{-2 pi i ky(jy) y / Y}
+// tyi[jy][y] holds the conjugate twiddles.  (One ky per thread took two shared
+// reads for four multiply-adds: 65 us at 128^3, 12 modes.)
+constexpr int kYJ = 8;
 __global__ void __launch_bounds__(256) k_dft_y(const float2 *__restrict__ src, float2 *__restrict__ dst,
-                                               const float2 *__restrict__ twy, int Y, int Mz, int m) {
+                                               const float2 *__restrict__ tyi, long long nslab, int NS, int Y, int Mz,
+                                               int m) {
     extern __shared__ __align__(16) float2 smy[];
-    float2 *tw = smy, *slab = smy + Y;
-    const long long r = blockIdx.x;
-    for (int e = threadIdx.x; e < Y; e += blockDim.x) tw[e] = twy[e];
-    const float2 *s = src + r * Y * Mz;
-    for (int e = threadIdx.x; e < Y * Mz; e += blockDim.x) slab[e] = s[e];
+    const int J = 2 * m, JG = (J + kYJ - 1) / kYJ;
+    float2 *slab = smy;                                          // [NS][Y][Mz]
+    const long long r0 = (long long)blockIdx.x * NS;
+    const int ns = (int)min((long long)NS, nslab - r0);
+    const float2 *s = src + r0 * Y * Mz;
+    for (int e = threadIdx.x; e < ns * Y * Mz; e += blockDim.x) slab[e] = s[e];
     __syncthreads();
-    const int nout = 2 * m * Mz;
-    for (int e = threadIdx.x; e < nout; e += blockDim.x) {
-        const int jy = e / Mz, kz = e - jy * Mz;
-        const int ky = kcorner(jy, m, Y);
-        float re = 0.f, im = 0.f;
-        int idx = 0;
-        for (int y = 0; y < Y; ++y) {
-            const float2 a = slab[y * Mz + kz], w = tw[idx];
-            re = fmaf(a.x, w.x, fmaf(-a.y, w.y, re));
-            im = fmaf(a.x, w.y, fmaf(a.y, w.x, im));
-            idx += ky;
-            if (idx >= Y) idx -= Y;
+    // kz fastest, then the slab: a warp shares the group of ky and its twiddles
+    for (int e = threadIdx.x; e < ns * Mz * JG; e += blockDim.x) {
+        const int jg = e / (ns * Mz), rem = e - jg * ns * Mz;
+        const int sl = rem / Mz, kz = rem - sl * Mz;
+        const float2 *a = slab + (long long)sl * Y * Mz + kz;
+        const float2 *w = tyi + (long long)jg * kYJ * Y;
+        const int nj = min(kYJ, J - jg * kYJ);
+        float re[kYJ], im[kYJ];
+#pragma unroll
+        for (int j = 0; j < kYJ; ++j) re[j] = im[j] = 0.f;
+        auto add = [&](int j, float2 v, float tx, float ty) {   // e^{-}: (tx, -ty)
+            re[j] = fmaf(v.x, tx, fmaf(-v.y, -ty, re[j]));
+            im[j] = fmaf(v.x, -ty, fmaf(v.y, tx, im[j]));
+        };
+        int y = 0;
+        if (Y % 2 == 0) {   // the twiddles of two positions per read
+            for (; y < Y; y += 2) {
+                const float2 v0 = a[y * Mz], v1 = a[(y + 1) * Mz];
+#pragma unroll
+                for (int j = 0; j < kYJ; ++j) {
+                    const float4 t = __ldg(reinterpret_cast<const float4 *>(w + (j < nj ? j : 0) * Y + y));
+                    add(j, v0, t.x, t.y);
+                    add(j, v1, t.z, t.w);
+                }
+            }
         }
-        dst[r * nout + e] = make_float2(re, im);
+        for (; y < Y; ++y) {
+            const float2 v = a[y * Mz];
+#pragma unroll
+            for (int j = 0; j < kYJ; ++j) {
+                const float2 t = __ldg(w + (j < nj ? j : 0) * Y + y);
+                add(j, v, t.x, t.y);
+            }
+        }
+        float2 *d = dst + (r0 + sl) * J * Mz + kz;
+#pragma unroll
+        for (int j = 0; j < kYJ; ++j)
+            if (j < nj) d[(jg * kYJ + j) * Mz] = make_float2(re[j], im[j]);
     }
 }
 
-// x forward (e^{-}) onto the corner blocks: one block per (channel, jx)
+// x forward (e^{-}) onto the corner blocks: kXJ retained kx per thread share
+// each value; block (channel, group of kx, chunk of q)
 // dst[c][jx][q] = sum_x src[c][x][q] e^{-2 pi i kx(jx) x / X},  q < Q
-__global__ void __launch_bounds__(256) k_dft_x(const float2 *__restrict__ src, float2 *__restrict__ dst,
+// (One kx per block read the whole channel 2m times: 115 us at 128^3, 12 modes.)
+constexpr int kXJ = 8, kXT = 96;
+__global__ void __launch_bounds__(kXT) k_dft_x(const float2 *__restrict__ src, float2 *__restrict__ dst,
                                                const float2 *__restrict__ twx, int X, int Q, int m) {
-    extern __shared__ __align__(16) float2 smx[];
-    const int c = blockIdx.x / (2 * m), jx = blockIdx.x % (2 * m);
-    const int kx = kcorner(jx, m, X);
-    for (int e = threadIdx.x; e < X; e += blockDim.x) smx[e] = twx[(int)(((long long)kx * e) % X)];
-    __syncthreads();
-    const float2 *s = src + (long long)c * X * Q;
-    for (int q = threadIdx.x; q < Q; q += blockDim.x) {
-        float re = 0.f, im = 0.f;
-#pragma unroll 8
-        for (int x = 0; x < X; ++x) {
-            const float2 a = s[(long long)x * Q + q], w = smx[x];
-            re = fmaf(a.x, w.x, fmaf(-a.y, w.y, re));
-            im = fmaf(a.x, w.y, fmaf(a.y, w.x, im));
-        }
-        dst[((long long)c * 2 * m + jx) * Q + q] = make_float2(re, im);
+    extern __shared__ __align__(16) float2 smx[];                // [X][kXJ]
+    const int J = 2 * m, c = blockIdx.y, j0 = blockIdx.z * kXJ, nj = min(kXJ, J - j0);
+    for (int e = threadIdx.x; e < X * kXJ; e += blockDim.x) {
+        const int x = e / kXJ, j = e - x * kXJ;
+        smx[e] = j < nj ? twx[(int)(((long long)kcorner(j0 + j, m, X) * x) % X)] : make_float2(0.f, 0.f);
     }
+    __syncthreads();
+    const int q = blockIdx.x * kXT + threadIdx.x;
+    if (q >= Q) return;
+    const float2 *s = src + (long long)c * X * Q + q;
+    float re[kXJ], im[kXJ];
+#pragma unroll
+    for (int j = 0; j < kXJ; ++j) re[j] = im[j] = 0.f;
+#pragma unroll 4
+    for (int x = 0; x < X; ++x) {
+        const float2 a = s[(long long)x * Q];
+#pragma unroll
+        for (int j = 0; j < kXJ; ++j) {
+            const float2 w = smx[x * kXJ + j];
+            re[j] = fmaf(a.x, w.x, fmaf(-a.y, w.y, re[j]));
+            im[j] = fmaf(a.x, w.y, fmaf(a.y, w.x, im[j]));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kXJ; ++j)
+        if (j < nj) dst[((long long)c * J + j0 + j) * Q + q] = make_float2(re[j], im[j]);
 }
 
 // x inverse (e^{+}) from the corner blocks: one block per (channel, x)
@@ -289,78 +372,111 @@ __global__ void __launch_bounds__(256) k_mode_grad(const float2 *__restrict__ C,
 // one spectral layer's output: z c2r of the mixed spectrum (weights 1, 2, 2,
 // ...) fused with the pointwise path
 //   pre[o] = spec[o] + b[o] + sum_i W[o][i] v[i];  vout = GELU(pre) or pre
-// One cell per thread, 256 consecutive cells per block; the block stages the
-// half-spectrum lines its cells lie on (at most 256/Z + 2 lines).
+// Two cells per thread (neighbours on one line when Z is even), 256 cells per
+// block; the block stages the half-spectrum lines its cells lie on (at most
+// 256/Z + 2 lines).  All 32 outputs of a cell are sums in registers, packed in
+// pairs: 16 bytes of weights or of spectrum feed four or two pairs of
+// multiply-adds for both cells.  (One cell per thread in scalar arithmetic was
+// bound by its 640 broadcast reads per cell: 395 us at 128^3, 12 modes.)
 // ---------------------------------------------------------------------------
 constexpr int kLayerCells = 256;
 __host__ __device__ constexpr int layer_lines(int Z) { return kLayerCells / Z + 2; }
 
-template <bool ACT, bool SAVE>
-__global__ void __launch_bounds__(kLayerCells, 2) k_layer_fwd(const float2 *__restrict__ A,
-                                                              const float *__restrict__ v,
-                                                              const __nv_bfloat16 *__restrict__ Ww,
-                                                              const float *__restrict__ bw, float *__restrict__ vout,
-                                                              float *__restrict__ pre,
-                                                              const float2 *__restrict__ gz, long long S, int Z,
-                                                              int Mz) {
+template <bool ACT, bool SAVE, bool PAIR>
+__global__ void __launch_bounds__(kLayerCells / 2, 3) k_layer_fwd(const float2 *__restrict__ A,
+                                                                  const float *__restrict__ v,
+                                                                  const __nv_bfloat16 *__restrict__ Ww,
+                                                                  const float *__restrict__ bw,
+                                                                  float *__restrict__ vout, float *__restrict__ pre,
+                                                                  const float2 *__restrict__ gz, long long S, int Z,
+                                                                  int Mz) {
     extern __shared__ __align__(16) float sml[];
-    float (*Wm)[kW] = reinterpret_cast<float (*)[kW]>(sml);   // rows read as float4 broadcasts
+    float (*WT)[kW] = reinterpret_cast<float (*)[kW]>(sml);   // WT[i][o], rows read as float4 broadcasts
     float *bs = sml + kW * kW;
-    float2 *G = reinterpret_cast<float2 *>(bs + kW);           // G[k][z] = c_k e(k z): conflict-free in z
-    float2 *At = G + Mz * Z;
+    float4 *At = reinterpret_cast<float4 *>(bs + kW);          // [line][k][pair of channels]: (re, re, im, im)
     const long long N = S * Z;
     const long long c0 = (long long)blockIdx.x * kLayerCells;
     const long long c1 = min(N, c0 + kLayerCells);
     const long long sf = c0 / Z;
     const int nl = (int)((c1 - 1) / Z - sf + 1);
-    for (int e = threadIdx.x; e < kW * kW; e += blockDim.x) Wm[e / kW][e % kW] = bf(Ww[e]);
+    float2 *G = reinterpret_cast<float2 *>(At + layer_lines(Z) * Mz * (kW / 2));   // G[k][z] = c_k e(k z)
+    for (int e = threadIdx.x; e < kW * kW; e += blockDim.x) WT[e % kW][e / kW] = bf(Ww[e]);
     if (threadIdx.x < kW) bs[threadIdx.x] = bw[threadIdx.x];
-    for (int e = threadIdx.x; e < Z; e += blockDim.x) G[e] = gz[e];   // k = 0: weight 1
-    for (int e = Z + threadIdx.x; e < Mz * Z; e += blockDim.x) {
-        const float2 t = gz[e];                                         // k > 0: weight 2
-        G[e] = make_float2(2.f * t.x, 2.f * t.y);
+    for (int e = threadIdx.x; e < Mz * Z; e += blockDim.x) {
+        const float2 t = gz[e];
+        const float w = e < Z ? 1.f : 2.f;   // k = 0 once, the others with their conjugates
+        G[e] = make_float2(w * t.x, w * t.y);
     }
     for (int e = threadIdx.x; e < kW * nl * Mz; e += blockDim.x) {
         const int c = e / (nl * Mz), rem = e - c * nl * Mz;
-        At[e] = A[(c * S + sf) * Mz + rem];
+        const float2 a = A[(c * S + sf) * Mz + rem];
+        float *d = reinterpret_cast<float *>(At + rem * (kW / 2) + (c >> 1)) + (c & 1);
+        d[0] = a.x;
+        d[2] = a.y;
     }
     __syncthreads();
-    const long long n = c0 + threadIdx.x;
-    if (n >= c1) return;
-    const int l = (int)(n / Z - sf), z = (int)(n % Z);
-    float acc[kW];
-    {
-        float x[kW];
+    const long long n0 = PAIR ? c0 + 2 * threadIdx.x : c0 + threadIdx.x, n1 = PAIR ? n0 + 1 : n0 + kLayerCells / 2;
+    if (n0 >= c1) return;
+    const bool two = n1 < c1;
+    const int l0 = (int)(n0 / Z - sf), z0 = (int)(n0 % Z);
+    const int l1 = PAIR || !two ? l0 : (int)(n1 / Z - sf), z1 = PAIR ? z0 + 1 : (two ? (int)(n1 % Z) : z0);
+    f2x::P s0[kW / 2], s1[kW / 2];
 #pragma unroll
-        for (int i = 0; i < kW; ++i) x[i] = v[i * N + n];
+    for (int p = 0; p < kW / 2; ++p) s0[p] = s1[p] = f2x::pk(make_float2(bs[2 * p], bs[2 * p + 1]));
+#pragma unroll 8
+    for (int i = 0; i < kW; ++i) {
+        float x0, x1;
+        if (PAIR) {
+            const float2 t = *reinterpret_cast<const float2 *>(v + i * N + n0);
+            x0 = t.x;
+            x1 = t.y;
+        } else {
+            x0 = v[i * N + n0];
+            x1 = two ? v[i * N + n1] : 0.f;
+        }
+        const f2x::P b0 = f2x::both(x0), b1 = f2x::both(x1);
+        const float4 *w4 = reinterpret_cast<const float4 *>(WT[i]);
 #pragma unroll
-        for (int o = 0; o < kW; ++o) {
-            float s = bs[o];
-            const float4 *w4 = reinterpret_cast<const float4 *>(Wm[o]);
-#pragma unroll
-            for (int q = 0; q < kW / 4; ++q) {
-                const float4 w = w4[q];
-                s = fmaf(w.x, x[4 * q], s);
-                s = fmaf(w.y, x[4 * q + 1], s);
-                s = fmaf(w.z, x[4 * q + 2], s);
-                s = fmaf(w.w, x[4 * q + 3], s);
-            }
-            acc[o] = s;
+        for (int q = 0; q < kW / 4; ++q) {
+            const float4 w = w4[q];
+            const f2x::P wa = f2x::pk(make_float2(w.x, w.y)), wb = f2x::pk(make_float2(w.z, w.w));
+            s0[2 * q] = f2x::fma(wa, b0, s0[2 * q]);
+            s0[2 * q + 1] = f2x::fma(wb, b0, s0[2 * q + 1]);
+            s1[2 * q] = f2x::fma(wa, b1, s1[2 * q]);
+            s1[2 * q + 1] = f2x::fma(wb, b1, s1[2 * q + 1]);
         }
     }
-    const float2 *Al = At + l * Mz;
     for (int k = 0; k < Mz; ++k) {
-        const float2 t = G[k * Z + z];
+        const float2 t0 = G[k * Z + z0], t1 = G[k * Z + z1];
+        const f2x::P x0 = f2x::both(t0.x), y0 = f2x::both(t0.y), x1 = f2x::both(t1.x), y1 = f2x::both(t1.y);
+        const float4 *a0 = At + (l0 * Mz + k) * (kW / 2), *a1 = At + (l1 * Mz + k) * (kW / 2);
 #pragma unroll
-        for (int c = 0; c < kW; ++c) {
-            const float2 a = Al[c * nl * Mz + k];
-            acc[c] = fmaf(a.x, t.x, fmaf(a.y, t.y, acc[c]));   // Re(a e^{+i theta})
+        for (int p = 0; p < kW / 2; ++p) {
+            // Re(a e^{+i theta}) of two channels
+            const float4 a = a0[p];
+            s0[p] = f2x::fma(f2x::pk(make_float2(a.x, a.y)), x0,
+                             f2x::fma(f2x::pk(make_float2(a.z, a.w)), y0, s0[p]));
+            const float4 b = PAIR ? a : a1[p];
+            s1[p] = f2x::fma(f2x::pk(make_float2(b.x, b.y)), x1,
+                             f2x::fma(f2x::pk(make_float2(b.z, b.w)), y1, s1[p]));
         }
     }
 #pragma unroll
     for (int o = 0; o < kW; ++o) {
-        if (SAVE) pre[o * N + n] = acc[o];
-        vout[o * N + n] = ACT ? gelu(acc[o]) : acc[o];
+        const float2 u0 = f2x::un(s0[o / 2]), u1 = f2x::un(s1[o / 2]);
+        const float p0 = o & 1 ? u0.y : u0.x, p1 = o & 1 ? u1.y : u1.x;
+        const float g0 = ACT ? gelu(p0) : p0, g1 = ACT ? gelu(p1) : p1;
+        if (PAIR) {
+            if (SAVE) *reinterpret_cast<float2 *>(pre + o * N + n0) = make_float2(p0, p1);
+            *reinterpret_cast<float2 *>(vout + o * N + n0) = make_float2(g0, g1);
+        } else {
+            if (SAVE) pre[o * N + n0] = p0;
+            vout[o * N + n0] = g0;
+            if (two) {
+                if (SAVE) pre[o * N + n1] = p1;
+                vout[o * N + n1] = g1;
+            }
+        }
     }
 }
 
@@ -398,43 +514,66 @@ __global__ void __launch_bounds__(256) k_idft_z_acc(const float2 *__restrict__ A
     }
 }
 
-// projection: y = out_scale (Q2 GELU(Q1 v + q1) + q2)
-__global__ void __launch_bounds__(256) k_project(const float *__restrict__ v, const __nv_bfloat16 *__restrict__ Q1w,
+// projection: y = out_scale (Q2 GELU(Q1 v + q1) + q2); two cells per thread,
+// four pairs of hidden units of each at a time in packed arithmetic
+__global__ void __launch_bounds__(128) k_project(const float *__restrict__ v, const __nv_bfloat16 *__restrict__ Q1w,
                                                  const float *__restrict__ q1, const __nv_bfloat16 *__restrict__ Q2w,
                                                  const float *__restrict__ q2, float4 os, float *__restrict__ y,
                                                  long long N) {
-    __shared__ __align__(16) float Q1[kH][kW];
+    __shared__ __align__(16) float Q1T[kW][kH];
     __shared__ float b1[kH], Q2[kOut][kH], b2[kOut];
-    for (int e = threadIdx.x; e < kH * kW; e += blockDim.x) Q1[e / kW][e % kW] = bf(Q1w[e]);
+    for (int e = threadIdx.x; e < kH * kW; e += blockDim.x) Q1T[e % kW][e / kW] = bf(Q1w[e]);
     for (int e = threadIdx.x; e < kOut * kH; e += blockDim.x) Q2[e / kH][e % kH] = bf(Q2w[e]);
     if (threadIdx.x < kH) b1[threadIdx.x] = q1[threadIdx.x];
     if (threadIdx.x < kOut) b2[threadIdx.x] = q2[threadIdx.x];
     __syncthreads();
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < N; n += (long long)gridDim.x * blockDim.x) {
-        float x[kW];
+    const long long half = (N + 1) / 2;   // cells n and n + half
+    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < half; n += (long long)gridDim.x * blockDim.x) {
+        const bool two = n + half < N;
+        const long long n1 = two ? n + half : n;
+        float x[kW], z[kW];
 #pragma unroll
-        for (int i = 0; i < kW; ++i) x[i] = v[i * N + n];
-        float o0 = b2[0], o1 = b2[1], o2 = b2[2];
-#pragma unroll 4
-        for (int j = 0; j < kH; ++j) {
-            float s = b1[j];
-            const float4 *w4 = reinterpret_cast<const float4 *>(Q1[j]);
+        for (int i = 0; i < kW; ++i) { x[i] = v[i * N + n]; z[i] = v[i * N + n1]; }
+        float o[kOut], p[kOut];
 #pragma unroll
-            for (int q = 0; q < kW / 4; ++q) {
-                const float4 w = w4[q];
-                s = fmaf(w.x, x[4 * q], s);
-                s = fmaf(w.y, x[4 * q + 1], s);
-                s = fmaf(w.z, x[4 * q + 2], s);
-                s = fmaf(w.w, x[4 * q + 3], s);
+        for (int c = 0; c < kOut; ++c) o[c] = p[c] = b2[c];
+#pragma unroll 1
+        for (int j = 0; j < kH; j += 8) {
+            f2x::P s[4], t[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q] = t[q] = f2x::pk(make_float2(b1[j + 2 * q], b1[j + 2 * q + 1]));
+#pragma unroll
+            for (int i = 0; i < kW; ++i) {
+                const float4 wa = *reinterpret_cast<const float4 *>(&Q1T[i][j]);
+                const float4 wb = *reinterpret_cast<const float4 *>(&Q1T[i][j + 4]);
+                const f2x::P w[4] = {f2x::pk(make_float2(wa.x, wa.y)), f2x::pk(make_float2(wa.z, wa.w)),
+                                     f2x::pk(make_float2(wb.x, wb.y)), f2x::pk(make_float2(wb.z, wb.w))};
+                const f2x::P bx = f2x::both(x[i]), bz = f2x::both(z[i]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    s[q] = f2x::fma(w[q], bx, s[q]);
+                    t[q] = f2x::fma(w[q], bz, t[q]);
+                }
             }
-            const float h = gelu(s);
-            o0 = fmaf(Q2[0][j], h, o0);
-            o1 = fmaf(Q2[1][j], h, o1);
-            o2 = fmaf(Q2[2][j], h, o2);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 a = f2x::un(s[q]), b = f2x::un(t[q]);
+                const float ha = gelu(a.x), hb = gelu(a.y), ga = gelu(b.x), gb = gelu(b.y);
+#pragma unroll
+                for (int c = 0; c < kOut; ++c) {
+                    o[c] = fmaf(Q2[c][j + 2 * q + 1], hb, fmaf(Q2[c][j + 2 * q], ha, o[c]));
+                    p[c] = fmaf(Q2[c][j + 2 * q + 1], gb, fmaf(Q2[c][j + 2 * q], ga, p[c]));
+                }
+            }
         }
-        y[n] = os.x * o0;
-        y[N + n] = os.y * o1;
-        y[2 * N + n] = os.z * o2;
+        y[n] = os.x * o[0];
+        y[N + n] = os.y * o[1];
+        y[2 * N + n] = os.z * o[2];
+        if (two) {
+            y[n1] = os.x * p[0];
+            y[N + n1] = os.y * p[1];
+            y[2 * N + n1] = os.z * p[2];
+        }
     }
 }
 
@@ -458,12 +597,22 @@ __global__ void __launch_bounds__(256) k_sumsq(const float *__restrict__ t, long
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// fixed-order float64 sum of nb partials into out[0] (one thread)
-__global__ void k_sum_partials(const double *__restrict__ part, int nb, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// fixed-order float64 sum of nb partials over a block of 256 threads
+__device__ __forceinline__ double block_sum256(const double *__restrict__ part, int nb) {
+    __shared__ double red[256];
     double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[b];
-    out[0] = s;
+    for (int b = threadIdx.x; b < nb; b += 256) s += part[b];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    return red[0];
+}
+__global__ void __launch_bounds__(256) k_sum_partials(const double *__restrict__ part, int nb, double *__restrict__ out) {
+    const double s = block_sum256(part, nb);
+    if (threadIdx.x == 0) out[0] = s;
 }
 
 // Projection backward with the loss L = sum (y - t)^2 / den.
@@ -718,23 +867,30 @@ __global__ void __launch_bounds__(kTile) k_lift_bwd(const float *__restrict__ g0
     if (t < kW) P[kW * kIn + t] = ab;
 }
 
-// grad[e] (+)= sum over blocks of part[b][e], float64, fixed order
-__global__ void __launch_bounds__(256) k_reduce_part(const float *__restrict__ part, int nb, int E,
-                                                     float *__restrict__ grad, int accumulate) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
+// grad[e] (+)= sum over blocks of part[b][e], float64, fixed order: a warp's
+// lanes take 32 entries, the block's 32 warps every 32nd partial (608 partials
+// of 2,307 entries: 98 us with one thread per entry, a chain of 608 loads)
+__global__ void __launch_bounds__(1024) k_reduce_part(const float *__restrict__ part, int nb, int E,
+                                                      float *__restrict__ grad, int accumulate) {
+    __shared__ double red[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += (double)part[(long long)b * E + e];
-    grad[e] = accumulate ? (float)((double)grad[e] + s) : (float)s;
+    if (e < E)
+        for (int b = w; b < nb; b += 32) s += (double)part[(long long)b * E + e];
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && e < E) {
+        double t = red[0][lane];
+        for (int k = 1; k < 32; ++k) t += red[k][lane];
+        grad[e] = accumulate ? (float)((double)grad[e] + t) : (float)t;
+    }
 }
 
 // loss = sum(lpart) / den
-__global__ void k_loss_final(const double *__restrict__ lpart, int nb, const double *__restrict__ den,
-                             double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += lpart[b];
-    out[0] = s / den[0];
+__global__ void __launch_bounds__(256) k_loss_final(const double *__restrict__ lpart, int nb,
+                                                    const double *__restrict__ den, double *__restrict__ out) {
+    const double s = block_sum256(lpart, nb);
+    if (threadIdx.x == 0) out[0] = s / den[0];
 }
 
 __global__ void __launch_bounds__(256) k_sumsq_f(const float *__restrict__ g, long long n, double *__restrict__ part) {
@@ -851,9 +1007,18 @@ pfgb_status upload_tw(pfgb_fno *f, float2 **dst, int n) {
 }
 
 constexpr size_t kSmemCap = 200 * 1024;
-size_t dft_z_smem(int Z, int Mz, int LB);
-int dft_z_lb(int Z, int Mz);
 size_t layer_smem(int Z, int Mz);
+// the models that are taken: the staging of a z line's DFT matrix and of about
+// 256 / (modes / 2) lines (64 KB at most), and of a y slab, within kSmemCap
+size_t dft_z_staging(int Z, int Mz) {
+    const int kg = pad2(Mz) / 2;
+    const int lb = std::max(1, std::min((256 + kg - 1) / kg, (64 * 1024) / (4 * (Z + 1))));
+    return sizeof(float) * (2 * (size_t)Z * pad2(Mz) + (size_t)lb * (Z + 1));
+}
+size_t layer_staging(int Z, int Mz) {
+    return sizeof(float) * ((size_t)kW * kW + kW) +
+           sizeof(float2) * ((size_t)Mz * Z + (size_t)kW * layer_lines(Z) * Mz);
+}
 
 pfgb_status validate(const pfgb_fno_config *c) {
     const int m = c->modes;
@@ -867,12 +1032,12 @@ pfgb_status validate(const pfgb_fno_config *c) {
         return PFGB_ERR_INVALID;
     }
     // the z and y transforms stage a whole DFT matrix / slab in shared memory
-    if (dft_z_smem(c->Nz, m, dft_z_lb(c->Nz, m)) > kSmemCap || sizeof(float2) * (size_t)c->Ny * (m + 1) > kSmemCap) {
+    if (dft_z_staging(c->Nz, m) > kSmemCap || sizeof(float2) * (size_t)c->Ny * (m + 1) > kSmemCap) {
         pfgb_set_error_msg("FNO: modes=%d too many for a %dx%dx%d grid (shared-memory staging)", m, c->Nx, c->Ny,
                            c->Nz);
         return PFGB_ERR_UNSUPPORTED;
     }
-    if (layer_smem(c->Nz, m) > kSmemCap) {
+    if (layer_staging(c->Nz, m) > kSmemCap) {
         pfgb_set_error_msg("FNO: modes=%d too many for Nz=%d (shared-memory staging)", m, c->Nz);
         return PFGB_ERR_UNSUPPORTED;
     }
@@ -945,31 +1110,32 @@ pfgb_status smem_opt_in(K kern, size_t bytes) {
     return PFGB_OK;
 }
 
-size_t dft_z_smem(int Z, int Mz, int LB) {
-    return sizeof(float) * (2 * (size_t)Z * pad2(Mz) + (size_t)LB * (Z + 1));
-}
-// about 256 tasks (2 wavenumbers of one line each) per block, lines within 64 KB
-int dft_z_lb(int Z, int Mz) {
-    const int kg = pad2(Mz) / 2;
-    return std::max(1, std::min((256 + kg - 1) / kg, (64 * 1024) / (4 * (Z + 1))));
+size_t dft_z_smem(int Mz, int LB) {
+    return sizeof(float) * (2 * (size_t)kZC * pad2(Mz) + (size_t)kZC * dft_z_stride(LB));
 }
 
 // spectral transform of src [W][N] onto the retained modes -> dst [W][M]
 pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, float w1) {
     const long long lines = (long long)kW * f->S;
-    const int LB = dft_z_lb(f->Z, f->Mz);
-    const size_t sz = dft_z_smem(f->Z, f->Mz, LB);
+    const int LB = dft_z_lines(f->Mz);
+    const size_t sz = dft_z_smem(f->Mz, LB);
     FNO_CHECK(smem_opt_in(k_dft_z, sz));
     k_dft_z<<<(unsigned)((lines + LB - 1) / LB), 256, sz, f->stream>>>(src, f->A, f->fz, lines, f->Z, f->Mz, LB,
                                                                        w0, w1);
     FNO_CHECK(check_launch("dft_z"));
-    const size_t sy = sizeof(float2) * ((size_t)f->Y + (size_t)f->Y * f->Mz);
-    FNO_CHECK(smem_opt_in(k_dft_y, sy));
-    k_dft_y<<<(unsigned)(kW * f->X), 256, sy, f->stream>>>(f->A, f->B, f->twy, f->Y, f->Mz, f->m);
+    // slabs per block: about 256 tasks within 96 KB, one at least
+    const size_t slab = sizeof(float2) * (size_t)f->Y * f->Mz;
+    const int tasks = f->Mz * ((2 * f->m + kYJ - 1) / kYJ);
+    const long long nslab = (long long)kW * f->X;
+    const int NS = (int)std::max<long long>(1, std::min<long long>(256 / std::max(1, tasks), (96 * 1024) / (long long)slab));
+    FNO_CHECK(smem_opt_in(k_dft_y, kSmemCap));
+    k_dft_y<<<(unsigned)((nslab + NS - 1) / NS), 256, slab * NS, f->stream>>>(f->A, f->B, f->tyi, nslab, NS, f->Y,
+                                                                              f->Mz, f->m);
     FNO_CHECK(check_launch("dft_y"));
-    const size_t sx = sizeof(float2) * (size_t)f->X;
+    const size_t sx = sizeof(float2) * (size_t)f->X * kXJ;
     FNO_CHECK(smem_opt_in(k_dft_x, sx));
-    k_dft_x<<<(unsigned)(kW * 2 * f->m), 256, sx, f->stream>>>(f->B, dst, f->twx, f->X, f->Q, f->m);
+    k_dft_x<<<dim3((f->Q + kXT - 1) / kXT, kW, (2 * f->m + kXJ - 1) / kXJ), kXT, sx, f->stream>>>(f->B, dst, f->twx,
+                                                                                              f->X, f->Q, f->m);
     return check_launch("dft_x");
 }
 
@@ -983,10 +1149,7 @@ pfgb_status spec_inverse_xy(pfgb_fno *f, const float2 *src) {
     return check_launch("idft_y");
 }
 
-size_t layer_smem(int Z, int Mz) {
-    return sizeof(float) * ((size_t)kW * kW + kW) +
-           sizeof(float2) * ((size_t)Mz * Z + (size_t)kW * layer_lines(Z) * Mz);
-}
+size_t layer_smem(int Z, int Mz) { return layer_staging(Z, Mz); }
 
 unsigned grid_cells(long long N) { return (unsigned)std::min<long long>((N + 255) / 256, 152LL * 16); }
 
@@ -1012,16 +1175,21 @@ pfgb_status forward_impl(pfgb_fno *f, const float *in, float *out, bool train) {
         const unsigned nb = (unsigned)((f->N + kLayerCells - 1) / kLayerCells);
         auto launch = [&](auto kern) -> pfgb_status {
             FNO_CHECK(smem_opt_in(kern, sl));
-            kern<<<nb, kLayerCells, sl, f->stream>>>(f->A, vin, f->wbf + f->offW[l], f->master + f->offb[l], vout,
+            kern<<<nb, kLayerCells / 2, sl, f->stream>>>(f->A, vin, f->wbf + f->offW[l], f->master + f->offb[l], vout,
                                                      train ? f->pres[l] : nullptr, f->gz, f->S, f->Z, f->Mz);
             return check_launch("layer_fwd");
         };
-        if (act) FNO_CHECK(train ? launch(k_layer_fwd<true, true>) : launch(k_layer_fwd<true, false>));
-        else FNO_CHECK(train ? launch(k_layer_fwd<false, true>) : launch(k_layer_fwd<false, false>));
+        if (f->Z % 2 == 0) {
+            if (act) FNO_CHECK(train ? launch(k_layer_fwd<true, true, true>) : launch(k_layer_fwd<true, false, true>));
+            else FNO_CHECK(train ? launch(k_layer_fwd<false, true, true>) : launch(k_layer_fwd<false, false, true>));
+        } else {
+            if (act) FNO_CHECK(train ? launch(k_layer_fwd<true, true, false>) : launch(k_layer_fwd<true, false, false>));
+            else FNO_CHECK(train ? launch(k_layer_fwd<false, true, false>) : launch(k_layer_fwd<false, false, false>));
+        }
     }
     if (!out) return PFGB_OK;   // training: the projection backward recomputes it
     const float *vl = train ? f->vs[f->L] : (f->L % 2 == 0 ? f->va : f->vb);
-    k_project<<<grid_cells(f->N), 256, 0, f->stream>>>(vl, f->wbf + f->offQ1, f->master + f->offq1,
+    k_project<<<grid_cells(f->N), 128, 0, f->stream>>>(vl, f->wbf + f->offQ1, f->master + f->offq1,
                                                        f->wbf + f->offQ2, f->master + f->offq2,
                                                        make_float4(osc[0], osc[1], osc[2], 0.f), out, f->N);
     return check_launch("project");
@@ -1052,7 +1220,7 @@ pfgb_status ensure_train(pfgb_fno *f) {
 }
 
 pfgb_status reduce_into(pfgb_fno *f, int nb, int E, long long off, int accumulate) {
-    k_reduce_part<<<(E + 255) / 256, 256, 0, f->stream>>>(f->part, nb, E, f->grad + off, accumulate);
+    k_reduce_part<<<(E + 31) / 32, 1024, 0, f->stream>>>(f->part, nb, E, f->grad + off, accumulate);
     return check_launch("reduce_part");
 }
 
@@ -1064,7 +1232,7 @@ pfgb_status loss_grad_impl(pfgb_fno *f, const float *in, const float *tgt, int a
     double *den = f->dscal, *loss = f->dscal + 1;
     k_sumsq<<<nbs, 256, 0, f->stream>>>(tgt, nt, f->dpart);
     FNO_CHECK(check_launch("sumsq"));
-    k_sum_partials<<<1, 1, 0, f->stream>>>(f->dpart, nbs, den);
+    k_sum_partials<<<1, 256, 0, f->stream>>>(f->dpart, nbs, den);
     FNO_CHECK(check_launch("sum_partials"));
     const long long ntiles = (f->N + kTile - 1) / kTile;
     const int nb = (int)std::min<long long>(ntiles, kRedBlocks);
@@ -1078,7 +1246,7 @@ pfgb_status loss_grad_impl(pfgb_fno *f, const float *in, const float *tgt, int a
                                                 f->dpart + kRedBlocks, f->N, ntiles);
     FNO_CHECK(check_launch("project_bwd"));
     FNO_CHECK(reduce_into(f, nb, kProjE, f->offQ1, accumulate));
-    k_loss_final<<<1, 1, 0, f->stream>>>(f->dpart + kRedBlocks, nb, den, loss);
+    k_loss_final<<<1, 256, 0, f->stream>>>(f->dpart + kRedBlocks, nb, den, loss);
     FNO_CHECK(check_launch("loss_final"));
     const float invN = (float)(1.0 / (double)f->N);
     const int LBz = lines_per_block(f->Z);
@@ -1339,7 +1507,7 @@ pfgb_status pfgb_fno_adam_step(pfgb_fno *f, const pfgb_fno_adam *opt) {
     if (opt->clip_norm > 0.f) {
         k_sumsq_f<<<4 * 152, 256, 0, f->stream>>>(f->grad, f->nparams, f->dpart);
         FNO_CHECK(check_launch("grad_norm"));
-        k_sum_partials<<<1, 1, 0, f->stream>>>(f->dpart, 4 * 152, gn);
+        k_sum_partials<<<1, 256, 0, f->stream>>>(f->dpart, 4 * 152, gn);
         FNO_CHECK(check_launch("grad_norm_sum"));
     }
     k_adam<<<1216, 256, 0, f->stream>>>(f->master, f->wbf, f->grad, f->am, f->av, f->nparams, opt->lr, opt->beta1,
