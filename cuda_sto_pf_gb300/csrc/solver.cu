@@ -83,7 +83,7 @@ enum { DS_MEAN_DY = 0, DS_RES_DIFF = 1, DS_RES_REF = 2, DS_ZM = 4, DS_BR = 12, D
 // elastic-iteration status on the device (slots of the same array): done,
 // updates taken, non-finite residual, converged.  While `done` is set, the
 // kernels of further iterations launched ahead return at once.
-enum { DS_EL = 56 };
+enum { DS_EL = 56, DS_CTR = 62 };   // DS_CTR: the residual's block counter (zero between launches)
 
 struct pfgb_ctx {
     pfgb_params p;
@@ -1972,6 +1972,70 @@ struct OpStrainFromUX {   // warm start: strain of the stored u, then inverse x
     }
 };
 
+// the stopping rule of the accelerated elastic solver on the device (loop
+// control of main_cuda.cu:28982-29050): after an update, rel = sqrt(diff /
+// max(ref, floor)); stop when iter >= iter_min and rel <= tol, at iter_max,
+// or on a non-finite / negative residual sum.  Slots DS_EL + 0..3: done,
+// updates taken, non-finite, converged.  Nothing changes once done is set.
+struct ResidArgs {
+    double *dscal;
+    unsigned *ctr;             // blocks whose residual sums are written
+    double floor_, tol;
+    int iter_min, iter_max;
+};
+__device__ __forceinline__ void resid_step(const ResidArgs &A) {
+    double *dscal = A.dscal, *st = dscal + DS_EL;
+    if (st[0] != 0.0) return;
+    const double d = dscal[DS_RES_DIFF], r = dscal[DS_RES_REF];
+    const double it = st[1] + 1.0;
+    st[1] = it;
+    if (!isfinite(d) || !isfinite(r) || d < 0.0 || r < 0.0) {
+        st[2] = 1.0;
+        st[0] = 1.0;
+        return;
+    }
+    const double rel = sqrt(d / fmax(r, A.floor_));
+    dscal[3] = rel;
+    if (it >= (double)A.iter_min && rel <= A.tol) {
+        st[3] = 1.0;
+        st[0] = 1.0;
+    } else if (it >= (double)A.iter_max) {
+        st[0] = 1.0;
+    }
+}
+static __global__ void k_resid_step(ResidArgs A) { resid_step(A); }
+
+// The residual of a Green pass without launches of its own: each block writes
+// its sums and counts itself in (resid_block, true in the last one), and the
+// last block, when its lines are stored, adds all sums in a fixed order and
+// takes the stopping decision (resid_finish).
+__device__ __forceinline__ bool resid_block(const ResidArgs &A, double *partials, AccSum2 s) {
+    __shared__ bool last;
+    block_reduce_acc(s);
+    if (threadIdx.x == 0) {
+        const unsigned nb = gridDim.x * gridDim.y;
+        reinterpret_cast<AccSum2 *>(partials)[blockIdx.y * gridDim.x + blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(A.ctr, 1u) == nb - 1;
+    }
+    __syncthreads();
+    return last;
+}
+__device__ __forceinline__ void resid_finish(const ResidArgs &A, const double *partials, int resid) {
+    __threadfence();
+    AccSum2 a = AccSum2::identity();
+    const int nb = gridDim.x * gridDim.y;
+    for (int i = threadIdx.x; i < nb; i += blockDim.x)
+        a = AccSum2::combine(a, AccSum2{__ldcg(partials + 2 * i), __ldcg(partials + 2 * i + 1)});
+    block_reduce_acc(a);
+    if (threadIdx.x == 0) {
+        A.dscal[DS_RES_DIFF] = a.a;
+        A.dscal[DS_RES_REF] = a.b;
+        *A.ctr = 0u;
+        if (resid == 2) resid_step(A);
+    }
+}
+
 // Green's function x pass.  Inputs: the 6 y-transformed components of the
 // source (eps0 for the cold start, h_ij during the iteration).
 //   t_i = k_j tau_ij  (tau = C0:eps0 for EIGEN)
@@ -1993,7 +2057,8 @@ struct GreenArgs {
     const double *skip;        // return at once when *skip != 0 (a finished solve)
     const float4 *btab;        // tensor-core 41-point stage: its B table (null: FP32 FMAs)
     int *tc_err;               // set when a bounded tensor-core wait runs out
-    int resid;
+    int resid;                 // accumulate the residual; 2: the last block also takes the stopping decision
+    ResidArgs res;
     int mode;                  // 0 u <- Phi(u); 1 first increment step; 2 delta <- r0 + L delta
 };
 
@@ -2226,13 +2291,9 @@ k_x_green(const __grid_constant__ GreenArgs<TE> A, const __grid_constant__ AxisP
 #pragma unroll
         for (int c = 0; c < 6; ++c) X[q * SP + c * TK + l] = strain_comp<TE>(c, kv[0], kv[1], kv[2], v);
     }
-    if (A.resid) {
-        AccSum2 s{double(rd), double(rr)};
-        block_reduce_acc(s);
-        if (threadIdx.x == 0)
-            reinterpret_cast<AccSum2 *>(A.partials)[blockIdx.y * gridDim.x + blockIdx.x] = s;
-    }
-    __syncthreads();
+    bool last = false;
+    if (A.resid) last = resid_block(A.res, A.partials, AccSum2{double(rd), double(rr)});
+    else __syncthreads();
     fft_lines<TE, +1>(X, tw, plan, td.out, SP, 1);
 #pragma unroll 1
     for (Walk w(fTK); w.q < n; w.step()) {
@@ -2241,42 +2302,16 @@ k_x_green(const __grid_constant__ GreenArgs<TE> A, const __grid_constant__ AxisP
             for (int cmp = 0; cmp < 6; ++cmp) A.E[cmp][base + w.q * es + w.l] = X[w.q * SP + cmp * TK + w.l];
         }
     }
-}
-
-// residual finalize: rel = sqrt(diff / max(ref, floor))
-static __global__ void k_resid_final(double *dscal, double floor_) {
-    const double d = dscal[DS_RES_DIFF], r = dscal[DS_RES_REF];
-    dscal[3] = sqrt(d / fmax(r, floor_));
-}
-
-// the stopping rule of the accelerated elastic solver on the device (loop
-// control of main_cuda.cu:28982-29050): after an update, rel = sqrt(diff /
-// max(ref, floor)); stop when iter >= iter_min and rel <= tol, at iter_max,
-// or on a non-finite / negative residual sum.  Slots DS_EL + 0..3: done,
-// updates taken, non-finite, converged.  Nothing changes once done is set.
-static __global__ void k_resid_step(double *dscal, double floor_, double tol, int iter_min, int iter_max) {
-    double *st = dscal + DS_EL;
-    if (st[0] != 0.0) return;
-    const double d = dscal[DS_RES_DIFF], r = dscal[DS_RES_REF];
-    const double it = st[1] + 1.0;
-    st[1] = it;
-    if (!isfinite(d) || !isfinite(r) || d < 0.0 || r < 0.0) {
-        st[2] = 1.0;
-        st[0] = 1.0;
-        return;
-    }
-    const double rel = sqrt(d / fmax(r, floor_));
-    dscal[3] = rel;
-    if (it >= (double)iter_min && rel <= tol) {
-        st[3] = 1.0;
-        st[0] = 1.0;
-    } else if (it >= (double)iter_max) {
-        st[0] = 1.0;
-    }
+    if (last) resid_finish(A.res, A.partials, A.resid);
 }
 
 static __global__ void k_el_status_reset(double *dscal) {
     if (threadIdx.x < 4) dscal[DS_EL + threadIdx.x] = 0.0;
+}
+
+static ResidArgs resid_args(const pfgb_ctx *c) {
+    return ResidArgs{c->dscal, (unsigned *)(c->dscal + DS_CTR), c->p.elastic_residual_absolute_floor,
+                     c->p.elastic_residual_tolerance, c->p.elastic_iter_min, std::max(1, c->p.elastic_iter_max)};
 }
 
 // spectra a Green pass moves besides its 6 sources, 6 strains and 3 written
@@ -2291,7 +2326,7 @@ static int green_extra(const pfgb_ctx *c, int mode, int resid) {
 }
 
 template <typename TE>
-static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks, int mode = 0) {
+static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int mode = 0) {
     using T2 = cplx_t<TE>;
     const int n = c->plx.n;
     const int TK = axis_tile<T2>(n, 6, c->g.kept_rows(), c->g.NzK);
@@ -2313,6 +2348,7 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
     A.btab = (const float4 *)c->tc_btab;
     A.tc_err = c->tc_err;
     A.resid = resid;
+    A.res = resid_args(c);
     A.mode = mode;
     dim3 grid((c->g.NzK + TK - 1) / TK, c->g.kept_rows());
     // reads 6 source spectra (+3 old u for the residual), writes 3 u + 6 strain spectra
@@ -2328,7 +2364,6 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int *nblocks
         kern<<<grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream>>>(A, c->plx, ft);
     }
     PFGB_CUDA_TRY(cudaGetLastError());
-    *nblocks = grid.x * grid.y;
     return PFGB_OK;
 }
 
@@ -2420,17 +2455,14 @@ k_x_green246(GreenArgs<float> A) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) pt[c * TC] = strain_comp<float>(c, kv[0], kv[1], kv[2], v);
     }
-    if (A.resid) {
-        AccSum2 sacc{double(rd), double(rr)};
-        block_reduce_acc(sacc);
-        if (threadIdx.x == 0)
-            reinterpret_cast<AccSum2 *>(A.partials)[blockIdx.y * gridDim.x + blockIdx.x] = sacc;
-    }
-    __syncthreads();
+    bool last = false;
+    if (A.resid) last = resid_block(A.res, A.partials, AccSum2{double(rd), double(rr)});
+    else __syncthreads();
     if constexpr (TCS) tc41::lines<+1, PSX, 1>(buf, tw, tcx);
     else lines<PSX, +1, PSX, 1>(buf, tw);
 #pragma unroll
     for (int s = 0; s < 6; ++s) tile_out<TC, PSX>(buf + s * TC, A.E[s] + base, es, kcnt, N, N);
+    if (last) resid_finish(A.res, A.partials, A.resid);
     if constexpr (TCS) tc41::end(tcx.tmem);
 }
 
@@ -2556,7 +2588,7 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
     return PFGB_OK;
 }
 
-static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblocks, int mode = 0) {
+static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int mode = 0) {
     using E = f246::Eng<42>;
     GreenArgs<float> A;
     A.g = c->g;
@@ -2575,6 +2607,7 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     A.btab = (const float4 *)c->tc_btab;
     A.tc_err = c->tc_err;
     A.resid = resid;
+    A.res = resid_args(c);
     A.mode = mode;
     const int TC = c->tc_x ? f246::TC : E::NL / 6;
     dim3 grid((c->g.NzK + TC - 1) / TC, c->g.kept_rows());
@@ -2590,7 +2623,6 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int *nblo
     else
         TRY(eigen ? go(k_x_green246<true, false>, E::SMEM) : go(k_x_green246<false, false>, E::SMEM));
     PFGB_CUDA_TRY(cudaGetLastError());
-    *nblocks = grid.x * grid.y;
     return PFGB_OK;
 }
 
@@ -2842,7 +2874,6 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
     const double Nf = (double)c->g.N;
     AxisIO<TE, 6, 6> io6;
     for (int i = 0; i < 6; ++i) { io6.in[i] = (const T2e *)c->E[i]; io6.out[i] = (T2e *)c->E[i]; }
-    int nb = 0;
     // the four passes of an iteration, on the 246-point engine where the axis allows
     auto ypass = [&](int dir, const char *tag) -> pfgb_status {
         if constexpr (std::is_same<TE, float>::value) {
@@ -2853,9 +2884,9 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
     };
     auto green = [&](bool eigen, int resid, int mode) -> pfgb_status {
         if constexpr (std::is_same<TE, float>::value) {
-            if (c->f246[0]) return launch_green246(c, eigen, resid, &nb, mode);
+            if (c->f246[0]) return launch_green246(c, eigen, resid, mode);
         }
-        return launch_green<TE>(c, eigen, resid, &nb, mode);
+        return launch_green<TE>(c, eigen, resid, mode);
     };
     auto hij = [&](int lin) -> pfgb_status {
         const double extra = lin ? 2.0 * Nf * sizeof(T) : (2.0 + pc.gp) * Nf * sizeof(T);
@@ -2927,13 +2958,23 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
             c->cheb_rho = cheb_it == 0 ? 2.0 / (2.0 - s2) : 1.0 / (1.0 - 0.25 * s2 * c->cheb_rho);
             ++cheb_it;
         }
-        TRY(green(false, accel, inc ? (lin ? 2 : 1) : 0));
+        // In the increment form the strain of the last iterate is not used
+        // (the final pass takes the strain of u0 + delta), so the stopping
+        // decision is taken in the Green pass and the y pass of the update
+        // that ends the solve returns at once, like the later ones.
+        TRY(green(false, accel ? (inc ? 2 : 1) : 0, inc ? (lin ? 2 : 1) : 0));
         if (cheb && lin)
             for (int i = 0; i < 3; ++i) std::swap(c->Dk[i], c->Dkm[i]);
-        return ypass(+1, "y_inv6");
+        TRY(ypass(+1, "y_inv6"));
+        if (accel && !inc) {
+            ProfScope ps(c, {"resid_step", 0.0});
+            k_resid_step<<<1, 1, 0, c->stream>>>(resid_args(c));
+            PFGB_CUDA_TRY(cudaGetLastError());
+        }
+        return PFGB_OK;
     };
     if (accel) {
-        // The residual test runs on the device (k_resid_step) and the host
+        // The residual test runs on the device (resid_step) and the host
         // launches the updates in batches, reading the status once per
         // batch: the first batch is the last solve's count (with the
         // extrapolated start the count moves by one at most from step to
@@ -2952,13 +2993,7 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
         int launched = 0;
         for (;;) {
             const int nbat = std::min(batch, imax - launched);
-            for (int b = 0; b < nbat; ++b) {
-                TRY(update(launched + b));
-                TRY(reduce_to<AccSum2>(c, nb, DS_RES_DIFF));
-                k_resid_step<<<1, 1, 0, c->stream>>>(c->dscal, P.elastic_residual_absolute_floor,
-                                                     P.elastic_residual_tolerance, P.elastic_iter_min, imax);
-                PFGB_CUDA_TRY(cudaGetLastError());
-            }
+            for (int b = 0; b < nbat; ++b) TRY(update(launched + b));
             launched += nbat;
             PFGB_CUDA_TRY(cudaMemcpyAsync(c->hscal + 3, c->dscal + 3, sizeof(double), cudaMemcpyDeviceToHost,
                                           c->stream));
@@ -4769,6 +4804,10 @@ pfgb_status pfgb_create(const pfgb_params *pin, int device, pfgb_ctx **out) {
     A_(&c->partials, sizeof(double) * c->npartials);
     A_(&c->dscal, sizeof(double) * 64);
 #undef A_
+    if (s == PFGB_OK && cudaMemset(c->dscal, 0, sizeof(double) * 64) != cudaSuccess) {
+        pfgb_set_error("cudaMemset", cudaGetLastError(), __FILE__, __LINE__);
+        s = PFGB_ERR_CUDA;
+    }
     if (s == PFGB_OK) s = make_ktab(c);
     if (s == PFGB_OK) s = upload_twiddles(c, 0, pin->Nx);
     if (s == PFGB_OK) s = upload_twiddles(c, 1, pin->Ny);
