@@ -255,6 +255,39 @@ PFGB_HD T logit_clip(T xB, T eps, T Yc) {
 }
 
 // ---------------------------------------------------------------------------
+// dependent launches.  A kernel launched with pfgb_launch starts while the one
+// before it in the stream drains: its first instruction waits for that one's
+// end (and its writes), then lets the next such kernel be scheduled.  It takes
+// the launch and the block scheduling out of the chain of short kernels.  Not for
+// a pass in FP64: blocks that come early fill the SMs that become free first, and
+// what is bound by the FP64 pipe then waits for the fullest SM (64^3 in FP64, ten
+// steps: 12.6 ms with such passes started early, 11.5 ms with them started at the
+// last block's end, 10.6 ms with plain launches).
+// ---------------------------------------------------------------------------
+template <typename T> constexpr bool kDependent = sizeof(T) == 4;
+template <typename T = float>
+__device__ __forceinline__ void dependent_begin() {
+    if constexpr (kDependent<T>) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+}
+template <typename T = float, typename... P, typename... A>
+static cudaError_t pfgb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = kDependent<T> ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // error handling
 // ---------------------------------------------------------------------------
 #define PFGB_CUDA_TRY(expr)                                                  \

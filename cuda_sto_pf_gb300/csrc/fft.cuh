@@ -382,6 +382,7 @@ template <typename T, int NIN, int NOUT, int DIN, int DOUT, class Op>
 __global__ void __launch_bounds__(256, pass_blocks<T>())
 k_axis_pass(Grid3 g, int axis, const __grid_constant__ AxisPlan plan, const cplx_t<T> *tw_g, TileDiv td,
             AxisIO<T, NIN, NOUT> io, Op op, const double *skip) {
+    dependent_begin<T>();
     if (skip && *skip != 0.0) return;   // a finished elastic iteration: launched ahead, nothing to do
     using T2 = cplx_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -519,6 +520,7 @@ template <typename T, int NFI, int NFO, class Op>
 __global__ void __launch_bounds__(256, 2)
 k_zpass(Grid3 g, const __grid_constant__ AxisPlan plan, const cplx_t<T> *tw_g, int R, Op op, ZDiv zd,
         const double *skip) {
+    dependent_begin<T>();
     if (skip && *skip != 0.0) return;
     using T2 = cplx_t<T>;
     extern __shared__ __align__(128) unsigned char smem_raw[];

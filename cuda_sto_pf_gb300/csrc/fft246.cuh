@@ -215,6 +215,7 @@ constexpr int Y_NL = 42;          // columns per block of the elastic y pass
 template <int DIR>
 __global__ void __launch_bounds__(f246::Eng<f246::Y_NL>::THREADS, f246::Eng<f246::Y_NL>::BLOCKS)
 k_y246(Grid3 g, const float2 *tw_g, AxisIO<float, 6, 6> io, const double *skip) {
+    dependent_begin();
     if (skip && *skip != 0.0) return;
     using namespace f246;
     constexpr int NLT = Y_NL;
@@ -262,6 +263,7 @@ template <int NIN, int NOUT, int DIN, int DOUT, class Op>
 __global__ void __launch_bounds__(f246::Eng<f246_axis_lines(NIN > NOUT ? NIN : NOUT)>::THREADS,
                                   f246::Eng<f246_axis_lines(NIN > NOUT ? NIN : NOUT)>::BLOCKS)
 k_axis246(Grid3 g, int axis, const float2 *tw_g, AxisIO<float, NIN, NOUT> io, Op op, const double *skip) {
+    dependent_begin();
     if (skip && *skip != 0.0) return;
     using namespace f246;
     constexpr int NW = NIN > NOUT ? NIN : NOUT;

@@ -560,9 +560,8 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
             PFGB_CUDA_TRY(allow_smem(kern, smem));
             dim3 grid((c->g.NzK + TCW - 1) / TCW, axis == 1 ? c->g.Nx : c->g.kept_rows());
             ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-            kern<<<grid, E::THREADS, smem, c->stream>>>(c->g, axis, (const float2 *)twp<T>(c, axis == 1 ? 1 : 0), io,
-                                                      op, c->skip);
-            PFGB_CUDA_TRY(cudaGetLastError());
+            PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, smem, c->stream, c->g, axis,
+                                      (const float2 *)twp<T>(c, axis == 1 ? 1 : 0), io, op, c->skip));
             return PFGB_OK;
         }
     }
@@ -576,9 +575,8 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
     dim3 grid((c->g.NzK + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.kept_rows(), Op::kInplace ? NIN : 1);
     const TileDiv ft = tile_div(TK, Op::kInplace ? 1 : NIN, Op::kInplace ? 1 : NOUT);
     ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-    kern<<<grid, pfgb_line_threads(pl, NW * TK), smem, c->stream>>>(c->g, axis, pl, twp<T>(c, axis == 1 ? 1 : 0), ft,
-                                                                    io, op, c->skip);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    PFGB_CUDA_TRY(pfgb_launch<T>(kern, grid, pfgb_line_threads(pl, NW * TK), smem, c->stream, c->g, axis, pl,
+                              twp<T>(c, axis == 1 ? 1 : 0), ft, io, op, c->skip));
     return PFGB_OK;
 }
 
@@ -596,6 +594,7 @@ template <int NFI, int NFO, class Op>
 __global__ void __launch_bounds__(f246::Eng<f246_z_lines(f246_z_width<NFI, NFO>())>::THREADS,
                                   f246::Eng<f246_z_lines(f246_z_width<NFI, NFO>())>::BLOCKS)
 k_zpass246g(Grid3 g, const float2 *tw_g, Op op, const double *skip) {
+    dependent_begin();
     if (skip && *skip != 0.0) return;
     using namespace f246;
     constexpr int LO = (NFO + 1) / 2, LW = f246_z_width<NFI, NFO>();
@@ -675,8 +674,8 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
             const long long rows = (long long)c->g.Nx * c->g.Ny;
             const int nb = (int)((rows + R - 1) / R);
             ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-            kern<<<nb, E::THREADS, smem, c->stream>>>(c->g, (const float2 *)twp<T>(c, 2), op, c->skip);
-            PFGB_CUDA_TRY(cudaGetLastError());
+            PFGB_CUDA_TRY(pfgb_launch(kern, nb, E::THREADS, smem, c->stream, c->g, (const float2 *)twp<T>(c, 2), op,
+                                      c->skip));
             if (nblocks) *nblocks = nb;
             return PFGB_OK;
         }
@@ -693,9 +692,8 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     const int nb = (int)((rows + R - 1) / R);
     ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-    kern<<<nb, pfgb_line_threads(c->plz, zpass_lines<NFI, NFO>(R)), smem, c->stream>>>(c->g, c->plz, twp<T>(c, 2), R,
-                                                                                       op, zdiv<NFI, NFO>(c->g, R), c->skip);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    PFGB_CUDA_TRY(pfgb_launch<T>(kern, nb, pfgb_line_threads(c->plz, zpass_lines<NFI, NFO>(R)), smem, c->stream, c->g,
+                              c->plz, twp<T>(c, 2), R, op, zdiv<NFI, NFO>(c->g, R), c->skip));
     if (nblocks) *nblocks = nb;
     return PFGB_OK;
 }
@@ -756,6 +754,7 @@ using AccZM = AccZMt<double>;
 template <class Acc>
 __global__ void k_reduce_partials(const Acc *part, int n, double *out, int slot, double scale,
                                   const double *skip = nullptr) {
+    dependent_begin();
     if (skip && *skip != 0.0) return;
     Acc a = Acc::identity();
     for (int i = threadIdx.x; i < n; i += blockDim.x) a = Acc::combine(a, part[i]);
@@ -769,9 +768,8 @@ __global__ void k_reduce_partials(const Acc *part, int n, double *out, int slot,
 template <class Acc>
 static pfgb_status reduce_to(pfgb_ctx *c, int nblocks, int slot, double scale = 1.0) {
     ProfScope ps(c, {"reduce_partials", (double)nblocks * sizeof(Acc)});
-    k_reduce_partials<Acc><<<1, 256, 0, c->stream>>>((const Acc *)c->partials, nblocks, c->dscal, slot, scale,
-                                                     c->skip);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    PFGB_CUDA_TRY(pfgb_launch(k_reduce_partials<Acc>, 1, 256, 0, c->stream, (const Acc *)c->partials, nblocks,
+                              c->dscal, slot, scale, c->skip));
     return PFGB_OK;
 }
 
@@ -2003,7 +2001,10 @@ __device__ __forceinline__ void resid_step(const ResidArgs &A) {
         st[0] = 1.0;
     }
 }
-static __global__ void k_resid_step(ResidArgs A) { resid_step(A); }
+static __global__ void k_resid_step(ResidArgs A) {
+    dependent_begin();
+    resid_step(A);
+}
 
 // The residual of a Green pass without launches of its own: each block writes
 // its sums and counts itself in (resid_block, true in the last one), and the
@@ -2215,6 +2216,7 @@ __device__ __forceinline__ void green_u(const TE *S, TE kx, TE ky, TE kz, const 
 template <typename TE, bool EIGEN>
 __global__ void __launch_bounds__(256, pass_blocks<TE>())
 k_x_green(const __grid_constant__ GreenArgs<TE> A, const __grid_constant__ AxisPlan plan, TileDiv td) {
+    dependent_begin<TE>();
     if (A.skip && *A.skip != 0.0) return;
     using T2 = cplx_t<TE>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -2306,6 +2308,7 @@ k_x_green(const __grid_constant__ GreenArgs<TE> A, const __grid_constant__ AxisP
 }
 
 static __global__ void k_el_status_reset(double *dscal) {
+    dependent_begin();
     if (threadIdx.x < 4) dscal[DS_EL + threadIdx.x] = 0.0;
 }
 
@@ -2357,11 +2360,11 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int mode = 0
     if (eigen) {
         auto kern = k_x_green<TE, true>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        kern<<<grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream>>>(A, c->plx, ft);
+        PFGB_CUDA_TRY(pfgb_launch<TE>(kern, grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream, A, c->plx, ft));
     } else {
         auto kern = k_x_green<TE, false>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        kern<<<grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream>>>(A, c->plx, ft);
+        PFGB_CUDA_TRY(pfgb_launch<TE>(kern, grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream, A, c->plx, ft));
     }
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
@@ -2378,6 +2381,7 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int mode = 0
 template <bool EIGEN, bool TCS>
 __global__ void __launch_bounds__(f246::Eng<TCS ? 48 : 42>::THREADS, 2)
 k_x_green246(GreenArgs<float> A) {
+    dependent_begin();
     if (A.skip && *A.skip != 0.0) return;
     using namespace f246;
     using T2 = float2;
@@ -2583,8 +2587,7 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
     for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
     dim3 grid((c->g.NzK + E::NL - 1) / E::NL, c->g.Nx, 6);
     ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
-    kern<<<grid, E::THREADS, smem, c->stream>>>(c->g, (const float2 *)c->tw[1][1], io, c->skip);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, smem, c->stream, c->g, (const float2 *)c->tw[1][1], io, c->skip));
     return PFGB_OK;
 }
 
@@ -2615,7 +2618,7 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int mode 
                      (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(float2)});
     auto go = [&](auto kern, size_t sm) -> pfgb_status {
         PFGB_CUDA_TRY(allow_smem(kern, sm));
-        kern<<<grid, E::THREADS, sm, c->stream>>>(A);
+        PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, sm, c->stream, A));
         return PFGB_OK;
     };
     if (c->tc_x)   // the 41-point stages on the tensor cores
@@ -2689,6 +2692,7 @@ template <typename TE>
 __global__ void __launch_bounds__(256)
 k_add_increment(Grid3 g, cplx_t<TE> *u0, cplx_t<TE> *u1, cplx_t<TE> *u2, const cplx_t<TE> *d0,
                 const cplx_t<TE> *d1, const cplx_t<TE> *d2) {
+    dependent_begin();
     for_kept(g, [&](long long i) {
         u0[i] = cadd(u0[i], d0[i]);
         u1[i] = cadd(u1[i], d1[i]);
@@ -2721,6 +2725,7 @@ struct ExtrapArgs { cplx_t<TE> *u[3], *h[5][3], *slot[3]; };
 template <typename TE>
 __global__ void __launch_bounds__(256)
 k_extrapolate_u(Grid3 g, ExtrapArgs<TE> a, int m) {
+    dependent_begin();
     for_kept(g, [&](long long i) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -2853,9 +2858,8 @@ static pfgb_status model_start(pfgb_ctx *c) {
     TRY((launch_axis<TE, 3, 3, -1, 0>(c, 2, io, OpCutU3<TE>{ktab(c)},
                                       "x_fwd3")));
     ProfScope ps(c, {"add_increment", 9.0 * c->g.kept() * sizeof(T2e)});
-    k_add_increment<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, (T2e *)c->U[0], (T2e *)c->U[1], (T2e *)c->U[2],
-                                                             E0, E1, E2);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    PFGB_CUDA_TRY(pfgb_launch(k_add_increment<TE>, 1216, dim3(32, 8), 0, c->stream, c->g, (T2e *)c->U[0],
+                              (T2e *)c->U[1], (T2e *)c->U[2], E0, E1, E2));
     return PFGB_OK;
 }
 
@@ -2925,8 +2929,7 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
                 for (int l = 0; l < 5; ++l) a.h[l][i] = (T2e *)c->Uhist[l][i];
                 a.slot[i] = (T2e *)c->Uhist[nh - 1][i];
             }
-            k_extrapolate_u<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, a, std::max(m, 0));
-            PFGB_CUDA_TRY(cudaGetLastError());
+            PFGB_CUDA_TRY(pfgb_launch(k_extrapolate_u<TE>, 1216, dim3(32, 8), 0, c->stream, c->g, a, std::max(m, 0)));
             for (int i = 0; i < 3; ++i) {
                 void *oldest = c->Uhist[nh - 1][i];
                 for (int l = nh - 1; l > 0; --l) c->Uhist[l][i] = c->Uhist[l - 1][i];
@@ -2968,8 +2971,7 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
         TRY(ypass(+1, "y_inv6"));
         if (accel && !inc) {
             ProfScope ps(c, {"resid_step", 0.0});
-            k_resid_step<<<1, 1, 0, c->stream>>>(resid_args(c));
-            PFGB_CUDA_TRY(cudaGetLastError());
+            PFGB_CUDA_TRY(pfgb_launch(k_resid_step, 1, 1, 0, c->stream, resid_args(c)));
         }
         return PFGB_OK;
     };
@@ -2984,8 +2986,7 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
         // batch a host round trip.  The Chebyshev buffer swaps the host made
         // for updates that returned at once are undone below.
         struct SkipGuard { pfgb_ctx *c; ~SkipGuard() { c->skip = nullptr; } } guard{c};
-        k_el_status_reset<<<1, 32, 0, c->stream>>>(c->dscal);
-        PFGB_CUDA_TRY(cudaGetLastError());
+        PFGB_CUDA_TRY(pfgb_launch(k_el_status_reset, 1, 32, 0, c->stream, c->dscal));
         c->skip = c->dscal + DS_EL;
         const int imax = std::max(1, P.elastic_iter_max);
         int batch = c->last_el_iters > 1 ? c->last_el_iters : 4;
@@ -3052,10 +3053,9 @@ static pfgb_status elastic_solve(pfgb_ctx *c, pfgb_step_stats *st) {
         // u = u0 + delta, and the strain of u for the final pass
         {
             ProfScope ps(c, {"add_increment", 9.0 * c->g.kept() * sizeof(T2e)});
-            k_add_increment<TE><<<1216, dim3(32, 8), 0, c->stream>>>(c->g, (T2e *)c->U[0], (T2e *)c->U[1],
-                                                                     (T2e *)c->U[2], (const T2e *)c->Dk[0],
-                                                                     (const T2e *)c->Dk[1], (const T2e *)c->Dk[2]);
-            PFGB_CUDA_TRY(cudaGetLastError());
+            PFGB_CUDA_TRY(pfgb_launch(k_add_increment<TE>, 1216, dim3(32, 8), 0, c->stream, c->g, (T2e *)c->U[0],
+                                      (T2e *)c->U[1], (T2e *)c->U[2], (const T2e *)c->Dk[0], (const T2e *)c->Dk[1],
+                                      (const T2e *)c->Dk[2]));
         }
         AxisIO<TE, 3, 6> io;
         for (int i = 0; i < 3; ++i) io.in[i] = (const T2e *)c->U[i];
@@ -5361,6 +5361,39 @@ struct OpRealOut {
     __device__ void store_spec(long long, int, const cplx_t<T> *) const {}
 };
 
+static size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// w_a[m] = exp(-2 pi i m / n_a) for the three axes, each table on a 256-byte
+// boundary
+template <typename T>
+__global__ void k_fill_twiddles(unsigned char *base, int n0, int n1, int n2, size_t off1, size_t off2) {
+    dependent_begin();
+    const int a = blockIdx.y;
+    const int n = a == 0 ? n0 : (a == 1 ? n1 : n2);
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= n) return;
+    cplx_t<T> *w = (cplx_t<T> *)(base + (a == 0 ? 0 : (a == 1 ? off1 : off2)));
+    double s, co;
+    sincospi(-2.0 * (double)m / (double)n, &s, &co);
+    w[m].x = (T)co;
+    w[m].y = (T)s;
+}
+template <typename T>
+static pfgb_status fill_twiddles(pfgb_ctx *c, unsigned char *base, size_t off1, size_t off2) {
+    const Grid3 &g = c->g;
+    const int pi = sizeof(T) == 8 ? 0 : 1, nmax = std::max(g.Nx, std::max(g.Ny, g.Nz));
+    c->tw[pi][0] = base;
+    c->tw[pi][1] = base + off1;
+    c->tw[pi][2] = base + off2;
+    PFGB_CUDA_TRY(pfgb_launch(k_fill_twiddles<T>, dim3((nmax + 255) / 256, 3), 256, 0, c->stream, base, g.Nx, g.Ny,
+                              g.Nz, off1, off2));
+    return PFGB_OK;
+}
+
+// the context of one standalone transform: its twiddle tables (the precision
+// asked for) in one stream-ordered allocation, filled on the device; six
+// synchronous allocations and copies from the host took 300 us of a call
+template <typename T>
 static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *stream) {
     if (Nx < 1 || Ny < 1 || Nz < 2 || Nx > PFGB_MAX_N || Ny > PFGB_MAX_N || Nz > PFGB_MAX_N) {
         pfgb_set_error_msg("transform size %dx%dx%d outside [1..%d] (Nz >= 2)", Nx, Ny, Nz, PFGB_MAX_N);
@@ -5374,17 +5407,26 @@ static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *strea
     pfgb_make_plan(Nx, &c->plx);
     pfgb_make_plan(Ny, &c->ply);
     pfgb_make_plan(Nz, &c->plz);
-    TRY(upload_twiddles(c, 0, Nx));
-    TRY(upload_twiddles(c, 1, Ny));
-    TRY(upload_twiddles(c, 2, Nz));
-    return PFGB_OK;
+    const size_t off1 = round256(sizeof(cplx_t<T>) * (size_t)Nx), off2 = off1 + round256(sizeof(cplx_t<T>) * (size_t)Ny);
+    void *base = nullptr;
+    const cudaError_t e = cudaMallocAsync(&base, off2 + sizeof(cplx_t<T>) * (size_t)Nz, c->stream);
+    if (e != cudaSuccess) {
+        pfgb_set_error("cudaMallocAsync", e, __FILE__, __LINE__);
+        return e == cudaErrorMemoryAllocation ? PFGB_ERR_NOMEM : PFGB_ERR_CUDA;
+    }
+    return fill_twiddles<T>(c, (unsigned char *)base, off1, off2);
 }
 
-static void fft_ctx_free(pfgb_ctx *c) {
-    cudaStreamSynchronize(c->stream);
-    for (int a = 0; a < 2; ++a)
-        for (int b = 0; b < 3; ++b)
-            if (c->tw[a][b]) cudaFree(c->tw[a][b]);
+// the tables are given back and the transform is complete on return
+static pfgb_status fft_ctx_free(pfgb_ctx *c, pfgb_status s) {
+    void *base = c->tw[0][0] ? c->tw[0][0] : c->tw[1][0];
+    if (base) cudaFreeAsync(base, c->stream);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    if (s == PFGB_OK && e != cudaSuccess) {
+        pfgb_set_error("cudaStreamSynchronize", e, __FILE__, __LINE__);
+        return PFGB_ERR_CUDA;
+    }
+    return s;
 }
 
 template <typename T>
@@ -5454,7 +5496,7 @@ pfgb_status pfgb_fft_y246x6(int tensor_cores, int dir, int Nx, int NzC, void *sp
     }
     TRY(check_transform_buffers(spec6, spec6));
     pfgb_ctx c;
-    pfgb_status s = fft_ctx_init(&c, Nx, f246::N, 2 * (NzC - 1), stream);
+    pfgb_status s = fft_ctx_init<float>(&c, Nx, f246::N, 2 * (NzC - 1), stream);
     c.g.NzC = NzC;
     c.g.Nk = (long long)Nx * f246::N * NzC;
     c.g.keep_all();
@@ -5471,7 +5513,7 @@ pfgb_status pfgb_fft_y246x6(int tensor_cores, int dir, int Nx, int NzC, void *sp
             cudaStreamSynchronize(c.stream) != cudaSuccess) s = PFGB_ERR_CUDA;
         else if (te) { pfgb_set_error_msg("tensor-core 41-point stage: a wait ran out"); s = PFGB_ERR_TIMEOUT; }
     }
-    fft_ctx_free(&c);
+    s = fft_ctx_free(&c, s);
     if (c.tc_btab) cudaFree(c.tc_btab);
     if (c.tc_err) cudaFree(c.tc_err);
     return s;
@@ -5480,24 +5522,24 @@ pfgb_status pfgb_fft_y246x6(int tensor_cores, int dir, int Nx, int NzC, void *sp
 pfgb_status pfgb_fft3d_r2c(int precision, int Nx, int Ny, int Nz, const void *in, void *out, void *stream) {
     TRY(check_transform_buffers(in, out));
     pfgb_ctx c;
-    pfgb_status s = fft_ctx_init(&c, Nx, Ny, Nz, stream);
+    pfgb_status s = precision == PFGB_PREC_FP64 ? fft_ctx_init<double>(&c, Nx, Ny, Nz, stream)
+                                                : fft_ctx_init<float>(&c, Nx, Ny, Nz, stream);
     if (s == PFGB_OK)
         s = precision == PFGB_PREC_FP64 ? fft_r2c_impl<double>(&c, (const double *)in, (double2 *)out)
                                         : fft_r2c_impl<float>(&c, (const float *)in, (float2 *)out);
-    fft_ctx_free(&c);
-    return s;
+    return fft_ctx_free(&c, s);
 }
 
 // The half-spectrum input is used as workspace and is overwritten.
 pfgb_status pfgb_fft3d_c2r(int precision, int Nx, int Ny, int Nz, const void *in, void *out, void *stream) {
     TRY(check_transform_buffers(in, out));
     pfgb_ctx c;
-    pfgb_status s = fft_ctx_init(&c, Nx, Ny, Nz, stream);
+    pfgb_status s = precision == PFGB_PREC_FP64 ? fft_ctx_init<double>(&c, Nx, Ny, Nz, stream)
+                                                : fft_ctx_init<float>(&c, Nx, Ny, Nz, stream);
     if (s == PFGB_OK)
         s = precision == PFGB_PREC_FP64 ? fft_c2r_impl<double>(&c, (double2 *)in, (double *)out)
                                         : fft_c2r_impl<float>(&c, (float2 *)in, (float *)out);
-    fft_ctx_free(&c);
-    return s;
+    return fft_ctx_free(&c, s);
 }
 
 }  // extern "C"
@@ -5513,22 +5555,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[PFGB_NOALLOC_SC
 static constexpr int kNoallocMaxDevices = 64;
 static std::mutex g_noalloc_mu;
 static void *g_noalloc_addr[kNoallocMaxDevices];
-
-static size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
-
-// w_a[m] = exp(-2 pi i m / n_a), the same table the allocating path uploads
-template <typename T>
-__global__ void k_fill_twiddles(unsigned char *base, int n0, int n1, int n2, size_t off1, size_t off2) {
-    const int a = blockIdx.y;
-    const int n = a == 0 ? n0 : (a == 1 ? n1 : n2);
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
-    cplx_t<T> *w = (cplx_t<T> *)(base + (a == 0 ? 0 : (a == 1 ? off1 : off2)));
-    double s, co;
-    sincospi(-2.0 * (double)m / (double)n, &s, &co);
-    w[m].x = (T)co;
-    w[m].y = (T)s;
-}
 
 // Address of the scratch array on the calling thread's current device,
 // looked up once per device.
@@ -5571,15 +5597,8 @@ static pfgb_status fft_r2c_noalloc(int Nx, int Ny, int Nz, const T *in, cplx_t<T
     pfgb_make_plan(Nx, &c.plx);
     pfgb_make_plan(Ny, &c.ply);
     pfgb_make_plan(Nz, &c.plz);
-    const int pi = sizeof(T) == 8 ? 0 : 1;
-    c.tw[pi][0] = base;
-    c.tw[pi][1] = base + off1;
-    c.tw[pi][2] = base + off2;
-    const int nmax = std::max(Nx, std::max(Ny, Nz));
-    k_fill_twiddles<T><<<dim3((nmax + 255) / 256, 3), 256, 0, c.stream>>>(base, Nx, Ny, Nz, off1, off2);
-    PFGB_CUDA_TRY(cudaGetLastError());
+    TRY(fill_twiddles<T>(&c, base, off1, off2));
     pfgb_status s = fft_r2c_impl<T>(&c, in, out);
-    c.tw[pi][0] = c.tw[pi][1] = c.tw[pi][2] = nullptr;
     return s;
 }
 
