@@ -367,6 +367,12 @@ struct AxisIO {
 
 template <int NIN, int NOUT> constexpr int axis_width() { return NIN > NOUT ? NIN : NOUT; }
 
+// ops may declare begin(): what a thread reads once before its points
+template <class Op, class = void>
+struct op_has_begin { static constexpr bool value = false; };
+template <class Op>
+struct op_has_begin<Op, std::void_t<decltype(std::declval<Op &>().begin())>> { static constexpr bool value = true; };
+
 // divisors of an axis pass's loops: the columns of a tile, the lines that it
 // transforms forward and back
 struct TileDiv {
@@ -433,6 +439,7 @@ k_axis_pass(Grid3 g, int axis, const __grid_constant__ AxisPlan plan, const cplx
     __syncthreads();
     if (DIN != 0) fft_lines<T, DIN>(A, tw, plan, td.in, SP, 1);
     if constexpr (!INPL) {
+        if constexpr (op_has_begin<Op>::value) op.begin();
 #pragma unroll 1
         for (Walk w(fTK); w.q < n; w.step()) {
             const int q = w.q, l = w.l;

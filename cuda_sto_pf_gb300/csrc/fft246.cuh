@@ -285,6 +285,7 @@ k_axis246(Grid3 g, int axis, const float2 *tw_g, AxisIO<float, NIN, NOUT> io, Op
     __syncthreads();
     if (DIN != 0) lines<NLT, DIN, NLT, 1>(buf, tw);
     if constexpr (!Op::kInplace) {
+        if constexpr (op_has_begin<Op>::value) op.begin();
         for (int e = threadIdx.x; e < N * TCW; e += blockDim.x) {
             const int q = e / TCW, t = e % TCW;
             const int i = axis == 1 ? slab : q, j = axis == 1 ? q : slab;

@@ -39,6 +39,7 @@ const char *pfgb_error_buffer(void);
 struct KTab {
     const double *kx, *ky, *kz;
     const float *fx, *fy, *fz;           // the same rounded to float
+    const float2 *qx, *qy, *qz;          // their squares as double-float pairs
     const unsigned char *mx, *my, *mz;   // 1 = removed by the 2/3 rule
     __device__ __forceinline__ bool cut(int i, int j, int k) const { return (mx[i] | my[j] | mz[k]) != 0; }
     // the wave numbers in the type of a pass (a conversion from double per point
@@ -54,6 +55,11 @@ struct KTab {
     template <typename T> __device__ __forceinline__ T z(int k) const {
         if constexpr (sizeof(T) == 4) return fz[k];
         else return kz[k];
+    }
+    // k^2 in double-float (FP32 passes: the FP64 pipe is 64 times slower)
+    __device__ __forceinline__ dfl k2f(int i, int j, int k) const {
+        const float2 a = qx[i], b = qy[j], c = qz[k];
+        return df_add(df_add(dfl{a.x, a.y}, dfl{b.x, b.y}), dfl{c.x, c.y});
     }
     __device__ __forceinline__ double k2(int i, int j, int k) const {
         double a = kx[i], b = ky[j], c = kz[k];
@@ -98,6 +104,7 @@ struct pfgb_ctx {
     void *tw[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};  // [fp64|fp32][x,y,z]
     double *kx = nullptr, *ky = nullptr, *kz = nullptr;
     float *kf = nullptr;      // the wave numbers of the three axes in float, one after another
+    float2 *kq = nullptr;     // and their squares as double-float pairs
     unsigned char *mx = nullptr, *my = nullptr, *mz = nullptr;
     void *phi[2] = {nullptr, nullptr}, *eta[2] = {nullptr, nullptr}, *Y = nullptr, *dYdt = nullptr;
     void *Yprev = nullptr;   // Y_f of the last step's start, for the stress export
@@ -166,7 +173,8 @@ struct pfgb_ctx {
 };
 
 static KTab ktab(const pfgb_ctx *c) {
-    return KTab{c->kx, c->ky, c->kz, c->kf, c->kf + c->g.Nx, c->kf + c->g.Nx + c->g.Ny, c->mx, c->my, c->mz};
+    return KTab{c->kx, c->ky, c->kz, c->kf, c->kf + c->g.Nx, c->kf + c->g.Nx + c->g.Ny, c->kq, c->kq + c->g.Nx,
+                c->kq + c->g.Nx + c->g.Ny, c->mx, c->my, c->mz};
 }
 
 // tag + algorithmic bytes of the next launch (set by the op-level wrappers)
@@ -723,6 +731,35 @@ struct AccSum2 {
         return {__shfl_down_sync(0xffffffffu, x.a, o), __shfl_down_sync(0xffffffffu, x.b, o)};
     }
 };
+// the same sums in an FP32 pass: double-float per thread and block (the FP64
+// pipe takes a conversion and an addition per cell otherwise)
+struct AccDf1 {
+    static constexpr bool kActive = true;
+    dfl s;
+    __device__ static AccDf1 identity() { return {dfl{0.f, 0.f}}; }
+    __device__ static AccDf1 combine(AccDf1 a, AccDf1 b) { return {df_add(a.s, b.s)}; }
+    __device__ static AccDf1 shfl_down(AccDf1 a, int o) {
+        return {dfl{__shfl_down_sync(0xffffffffu, a.s.hi, o), __shfl_down_sync(0xffffffffu, a.s.lo, o)}};
+    }
+};
+struct AccDf2 {
+    static constexpr bool kActive = true;
+    dfl a, b;
+    __device__ static AccDf2 identity() { return {dfl{0.f, 0.f}, dfl{0.f, 0.f}}; }
+    __device__ static AccDf2 combine(AccDf2 x, AccDf2 y) { return {df_add(x.a, y.a), df_add(x.b, y.b)}; }
+    __device__ static AccDf2 shfl_down(AccDf2 x, int o) {
+        return {AccDf1::shfl_down(AccDf1{x.a}, o).s, AccDf1::shfl_down(AccDf1{x.b}, o).s};
+    }
+};
+__device__ __forceinline__ void acc_add(double &s, double v) { s += v; }
+__device__ __forceinline__ void acc_add(dfl &s, float v) { s = df_add_f(s, v); }
+__device__ __forceinline__ AccSum1 acc_out(const AccSum1 &a) { return a; }
+__device__ __forceinline__ AccSum1 acc_out(const AccDf1 &a) { return {df_to_double(a.s)}; }
+__device__ __forceinline__ AccSum2 acc_out(const AccSum2 &a) { return a; }
+__device__ __forceinline__ AccSum2 acc_out(const AccDf2 &a) { return {df_to_double(a.a), df_to_double(a.b)}; }
+template <typename T> using AccSum1Of = std::conditional_t<sizeof(T) == 8, AccSum1, AccDf1>;
+template <typename T> using AccSum2Of = std::conditional_t<sizeof(T) == 8, AccSum2, AccDf2>;
+
 // zero-mode statistics: min, max of Y*, and the Taylor moments
 // M_p = sum (1-h) sigma^{(p)}(Y*) (M_0 also + h v_B), p = 0..4
 // (m[5] = sum |1 - h|, the curvature bound of the zero-mode certification).
@@ -837,13 +874,30 @@ struct OpEtaR2C {   // z pass producer: eta - L_eta dt rhs_eta (phi = updated ph
     }
 };
 
+// T(num / (1 + m k^2)): in double, or for float values in double-float, one
+// correction of the float quotient rounding it like the double one
+template <typename T>
+__device__ __forceinline__ T damped(const KTab &kt, int i, int j, int k, double num, double m, dfl numf, dfl mf) {
+    if constexpr (sizeof(T) == 8) {
+        return T(num / (1.0 + m * kt.k2(i, j, k)));
+    } else {
+        const dfl den = df_add_f(df_mul(mf, kt.k2f(i, j, k)), 1.0f);
+        const float q = 1.0f / den.hi, f = numf.hi * q;
+        const float e = fmaf(-f, den.hi, numf.hi) + fmaf(-f, den.lo, numf.lo);
+        return fmaf(e, q, f);
+    }
+}
+static dfl host_df(double v) { return dfl{(float)v, (float)(v - (double)(float)v)}; }
+
 template <typename T>
 struct OpACFilterX {   // x pass: mask / (1 + L dt kappa k^2) / N
     static constexpr bool kInplace = false;
     KTab kt; double Ldtk, invN;
+    dfl Lf, nf;
+    OpACFilterX(const KTab &k, double L, double n) : kt(k), Ldtk(L), invN(n), Lf(host_df(L)), nf(host_df(n)) {}
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         if (kt.cut(i, j, k)) { out[0] = mk2<cplx_t<T>>(T(0), T(0)); return; }
-        const T f = T(invN / (1.0 + Ldtk * kt.k2(i, j, k)));
+        const T f = damped<T>(kt, i, j, k, invN, Ldtk, nf, Lf);
         out[0] = cscale(in[0], f);
     }
 };
@@ -871,7 +925,7 @@ struct OpACStoreZ {   // z pass consumer: clamp and store the new order paramete
 // paths carry none of its code)
 template <typename T, typename TE, bool GPC = false>
 struct OpMuR2C {
-    using Acc = AccSum1;
+    using Acc = AccSum1Of<T>;
     DevState<T, TE> d; PhysCT<T> c; ElasC<TE> ec;
     // the fields of two cells read ahead of their work
     static constexpr int kBatch = 2;
@@ -921,7 +975,7 @@ struct OpMuR2C {
             // at eta_for_Y_explicit (main_cuda.cu:30292)
             const T hp = pf_h(phiY), he = pf_h(c.prev_level ? d.eta_old[cell] : d.eta_new[cell]);
             const T xs = sigmoid_clip(Yv, T(20), T(1e-12));
-            acc.s += double((T(1) - hp) * (T(1) - he) * T(c.Da) * (xs * (T(1) - xs)));
+            acc_add(acc.s, (T(1) - hp) * (T(1) - he) * T(c.Da) * (xs * (T(1) - xs)));
             return;
         }
         const T h = pf_h(phiY);
@@ -929,13 +983,13 @@ struct OpMuR2C {
         T x = lg.x;
         if (x < T(1e-12)) x = T(1e-12);
         if (x > T(1) - T(1e-12)) x = T(1) - T(1e-12);
-        acc.s += double(Dm * x * (T(1) - x));
+        acc_add(acc.s, Dm * x * (T(1) - x));
     }
     __device__ void load_spec(long long, int, cplx_t<T> *) const {}
     __device__ void store_spec(long long row, int k, const cplx_t<T> *v) const {
         d.S[0][row * d.g.NzC + k] = v[0];
     }
-    __device__ void finish(int b, const Acc &a) const { reinterpret_cast<Acc *>(d.partials)[b] = a; }
+    __device__ void finish(int b, const Acc &a) const { reinterpret_cast<AccSum1 *>(d.partials)[b] = acc_out(a); }
 };
 
 // (2) gradient: g_a = IFFT(mask i k_a mask mu_k)/N, three outputs
@@ -1080,11 +1134,13 @@ template <typename T>
 struct OpYUpdX {
     static constexpr bool kInplace = false;
     KTab kt; double dt, invN; const double *meanDY;
+    double m = 0.0;      // dt <DY>, read once per thread
+    dfl mf{}, tf{};
+    __device__ void begin() { m = dt * (*meanDY); mf = df_from_double(m); tf = df_from_double(dt); }
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         using T2 = cplx_t<T>;
         if (kt.cut(i, j, k)) { out[0] = mk2<T2>(T(0), T(0)); return; }
-        const double den = 1.0 + dt * (*meanDY) * kt.k2(i, j, k);
-        const T a = T(dt / den);
+        const T a = damped<T>(kt, i, j, k, dt, m, tf, mf);
         const T2 div = cadd(cmul_is(in[0], kt.template x<T>(i)), in[1]);
         out[0] = cscale(cadd(in[2], cscale(div, a)), T(invN));
     }
@@ -1162,10 +1218,12 @@ template <typename T>
 struct OpXSplitX {
     static constexpr bool kInplace = false;
     KTab kt; double dt, invN, m;
+    dfl mf{}, tf{};
+    __device__ void begin() { m = dt * m; mf = df_from_double(m); tf = df_from_double(dt); }
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         using T2 = cplx_t<T>;
         if (kt.cut(i, j, k)) { out[0] = mk2<T2>(T(0), T(0)); return; }
-        const T a = T(dt / (1.0 + dt * m * kt.k2(i, j, k)));
+        const T a = damped<T>(kt, i, j, k, dt, m, tf, mf);
         out[0] = cscale(cadd(in[1], cscale(in[0], a)), T(invN));
     }
 };
@@ -1485,10 +1543,13 @@ template <typename T>
 struct OpYUpdRX {
     static constexpr bool kInplace = false;
     KTab kt; double dt, invN; const double *meanDY;
+    double m = 0.0;      // dt <DY>, read once per thread
+    dfl mf{}, tf{};
+    __device__ void begin() { m = dt * (*meanDY); mf = df_from_double(m); tf = df_from_double(dt); }
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         using T2 = cplx_t<T>;
         if (kt.cut(i, j, k)) { out[0] = mk2<T2>(T(0), T(0)); return; }
-        const T a = T(dt / (1.0 + dt * (*meanDY) * kt.k2(i, j, k)));
+        const T a = damped<T>(kt, i, j, k, dt, m, tf, mf);
         out[0] = cscale(cadd(in[1], cscale(in[0], a)), T(invN));
     }
 };
@@ -3694,9 +3755,14 @@ template <typename T>
 struct OpLapX {
     static constexpr bool kInplace = false;
     KTab kt; double invN;
+    dfl nf{};
+    __device__ void begin() { nf = df_from_double(invN); }
     __device__ void apply(int i, int j, int k, const cplx_t<T> *in, cplx_t<T> *out) const {
         if (kt.cut(i, j, k)) { out[0] = mk2<cplx_t<T>>(T(0), T(0)); return; }
-        out[0] = cscale(in[0], T(-kt.k2(i, j, k) * invN));
+        T f;
+        if constexpr (sizeof(T) == 8) f = T(-kt.k2(i, j, k) * invN);
+        else f = -df_mul(kt.k2f(i, j, k), nf).hi;
+        out[0] = cscale(in[0], f);
     }
 };
 
@@ -3704,7 +3770,7 @@ struct OpLapX {
 // g_full = g_e - kappa Lap (the volume multiplier, :29484-29489)
 template <typename T, typename TE>
 struct OpMinLapZ {
-    using Acc = AccSum2;
+    using Acc = AccSum2Of<T>;
     DevState<T, TE> d; const T *phi; double kappa;
     __device__ void load_spec(long long row, int k, cplx_t<T> *v) const { v[0] = d.S[0][row * d.g.NzC + k]; }
     __device__ void point(long long cell, const T *in, T *, Acc &acc) const {
@@ -3712,11 +3778,11 @@ struct OpMinLapZ {
         d.mlap[cell] = lap;
         const T gf = d.mge[cell] - T(kappa) * lap;
         const T hp = pf_hp(phi[cell]);
-        acc.a += double(hp * gf);
-        acc.b += double(hp * hp);
+        acc_add(acc.a, hp * gf);
+        acc_add(acc.b, hp * hp);
     }
     __device__ void store_spec(long long, int, const cplx_t<T> *) const {}
-    __device__ void finish(int b, const Acc &a) const { reinterpret_cast<Acc *>(d.partials)[b] = a; }
+    __device__ void finish(int b, const Acc &a) const { reinterpret_cast<AccSum2 *>(d.partials)[b] = acc_out(a); }
 };
 
 // z pass producer of the constrained step: phi - L dt [(g_full + kappa Lap) + lambda h']
@@ -3757,12 +3823,34 @@ struct AccMinE {
     }
 };
 
+// the cell's terms in the arithmetic R: double for FP64 fields, double-float for
+// FP32 fields (per cell in FP64: 163 us at 96^3; in double-float 90 us)
+__device__ __forceinline__ double w_const(double v, double) { return v; }
+__device__ __forceinline__ dfl w_const(double v, dfl) { return df_from_double(v); }
+__device__ __forceinline__ double w_diff(double a, double b) { return a - b; }
+__device__ __forceinline__ dfl w_diff(float a, float b) { return df_two_sum(a, -b); }
+__device__ __forceinline__ double w_add(double a, double b) { return a + b; }
+__device__ __forceinline__ dfl w_add(dfl a, dfl b) { return df_add(a, b); }
+__device__ __forceinline__ double w_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ dfl w_mul(dfl a, dfl b) { return df_mul(a, b); }
+__device__ __forceinline__ double w_of(double v, double) { return v; }
+__device__ __forceinline__ dfl w_of(float v, dfl) { return {v, 0.f}; }
+__device__ __forceinline__ double w_round(double v, double) { return v; }
+__device__ __forceinline__ float w_round(dfl v, float) { return v.hi; }
+__device__ __forceinline__ double w_out(double v) { return v; }
+__device__ __forceinline__ double w_out(dfl v) { return df_to_double(v); }
+
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
-k_min_energy(DevState<T, TE> d, PhysC c, ElasC<TE> ec, const T *phi, double g0, int chem, AccMinE *part) {
-    AccMinE a = AccMinE::identity();
+k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *phi, double g0, int chem, AccMinE *part) {
+    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
+    R mh = w_const(0.0, R{}), grad = mh, dw = mh, gel = mh, gelh = mh, ch = mh;
     const int Nx = d.g.Nx, Ny = d.g.Ny, Nz = d.g.Nz;
-    const double idx2 = 0.5 / c.dx, idy2 = 0.5 / c.dy, idz2 = 0.5 / c.dz;
+    // 0.5 kappa (0.5 / dx)^2 and so on
+    const R wx = w_const(0.125 * cd.kappa / (cd.dx * cd.dx), R{}), wy = w_const(0.125 * cd.kappa / (cd.dy * cd.dy), R{}),
+            wz = w_const(0.125 * cd.kappa / (cd.dz * cd.dz), R{});
+    const R GA = w_const(cd.tc.GA_s, R{}), GB = w_const(cd.tc.GB_s, R{}), mu0 = w_const(cd.mu0, R{}),
+            mg0 = w_const(-g0, R{});
     for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < d.g.N;
          cell += (long long)gridDim.x * blockDim.x) {
         const int k = (int)(cell % Nz);
@@ -3771,35 +3859,39 @@ k_min_energy(DevState<T, TE> d, PhysC c, ElasC<TE> ec, const T *phi, double g0, 
         const int ip = i + 1 == Nx ? 0 : i + 1, im = i == 0 ? Nx - 1 : i - 1;
         const int jp = j + 1 == Ny ? 0 : j + 1, jm = j == 0 ? Ny - 1 : j - 1;
         const int kp = k + 1 == Nz ? 0 : k + 1, km = k == 0 ? Nz - 1 : k - 1;
-        const double gx = (double(phi[((long long)ip * Ny + j) * Nz + k]) - double(phi[((long long)im * Ny + j) * Nz + k])) * idx2;
-        const double gy = (double(phi[((long long)i * Ny + jp) * Nz + k]) - double(phi[((long long)i * Ny + jm) * Nz + k])) * idy2;
-        const double gz = (double(phi[r * Nz + kp]) - double(phi[r * Nz + km])) * idz2;
+        const R gx = w_diff(phi[((long long)ip * Ny + j) * Nz + k], phi[((long long)im * Ny + j) * Nz + k]);
+        const R gy = w_diff(phi[((long long)i * Ny + jp) * Nz + k], phi[((long long)i * Ny + jm) * Nz + k]);
+        const R gz = w_diff(phi[r * Nz + kp], phi[r * Nz + km]);
         const T p = phi[cell];
-        a.grad += 0.5 * c.kappa * (gx * gx + gy * gy + gz * gz);
-        a.dw += c.W * double(pf_g(p));
+        grad = w_add(grad, w_add(w_add(w_mul(wx, w_mul(gx, gx)), w_mul(wy, w_mul(gy, gy))), w_mul(wz, w_mul(gz, gz))));
+        dw = w_add(dw, w_of(pf_g(p), R{}));
         const T h = pf_h(clamp01(p));
-        a.mh += double(h);
+        const R hr = w_of(h, R{});
+        mh = w_add(mh, hr);
         // the monitor's composition: sigmoid(Y), capped once clamped
         const T xB = xB_of_Y<T>(c, d.Y[cell] + T(d.Yc));
         const T xm = xB < T(c.xbcap) ? xB : T(c.xbcap);
         if (c.elastic) {
             TE e0[6];
             eigenstrain<T, TE>(c, ec, p, c.gp ? d.eta_old[cell] : T(0), clamp01(xm), c.gp_el != 0, e0);
-            double sd = 0.0;
+            R sd = w_const(0.0, R{});
 #pragma unroll
-            for (int q = 0; q < 6; ++q)
-                sd += (q < 3 ? 1.0 : 2.0) * double(d.sig[q][cell]) * (double(d.eps[q][cell]) - double(e0[q]));
-            a.gel += 0.5 * sd;
-            a.gelh += 0.5 * sd * double(h);
+            for (int q = 0; q < 6; ++q)   // 1/2 sigma : (eps - e0); shear enters twice
+                sd = w_add(sd, w_mul(w_of(T(d.sig[q][cell]) * (q < 3 ? T(0.5) : T(1)), R{}),
+                                     w_diff(T(d.eps[q][cell]), T(e0[q]))));
+            gel = w_add(gel, sd);
+            gelh = w_add(gelh, w_mul(sd, hr));
         }
         if (chem) {
             const T x = clamp_eps(xm, T(1e-12));
             T offA, offB;
             thermo_mu_off<T>(c.tc, x, offA, offB);
-            const double mix = (1.0 - double(x)) * (c.tc.GA_s + double(offA)) + double(x) * (c.tc.GB_s + double(offB));
-            a.chem += (1.0 - double(h)) * mix + double(h) * c.mu0 - g0;
+            const R xr = w_of(x, R{}), omx = w_diff(T(1), x), omh = w_diff(T(1), h);
+            const R mix = w_add(w_mul(omx, w_add(GA, w_of(offA, R{}))), w_mul(xr, w_add(GB, w_of(offB, R{}))));
+            ch = w_add(ch, w_add(w_add(w_mul(omh, mix), w_mul(hr, mu0)), mg0));
         }
     }
+    AccMinE a{w_out(mh), w_out(grad), cd.W * w_out(dw), w_out(gel), w_out(gelh), w_out(ch)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
@@ -3808,16 +3900,18 @@ k_min_energy(DevState<T, TE> d, PhysC c, ElasC<TE> ec, const T *phi, double g0, 
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_resid(DevState<T, TE> d, const T *phi, const T *phin, double kappa, double lk, AccSum2 *part) {
-    AccSum2 a = AccSum2::identity();
+    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
+    R sa = w_const(0.0, R{}), sb = sa;
     for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < d.g.N;
          cell += (long long)gridDim.x * blockDim.x) {
         const T p = phi[cell];
         T rr = (d.mge[cell] - T(kappa) * d.mlap[cell]) + T(lk) * pf_hp(p);
         if ((p <= T(1e-12) && rr > T(0)) || (p >= T(1) - T(1e-12) && rr < T(0))) rr = T(0);
-        a.a += double(rr) * double(rr);
-        const double dp = double(p) - double(phin[cell]);
-        a.b += dp * dp;
+        sa = w_add(sa, w_mul(w_of(rr, R{}), w_of(rr, R{})));
+        const R dp = w_diff(p, phin[cell]);
+        sb = w_add(sb, w_mul(dp, dp));
     }
+    AccSum2 a{w_out(sa), w_out(sb)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
@@ -3826,14 +3920,16 @@ k_min_resid(DevState<T, TE> d, const T *phi, const T *phin, double kappa, double
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_min_hsums(const T *phi, long long N, AccSum2 *part) {
-    AccSum2 a = AccSum2::identity();
+    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
+    R sa = w_const(0.0, R{}), sb = sa;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
          i += (long long)gridDim.x * blockDim.x) {
         const T p = phi[i];
-        a.a += double(pf_h(clamp01(p)));
+        sa = w_add(sa, w_of(pf_h(clamp01(p)), R{}));
         const T hp = pf_hp(p);
-        a.b += double(hp * hp);
+        sb = w_add(sb, w_of(hp * hp, R{}));
     }
+    AccSum2 a{w_out(sa), w_out(sb)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
@@ -3861,13 +3957,19 @@ struct AccSumMax {
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_dy(DevState<T, TE> d, PhysCT<T> c, double yc_prev, AccSumMax *part) {
-    AccSumMax a = AccSumMax::identity();
+    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
+    R ss = w_const(0.0, R{});
+    T mx = T(-3e38);
+    const R dc = w_const(d.Yc - yc_prev, R{}), yc = w_const(d.Yc, R{});
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < d.g.N;
          i += (long long)gridDim.x * blockDim.x) {
-        const double y = double(d.Y[i]) + d.Yc, yp = double(d.Yprev[i]) + yc_prev;
-        a.s += (y - yp) * (y - yp);
-        a.m = fmax(a.m, double(xB_of_Y<T>(c, T(y))));
+        const T Y = d.Y[i];
+        const R dy = w_add(w_diff(Y, d.Yprev[i]), dc);
+        ss = w_add(ss, w_mul(dy, dy));
+        const T y = w_round(w_add(w_of(Y, R{}), yc), T(0));
+        mx = fmax(mx, xB_of_Y<T>(c, y));
     }
+    AccSumMax a{w_out(ss), double(mx)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
@@ -3953,7 +4055,7 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     const double muAr = c->pc.tc.GA_s + oA, muBf = c->pc.tc.GB_s + oB;
     const double g0 = (1.0 - xref) * muAr + xref * muBf;
     TRY((min_reduce<AccMinE>(c, "min_energy", (2.0 * Nf) * sizeof(T) + 12.0 * Nf * sizeof(TE), 42, 6,
-                             k_min_energy<T, TE>, d, c->pc, ec, (const T *)pa, g0, phi_only ? 0 : 1)));
+                             k_min_energy<T, TE>, d, pc, c->pc, ec, (const T *)pa, g0, phi_only ? 0 : 1)));
     const double *E = c->hscal + 42;
     double mean_h = E[0] / Nf;
     if (it == 1 && !(c->V0_target > 0.0)) {
@@ -4274,6 +4376,11 @@ static pfgb_status make_ktab(pfgb_ctx *c) {
     std::vector<float> kf(kx.begin(), kx.end());
     kf.insert(kf.end(), ky.begin(), ky.end());
     kf.insert(kf.end(), kz.begin(), kz.end());
+    std::vector<float2> kq;
+    for (const auto *v : {&kx, &ky, &kz})
+        for (double k : *v) kq.push_back(make_float2((float)(k * k), (float)(k * k - (double)(float)(k * k))));
+    TRY(dalloc(c, (void **)&c->kq, sizeof(float2) * kq.size()));
+    PFGB_CUDA_TRY(cudaMemcpy(c->kq, kq.data(), sizeof(float2) * kq.size(), cudaMemcpyHostToDevice));
     TRY(dalloc(c, (void **)&c->kf, sizeof(float) * kf.size()));
     PFGB_CUDA_TRY(cudaMemcpy(c->kf, kf.data(), sizeof(float) * kf.size(), cudaMemcpyHostToDevice));
     PFGB_CUDA_TRY(cudaMemcpy(c->mx, mx.data(), P.Nx, cudaMemcpyHostToDevice));
@@ -4496,7 +4603,7 @@ static void ctx_free(pfgb_ctx *c) {
     for (int a = 0; a < 2; ++a) for (int b = 0; b < 3; ++b) f(c->tw[a][b]);
     f(c->tc_btab);
     f(c->tc_err);
-    f(c->kx); f(c->ky); f(c->kz); f(c->kf); f(c->mx); f(c->my); f(c->mz);
+    f(c->kx); f(c->ky); f(c->kz); f(c->kf); f(c->kq); f(c->mx); f(c->my); f(c->mz);
     for (int i = 0; i < 2; ++i) f(c->phi[i]);
     f(c->eta[0]);
     if (c->eta[1] != c->eta[0]) f(c->eta[1]);
