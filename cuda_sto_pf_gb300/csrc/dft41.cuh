@@ -58,7 +58,6 @@ __host__ __device__ constexpr double cval(int which, int b) {
 }
 
 using namespace f2x;
-__device__ __forceinline__ P sub(P a, P b) { return fma(b, both(-1.f), a); }
 template <int W, int B, bool NEG = false> __device__ __forceinline__ P kc() {
     constexpr float k = (float)(NEG ? -cval(W, B) : cval(W, B));
     return both(k);

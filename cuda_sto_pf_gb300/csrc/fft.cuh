@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "rader41.cuh"
 
 #define PFGB_MAX_STAGES 16
@@ -141,6 +142,10 @@ template <int DIR, typename T2> __device__ __forceinline__ T2 rot_mi(T2 a) {
     // forward: multiply by -i ; inverse: by +i
     return DIR < 0 ? mk2<T2>(a.y, -a.x) : mk2<T2>(-a.y, a.x);
 }
+
+// complex sums in FP32: one packed instruction for both parts, rounded as two
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return f2x::un(f2x::add(f2x::pk(a), f2x::pk(b))); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return f2x::un(f2x::sub(f2x::pk(a), f2x::pk(b))); }
 
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly2(cplx_t<T> *v) {
