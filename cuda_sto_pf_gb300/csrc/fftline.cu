@@ -136,6 +136,10 @@ __device__ __forceinline__ void sts2(uint32_t a, double2 v) {
     asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
 }
 
+// a += s, each time anew: as a + r s the offsets r s would be kept in registers
+// over the loop of a stage, and a stage saves to the stack what it uses of them
+__device__ __forceinline__ void advance(uint32_t &a, uint32_t s) { asm volatile("add.u32 %0, %0, %1;" : "+r"(a) : "r"(s)); }
+
 // natural position of output r = 0 of block b of the last stage: b's digits
 // (k_1 most significant) in the reverse order of significance
 __device__ __forceinline__ int reversed_block(const AxisPlan &p, int b) {
@@ -156,16 +160,19 @@ __device__ __noinline__ void stage_mid(LineTile t, int nb, int B, int m, int tws
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
         const int j = (int)t.fL.div((unsigned)it), l = it - j * L;
         const int b = (int)fm.div((unsigned)j), jp = j - b * m;
-        const uint32_t a = t.buf + (uint32_t)((b * B + jp) * t.PS + l * t.LS);
+        const uint32_t a0 = t.buf + (uint32_t)((b * B + jp) * t.PS + l * t.LS);
+        uint32_t a = a0;
         T2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = lds2(a + r * step, T(0));
+        for (int r = 0; r < R; ++r) { v[r] = lds2(a, T(0)); advance(a, step); }
         bfly<T, DIR, R>(v);
         const uint32_t wst = (uint32_t)(jp * twst) * (uint32_t)sizeof(T2);
+        uint32_t wa = t.tw;
 #pragma unroll
-        for (int r = 1; r < R; ++r) v[r] = twmul<DIR>(v[r], lds2(t.tw + r * wst, T(0)));
+        for (int r = 1; r < R; ++r) { advance(wa, wst); v[r] = twmul<DIR>(v[r], lds2(wa, T(0))); }
+        a = a0;
 #pragma unroll
-        for (int r = 0; r < R; ++r) sts2(a + r * step, v[r]);
+        for (int r = 0; r < R; ++r) { sts2(a, v[r]); advance(a, step); }
     }
 }
 
@@ -185,14 +192,16 @@ __device__ __noinline__ void stage_last(LineTile t, const AxisPlan *plan, int nb
         const uint32_t lo = (uint32_t)((l0 + l) * t.LS);
         T2 v[R];
         if (act) {
+            uint32_t a = in + lo;
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = lds2(in + lo + r * t.PS, T(0));
+            for (int r = 0; r < R; ++r) { v[r] = lds2(a, T(0)); advance(a, t.PS); }
             bfly<T, DIR, R>(v);
         }
         __syncthreads();
         if (act) {
+            uint32_t a = out + lo;
 #pragma unroll
-            for (int r = 0; r < R; ++r) sts2(out + lo + r * ost, v[r]);
+            for (int r = 0; r < R; ++r) { sts2(a, v[r]); advance(a, ost); }
         }
     }
 }
