@@ -618,10 +618,15 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double *__restrict__
 // Projection backward with the loss L = sum (y - t)^2 / den.
 // Per block partials (float): G_Q1 [64][32], g_q1 [64], G_Q2 [3][64], g_q2 [3]
 // in that order (the flat layout of Q1 q1 Q2 q2); loss numerator in lpart.
+// Bound by instruction issue (6,000 fused multiply-adds a cell, two
+// blocks per SM).  A cell's 64 hidden values stay in its row of the tile and the
+// 32 outputs of g_v in registers, so that the loops over hidden units stay
+// rolled (with the hidden values in registers they were 100 KB of code, 236
+// registers), and the bias and Q2 sums run along with the weights' loop.
 constexpr int kProjE = kH * kW + kH + kOut * kH + kOut;   // 2307
 constexpr int kVS = kW + 4;                               // v tile row stride (16-byte rows)
 __host__ __device__ constexpr size_t project_bwd_smem_floats() {
-    return (size_t)2 * kH * kW + kOut * kH + kH + 4 + (size_t)kTile * (2 * (kH + 1) + kVS + 4);
+    return (size_t)kH * kW + kOut * kH + kH + 4 + (size_t)kTile * (2 * (kH + 1) + kVS + 4);
 }
 __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__ v, const float *__restrict__ tgt,
                                                        const __nv_bfloat16 *__restrict__ Q1w,
@@ -633,21 +638,16 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
                                                        long long N, long long ntiles) {
     extern __shared__ __align__(16) float smp[];
     float (*Q1)[kW] = reinterpret_cast<float (*)[kW]>(smp);                   // [64][32]
-    float (*Q1T)[kH] = reinterpret_cast<float (*)[kH]>(smp + kH * kW);       // [32][64]
-    float (*Q2)[kH] = reinterpret_cast<float (*)[kH]>(smp + 2 * kH * kW);
-    float *b1 = smp + 2 * kH * kW + kOut * kH;
+    float (*Q2)[kH] = reinterpret_cast<float (*)[kH]>(smp + kH * kW);
+    float *b1 = smp + kH * kW + kOut * kH;
     float *b2 = b1 + kH;
     float (*Vs)[kVS] = reinterpret_cast<float (*)[kVS]>(b2 + 4);             // v tile (16-byte rows)
-    float (*Gs)[kH + 1] = reinterpret_cast<float (*)[kH + 1]>(&Vs[kTile][0]); // g_hpre tile
+    float (*Gs)[kH + 1] = reinterpret_cast<float (*)[kH + 1]>(&Vs[kTile][0]); // hpre, then g_hpre tile
     float (*Hs)[kH + 1] = reinterpret_cast<float (*)[kH + 1]>(&Gs[kTile][0]); // h tile
     float (*Ys)[4] = reinterpret_cast<float (*)[4]>(&Hs[kTile][0]);           // g_y tile
     __shared__ double lred[kTile];
     const int t = threadIdx.x;
-    for (int e = t; e < kH * kW; e += blockDim.x) {
-        const float w = bf(Q1w[e]);
-        Q1[e / kW][e % kW] = w;
-        Q1T[e % kW][e / kW] = w;
-    }
+    for (int e = t; e < kH * kW; e += blockDim.x) Q1[e / kW][e % kW] = bf(Q1w[e]);
     for (int e = t; e < kOut * kH; e += blockDim.x) Q2[e / kH][e % kH] = bf(Q2w[e]);
     if (t < kH) b1[t] = q1[t];
     if (t < kOut) b2[t] = q2[t];
@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long long n = tile * kTile + t;
         const bool ok = n < N;
-        float x[kW], g[kH];
+        float x[kW];
 #pragma unroll
         for (int i = 0; i < kW; ++i) x[i] = ok ? v[i * N + n] : 0.f;
         float y[kOut];
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
                 s = fmaf(w.z, x[4 * q + 2], s);
                 s = fmaf(w.w, x[4 * q + 3], s);
             }
-            g[j] = s;   // hpre for now
+            Gs[t][j] = s;   // hpre for now
             const float h = gelu(s);
             Hs[t][j] = ok ? h : 0.f;
 #pragma unroll
@@ -695,33 +695,35 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
             gy[c] = 2.f * r * inv * osc[c];
             Ys[t][c] = gy[c];
         }
-#pragma unroll 4
+        float sg[kW];
+#pragma unroll
+        for (int i = 0; i < kW; ++i) sg[i] = 0.f;
+#pragma unroll 2
         for (int j = 0; j < kH; ++j) {
             float gh = 0.f;
 #pragma unroll
             for (int c = 0; c < kOut; ++c) gh = fmaf(Q2[c][j], gy[c], gh);
-            g[j] = ok ? gh * gelu_d(g[j]) : 0.f;
-            Gs[t][j] = g[j];
+            const float gj = ok ? gh * gelu_d(Gs[t][j]) : 0.f;
+            Gs[t][j] = gj;
+            const float4 *w4 = reinterpret_cast<const float4 *>(Q1[j]);
+#pragma unroll
+            for (int q = 0; q < kW / 4; ++q) {
+                const float4 w = w4[q];
+                sg[4 * q] = fmaf(w.x, gj, sg[4 * q]);
+                sg[4 * q + 1] = fmaf(w.y, gj, sg[4 * q + 1]);
+                sg[4 * q + 2] = fmaf(w.z, gj, sg[4 * q + 2]);
+                sg[4 * q + 3] = fmaf(w.w, gj, sg[4 * q + 3]);
+            }
         }
         if (ok) {
-#pragma unroll 2
-            for (int i = 0; i < kW; ++i) {
-                float s = 0.f;
-                const float4 *w4 = reinterpret_cast<const float4 *>(Q1T[i]);
 #pragma unroll
-                for (int q = 0; q < kH / 4; ++q) {
-                    const float4 w = w4[q];
-                    s = fmaf(w.x, g[4 * q], s);
-                    s = fmaf(w.y, g[4 * q + 1], s);
-                    s = fmaf(w.z, g[4 * q + 2], s);
-                    s = fmaf(w.w, g[4 * q + 3], s);
-                }
-                gv[i * N + n] = s;
-            }
+            for (int i = 0; i < kW; ++i) gv[i * N + n] = sg[i];
         }
 #pragma unroll
         for (int i = 0; i < kW; ++i) Vs[t][i] = x[i];
         __syncthreads();
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
         for (int c = 0; c < kTile; ++c) {
             const float gj = Gs[c][jo];
             const float4 *v4 = reinterpret_cast<const float4 *>(&Vs[c][i0]);
@@ -733,29 +735,24 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
                 a1[4 * q + 2] = fmaf(gj, w.z, a1[4 * q + 2]);
                 a1[4 * q + 3] = fmaf(gj, w.w, a1[4 * q + 3]);
             }
+            ab1 += gj;
+            s0 = fmaf(Ys[c][t / kH], Hs[c][t % kH], s0);
+            if (t < kH) s1 = fmaf(Ys[c][2], Hs[c][t], s1);
+            else if (t < kH + kOut) ab2 += Ys[c][t - kH];
         }
-        for (int r = 0; r < 2; ++r) {
-            const int e = t + r * kTile;
-            if (e < kOut * kH) {
-                const int cc = e / kH, j = e - cc * kH;
-                float s = 0.f;
-                for (int c = 0; c < kTile; ++c) s = fmaf(Ys[c][cc], Hs[c][j], s);
-                a2[r] += s;
-            }
-        }
-        if (t < kH) for (int c = 0; c < kTile; ++c) ab1 += Gs[c][t];
-        if (t < kOut) for (int c = 0; c < kTile; ++c) ab2 += Ys[c][t];
+        a2[0] += s0;
+        a2[1] += s1;
         __syncthreads();
     }
     float *P = part + (long long)blockIdx.x * kProjE;
 #pragma unroll
     for (int k = 0; k < 16; ++k) P[jo * kW + i0 + k] = a1[k];
-    if (t < kH) P[kH * kW + t] = ab1;
+    if (t % 2 == 0) P[kH * kW + jo] = ab1;
     for (int r = 0; r < 2; ++r) {
         const int e = t + r * kTile;
         if (e < kOut * kH) P[kH * kW + kH + e] = a2[r];
     }
-    if (t < kOut) P[kH * kW + kH + kOut * kH + t] = ab2;
+    if (t >= kH && t < kH + kOut) P[kH * kW + kH + kOut * kH + t - kH] = ab2;
     lred[t] = lsum;
     __syncthreads();
     if (t == 0) {
@@ -767,18 +764,21 @@ __global__ void __launch_bounds__(kTile) k_project_bwd(const float *__restrict__
 
 // Pointwise backward of one layer: g_pre = g_out * act'(pre); g_v = W^T g_pre
 // (the spectral adjoint is added later); per block partials of G_W [32][32]
-// and g_b [32] (the flat layout of W_l b_l).
+// and g_b [32] (the flat layout of W_l b_l).  Eight channels at a time: their
+// reads go out together and their part of g_v is added at once, so that the
+// channels' loop stays rolled (unrolled, with erf in every channel, it was 40 KB
+// of code).
 constexpr int kLayerE = kW * kW + kW;   // 1056
 template <bool LAST>
 __global__ void __launch_bounds__(kTile) k_layer_bwd(const float *__restrict__ gout, const float *__restrict__ pre,
                                                      const float *__restrict__ v, const __nv_bfloat16 *__restrict__ Ww,
                                                      float *__restrict__ gpre, float *__restrict__ gv,
                                                      float *__restrict__ part, long long N, long long ntiles) {
-    __shared__ __align__(16) float WmT[kW][kW];   // WmT[i][o] = W[o][i]
+    __shared__ __align__(16) float Wm[kW][kW];
     __shared__ float Gs[kTile][kW + 1];
     __shared__ __align__(16) float Vs[kTile][kVS];
     const int t = threadIdx.x;
-    for (int e = t; e < kW * kW; e += blockDim.x) WmT[e % kW][e / kW] = bf(Ww[e]);
+    for (int e = t; e < kW * kW; e += blockDim.x) Wm[e / kW][e % kW] = bf(Ww[e]);
     __syncthreads();
     const int oo = t >> 2, i0 = (t & 3) * 8;
     float aw[8], ab = 0.f;
@@ -787,36 +787,44 @@ __global__ void __launch_bounds__(kTile) k_layer_bwd(const float *__restrict__ g
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long long n = tile * kTile + t;
         const bool ok = n < N;
-        float g[kW];
+        float sg[kW];
 #pragma unroll
-        for (int c = 0; c < kW; ++c) {
-            float x = 0.f;
-            if (ok) {
-                x = gout[c * N + n];
-                if (!LAST) x *= gelu_d(pre[c * N + n]);
-                gpre[c * N + n] = x;
+        for (int i = 0; i < kW; ++i) sg[i] = 0.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < kW; c0 += 8) {
+            float x[8], p[8], y[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                x[u] = ok ? gout[(c0 + u) * N + n] : 0.f;
+                p[u] = ok && !LAST ? pre[(c0 + u) * N + n] : 0.f;
+                y[u] = ok ? v[(c0 + u) * N + n] : 0.f;
             }
-            g[c] = x;
-            Gs[t][c] = x;
-            Vs[t][c] = ok ? v[c * N + n] : 0.f;
-        }
-        if (ok) {
-#pragma unroll 4
-            for (int i = 0; i < kW; ++i) {
-                float s = 0.f;
-                const float4 *w4 = reinterpret_cast<const float4 *>(WmT[i]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (!LAST) x[u] *= gelu_d(p[u]);
+                if (ok) gpre[(c0 + u) * N + n] = x[u];
+                Gs[t][c0 + u] = x[u];
+                Vs[t][c0 + u] = y[u];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float4 *w4 = reinterpret_cast<const float4 *>(Wm[c0 + u]);
 #pragma unroll
                 for (int q = 0; q < kW / 4; ++q) {
                     const float4 w = w4[q];
-                    s = fmaf(w.x, g[4 * q], s);
-                    s = fmaf(w.y, g[4 * q + 1], s);
-                    s = fmaf(w.z, g[4 * q + 2], s);
-                    s = fmaf(w.w, g[4 * q + 3], s);
+                    sg[4 * q] = fmaf(w.x, x[u], sg[4 * q]);
+                    sg[4 * q + 1] = fmaf(w.y, x[u], sg[4 * q + 1]);
+                    sg[4 * q + 2] = fmaf(w.z, x[u], sg[4 * q + 2]);
+                    sg[4 * q + 3] = fmaf(w.w, x[u], sg[4 * q + 3]);
                 }
-                gv[i * N + n] = s;
             }
         }
+        if (ok) {
+#pragma unroll
+            for (int i = 0; i < kW; ++i) gv[i * N + n] = sg[i];
+        }
         __syncthreads();
+#pragma unroll 4
         for (int c = 0; c < kTile; ++c) {
             const float go = Gs[c][oo];
             const float4 va = *reinterpret_cast<const float4 *>(&Vs[c][i0]);
@@ -825,14 +833,14 @@ __global__ void __launch_bounds__(kTile) k_layer_bwd(const float *__restrict__ g
             aw[2] = fmaf(go, va.z, aw[2]); aw[3] = fmaf(go, va.w, aw[3]);
             aw[4] = fmaf(go, vb.x, aw[4]); aw[5] = fmaf(go, vb.y, aw[5]);
             aw[6] = fmaf(go, vb.z, aw[6]); aw[7] = fmaf(go, vb.w, aw[7]);
+            ab += go;
         }
-        if (t < kW) for (int c = 0; c < kTile; ++c) ab += Gs[c][t];
         __syncthreads();
     }
     float *P = part + (long long)blockIdx.x * kLayerE;
 #pragma unroll
     for (int k = 0; k < 8; ++k) P[oo * kW + i0 + k] = aw[k];
-    if (t < kW) P[kW * kW + t] = ab;
+    if (t % 4 == 0) P[kW * kW + oo] = ab;
 }
 
 // lift backward: G_P [32][8] and g_p [32] (the flat layout of P p)
