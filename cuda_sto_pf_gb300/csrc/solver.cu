@@ -102,6 +102,7 @@ struct pfgb_ctx {
     Grid3 g;
     AxisPlan plx, ply, plz;
     void *tw[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};  // [fp64|fp32][x,y,z]
+    int tab_dev = 0, tab_slot = -1;   // a standalone transform's table slot
     double *kx = nullptr, *ky = nullptr, *kz = nullptr;
     float *kf = nullptr;      // the wave numbers of the three axes in float, one after another
     float2 *kq = nullptr;     // and their squares as double-float pairs
@@ -5508,9 +5509,45 @@ static pfgb_status fill_twiddles(pfgb_ctx *c, unsigned char *base, size_t off1, 
     return PFGB_OK;
 }
 
+// Room for the twiddle tables of standalone transforms: kTabSlots of the largest
+// size in the module's memory, taken for the length of a call (which ends with
+// the stream idle, so that a returned slot is in no kernel's use); a call that
+// finds all taken allocates.  An allocation and its release cost 190 us a call:
+// 130 us of kernels for FP64 c2r at 90x75x126 took 320.
+constexpr int kTabSlots = 8;
+constexpr size_t kTabBytes = 3 * (size_t)PFGB_MAX_N * sizeof(double2);
+static __device__ __align__(256) unsigned char g_fft_tables[kTabSlots * kTabBytes];
+struct TabSlots { unsigned used = 0; unsigned char *addr = nullptr; };
+static std::mutex g_tab_mu;
+static std::map<int, TabSlots> g_tab;   // by device
+// a free slot's address, null if there is none (or the device cannot be asked)
+static unsigned char *take_table(int *dev, int *slot) {
+    if (cudaGetDevice(dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lk(g_tab_mu);
+    TabSlots &t = g_tab[*dev];
+    if (!t.addr) {
+        void *p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_fft_tables) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        t.addr = (unsigned char *)p;
+    }
+    for (int i = 0; i < kTabSlots; ++i)
+        if (!(t.used >> i & 1u)) {
+            t.used |= 1u << i;
+            *slot = i;
+            return t.addr + i * kTabBytes;
+        }
+    return nullptr;
+}
+static void return_table(int dev, int slot) {
+    std::lock_guard<std::mutex> lk(g_tab_mu);
+    g_tab[dev].used &= ~(1u << slot);
+}
+
 // the context of one standalone transform: its twiddle tables (the precision
-// asked for) in one stream-ordered allocation, filled on the device; six
-// synchronous allocations and copies from the host took 300 us of a call
+// asked for), filled on the device
 template <typename T>
 static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *stream) {
     if (Nx < 1 || Ny < 1 || Nz < 2 || Nx > PFGB_MAX_N || Ny > PFGB_MAX_N || Nz > PFGB_MAX_N) {
@@ -5526,11 +5563,13 @@ static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *strea
     pfgb_make_plan(Ny, &c->ply);
     pfgb_make_plan(Nz, &c->plz);
     const size_t off1 = round256(sizeof(cplx_t<T>) * (size_t)Nx), off2 = off1 + round256(sizeof(cplx_t<T>) * (size_t)Ny);
-    void *base = nullptr;
-    const cudaError_t e = cudaMallocAsync(&base, off2 + sizeof(cplx_t<T>) * (size_t)Nz, c->stream);
-    if (e != cudaSuccess) {
-        pfgb_set_error("cudaMallocAsync", e, __FILE__, __LINE__);
-        return e == cudaErrorMemoryAllocation ? PFGB_ERR_NOMEM : PFGB_ERR_CUDA;
+    void *base = take_table(&c->tab_dev, &c->tab_slot);
+    if (!base) {
+        const cudaError_t e = cudaMallocAsync(&base, off2 + sizeof(cplx_t<T>) * (size_t)Nz, c->stream);
+        if (e != cudaSuccess) {
+            pfgb_set_error("cudaMallocAsync", e, __FILE__, __LINE__);
+            return e == cudaErrorMemoryAllocation ? PFGB_ERR_NOMEM : PFGB_ERR_CUDA;
+        }
     }
     return fill_twiddles<T>(c, (unsigned char *)base, off1, off2);
 }
@@ -5538,8 +5577,9 @@ static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *strea
 // the tables are given back and the transform is complete on return
 static pfgb_status fft_ctx_free(pfgb_ctx *c, pfgb_status s) {
     void *base = c->tw[0][0] ? c->tw[0][0] : c->tw[1][0];
-    if (base) cudaFreeAsync(base, c->stream);
+    if (base && c->tab_slot < 0) cudaFreeAsync(base, c->stream);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
+    if (c->tab_slot >= 0) return_table(c->tab_dev, c->tab_slot);
     if (s == PFGB_OK && e != cudaSuccess) {
         pfgb_set_error("cudaStreamSynchronize", e, __FILE__, __LINE__);
         return PFGB_ERR_CUDA;
