@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dfloat.cuh"
 #include "f32x2.cuh"
 
 namespace {
@@ -903,12 +904,12 @@ __global__ void __launch_bounds__(256) k_loss_final(const double *__restrict__ l
 
 __global__ void __launch_bounds__(256) k_sumsq_f(const float *__restrict__ g, long long n, double *__restrict__ part) {
     __shared__ double red[256];
-    double s = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const double x = g[i];
-        s += x * x;
-    }
-    red[threadIdx.x] = s;
+    // a thread's sum in double-float (in FP64, whose pipe is 64 times slower, a
+    // conversion and a multiply-add per entry took 70 us for 17M entries)
+    dfl s = {0.f, 0.f};
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        s = df_add(s, df_two_prod(g[i], g[i]));
+    red[threadIdx.x] = df_to_double(s);
     __syncthreads();
     for (int w = 128; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
@@ -918,26 +919,48 @@ __global__ void __launch_bounds__(256) k_sumsq_f(const float *__restrict__ g, lo
 }
 
 // Adam with decoupled weight decay on the float32 master weights; the
-// bfloat16 copy is refreshed.  gscale = min(1, clip / ||g||) when clip > 0.
+// bfloat16 copy is refreshed.  gscale = min(1, clip / ||g||) when clip > 0, once
+// a block (its FP64 square root and quotient in every thread took 30 us).  Bound
+// by memory, 30 bytes a weight: four weights a thread and trip.
 __global__ void __launch_bounds__(256) k_adam(float *__restrict__ w, __nv_bfloat16 *__restrict__ wb,
                                               const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                                               long long n, float lr, float b1, float b2, float eps, float wd,
                                               float bc1, float bc2, float clip, const double *__restrict__ gnorm2) {
-    float gs = 1.f;
-    if (clip > 0.f) {
-        const double nrm = sqrt(gnorm2[0]);
-        if (nrm > (double)clip) gs = (float)((double)clip / nrm);
+    __shared__ float gsh;
+    if (threadIdx.x == 0) {
+        gsh = 1.f;
+        if (clip > 0.f) {
+            const double nrm = sqrt(gnorm2[0]);
+            if (nrm > (double)clip) gsh = (float)((double)clip / nrm);
+        }
     }
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gi = g[i] * gs;
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
+    __syncthreads();
+    const float gs = gsh;
+    auto one = [&](float &wi, float g0, float &mi, float &vi) {
+        const float gi = g0 * gs;
+        mi = b1 * mi + (1.f - b1) * gi;
+        vi = b2 * vi + (1.f - b2) * gi * gi;
         const float mh = mi / bc1, vh = vi / bc2;
-        const float wi = w[i] - lr * (mh / (sqrtf(vh) + eps) + wd * w[i]);
-        w[i] = wi;
-        wb[i] = __float2bfloat16_rn(wi);
+        wi = wi - lr * (mh / (sqrtf(vh) + eps) + wd * wi);
+    };
+    const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, st = (long long)gridDim.x * blockDim.x;
+    for (long long q = i0; q < n / 4; q += st) {
+        float4 w4 = reinterpret_cast<const float4 *>(w)[q], m4 = reinterpret_cast<const float4 *>(m)[q],
+               v4 = reinterpret_cast<const float4 *>(v)[q];
+        const float4 g4 = reinterpret_cast<const float4 *>(g)[q];
+        one(w4.x, g4.x, m4.x, v4.x);
+        one(w4.y, g4.y, m4.y, v4.y);
+        one(w4.z, g4.z, m4.z, v4.z);
+        one(w4.w, g4.w, m4.w, v4.w);
+        reinterpret_cast<float4 *>(m)[q] = m4;
+        reinterpret_cast<float4 *>(v)[q] = v4;
+        reinterpret_cast<float4 *>(w)[q] = w4;
+        reinterpret_cast<__nv_bfloat162 *>(wb)[2 * q] = __floats2bfloat162_rn(w4.x, w4.y);
+        reinterpret_cast<__nv_bfloat162 *>(wb)[2 * q + 1] = __floats2bfloat162_rn(w4.z, w4.w);
+    }
+    for (long long i = n / 4 * 4 + i0; i < n; i += st) {
+        one(w[i], g[i], m[i], v[i]);
+        wb[i] = __float2bfloat16_rn(w[i]);
     }
 }
 
