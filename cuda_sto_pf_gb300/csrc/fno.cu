@@ -180,60 +180,65 @@ __global__ void __launch_bounds__(256) k_dft_z(const float *__restrict__ src, fl
 }
 
 // y forward (e^{-}) onto the corner blocks: kYJ retained ky per thread share
-// each slab value, NS slabs (channel, x) per block
+// each value, NS slabs (channel, x) per block
 // dst[r][jy][kz] = sum_y src[r][y][kz] e^{-2 pi i ky(jy) y / Y}
-// tyi[jy][y] holds the conjugate twiddles.  (One ky per thread took two shared
-// reads for four multiply-adds: 65 us at 128^3, 12 modes.)
-constexpr int kYJ = 8;
+// tyi[jy][y] holds the conjugate twiddles; they are staged in shared memory,
+// transposed, kYTab of them at a time, and read as broadcasts; the values come
+// straight from memory.  (Twiddles from the cache and slabs staged instead: the
+// warps waited for the twiddles, 107 us at 128^3, 12 modes, issue 26%; now 48.)
+constexpr int kYJ = 8, kYTab = 4096;
+__host__ __device__ constexpr int dft_y_groups(int m) { return (2 * m + kYJ - 1) / kYJ; }
+// positions staged at a time
+__host__ __device__ constexpr int dft_y_chunk(int Y, int m) {
+    const int c = kYTab / (dft_y_groups(m) * kYJ);
+    return Y < c ? Y : c;
+}
 __global__ void __launch_bounds__(256) k_dft_y(const float2 *__restrict__ src, float2 *__restrict__ dst,
                                                const float2 *__restrict__ tyi, long long nslab, int NS, int Y, int Mz,
                                                int m) {
-    extern __shared__ __align__(16) float2 smy[];
-    const int J = 2 * m, JG = (J + kYJ - 1) / kYJ;
-    float2 *slab = smy;                                          // [NS][Y][Mz]
+    extern __shared__ __align__(16) float2 smy[];                // [YC][JP]
+    const int J = 2 * m, JG = dft_y_groups(m), JP = JG * kYJ, YC = dft_y_chunk(Y, m);
     const long long r0 = (long long)blockIdx.x * NS;
-    const int ns = (int)min((long long)NS, nslab - r0);
+    const int ns = (int)min((long long)NS, nslab - r0), ntask = ns * Mz * JG;
     const float2 *s = src + r0 * Y * Mz;
-    for (int e = threadIdx.x; e < ns * Y * Mz; e += blockDim.x) slab[e] = s[e];
-    __syncthreads();
     // kz fastest, then the slab: a warp shares the group of ky and its twiddles
-    for (int e = threadIdx.x; e < ns * Mz * JG; e += blockDim.x) {
-        const int jg = e / (ns * Mz), rem = e - jg * ns * Mz;
+    for (int e0 = 0; e0 < ntask; e0 += blockDim.x) {
+        const int e = e0 + threadIdx.x;
+        const bool act = e < ntask;
+        const int jg = act ? e / (ns * Mz) : 0, rem = act ? e - jg * ns * Mz : 0;
         const int sl = rem / Mz, kz = rem - sl * Mz;
-        const float2 *a = slab + (long long)sl * Y * Mz + kz;
-        const float2 *w = tyi + (long long)jg * kYJ * Y;
-        const int nj = min(kYJ, J - jg * kYJ);
+        const float2 *a = s + (long long)sl * Y * Mz + kz;
         float re[kYJ], im[kYJ];
 #pragma unroll
         for (int j = 0; j < kYJ; ++j) re[j] = im[j] = 0.f;
-        auto add = [&](int j, float2 v, float tx, float ty) {   // e^{-}: (tx, -ty)
-            re[j] = fmaf(v.x, tx, fmaf(-v.y, -ty, re[j]));
-            im[j] = fmaf(v.x, -ty, fmaf(v.y, tx, im[j]));
-        };
-        int y = 0;
-        if (Y % 2 == 0) {   // the twiddles of two positions per read
-            for (; y < Y; y += 2) {
-                const float2 v0 = a[y * Mz], v1 = a[(y + 1) * Mz];
+        for (int yb = 0; yb < Y; yb += YC) {
+            const int ny = min(YC, Y - yb);
+            __syncthreads();
+            for (int i = threadIdx.x; i < ny * JP; i += blockDim.x) {
+                const int j = i / ny, y = i - j * ny;
+                smy[y * JP + j] = j < J ? tyi[j * Y + yb + y] : make_float2(0.f, 0.f);
+            }
+            __syncthreads();
+            if (!act) continue;
+#pragma unroll 4
+            for (int y = 0; y < ny; ++y) {
+                const float2 v = a[(yb + y) * Mz];
+                const float4 *w = reinterpret_cast<const float4 *>(smy + y * JP + jg * kYJ);
 #pragma unroll
-                for (int j = 0; j < kYJ; ++j) {
-                    const float4 t = __ldg(reinterpret_cast<const float4 *>(w + (j < nj ? j : 0) * Y + y));
-                    add(j, v0, t.x, t.y);
-                    add(j, v1, t.z, t.w);
+                for (int q = 0; q < kYJ / 2; ++q) {              // e^{-}: (tx, -ty)
+                    const float4 t = w[q];
+                    re[2 * q] = fmaf(v.x, t.x, fmaf(-v.y, -t.y, re[2 * q]));
+                    im[2 * q] = fmaf(v.x, -t.y, fmaf(v.y, t.x, im[2 * q]));
+                    re[2 * q + 1] = fmaf(v.x, t.z, fmaf(-v.y, -t.w, re[2 * q + 1]));
+                    im[2 * q + 1] = fmaf(v.x, -t.w, fmaf(v.y, t.z, im[2 * q + 1]));
                 }
             }
         }
-        for (; y < Y; ++y) {
-            const float2 v = a[y * Mz];
-#pragma unroll
-            for (int j = 0; j < kYJ; ++j) {
-                const float2 t = __ldg(w + (j < nj ? j : 0) * Y + y);
-                add(j, v, t.x, t.y);
-            }
-        }
+        if (!act) continue;
         float2 *d = dst + (r0 + sl) * J * Mz + kz;
 #pragma unroll
         for (int j = 0; j < kYJ; ++j)
-            if (j < nj) d[(jg * kYJ + j) * Mz] = make_float2(re[j], im[j]);
+            if (jg * kYJ + j < J) d[(jg * kYJ + j) * Mz] = make_float2(re[j], im[j]);
     }
 }
 
@@ -1154,14 +1159,15 @@ pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, f
     k_dft_z<<<(unsigned)((lines + LB - 1) / LB), 256, sz, f->stream>>>(src, f->A, f->fz, lines, f->Z, f->Mz, LB,
                                                                        w0, w1);
     FNO_CHECK(check_launch("dft_z"));
-    // slabs per block: about 256 tasks within 96 KB, one at least
-    const size_t slab = sizeof(float2) * (size_t)f->Y * f->Mz;
-    const int tasks = f->Mz * ((2 * f->m + kYJ - 1) / kYJ);
+    // slabs per block: about 256 tasks, fewer where the grid would leave SMs
+    // without two blocks
+    const int tasks = f->Mz * dft_y_groups(f->m);
     const long long nslab = (long long)kW * f->X;
-    const int NS = (int)std::max<long long>(1, std::min<long long>(256 / std::max(1, tasks), (96 * 1024) / (long long)slab));
-    FNO_CHECK(smem_opt_in(k_dft_y, kSmemCap));
-    k_dft_y<<<(unsigned)((nslab + NS - 1) / NS), 256, slab * NS, f->stream>>>(f->A, f->B, f->tyi, nslab, NS, f->Y,
-                                                                              f->Mz, f->m);
+    const int NS = (int)std::max<long long>(1, std::min<long long>(256 / std::max(1, tasks), nslab / 304));
+    const int ny_thr = std::min(256, (NS * tasks + 31) / 32 * 32);
+    const size_t sy = sizeof(float2) * (size_t)dft_y_chunk(f->Y, f->m) * dft_y_groups(f->m) * kYJ;
+    k_dft_y<<<(unsigned)((nslab + NS - 1) / NS), ny_thr, sy, f->stream>>>(f->A, f->B, f->tyi, nslab, NS, f->Y, f->Mz,
+                                                                         f->m);
     FNO_CHECK(check_launch("dft_y"));
     const size_t sx = sizeof(float2) * (size_t)f->X * kXJ;
     FNO_CHECK(smem_opt_in(k_dft_x, sx));

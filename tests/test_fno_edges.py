@@ -1,7 +1,7 @@
 """The learned start's kernels at the edges of their tiles, against the float64
 oracle: an odd z axis (cells taken one by one, not in pairs), a last tile of
 cells that is partly empty, a z axis one position past a staged chunk, an odd
-number of modes.  Tolerances as on the regular shapes (test_fno.py): FP32 sums
+number of modes, a y axis of two chunks of twiddles.  Tolerances as on the regular shapes (test_fno.py): FP32 sums
 forward, central differences for gradients."""
 import numpy as np
 import pytest
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape,modes,layers", [((5, 6, 9), 2, 2), ((4, 3, 65), 1, 1), ((10, 11, 64), 5, 2),
-                                                ((2, 2, 2), 1, 1)], ids=str)
+                                                ((2, 2, 2), 1, 1), ((2, 520, 3), 1, 1)], ids=str)
 def test_forward_and_gradients_at_tile_edges(capi, shape, modes, layers):
     import torch
     rng = np.random.default_rng(31)
