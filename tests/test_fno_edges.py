@@ -1,8 +1,9 @@
 """The learned start's kernels at the edges of their tiles, against the float64
 oracle: an odd z axis (cells taken one by one, not in pairs), a last tile of
 cells that is partly empty, a z axis one position past a staged chunk, an odd
-number of modes, a y axis of two chunks of twiddles.  Tolerances as on the regular shapes (test_fno.py): FP32 sums
-forward, central differences for gradients."""
+number of modes, a y axis of two chunks of twiddles.  Tolerances as on the
+regular shapes (test_fno.py): FP32 sums forward, central differences for
+gradients."""
 import numpy as np
 import pytest
 
