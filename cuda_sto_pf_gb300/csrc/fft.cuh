@@ -29,6 +29,8 @@
 
 #define PFGB_MAX_STAGES 16
 #define PFGB_MAX_N 1024
+#define PFGB_LINE_THREADS 256   // threads of a generic pass's block at most
+#define PFGB_DIRECT_SUMS 8      // sums of a direct stage that a thread holds
 
 // Division by a run-time constant d via a multiply-high (round-up method):
 // valid for every 32-bit dividend.
@@ -102,13 +104,18 @@ static inline void pfgb_best_radices(int q, int lim, std::vector<int> &cur, std:
     }
 }
 
-// host: the stages of an n-point line.  A factor 41 goes first (Rader's
-// convolution), then the other primes above 13 as direct sums, then the
-// smooth part with radices up to 16, the largest first.
-static inline void pfgb_make_plan(int n, AxisPlan *p) {
+// host: the stages of an n-point line, false if the kernels could not run
+// them.  A factor 41 goes first (Rader's convolution), then the other primes
+// above 13 as direct sums, then the smooth part with radices up to 16, the
+// largest first.  The last butterfly stage holds a whole line, one butterfly
+// per thread: where the smallest radix leaves it more than a block's threads
+// (n / R > 256: 598 = 23 x 13 x 2), the largest smooth radix goes last, and
+// where that is still too few points (n = 514, 578, 771, ...), a direct stage does,
+// which holds eight sums per thread and so any n up to 2,048.
+static inline bool pfgb_make_plan(int n, AxisPlan *p) {
     p->n = n;
     p->nst = 0;
-    std::vector<std::pair<int, int>> rad;   // radix, kind
+    std::vector<std::pair<int, int>> rad, dir;   // radix, kind
     int q = n;
     if (q % 41 == 0) { rad.push_back({41, 1}); q /= 41; }
     for (int f = 17; f <= q; ++f)
@@ -116,12 +123,18 @@ static inline void pfgb_make_plan(int n, AxisPlan *p) {
             bool prime = true;
             for (int d = 2; d * d <= f; ++d) prime = prime && f % d;
             if (!prime) break;
-            rad.push_back({f, 2});
+            dir.push_back({f, 2});
             q /= f;
         }
     std::vector<int> cur, best;
     if (q > 1) pfgb_best_radices(q, 16, cur, best);
+    auto fits = [&] { return best.empty() || n / best.back() <= PFGB_LINE_THREADS; };
+    if (!fits()) std::reverse(best.begin(), best.end());
+    const bool direct_last = !fits();
+    if (!direct_last) rad.insert(rad.end(), dir.begin(), dir.end());
     for (int r : best) rad.push_back({r, 0});
+    if (direct_last) rad.insert(rad.end(), dir.begin(), dir.end());
+    if (rad.size() > PFGB_MAX_STAGES) return false;
     int B = n;
     for (auto &rk : rad) {
         StagePlan &st = p->st[p->nst++];
@@ -133,6 +146,13 @@ static inline void pfgb_make_plan(int n, AxisPlan *p) {
         st.fR.init((unsigned)st.R);
         B = st.m;
     }
+    for (int i = 0; i < p->nst; ++i) {
+        const StagePlan &st = p->st[i];
+        if (st.kind == 1 && i > 0) return false;
+        if (st.kind == 2 && n > PFGB_LINE_THREADS * PFGB_DIRECT_SUMS) return false;
+        if (st.kind == 0 && i == p->nst - 1 && n / st.R > PFGB_LINE_THREADS) return false;
+    }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -260,9 +280,11 @@ __device__ __forceinline__ void bfly6(cplx_t<T> *v) {
 // (line l, position p) at buf[p * PS + l * LS] (PS = L, LS = 1 for strided
 // axes; PS = 1, LS odd for z rows).  The lanes of a warp walk the lines, so
 // every access is contiguous in l (or has the odd stride LS): no bank
-// conflicts at any stage, and the index arithmetic is per butterfly of up to
-// 16 points.  A line makes one trip through shared memory per stage: two
-// stages up to 256 points, three up to 1024.
+// conflicts at any stage but the last, whose chunks can be narrower than a
+// warp, and the index arithmetic is per butterfly of up to 16 points.  A line
+// makes one trip through shared memory per stage: at most two stages for most
+// lengths up to 256 (125, 200, 243 and 13 others take three), at most three up
+// to 1024 (625 and 875 take four).
 //
 // The transform is a device function of its own translation unit
 // (fftline.cu), one per precision and direction: every pass kernel calls the
@@ -309,12 +331,16 @@ static inline int pfgb_line_threads(const AxisPlan &p, int L) {
         int per = 1;                                   // work items of a thread and trip
         long long items = (long long)L * nb;
         if (p.st[s].kind == 1) items *= 8;             // eight lanes per butterfly
-        else if (p.st[s].kind == 2) { items = (long long)L * p.n; per = 8; least = std::max(least, (p.n + 7) / 8); }
-        else if (s == p.nst - 1) least = std::max(least, nb);
-        const long long trips = (items + 256 * per - 1) / (256 * per);
+        else if (p.st[s].kind == 2) {
+            items = (long long)L * p.n;
+            per = PFGB_DIRECT_SUMS;
+            least = std::max(least, (p.n + per - 1) / per);
+        } else if (s == p.nst - 1) least = std::max(least, nb);
+        const long long trips = (items + PFGB_LINE_THREADS * per - 1) / (PFGB_LINE_THREADS * per);
         t = std::max(t, (int)((items + trips * per - 1) / (trips * per)));
     }
-    return std::min(256, (std::max(t, least) + 31) / 32 * 32);
+    // (pfgb_make_plan keeps `least` within a block)
+    return std::min(PFGB_LINE_THREADS, (std::max(t, least) + 31) / 32 * 32);
 }
 
 // blocks per SM that the pass kernels' registers allow for (80 or 128 per

@@ -177,7 +177,9 @@ __device__ __noinline__ void stage_mid(LineTile t, int nb, int B, int m, int tws
 }
 
 // the last stage: a chunk of lines at a time, one butterfly per thread, whose
-// points are all in registers before the block writes them back
+// points are all in registers before the block writes them back.  A block has
+// a thread for every butterfly of a line (pfgb_make_plan, pfgb_line_threads),
+// so that a chunk holds at least one line.
 template <typename T, int DIR, int R>
 __device__ __noinline__ void stage_last(LineTile t, const AxisPlan *plan, int nb) {
     using T2 = cplx_t<T>;
@@ -212,7 +214,7 @@ __device__ __noinline__ void stage_last(LineTile t, const AxisPlan *plan, int nb
 template <typename T, int DIR>
 __device__ __noinline__ void stage_direct(LineTile t, const AxisPlan *plan, int s) {
     using T2 = cplx_t<T>;
-    constexpr int H = 8;
+    constexpr int H = PFGB_DIRECT_SUMS;
     const AxisPlan &p = *plan;
     const int n = p.n, R = p.st[s].R, B = p.st[s].B, m = p.st[s].m, twst = n / B;
     const FastDiv fm = p.st[s].fm;

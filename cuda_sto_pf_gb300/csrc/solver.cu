@@ -173,6 +173,18 @@ struct pfgb_ctx {
     bool tc_y = false, tc_x = false, tc_z = false;   // passes that use it
 };
 
+// the line transforms of the grid's axes
+[[maybe_unused]] static pfgb_status make_plans(pfgb_ctx *c) {
+    const int n[3] = {c->g.Nx, c->g.Ny, c->g.Nz};
+    AxisPlan *pl[3] = {&c->plx, &c->ply, &c->plz};
+    for (int a = 0; a < 3; ++a)
+        if (!pfgb_make_plan(n[a], pl[a])) {
+            pfgb_set_error_msg("no line transform for an axis of %d points", n[a]);
+            return PFGB_ERR_UNSUPPORTED;
+        }
+    return PFGB_OK;
+}
+
 static KTab ktab(const pfgb_ctx *c) {
     return KTab{c->kx, c->ky, c->kz, c->kf, c->kf + c->g.Nx, c->kf + c->g.Nx + c->g.Ny, c->kq, c->kq + c->g.Nx,
                 c->kq + c->g.Nx + c->g.Ny, c->mx, c->my, c->mz};
@@ -4856,9 +4868,10 @@ pfgb_status pfgb_create(const pfgb_params *pin, int device, pfgb_ctx **out) {
     c->g.N = (long long)pin->Nx * pin->Ny * pin->Nz;
     c->g.Nk = (long long)pin->Nx * pin->Ny * c->g.NzC;
     c->g.keep_all();   // make_ktab sets the dealias box
-    pfgb_make_plan(pin->Nx, &c->plx);
-    pfgb_make_plan(pin->Ny, &c->ply);
-    pfgb_make_plan(pin->Nz, &c->plz);
+    if (pfgb_status ps = make_plans(c)) {
+        delete c;
+        return ps;
+    }
     {
         // the strided-axis kernels copy column pairs with 16-byte accesses
         const bool e32 = pin->elastic_precision == PFGB_PREC_FP32, evenc = ((pin->Nz / 2 + 1) % 2) == 0;
@@ -5559,9 +5572,7 @@ static pfgb_status fft_ctx_init(pfgb_ctx *c, int Nx, int Ny, int Nz, void *strea
     c->g.N = (long long)Nx * Ny * Nz;
     c->g.Nk = (long long)Nx * Ny * c->g.NzC;
     c->g.keep_all();
-    pfgb_make_plan(Nx, &c->plx);
-    pfgb_make_plan(Ny, &c->ply);
-    pfgb_make_plan(Nz, &c->plz);
+    TRY(make_plans(c));
     const size_t off1 = round256(sizeof(cplx_t<T>) * (size_t)Nx), off2 = off1 + round256(sizeof(cplx_t<T>) * (size_t)Ny);
     void *base = take_table(&c->tab_dev, &c->tab_slot);
     if (!base) {
@@ -5752,9 +5763,7 @@ static pfgb_status fft_r2c_noalloc(int Nx, int Ny, int Nz, const T *in, cplx_t<T
     c.g.N = (long long)Nx * Ny * Nz;
     c.g.Nk = (long long)Nx * Ny * c.g.NzC;
     c.g.keep_all();
-    pfgb_make_plan(Nx, &c.plx);
-    pfgb_make_plan(Ny, &c.ply);
-    pfgb_make_plan(Nz, &c.plz);
+    TRY(make_plans(&c));
     TRY(fill_twiddles<T>(&c, base, off1, off2));
     pfgb_status s = fft_r2c_impl<T>(&c, in, out);
     return s;
