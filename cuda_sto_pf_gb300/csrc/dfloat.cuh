@@ -61,6 +61,47 @@ __device__ __forceinline__ dfl df_from_double(double v) {
     return {hi, (float)(v - (double)hi)};
 }
 
+// ---------------------------------------------------------------------------
+// A sum of floats, or of their exact products, in more than a double's 53 bits
+// on the FP32 pipe: h + m + l, where m holds the rounding errors of h and l
+// those of m (cascaded compensated summation, Ogita, Rump and Oishi, 2005: as
+// if summed with 72 bits), and in x what float arithmetic has no room for (sums
+// that could overflow, products whose error term would underflow, infinities and
+// NaN), in FP64 as a plain double sum has it.
+// ---------------------------------------------------------------------------
+struct fsum { float h, m, l; double x; };
+
+__device__ __forceinline__ fsum fs_zero() { return {0.f, 0.f, 0.f, 0.0}; }
+// v below 2^-24 of what the sum holds (an error term), added to m
+__device__ __forceinline__ void fs_add_low(fsum &s, float v) {
+    const dfl u = df_two_sum(s.m, v);
+    s.m = u.hi;
+    s.l += u.lo;
+}
+__device__ __forceinline__ void fs_add_in_range(fsum &s, float v) {
+    const dfl t = df_two_sum(s.h, v);
+    s.h = t.hi;
+    fs_add_low(s, t.lo);
+}
+__device__ __forceinline__ void fs_add(fsum &s, float v) {
+    if (fabsf(v) < 0x1p100f) fs_add_in_range(s, v);
+    else s.x += (double)v;
+}
+// s += v^2: the two-product is exact for 2^-50 < |v| < 2^50 and for 0
+__device__ __forceinline__ void fs_add_square(fsum &s, float v) {
+    const float a = fabsf(v);
+    if ((a > 0x1p-50f && a < 0x1p50f) || a == 0.f) {
+        const dfl p = df_two_prod(v, v);
+        fs_add_in_range(s, p.hi);
+        fs_add_low(s, p.lo);
+    } else {
+        s.x += (double)v * (double)v;
+    }
+}
+__device__ __forceinline__ double fs_to_double(const fsum &s) {
+    return s.x + ((double)s.h + ((double)s.m + (double)s.l));
+}
+
 // e^w for -40 <= w <= 0 by Tang's table-driven method (ACM TOMS 15, 1989):
 // w = N ln2/64 + r (N = 64 k + j, |r| <= ln2/128),
 // e^r = 1 + r + r^2/2 + (r^3/6 + r^4/24 + r^5/120) with the bracket in

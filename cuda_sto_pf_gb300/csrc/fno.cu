@@ -936,12 +936,13 @@ __global__ void __launch_bounds__(256) k_loss_final(const double *__restrict__ l
 
 __global__ void __launch_bounds__(256) k_sumsq_f(const float *__restrict__ g, long long n, double *__restrict__ part) {
     __shared__ double red[256];
-    // a thread's sum in double-float (in FP64, whose pipe is 64 times slower, a
-    // conversion and a multiply-add per entry took 70 us for 17M entries)
-    dfl s = {0.f, 0.f};
+    // a thread's sum on the FP32 pipe, to more bits than a double's and over its
+    // range (in FP64, whose pipe is 64 times slower, a conversion and a multiply-add
+    // per entry take 70 us for 17M entries)
+    fsum s = fs_zero();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        s = df_add(s, df_two_prod(g[i], g[i]));
-    red[threadIdx.x] = df_to_double(s);
+        fs_add_square(s, g[i]);
+    red[threadIdx.x] = fs_to_double(s);
     __syncthreads();
     for (int w = 128; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
