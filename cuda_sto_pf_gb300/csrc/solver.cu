@@ -222,9 +222,10 @@ struct ProfScope {
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
-// A tile of the generic engine: at most 72 KiB, three blocks per SM.  Tiles
-// narrower than 32 bytes of columns leave part of every DRAM sector unused:
-// long axes take that width at up to kSmemWide instead.
+// A tile of the generic engine: 72 KiB, so that three blocks fit on an SM.
+// Tiles narrower than 32 bytes of columns leave part of every DRAM sector
+// unused: long axes take that width at up to kSmemWide instead, one or two
+// blocks per SM.
 static const size_t kSmemBudget = 72 * 1024;
 static const size_t kSmemWide = 220 * 1024;
 
@@ -470,10 +471,12 @@ static int tuned_tk(pfgb_ctx *c, int axis, const AxisPlan &pl, const Op &op, int
                 for (int a = 0; a < NIN; ++a) io[i].in[a] = (const T2 *)ts.sc[i]->p[a];
                 for (int b = 0; b < NOUT; ++b) io[i].out[b] = (T2 *)ts.sc[i]->p[NIN + b];
             }
-            for (int tk = 1; tk <= 32; tk <<= 1) {
-                if (tk > 1 && tk / 2 >= c->g.NzK) break;
+            // powers of two, and the rule's own width, which can be any
+            for (int i = 0; i <= 6; ++i) {
+                const int tk = i < 6 ? 1 << i : rule;
+                if (i < 6 && (tk == rule || (tk > 1 && tk / 2 >= c->g.NzK))) continue;
                 const size_t smem = axis_tile_bytes<T2>(n, NW, tk);
-                if (smem > kSmemWide || allow_smem(kern, smem) != cudaSuccess) break;
+                if (smem > kSmemWide || allow_smem(kern, smem) != cudaSuccess) continue;
                 const dim3 grid((c->g.NzK + tk - 1) / tk, gy, nz);
                 const T2 *tw = twp<T>(c, axis == 1 ? 1 : 0);
                 const TileDiv ft = tile_div(tk, Op::kInplace ? 1 : NIN, Op::kInplace ? 1 : NOUT);

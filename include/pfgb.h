@@ -156,9 +156,11 @@ typedef struct pfgb_params {
        and keeps the fastest for the life of the process: 1 the columns per
        block of the x and y passes (timed as themselves), 2 the rows per
        block of the z passes (timed through a copy op with the same field
-       counts); pfgb_tile_report lists them.  0 (default): the fixed rule,
-       the largest tile within 112 KiB of shared memory.  No counterpart key
-       in the reference. */
+       counts); pfgb_tile_report lists them.  The candidates are powers of
+       two and the rule's own width.  0 (default): the fixed rule, the
+       largest tile within 72 KiB of shared memory (long axes: 32 bytes of
+       columns, within 220 KiB), smaller where the grid would leave SMs
+       without two blocks.  No counterpart key in the reference. */
     int32_t fft_autotune;
     int32_t pad_fft;
     double elastic_residual_tolerance;
