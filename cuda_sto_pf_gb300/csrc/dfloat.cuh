@@ -62,6 +62,35 @@ __device__ __forceinline__ dfl df_from_double(double v) {
 }
 
 // ---------------------------------------------------------------------------
+// Values that end as floats: the float that the same expression in FP64 rounds
+// to, found in double-float arithmetic wherever it decides it (Ziv, "Fast
+// Evaluation of Elementary Mathematical Functions with Correctly Rounded Last
+// Bit", ACM TOMS 17, 1991).  The double-float value is f + c; if everything
+// within 2^-40 of it rounds to one float, so does the double value, which lies
+// within 2^-42.  The rest, one value in some 2^15, and what leaves the range that
+// this holds for, is the caller's to compute in FP64.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool df_rounds(float f, float c, float *out) {
+    const float err = fabsf(f) * 0x1p-40f;
+    const float lo = f + (c - err), hi = f + (c + err);
+    *out = lo;
+    return lo == hi && fabsf(f) > 0x1p-80f && fabsf(f) < 0x1p100f;
+}
+// float(a b) for |a b| in (2^-80, 2^100)
+__device__ __forceinline__ bool df_round_product(dfl a, dfl b, float *out) {
+    const dfl p = df_mul(a, b);
+    return df_rounds(p.hi, p.lo, out);
+}
+// float(num / (1 + m k2)) for 1 + m k2 in [1/2, 2^60): one correction of the
+// float quotient
+__device__ __forceinline__ bool df_round_damped(dfl num, dfl m, dfl k2, float *out) {
+    const dfl den = df_add_f(df_mul(m, k2), 1.0f);
+    const float q = 1.0f / den.hi, f = num.hi * q;
+    const float e = fmaf(-f, den.hi, num.hi) + fmaf(-f, den.lo, num.lo);
+    return df_rounds(f, e * q, out) && den.hi >= 0.5f && den.hi < 0x1p60f && fabsf(m.hi) < 0x1p60f && k2.hi < 0x1p60f;
+}
+
+// ---------------------------------------------------------------------------
 // A sum of floats, or of their exact products, in more than a double's 53 bits
 // on the FP32 pipe: h + m + l, where m holds the rounding errors of h and l
 // those of m (cascaded compensated summation, Ogita, Rump and Oishi, 2005: as
