@@ -101,7 +101,7 @@ __device__ __forceinline__ bool df_round_damped(dfl num, dfl m, dfl k2, float *o
 struct fsum { float h, m, l; double x; };
 
 __device__ __forceinline__ fsum fs_zero() { return {0.f, 0.f, 0.f, 0.0}; }
-// v below 2^-24 of what the sum holds (an error term), added to m
+// s += v at the level of m (an error term of what h takes)
 __device__ __forceinline__ void fs_add_low(fsum &s, float v) {
     const dfl u = df_two_sum(s.m, v);
     s.m = u.hi;
@@ -113,19 +113,30 @@ __device__ __forceinline__ void fs_add_in_range(fsum &s, float v) {
     fs_add_low(s, t.lo);
 }
 __device__ __forceinline__ void fs_add(fsum &s, float v) {
-    if (fabsf(v) < 0x1p100f) fs_add_in_range(s, v);
+    if (fabsf(v) < 0x1p96f) fs_add_in_range(s, v);   // 2^31 of them stay below a float's range
     else s.x += (double)v;
 }
-// s += v^2: the two-product is exact for 2^-50 < |v| < 2^50 and for 0
+// s += v^2: the two-product is exact for 2^-46 < |v| < 2^48 and for 0
 __device__ __forceinline__ void fs_add_square(fsum &s, float v) {
     const float a = fabsf(v);
-    if ((a > 0x1p-50f && a < 0x1p50f) || a == 0.f) {
+    if ((a > 0x1p-46f && a < 0x1p48f) || a == 0.f) {
         const dfl p = df_two_prod(v, v);
         fs_add_in_range(s, p.hi);
         fs_add_low(s, p.lo);
     } else {
         s.x += (double)v * (double)v;
     }
+}
+__device__ __forceinline__ void fs_merge(fsum &s, const fsum &b) {
+    fs_add_in_range(s, b.h);
+    fs_add_low(s, b.m);
+    s.l += b.l;
+    if (__double_as_longlong(b.x) != 0) s.x += b.x;   // (a branch, not an FP64 addition)
+}
+__device__ __forceinline__ fsum fs_shfl_down(const fsum &s, int o) {
+    const unsigned all = 0xffffffffu;
+    return {__shfl_down_sync(all, s.h, o), __shfl_down_sync(all, s.m, o), __shfl_down_sync(all, s.l, o),
+            __shfl_down_sync(all, s.x, o)};
 }
 __device__ __forceinline__ double fs_to_double(const fsum &s) {
     return s.x + ((double)s.h + ((double)s.m + (double)s.l));

@@ -747,34 +747,30 @@ struct AccSum2 {
         return {__shfl_down_sync(0xffffffffu, x.a, o), __shfl_down_sync(0xffffffffu, x.b, o)};
     }
 };
-// the same sums in an FP32 pass: double-float per thread and block (the FP64
-// pipe takes a conversion and an addition per cell otherwise)
-struct AccDf1 {
+// the same sums of floats in an FP32 pass, to more bits than a double's on the
+// FP32 pipe (the FP64 pipe takes a conversion and an addition per cell otherwise)
+struct AccFs1 {
     static constexpr bool kActive = true;
-    dfl s;
-    __device__ static AccDf1 identity() { return {dfl{0.f, 0.f}}; }
-    __device__ static AccDf1 combine(AccDf1 a, AccDf1 b) { return {df_add(a.s, b.s)}; }
-    __device__ static AccDf1 shfl_down(AccDf1 a, int o) {
-        return {dfl{__shfl_down_sync(0xffffffffu, a.s.hi, o), __shfl_down_sync(0xffffffffu, a.s.lo, o)}};
-    }
+    fsum s;
+    __device__ static AccFs1 identity() { return {fs_zero()}; }
+    __device__ static AccFs1 combine(AccFs1 a, const AccFs1 &b) { fs_merge(a.s, b.s); return a; }
+    __device__ static AccFs1 shfl_down(const AccFs1 &a, int o) { return {fs_shfl_down(a.s, o)}; }
 };
-struct AccDf2 {
+struct AccFs2 {
     static constexpr bool kActive = true;
-    dfl a, b;
-    __device__ static AccDf2 identity() { return {dfl{0.f, 0.f}, dfl{0.f, 0.f}}; }
-    __device__ static AccDf2 combine(AccDf2 x, AccDf2 y) { return {df_add(x.a, y.a), df_add(x.b, y.b)}; }
-    __device__ static AccDf2 shfl_down(AccDf2 x, int o) {
-        return {AccDf1::shfl_down(AccDf1{x.a}, o).s, AccDf1::shfl_down(AccDf1{x.b}, o).s};
-    }
+    fsum a, b;
+    __device__ static AccFs2 identity() { return {fs_zero(), fs_zero()}; }
+    __device__ static AccFs2 combine(AccFs2 x, const AccFs2 &y) { fs_merge(x.a, y.a); fs_merge(x.b, y.b); return x; }
+    __device__ static AccFs2 shfl_down(const AccFs2 &x, int o) { return {fs_shfl_down(x.a, o), fs_shfl_down(x.b, o)}; }
 };
 __device__ __forceinline__ void acc_add(double &s, double v) { s += v; }
-__device__ __forceinline__ void acc_add(dfl &s, float v) { s = df_add_f(s, v); }
+__device__ __forceinline__ void acc_add(fsum &s, float v) { fs_add(s, v); }
 __device__ __forceinline__ AccSum1 acc_out(const AccSum1 &a) { return a; }
-__device__ __forceinline__ AccSum1 acc_out(const AccDf1 &a) { return {df_to_double(a.s)}; }
+__device__ __forceinline__ AccSum1 acc_out(const AccFs1 &a) { return {fs_to_double(a.s)}; }
 __device__ __forceinline__ AccSum2 acc_out(const AccSum2 &a) { return a; }
-__device__ __forceinline__ AccSum2 acc_out(const AccDf2 &a) { return {df_to_double(a.a), df_to_double(a.b)}; }
-template <typename T> using AccSum1Of = std::conditional_t<sizeof(T) == 8, AccSum1, AccDf1>;
-template <typename T> using AccSum2Of = std::conditional_t<sizeof(T) == 8, AccSum2, AccDf2>;
+__device__ __forceinline__ AccSum2 acc_out(const AccFs2 &a) { return {fs_to_double(a.a), fs_to_double(a.b)}; }
+template <typename T> using AccSum1Of = std::conditional_t<sizeof(T) == 8, AccSum1, AccFs1>;
+template <typename T> using AccSum2Of = std::conditional_t<sizeof(T) == 8, AccSum2, AccFs2>;
 
 // zero-mode statistics: min, max of Y*, and the Taylor moments
 // M_p = sum (1-h) sigma^{(p)}(Y*) (M_0 also + h v_B), p = 0..4

@@ -1,0 +1,85 @@
+"""Sums of floats and of their squares on the FP32 pipe (fsum, dfloat.cuh) against
+exactly rounded sums: no further off than float64 sums are, over a float's whole
+range."""
+import ctypes
+import math
+import subprocess
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one block; its threads' sums are merged as the solver's block reductions do
+SRC = r"""
+#include "dfloat.cuh"
+template <bool SQ> __global__ void k_sum(const float *v, int n, double *out) {
+    __shared__ fsum red[32];
+    fsum s = fs_zero();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) SQ ? fs_add_square(s, v[i]) : fs_add(s, v[i]);
+    for (int o = 16; o > 0; o >>= 1) fs_merge(s, fs_shfl_down(s, o));
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)blockDim.x / 32; ++w) fs_merge(s, red[w]);
+        out[0] = fs_to_double(s);
+    }
+}
+extern "C" int run(int square, const float *v, int n, double *out) {
+    if (square) k_sum<true><<<1, 256>>>(v, n, out);
+    else k_sum<false><<<1, 256>>>(v, n, out);
+    return (int)cudaDeviceSynchronize();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    from cuda_sto_pf_gb300 import build
+    d = tmp_path_factory.mktemp("fs")
+    (d / "fs.cu").write_text(SRC)
+    subprocess.run([build.NVCC, *build.NVCC_FLAGS, "-I", build.CSRC, "-shared", "-o", str(d / "fs.so"), str(d / "fs.cu")],
+                   check=True)
+    return ctypes.CDLL(str(d / "fs.so"))
+
+
+def _sum(lib, v, square):
+    import torch
+    d = torch.from_numpy(np.ascontiguousarray(v, dtype=np.float32)).cuda()
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.run(int(square), ctypes.c_void_p(d.data_ptr()), v.size, ctypes.c_void_p(out.data_ptr())) == 0
+    return out.item()
+
+
+def _values(kind, n):
+    rng = np.random.default_rng(n)
+    u = rng.uniform(-1.0, 1.0, n)
+    return {"near": np.abs(u) + 0.25, "signed": u, "wide": u * 10.0 ** rng.uniform(-12, 12, n),
+            "small": u * 1e-24, "tiny": u * 1e-38, "large": np.abs(u) * 1e30, "huge": np.abs(u) * 3e38,
+            "zeros": 0.0 * u, "mixed": u * 10.0 ** rng.uniform(-37, 38, n)}[kind].astype(np.float32)
+
+
+@pytest.mark.parametrize("square", [False, True])
+@pytest.mark.parametrize("n", [1, 255, 100003])
+@pytest.mark.parametrize("kind", ["near", "signed", "wide", "small", "tiny", "large", "huge", "zeros", "mixed"])
+def test_sums_hold_float64_precision(lib, kind, n, square):
+    """Within 2^-53 of the sum of magnitudes for each rounding to float64: three in
+    the final conversion (and the compensated sum's own error, below one), and
+    where values are beyond its range, a thread's terms with their squares and
+    twelve merges, as in a plain float64 sum."""
+    v = _values(kind, n)
+    a = np.abs(v.astype(np.float64))
+    t = (v.astype(np.float64) ** 2 if square else v.astype(np.float64)).tolist()
+    beyond = ((a != 0) & ((a <= 2.0 ** -46) | (a >= 2.0 ** 48))).any() if square else (a >= 2.0 ** 96).any()
+    roundings = 4 + (math.ceil(n / 256) + 13 if beyond else 0)
+    assert abs(_sum(lib, v, square) - math.fsum(t)) <= 2.0 ** -53 * roundings * math.fsum(map(abs, t))
+
+
+@pytest.mark.parametrize("square", [False, True])
+def test_infinities_and_nan_reach_the_sum(lib, square):
+    v = np.ones(300, dtype=np.float32)
+    v[200] = np.inf
+    assert _sum(lib, v, square) == math.inf
+    v[17] = np.nan
+    assert math.isnan(_sum(lib, v, square))
