@@ -127,6 +127,13 @@ __device__ __forceinline__ void fs_add_square(fsum &s, float v) {
         s.x += (double)v * (double)v;
     }
 }
+// s += (p - q)^2, where the difference is a float (it is for values within a factor
+// of two), and in FP64 where it is not
+__device__ __forceinline__ void fs_add_square_diff(fsum &s, float p, float q) {
+    const dfl d = df_two_sum(p, -q);
+    if (d.lo == 0.f) fs_add_square(s, d.hi);
+    else s.x += ((double)p - (double)q) * ((double)p - (double)q);
+}
 __device__ __forceinline__ void fs_merge(fsum &s, const fsum &b) {
     fs_add_in_range(s, b.h);
     fs_add_low(s, b.m);

@@ -765,6 +765,10 @@ struct AccFs2 {
 };
 __device__ __forceinline__ void acc_add(double &s, double v) { s += v; }
 __device__ __forceinline__ void acc_add(fsum &s, float v) { fs_add(s, v); }
+__device__ __forceinline__ void acc_add_square(double &s, double v) { s += v * v; }
+__device__ __forceinline__ void acc_add_square(fsum &s, float v) { fs_add_square(s, v); }
+__device__ __forceinline__ void acc_add_square_diff(double &s, double p, double q) { s += (p - q) * (p - q); }
+__device__ __forceinline__ void acc_add_square_diff(fsum &s, float p, float q) { fs_add_square_diff(s, p, q); }
 __device__ __forceinline__ AccSum1 acc_out(const AccSum1 &a) { return a; }
 __device__ __forceinline__ AccSum1 acc_out(const AccFs1 &a) { return {fs_to_double(a.s)}; }
 __device__ __forceinline__ AccSum2 acc_out(const AccSum2 &a) { return a; }
@@ -3852,34 +3856,13 @@ struct AccMinE {
     }
 };
 
-// the cell's terms in the arithmetic R: double for FP64 fields, double-float for
-// FP32 fields (per cell in FP64: 163 us at 96^3; in double-float 90 us)
-__device__ __forceinline__ double w_const(double v, double) { return v; }
-__device__ __forceinline__ dfl w_const(double v, dfl) { return df_from_double(v); }
-__device__ __forceinline__ double w_diff(double a, double b) { return a - b; }
-__device__ __forceinline__ dfl w_diff(float a, float b) { return df_two_sum(a, -b); }
-__device__ __forceinline__ double w_add(double a, double b) { return a + b; }
-__device__ __forceinline__ dfl w_add(dfl a, dfl b) { return df_add(a, b); }
-__device__ __forceinline__ double w_mul(double a, double b) { return a * b; }
-__device__ __forceinline__ dfl w_mul(dfl a, dfl b) { return df_mul(a, b); }
-__device__ __forceinline__ double w_of(double v, double) { return v; }
-__device__ __forceinline__ dfl w_of(float v, dfl) { return {v, 0.f}; }
-__device__ __forceinline__ double w_round(double v, double) { return v; }
-__device__ __forceinline__ float w_round(dfl v, float) { return v.hi; }
-__device__ __forceinline__ double w_out(double v) { return v; }
-__device__ __forceinline__ double w_out(dfl v) { return df_to_double(v); }
-
+// (in FP64 per cell; 163 us at 96^3, bound by the FP64 pipe)
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *phi, double g0, int chem, AccMinE *part) {
-    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
-    R mh = w_const(0.0, R{}), grad = mh, dw = mh, gel = mh, gelh = mh, ch = mh;
+    AccMinE a = AccMinE::identity();
     const int Nx = d.g.Nx, Ny = d.g.Ny, Nz = d.g.Nz;
-    // 0.5 kappa (0.5 / dx)^2 and so on
-    const R wx = w_const(0.125 * cd.kappa / (cd.dx * cd.dx), R{}), wy = w_const(0.125 * cd.kappa / (cd.dy * cd.dy), R{}),
-            wz = w_const(0.125 * cd.kappa / (cd.dz * cd.dz), R{});
-    const R GA = w_const(cd.tc.GA_s, R{}), GB = w_const(cd.tc.GB_s, R{}), mu0 = w_const(cd.mu0, R{}),
-            mg0 = w_const(-g0, R{});
+    const double idx2 = 0.5 / cd.dx, idy2 = 0.5 / cd.dy, idz2 = 0.5 / cd.dz;
     for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < d.g.N;
          cell += (long long)gridDim.x * blockDim.x) {
         const int k = (int)(cell % Nz);
@@ -3888,39 +3871,35 @@ k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *ph
         const int ip = i + 1 == Nx ? 0 : i + 1, im = i == 0 ? Nx - 1 : i - 1;
         const int jp = j + 1 == Ny ? 0 : j + 1, jm = j == 0 ? Ny - 1 : j - 1;
         const int kp = k + 1 == Nz ? 0 : k + 1, km = k == 0 ? Nz - 1 : k - 1;
-        const R gx = w_diff(phi[((long long)ip * Ny + j) * Nz + k], phi[((long long)im * Ny + j) * Nz + k]);
-        const R gy = w_diff(phi[((long long)i * Ny + jp) * Nz + k], phi[((long long)i * Ny + jm) * Nz + k]);
-        const R gz = w_diff(phi[r * Nz + kp], phi[r * Nz + km]);
+        const double gx = (double(phi[((long long)ip * Ny + j) * Nz + k]) - double(phi[((long long)im * Ny + j) * Nz + k])) * idx2;
+        const double gy = (double(phi[((long long)i * Ny + jp) * Nz + k]) - double(phi[((long long)i * Ny + jm) * Nz + k])) * idy2;
+        const double gz = (double(phi[r * Nz + kp]) - double(phi[r * Nz + km])) * idz2;
         const T p = phi[cell];
-        grad = w_add(grad, w_add(w_add(w_mul(wx, w_mul(gx, gx)), w_mul(wy, w_mul(gy, gy))), w_mul(wz, w_mul(gz, gz))));
-        dw = w_add(dw, w_of(pf_g(p), R{}));
+        a.grad += 0.5 * cd.kappa * (gx * gx + gy * gy + gz * gz);
+        a.dw += cd.W * double(pf_g(p));
         const T h = pf_h(clamp01(p));
-        const R hr = w_of(h, R{});
-        mh = w_add(mh, hr);
+        a.mh += double(h);
         // the monitor's composition: sigmoid(Y), capped once clamped
         const T xB = xB_of_Y<T>(c, d.Y[cell] + T(d.Yc));
         const T xm = xB < T(c.xbcap) ? xB : T(c.xbcap);
         if (c.elastic) {
             TE e0[6];
             eigenstrain<T, TE>(c, ec, p, c.gp ? d.eta_old[cell] : T(0), clamp01(xm), c.gp_el != 0, e0);
-            R sd = w_const(0.0, R{});
+            double sd = 0.0;
 #pragma unroll
-            for (int q = 0; q < 6; ++q)   // 1/2 sigma : (eps - e0); shear enters twice
-                sd = w_add(sd, w_mul(w_of(T(d.sig[q][cell]) * (q < 3 ? T(0.5) : T(1)), R{}),
-                                     w_diff(T(d.eps[q][cell]), T(e0[q]))));
-            gel = w_add(gel, sd);
-            gelh = w_add(gelh, w_mul(sd, hr));
+            for (int q = 0; q < 6; ++q)
+                sd += (q < 3 ? 1.0 : 2.0) * double(d.sig[q][cell]) * (double(d.eps[q][cell]) - double(e0[q]));
+            a.gel += 0.5 * sd;
+            a.gelh += 0.5 * sd * double(h);
         }
         if (chem) {
             const T x = clamp_eps(xm, T(1e-12));
             T offA, offB;
             thermo_mu_off<T>(c.tc, x, offA, offB);
-            const R xr = w_of(x, R{}), omx = w_diff(T(1), x), omh = w_diff(T(1), h);
-            const R mix = w_add(w_mul(omx, w_add(GA, w_of(offA, R{}))), w_mul(xr, w_add(GB, w_of(offB, R{}))));
-            ch = w_add(ch, w_add(w_add(w_mul(omh, mix), w_mul(hr, mu0)), mg0));
+            const double mix = (1.0 - double(x)) * (cd.tc.GA_s + double(offA)) + double(x) * (cd.tc.GB_s + double(offB));
+            a.chem += (1.0 - double(h)) * mix + double(h) * cd.mu0 - g0;
         }
     }
-    AccMinE a{w_out(mh), w_out(grad), cd.W * w_out(dw), w_out(gel), w_out(gelh), w_out(ch)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
@@ -3929,38 +3908,33 @@ k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *ph
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_resid(DevState<T, TE> d, const T *phi, const T *phin, double kappa, double lk, AccSum2 *part) {
-    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
-    R sa = w_const(0.0, R{}), sb = sa;
+    AccSum2Of<T> a = AccSum2Of<T>::identity();
     for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < d.g.N;
          cell += (long long)gridDim.x * blockDim.x) {
         const T p = phi[cell];
         T rr = (d.mge[cell] - T(kappa) * d.mlap[cell]) + T(lk) * pf_hp(p);
         if ((p <= T(1e-12) && rr > T(0)) || (p >= T(1) - T(1e-12) && rr < T(0))) rr = T(0);
-        sa = w_add(sa, w_mul(w_of(rr, R{}), w_of(rr, R{})));
-        const R dp = w_diff(p, phin[cell]);
-        sb = w_add(sb, w_mul(dp, dp));
+        acc_add_square(a.a, rr);
+        acc_add_square_diff(a.b, p, phin[cell]);
     }
-    AccSum2 a{w_out(sa), w_out(sb)};
     block_reduce_acc(a);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
+    if (threadIdx.x == 0) part[blockIdx.x] = acc_out(a);
 }
 
 // sum h(clamp01 phi) and sum h'(phi)^2 (gpu_compute_vf_from_h, :5609; hprime_sq)
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_min_hsums(const T *phi, long long N, AccSum2 *part) {
-    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
-    R sa = w_const(0.0, R{}), sb = sa;
+    AccSum2Of<T> a = AccSum2Of<T>::identity();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
          i += (long long)gridDim.x * blockDim.x) {
         const T p = phi[i];
-        sa = w_add(sa, w_of(pf_h(clamp01(p)), R{}));
+        acc_add(a.a, pf_h(clamp01(p)));
         const T hp = pf_hp(p);
-        sb = w_add(sb, w_of(hp * hp, R{}));
+        acc_add(a.b, hp * hp);
     }
-    AccSum2 a{w_out(sa), w_out(sb)};
     block_reduce_acc(a);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
+    if (threadIdx.x == 0) part[blockIdx.x] = acc_out(a);
 }
 
 // apply_volume_projection_kernel (:636-645)
@@ -3986,19 +3960,13 @@ struct AccSumMax {
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_dy(DevState<T, TE> d, PhysCT<T> c, double yc_prev, AccSumMax *part) {
-    using R = std::conditional_t<sizeof(T) == 8, double, dfl>;
-    R ss = w_const(0.0, R{});
-    T mx = T(-3e38);
-    const R dc = w_const(d.Yc - yc_prev, R{}), yc = w_const(d.Yc, R{});
+    AccSumMax a = AccSumMax::identity();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < d.g.N;
          i += (long long)gridDim.x * blockDim.x) {
-        const T Y = d.Y[i];
-        const R dy = w_add(w_diff(Y, d.Yprev[i]), dc);
-        ss = w_add(ss, w_mul(dy, dy));
-        const T y = w_round(w_add(w_of(Y, R{}), yc), T(0));
-        mx = fmax(mx, xB_of_Y<T>(c, y));
+        const double y = double(d.Y[i]) + d.Yc, yp = double(d.Yprev[i]) + yc_prev;
+        a.s += (y - yp) * (y - yp);
+        a.m = fmax(a.m, double(xB_of_Y<T>(c, T(y))));
     }
-    AccSumMax a{w_out(ss), double(mx)};
     block_reduce_acc(a);
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }

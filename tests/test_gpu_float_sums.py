@@ -13,10 +13,13 @@ pytestmark = pytest.mark.gpu
 # one block; its threads' sums are merged as the solver's block reductions do
 SRC = r"""
 #include "dfloat.cuh"
-template <bool SQ> __global__ void k_sum(const float *v, int n, double *out) {
+template <int KIND> __global__ void k_sum(const float *v, const float *q, int n, double *out) {
     __shared__ fsum red[32];
     fsum s = fs_zero();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) SQ ? fs_add_square(s, v[i]) : fs_add(s, v[i]);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        if (KIND == 2) fs_add_square_diff(s, v[i], q[i]);
+        else KIND ? fs_add_square(s, v[i]) : fs_add(s, v[i]);
+    }
     for (int o = 16; o > 0; o >>= 1) fs_merge(s, fs_shfl_down(s, o));
     if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
     __syncthreads();
@@ -25,9 +28,10 @@ template <bool SQ> __global__ void k_sum(const float *v, int n, double *out) {
         out[0] = fs_to_double(s);
     }
 }
-extern "C" int run(int square, const float *v, int n, double *out) {
-    if (square) k_sum<true><<<1, 256>>>(v, n, out);
-    else k_sum<false><<<1, 256>>>(v, n, out);
+extern "C" int run(int kind, const float *v, const float *q, int n, double *out) {
+    if (kind == 2) k_sum<2><<<1, 256>>>(v, q, n, out);
+    else if (kind) k_sum<1><<<1, 256>>>(v, q, n, out);
+    else k_sum<0><<<1, 256>>>(v, q, n, out);
     return (int)cudaDeviceSynchronize();
 }
 """
@@ -43,12 +47,13 @@ def lib(tmp_path_factory):
     return ctypes.CDLL(str(d / "fs.so"))
 
 
-def _sum(lib, v, square):
+def _sum(lib, v, square, q=None):
     import torch
-    d = torch.from_numpy(np.ascontiguousarray(v, dtype=np.float32)).cuda()
+    d, e = [torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).cuda() for x in (v, v if q is None else q)]
     out = torch.zeros(1, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
-    assert lib.run(int(square), ctypes.c_void_p(d.data_ptr()), v.size, ctypes.c_void_p(out.data_ptr())) == 0
+    p = [ctypes.c_void_p(x.data_ptr()) for x in (d, e, out)]
+    assert lib.run(2 if q is not None else int(square), p[0], p[1], v.size, p[2]) == 0
     return out.item()
 
 
@@ -83,3 +88,15 @@ def test_infinities_and_nan_reach_the_sum(lib, square):
     assert _sum(lib, v, square) == math.inf
     v[17] = np.nan
     assert math.isnan(_sum(lib, v, square))
+
+
+@pytest.mark.parametrize("step", [0.0, 1e-9, 1e-3, 0.7])
+def test_squared_differences(lib, step):
+    """Squares of differences, exact in a float or not: two roundings to float64 a
+    term where they are not, a thread's terms and twelve merges."""
+    rng = np.random.default_rng(8)
+    p = (rng.uniform(0.0, 1.0, 4099) ** 8).astype(np.float32)
+    q = np.clip(p + step * rng.uniform(-1.0, 1.0, p.size), 0.0, 1.0).astype(np.float32)
+    t = ((p.astype(np.float64) - q.astype(np.float64)) ** 2).tolist()
+    want = math.fsum(t)
+    assert abs(_sum(lib, p, True, q) - want) <= 2.0 ** -53 * (math.ceil(p.size / 256) + 19) * want
