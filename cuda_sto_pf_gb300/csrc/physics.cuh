@@ -154,6 +154,15 @@ __device__ __forceinline__ void split_hl(T h, TE &hi, TE &lo) {
 }
 template <typename TE>
 __device__ __forceinline__ TE hl_mul(TE hi, TE lo, TE s) { return fma(hi, s, lo * s); }
+// h w s of a value h of [-1, 2]: h w first where h is a float; a double's bits are
+// kept by the pair
+template <typename T, typename TE>
+__device__ __forceinline__ TE h_scaled(T h, TE w, TE s) {
+    if constexpr (sizeof(T) == sizeof(TE)) return h * w * s;
+    TE hi, lo;
+    split_hl<T, TE>(h, hi, lo);
+    return hl_mul(hi, lo, w * s);
+}
 
 // c_xB_phi where the molar volume may be constant (no division then)
 template <typename T, typename PC>
