@@ -284,7 +284,9 @@ static cudaError_t pfgb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = kDependent<T> ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // reported here, not by the thread's next call
+    return e;
 }
 
 // ---------------------------------------------------------------------------
