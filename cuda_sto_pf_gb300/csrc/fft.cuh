@@ -21,7 +21,6 @@
 #include <algorithm>
 #include <type_traits>
 #include <utility>
-#include <vector>
 
 #include "common.cuh"
 #include "f32x2.cuh"
@@ -86,21 +85,25 @@ struct AxisPlan {
     StagePlan st[PFGB_MAX_STAGES];
 };
 
-// host: the smooth part's radices, at most 16 each: as few stages as there
-// can be, the largest radix as small as it can be
-static inline void pfgb_best_radices(int q, int lim, std::vector<int> &cur, std::vector<int> &best) {
+// radices of a line (1024 = 2^10: no length has more than ten factors); plans
+// are made at C entries, which must not throw, so nothing here allocates
+struct RadixList {
+    int n = 0, r[10];
+    void push(int f) { r[n++] = f; }
+};
+
+// host: the smooth part's radices in falling order, at most 16 each: as few
+// stages as there can be, the largest radix as small as it can be
+static inline void pfgb_best_radices(int q, int lim, RadixList &cur, RadixList &best) {
     if (q == 1) {
-        if (best.empty() || cur.size() < best.size() ||
-            (cur.size() == best.size() && *std::max_element(cur.begin(), cur.end()) <
-                                              *std::max_element(best.begin(), best.end())))
-            best = cur;
+        if (!best.n || cur.n < best.n || (cur.n == best.n && cur.r[0] < best.r[0])) best = cur;
         return;
     }
     for (int r = std::min(lim, q); r >= 2; --r) {
         if (q % r) continue;
-        cur.push_back(r);
+        cur.push(r);
         pfgb_best_radices(q / r, r, cur, best);
-        cur.pop_back();
+        --cur.n;
     }
 }
 
@@ -115,37 +118,35 @@ static inline void pfgb_best_radices(int q, int lim, std::vector<int> &cur, std:
 static inline bool pfgb_make_plan(int n, AxisPlan *p) {
     p->n = n;
     p->nst = 0;
-    std::vector<std::pair<int, int>> rad, dir;   // radix, kind
-    int q = n;
-    if (q % 41 == 0) { rad.push_back({41, 1}); q /= 41; }
+    if (n < 1 || n > PFGB_MAX_N) return false;
+    RadixList dir, cur, best;
+    int q = n, B = n;
+    auto stage = [&](int R, int kind) {
+        StagePlan &st = p->st[p->nst++];
+        st.R = R;
+        st.kind = kind;
+        st.B = B;
+        st.m = B / R;
+        st.fm.init((unsigned)st.m);
+        st.fR.init((unsigned)R);
+        B = st.m;
+    };
+    if (q % 41 == 0) { stage(41, 1); q /= 41; }
     for (int f = 17; f <= q; ++f)
         while (q % f == 0) {
             bool prime = true;
             for (int d = 2; d * d <= f; ++d) prime = prime && f % d;
             if (!prime) break;
-            dir.push_back({f, 2});
+            dir.push(f);
             q /= f;
         }
-    std::vector<int> cur, best;
     if (q > 1) pfgb_best_radices(q, 16, cur, best);
-    auto fits = [&] { return best.empty() || n / best.back() <= PFGB_LINE_THREADS; };
-    if (!fits()) std::reverse(best.begin(), best.end());
+    auto fits = [&] { return !best.n || n / best.r[best.n - 1] <= PFGB_LINE_THREADS; };
+    if (!fits()) std::reverse(best.r, best.r + best.n);
     const bool direct_last = !fits();
-    if (!direct_last) rad.insert(rad.end(), dir.begin(), dir.end());
-    for (int r : best) rad.push_back({r, 0});
-    if (direct_last) rad.insert(rad.end(), dir.begin(), dir.end());
-    if (rad.size() > PFGB_MAX_STAGES) return false;
-    int B = n;
-    for (auto &rk : rad) {
-        StagePlan &st = p->st[p->nst++];
-        st.R = rk.first;
-        st.kind = rk.second;
-        st.B = B;
-        st.m = B / rk.first;
-        st.fm.init((unsigned)st.m);
-        st.fR.init((unsigned)st.R);
-        B = st.m;
-    }
+    if (!direct_last) for (int i = 0; i < dir.n; ++i) stage(dir.r[i], 2);
+    for (int i = 0; i < best.n; ++i) stage(best.r[i], 0);
+    if (direct_last) for (int i = 0; i < dir.n; ++i) stage(dir.r[i], 2);
     for (int i = 0; i < p->nst; ++i) {
         const StagePlan &st = p->st[i];
         if (st.kind == 1 && i > 0) return false;

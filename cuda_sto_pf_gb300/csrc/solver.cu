@@ -5505,11 +5505,12 @@ constexpr int kTabSlots = 8;
 constexpr size_t kTabBytes = 3 * (size_t)PFGB_MAX_N * sizeof(double2);
 static __device__ __align__(256) unsigned char g_fft_tables[kTabSlots * kTabBytes];
 struct TabSlots { unsigned used = 0; unsigned char *addr = nullptr; };
+constexpr int kTabDevices = 64;
 static std::mutex g_tab_mu;
-static std::map<int, TabSlots> g_tab;   // by device
+static TabSlots g_tab[kTabDevices];
 // a free slot's address, null if there is none (or the device cannot be asked)
 static unsigned char *take_table(int *dev, int *slot) {
-    if (cudaGetDevice(dev) != cudaSuccess) return nullptr;
+    if (cudaGetDevice(dev) != cudaSuccess || *dev < 0 || *dev >= kTabDevices) return nullptr;
     std::lock_guard<std::mutex> lk(g_tab_mu);
     TabSlots &t = g_tab[*dev];
     if (!t.addr) {

@@ -15,12 +15,25 @@ from test_gpu_fft import _run
 # of threads over every count of lines that a tile can have
 SRC = r"""
 #include <cstdio>
+#include <cstdlib>
+#include <new>
 #include "fft.cuh"
+static int g_news = 0;
+__host__ __device__ void *operator new(size_t n) {
+#ifndef __CUDA_ARCH__
+    ++g_news;
+#endif
+    return malloc(n);
+}
+__host__ __device__ void operator delete(void *p) noexcept { free(p); }
+__host__ __device__ void operator delete(void *p, size_t) noexcept { free(p); }
 int main() {
     for (int n = 1; n <= PFGB_MAX_N; ++n) {
         AxisPlan p;
+        const int before = g_news;
         const bool ok = pfgb_make_plan(n, &p);
-        std::printf("{\"n\": %d, \"ok\": %s, \"stages\": [", n, ok ? "true" : "false");
+        const int news = g_news - before;
+        std::printf("{\"n\": %d, \"ok\": %s, \"news\": %d, \"stages\": [", n, ok ? "true" : "false", news);
         for (int s = 0; s < p.nst; ++s)
             std::printf("%s[%d, %d, %d, %d, %u, %u]", s ? ", " : "", p.st[s].R, p.st[s].B, p.st[s].m, p.st[s].kind,
                         p.st[s].fm.d, p.st[s].fR.d);
@@ -70,6 +83,11 @@ def test_every_length_fits_its_stages(plans):
                 assert kind == 0 and 2 <= R <= 16, p
                 if i == len(st) - 1:
                     assert lo // (n // R) >= 1, p
+
+
+def test_plans_allocate_nothing(plans):
+    """They are made at C entries, one of which promises no allocation."""
+    assert not any(p["news"] for p in plans)
 
 
 def _emulate(x, stages):
