@@ -1025,7 +1025,7 @@ struct pfgb_fno {
     std::vector<long long> offW, offb, offR;
     float *master = nullptr;
     __nv_bfloat16 *wbf = nullptr;
-    float2 *twx = nullptr, *twy = nullptr;
+    float2 *twx = nullptr;
     float2 *tyi = nullptr;   // [2m][Y] inverse y twiddles of the retained ky
     float4 *fz = nullptr;    // [Z][pad2(m)] e^{-2 pi i k z / Z}, read as float4 pairs of k
     float2 *gz = nullptr;    // [m][Z] the same values, z fastest
@@ -1072,8 +1072,12 @@ pfgb_status upload_tw(pfgb_fno *f, float2 **dst, int n) {
 
 constexpr size_t kSmemCap = 200 * 1024;
 size_t layer_smem(int Z, int Mz);
-// the models that are taken: the staging of a z line's DFT matrix and of about
-// 256 / (modes / 2) lines (64 KB at most), and of a y slab, within kSmemCap
+// The models that are taken: those whose z pass could stage the DFT matrix of a
+// whole line with about 256 / (modes / 2) lines (64 KB at most), whose y pass a
+// slab, and whose layer kernel its lines within kSmemCap.  The z and y passes
+// stage less than that (kZC positions, kYTab twiddles); the set of accepted
+// models stayed, and every launch of one is within the limits (dft_z_smem:
+// 64 KB; k_dft_x: 64 bytes an x position; layer_staging).
 size_t dft_z_staging(int Z, int Mz) {
     const int kg = pad2(Mz) / 2;
     const int lb = std::max(1, std::min((256 + kg - 1) / kg, (64 * 1024) / (4 * (Z + 1))));
@@ -1095,7 +1099,6 @@ pfgb_status validate(const pfgb_fno_config *c) {
                            c->Ny, c->Nz);
         return PFGB_ERR_INVALID;
     }
-    // the z and y transforms stage a whole DFT matrix / slab in shared memory
     if (dft_z_staging(c->Nz, m) > kSmemCap || sizeof(float2) * (size_t)c->Ny * (m + 1) > kSmemCap) {
         pfgb_set_error_msg("FNO: modes=%d too many for a %dx%dx%d grid (shared-memory staging)", m, c->Nx, c->Ny,
                            c->Nz);
@@ -1385,7 +1388,6 @@ pfgb_status create_impl(const pfgb_fno_config *cfg, int device, const float *par
     auto fail = [&](pfgb_status s) { fno_free(f); return s; };
     pfgb_status s;
     if ((s = upload_tw(f, &f->twx, f->X)) != PFGB_OK) return fail(s);
-    if ((s = upload_tw(f, &f->twy, f->Y)) != PFGB_OK) return fail(s);
     {
         std::vector<float2> h((size_t)2 * f->m * f->Y);
         for (int j = 0; j < 2 * f->m; ++j) {
