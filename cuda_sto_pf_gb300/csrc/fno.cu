@@ -1172,8 +1172,9 @@ pfgb_status check_launch(const char *what) {
 template <typename K>
 pfgb_status smem_opt_in(K kern, size_t bytes) {
     if (bytes <= 48 * 1024) return PFGB_OK;
-    // one fixed value per kernel, the same from every caller
-    FNO_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // one fixed value, the same from every caller: the limit belongs to the kernel,
+    // and another model's smaller one could come between this and the launch
+    FNO_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
     return PFGB_OK;
 }
 
