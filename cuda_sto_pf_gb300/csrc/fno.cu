@@ -183,62 +183,78 @@ __global__ void __launch_bounds__(256) k_dft_z(const float *__restrict__ src, fl
 // each value, NS slabs (channel, x) per block
 // dst[r][jy][kz] = sum_y src[r][y][kz] e^{-2 pi i ky(jy) y / Y}
 // tyi[jy][y] holds the conjugate twiddles; they are staged in shared memory,
-// transposed, kYTab of them at a time, and read as broadcasts; the values come
-// straight from memory.  (Twiddles from the cache and slabs staged instead: the
+// transposed, and read as broadcasts; the values come straight from memory.
+// (Twiddles from the cache and slabs staged instead: the
 // warps waited for the twiddles, 107 us at 128^3, 12 modes, issue 26%; now 48.)
 constexpr int kYJ = 8, kYTab = 4096;
 __host__ __device__ constexpr int dft_y_groups(int m) { return (2 * m + kYJ - 1) / kYJ; }
-// positions staged at a time
-__host__ __device__ constexpr int dft_y_chunk(int Y, int m) {
-    const int c = kYTab / (dft_y_groups(m) * kYJ);
-    return Y < c ? Y : c;
-}
+// positions whose twiddles fit
+__host__ __device__ constexpr int dft_y_positions(int m) { return kYTab / (dft_y_groups(m) * kYJ); }
 __global__ void __launch_bounds__(256) k_dft_y(const float2 *__restrict__ src, float2 *__restrict__ dst,
                                                const float2 *__restrict__ tyi, long long nslab, int NS, int Y, int Mz,
                                                int m) {
-    extern __shared__ __align__(16) float2 smy[];                // [YC][JP]
-    const int J = 2 * m, JG = dft_y_groups(m), JP = JG * kYJ, YC = dft_y_chunk(Y, m);
+    extern __shared__ __align__(16) float2 smy[];                // [Y][JP]
+    const int J = 2 * m, JG = dft_y_groups(m), JP = JG * kYJ;
     const long long r0 = (long long)blockIdx.x * NS;
     const int ns = (int)min((long long)NS, nslab - r0), ntask = ns * Mz * JG;
     const float2 *s = src + r0 * Y * Mz;
+    for (int i = threadIdx.x; i < Y * JP; i += blockDim.x) {
+        const int j = i / Y, y = i - j * Y;
+        smy[y * JP + j] = j < J ? tyi[j * Y + y] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
     // kz fastest, then the slab: a warp shares the group of ky and its twiddles
-    for (int e0 = 0; e0 < ntask; e0 += blockDim.x) {
-        const int e = e0 + threadIdx.x;
-        const bool act = e < ntask;
-        const int jg = act ? e / (ns * Mz) : 0, rem = act ? e - jg * ns * Mz : 0;
+    for (int e = threadIdx.x; e < ntask; e += blockDim.x) {
+        const int jg = e / (ns * Mz), rem = e - jg * ns * Mz;
         const int sl = rem / Mz, kz = rem - sl * Mz;
         const float2 *a = s + (long long)sl * Y * Mz + kz;
         float re[kYJ], im[kYJ];
 #pragma unroll
         for (int j = 0; j < kYJ; ++j) re[j] = im[j] = 0.f;
-        for (int yb = 0; yb < Y; yb += YC) {
-            const int ny = min(YC, Y - yb);
-            __syncthreads();
-            for (int i = threadIdx.x; i < ny * JP; i += blockDim.x) {
-                const int j = i / ny, y = i - j * ny;
-                smy[y * JP + j] = j < J ? tyi[j * Y + yb + y] : make_float2(0.f, 0.f);
-            }
-            __syncthreads();
-            if (!act) continue;
 #pragma unroll 4
-            for (int y = 0; y < ny; ++y) {
-                const float2 v = a[(yb + y) * Mz];
-                const float4 *w = reinterpret_cast<const float4 *>(smy + y * JP + jg * kYJ);
+        for (int y = 0; y < Y; ++y) {
+            const float2 v = a[y * Mz];
+            const float4 *w = reinterpret_cast<const float4 *>(smy + y * JP + jg * kYJ);
 #pragma unroll
-                for (int q = 0; q < kYJ / 2; ++q) {              // e^{-}: (tx, -ty)
-                    const float4 t = w[q];
-                    re[2 * q] = fmaf(v.x, t.x, fmaf(-v.y, -t.y, re[2 * q]));
-                    im[2 * q] = fmaf(v.x, -t.y, fmaf(v.y, t.x, im[2 * q]));
-                    re[2 * q + 1] = fmaf(v.x, t.z, fmaf(-v.y, -t.w, re[2 * q + 1]));
-                    im[2 * q + 1] = fmaf(v.x, -t.w, fmaf(v.y, t.z, im[2 * q + 1]));
-                }
+            for (int q = 0; q < kYJ / 2; ++q) {                  // e^{-}: (tx, -ty)
+                const float4 t = w[q];
+                re[2 * q] = fmaf(v.x, t.x, fmaf(-v.y, -t.y, re[2 * q]));
+                im[2 * q] = fmaf(v.x, -t.y, fmaf(v.y, t.x, im[2 * q]));
+                re[2 * q + 1] = fmaf(v.x, t.z, fmaf(-v.y, -t.w, re[2 * q + 1]));
+                im[2 * q + 1] = fmaf(v.x, -t.w, fmaf(v.y, t.z, im[2 * q + 1]));
             }
         }
-        if (!act) continue;
         float2 *d = dst + (r0 + sl) * J * Mz + kz;
 #pragma unroll
         for (int j = 0; j < kYJ; ++j)
             if (jg * kYJ + j < J) d[(jg * kYJ + j) * Mz] = make_float2(re[j], im[j]);
+    }
+}
+
+// the same for few slabs: a block stages one, one output per thread
+__global__ void __launch_bounds__(256) k_dft_y_slab(const float2 *__restrict__ src, float2 *__restrict__ dst,
+                                                    const float2 *__restrict__ twy, int Y, int Mz, int m) {
+    extern __shared__ __align__(16) float2 smy[];
+    float2 *tw = smy, *slab = smy + Y;
+    const long long r = blockIdx.x;
+    for (int e = threadIdx.x; e < Y; e += blockDim.x) tw[e] = twy[e];
+    const float2 *s = src + r * Y * Mz;
+    for (int e = threadIdx.x; e < Y * Mz; e += blockDim.x) slab[e] = s[e];
+    __syncthreads();
+    const int nout = 2 * m * Mz;
+    for (int e = threadIdx.x; e < nout; e += blockDim.x) {
+        const int jy = e / Mz, kz = e - jy * Mz;
+        const int ky = kcorner(jy, m, Y);
+        float re = 0.f, im = 0.f;
+        int idx = 0;
+        for (int y = 0; y < Y; ++y) {
+            const float2 a = slab[y * Mz + kz], w = tw[idx];
+            re = fmaf(a.x, w.x, fmaf(-a.y, w.y, re));
+            im = fmaf(a.x, w.y, fmaf(a.y, w.x, im));
+            idx += ky;
+            if (idx >= Y) idx -= Y;
+        }
+        dst[r * nout + e] = make_float2(re, im);
     }
 }
 
@@ -349,6 +365,28 @@ __global__ void __launch_bounds__(256) k_idft_y(const float2 *__restrict__ src, 
 #pragma unroll
         for (int p = 0; p < kYP; ++p)
             if (g * kYP + p < ny) d[p * Mz] = make_float2(re[p], im[p]);
+    }
+}
+
+// the same for few slabs: a block stages one, one output per thread
+__global__ void __launch_bounds__(256) k_idft_y_slab(const float2 *__restrict__ src, float2 *__restrict__ dst,
+                                                     const float2 *__restrict__ tyi, int Y, int Mz, int m) {
+    extern __shared__ __align__(16) float2 smiy[];
+    const long long r = blockIdx.x;
+    const float2 *s = src + r * 2 * m * Mz;
+    for (int e = threadIdx.x; e < 2 * m * Mz; e += blockDim.x) smiy[e] = s[e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < Y * Mz; e += blockDim.x) {
+        const int y = e / Mz, kz = e - y * Mz;
+        float re = 0.f, im = 0.f;
+#pragma unroll 4
+        for (int j = 0; j < 2 * m; ++j) {
+            const float2 a = smiy[j * Mz + kz];
+            const float2 t = __ldg(&tyi[j * Y + y]);
+            re = fmaf(a.x, t.x, fmaf(-a.y, t.y, re));
+            im = fmaf(a.x, t.y, fmaf(a.y, t.x, im));
+        }
+        dst[r * (long long)Y * Mz + e] = make_float2(re, im);
     }
 }
 
@@ -1025,7 +1063,7 @@ struct pfgb_fno {
     std::vector<long long> offW, offb, offR;
     float *master = nullptr;
     __nv_bfloat16 *wbf = nullptr;
-    float2 *twx = nullptr;
+    float2 *twx = nullptr, *twy = nullptr;
     float2 *tyi = nullptr;   // [2m][Y] inverse y twiddles of the retained ky
     float4 *fz = nullptr;    // [Z][pad2(m)] e^{-2 pi i k z / Z}, read as float4 pairs of k
     float2 *gz = nullptr;    // [m][Z] the same values, z fastest
@@ -1072,12 +1110,11 @@ pfgb_status upload_tw(pfgb_fno *f, float2 **dst, int n) {
 
 constexpr size_t kSmemCap = 200 * 1024;
 size_t layer_smem(int Z, int Mz);
-// The models that are taken: those whose z pass could stage the DFT matrix of a
-// whole line with about 256 / (modes / 2) lines (64 KB at most), whose y pass a
-// slab, and whose layer kernel its lines within kSmemCap.  The z and y passes
-// stage less than that (kZC positions, kYTab twiddles); the set of accepted
-// models stayed, and every launch of one is within the limits (dft_z_smem:
-// 64 KB; k_dft_x: 64 bytes an x position; layer_staging).
+// The models that are taken: those whose y pass can stage a slab (k_dft_y_slab),
+// whose layer kernel its lines, and whose z pass could stage the DFT matrix of a
+// whole line with about 256 / (modes / 2) lines (64 KB at most), within kSmemCap.
+// The z pass stages less than that (kZC positions: at most 64 KB); the set of
+// accepted models stayed.
 size_t dft_z_staging(int Z, int Mz) {
     const int kg = pad2(Mz) / 2;
     const int lb = std::max(1, std::min((256 + kg - 1) / kg, (64 * 1024) / (4 * (Z + 1))));
@@ -1182,6 +1219,21 @@ size_t dft_z_smem(int Mz, int LB) {
     return sizeof(float) * (2 * (size_t)kZC * pad2(Mz) + (size_t)kZC * dft_z_stride(LB));
 }
 
+// The forms for few threads.  k_dft_y and k_idft_y give a thread eight sums, whose
+// chain of reads from memory needs 15 warps an SM beside it to be hidden, and
+// k_dft_y the twiddles of all positions at once.  Either side gives the same
+// results.  us a pass, eight sums against one:
+//   y forward  12 modes: 56^3 -> 2.1 more, 64^3 1.1 less, 128^3 16 less; 8 modes: 64^3
+//              6.6, 128^3 13 more; 4 modes: 8x1000x16 172 more; 24 modes (Y > chunk): 96^3 7.6 more
+//   y inverse   8 modes: 32^3 4.2 more, 48^3 1.4, 64^3 4.3 less; 4 modes: 64^3 1.9 more
+constexpr long long kFewThreads = 152 * 480;
+bool few_slabs_fwd(const pfgb_fno *f) {
+    return (long long)kW * f->X * f->Mz * dft_y_groups(f->m) < kFewThreads || f->Y > dft_y_positions(f->m);
+}
+bool few_slabs_inv(const pfgb_fno *f) {
+    return (long long)kW * f->X * f->Mz * ((f->Y + kYP - 1) / kYP) < kFewThreads;
+}
+
 // spectral transform of src [W][N] onto the retained modes -> dst [W][M]
 pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, float w1) {
     const long long lines = (long long)kW * f->S;
@@ -1191,15 +1243,21 @@ pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, f
     k_dft_z<<<(unsigned)((lines + LB - 1) / LB), 256, sz, f->stream>>>(src, f->A, f->fz, lines, f->Z, f->Mz, LB,
                                                                        w0, w1);
     FNO_CHECK(check_launch("dft_z"));
-    // slabs per block: about 256 tasks, fewer where the grid would leave SMs
-    // without two blocks
-    const int tasks = f->Mz * dft_y_groups(f->m);
-    const long long nslab = (long long)kW * f->X;
-    const int NS = (int)std::max<long long>(1, std::min<long long>(256 / std::max(1, tasks), nslab / 304));
-    const int ny_thr = std::min(256, (NS * tasks + 31) / 32 * 32);
-    const size_t sy = sizeof(float2) * (size_t)dft_y_chunk(f->Y, f->m) * dft_y_groups(f->m) * kYJ;
-    k_dft_y<<<(unsigned)((nslab + NS - 1) / NS), ny_thr, sy, f->stream>>>(f->A, f->B, f->tyi, nslab, NS, f->Y, f->Mz,
-                                                                         f->m);
+    if (few_slabs_fwd(f)) {
+        const size_t sy = sizeof(float2) * ((size_t)f->Y + (size_t)f->Y * f->Mz);
+        FNO_CHECK(smem_opt_in(k_dft_y_slab, sy));
+        k_dft_y_slab<<<(unsigned)(kW * f->X), 256, sy, f->stream>>>(f->A, f->B, f->twy, f->Y, f->Mz, f->m);
+    } else {
+        // slabs per block: about 256 tasks, fewer where the grid would leave SMs
+        // without two blocks
+        const int tasks = f->Mz * dft_y_groups(f->m);
+        const long long nslab = (long long)kW * f->X;
+        const int NS = (int)std::max<long long>(1, std::min<long long>(256 / std::max(1, tasks), nslab / 304));
+        const int ny_thr = std::min(256, (NS * tasks + 31) / 32 * 32);
+        const size_t sy = sizeof(float2) * (size_t)f->Y * dft_y_groups(f->m) * kYJ;
+        k_dft_y<<<(unsigned)((nslab + NS - 1) / NS), ny_thr, sy, f->stream>>>(f->A, f->B, f->tyi, nslab, NS, f->Y, f->Mz,
+                                                                             f->m);
+    }
     FNO_CHECK(check_launch("dft_y"));
     const size_t sx = sizeof(float2) * (size_t)f->X * kXJ;
     FNO_CHECK(smem_opt_in(k_dft_x, sx));
@@ -1212,6 +1270,12 @@ pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, f
 pfgb_status spec_inverse_xy(pfgb_fno *f, const float2 *src) {
     k_idft_x<<<(unsigned)(kW * f->X), 256, 0, f->stream>>>(src, f->B, f->twx, f->X, f->Q, f->m);
     FNO_CHECK(check_launch("idft_x"));
+    if (few_slabs_inv(f)) {
+        const size_t sy = sizeof(float2) * (2 * (size_t)f->m * f->Mz);
+        FNO_CHECK(smem_opt_in(k_idft_y_slab, sy));
+        k_idft_y_slab<<<(unsigned)(kW * f->X), 256, sy, f->stream>>>(f->B, f->A, f->tyi, f->Y, f->Mz, f->m);
+        return check_launch("idft_y");
+    }
     // slabs per block: a few trips over the staged twiddles, fewer where the grid
     // would leave SMs without four blocks
     const int YC = idft_y_chunk(f->Y, f->m), tasks = f->Mz * (YC / kYP);
@@ -1389,6 +1453,7 @@ pfgb_status create_impl(const pfgb_fno_config *cfg, int device, const float *par
     auto fail = [&](pfgb_status s) { fno_free(f); return s; };
     pfgb_status s;
     if ((s = upload_tw(f, &f->twx, f->X)) != PFGB_OK) return fail(s);
+    if ((s = upload_tw(f, &f->twy, f->Y)) != PFGB_OK) return fail(s);
     {
         std::vector<float2> h((size_t)2 * f->m * f->Y);
         for (int j = 0; j < 2 * f->m; ++j) {
