@@ -31,6 +31,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -453,8 +454,9 @@ __global__ void __launch_bounds__(256) k_mode_grad(const float2 *__restrict__ C,
 constexpr int kLayerCells = 256;
 __host__ __device__ constexpr int layer_lines(int Z) { return kLayerCells / Z + 2; }
 
-template <bool ACT, bool SAVE, bool PAIR>
-__global__ void __launch_bounds__(kLayerCells / 2, 3) k_layer_fwd(const float2 *__restrict__ A,
+enum { kCellsPair, kCellsApart, kCellsOne };
+template <bool ACT, bool SAVE, int CELLS>
+__global__ void __launch_bounds__(CELLS == kCellsOne ? kLayerCells : kLayerCells / 2, CELLS == kCellsOne ? 2 : 3) k_layer_fwd(const float2 *__restrict__ A,
                                                                   const float *__restrict__ v,
                                                                   const __nv_bfloat16 *__restrict__ Ww,
                                                                   const float *__restrict__ bw,
@@ -486,9 +488,10 @@ __global__ void __launch_bounds__(kLayerCells / 2, 3) k_layer_fwd(const float2 *
         d[2] = a.y;
     }
     __syncthreads();
+    constexpr bool PAIR = CELLS == kCellsPair;
     const long long n0 = PAIR ? c0 + 2 * threadIdx.x : c0 + threadIdx.x, n1 = PAIR ? n0 + 1 : n0 + kLayerCells / 2;
     if (n0 >= c1) return;
-    const bool two = n1 < c1;
+    const bool two = CELLS != kCellsOne && n1 < c1;
     const int l0 = (int)(n0 / Z - sf), z0 = (int)(n0 % Z);
     const int l1 = PAIR || !two ? l0 : (int)(n1 / Z - sf), z1 = PAIR ? z0 + 1 : (two ? (int)(n1 % Z) : z0);
     f2x::P s0[kW / 2], s1[kW / 2];
@@ -1221,18 +1224,21 @@ size_t dft_z_smem(int Mz, int LB) {
 
 // The forms for few threads.  k_dft_y and k_idft_y give a thread eight sums, whose
 // chain of reads from memory needs 15 warps an SM beside it to be hidden, and
-// k_dft_y the twiddles of all positions at once.  Either side gives the same
-// results.  us a pass, eight sums against one:
+// k_dft_y the twiddles of all positions at once; k_layer_fwd gives a thread two cells,
+// which below a block an SM only leaves threads out.  Either side gives the same
+// results.  us a pass, eight sums / one (two cells / one), 4 layers:
 //   y forward  12 modes: 56^3 -> 2.1 more, 64^3 1.1 less, 128^3 16 less; 8 modes: 64^3
 //              6.6, 128^3 13 more; 4 modes: 8x1000x16 172 more; 24 modes (Y > chunk): 96^3 7.6 more
 //   y inverse   8 modes: 32^3 4.2 more, 48^3 1.4, 64^3 4.3 less; 4 modes: 64^3 1.9 more
-constexpr long long kFewThreads = 152 * 480;
+//   layer      24^3 to 32^3 1 to 2.6 more, 40^3 0.4 to 2, 64^3 6 less
+constexpr long long kFewThreads = 152 * 480, kFewCells = 152 * kLayerCells;
 bool few_slabs_fwd(const pfgb_fno *f) {
     return (long long)kW * f->X * f->Mz * dft_y_groups(f->m) < kFewThreads || f->Y > dft_y_positions(f->m);
 }
 bool few_slabs_inv(const pfgb_fno *f) {
     return (long long)kW * f->X * f->Mz * ((f->Y + kYP - 1) / kYP) < kFewThreads;
 }
+bool few_cells(const pfgb_fno *f) { return f->N <= kFewCells; }
 
 // spectral transform of src [W][N] onto the retained modes -> dst [W][M]
 pfgb_status spec_forward(pfgb_fno *f, const float *src, float2 *dst, float w0, float w1) {
@@ -1310,19 +1316,22 @@ pfgb_status forward_impl(pfgb_fno *f, const float *in, float *out, bool train) {
         FNO_CHECK(spec_inverse_xy(f, f->O));
         const bool act = l < f->L - 1;
         const unsigned nb = (unsigned)((f->N + kLayerCells - 1) / kLayerCells);
+        const bool one = few_cells(f);
+        const int threads = one ? kLayerCells : kLayerCells / 2;
         auto launch = [&](auto kern) -> pfgb_status {
             FNO_CHECK(smem_opt_in(kern, sl));
-            kern<<<nb, kLayerCells / 2, sl, f->stream>>>(f->A, vin, f->wbf + f->offW[l], f->master + f->offb[l], vout,
-                                                     train ? f->pres[l] : nullptr, f->gz, f->S, f->Z, f->Mz);
+            kern<<<nb, threads, sl, f->stream>>>(f->A, vin, f->wbf + f->offW[l], f->master + f->offb[l], vout,
+                                                 train ? f->pres[l] : nullptr, f->gz, f->S, f->Z, f->Mz);
             return check_launch("layer_fwd");
         };
-        if (f->Z % 2 == 0) {
-            if (act) FNO_CHECK(train ? launch(k_layer_fwd<true, true, true>) : launch(k_layer_fwd<true, false, true>));
-            else FNO_CHECK(train ? launch(k_layer_fwd<false, true, true>) : launch(k_layer_fwd<false, false, true>));
-        } else {
-            if (act) FNO_CHECK(train ? launch(k_layer_fwd<true, true, false>) : launch(k_layer_fwd<true, false, false>));
-            else FNO_CHECK(train ? launch(k_layer_fwd<false, true, false>) : launch(k_layer_fwd<false, false, false>));
-        }
+        auto cells = [&](auto form) -> pfgb_status {
+            constexpr int C = decltype(form)::value;
+            if (act) return train ? launch(k_layer_fwd<true, true, C>) : launch(k_layer_fwd<true, false, C>);
+            return train ? launch(k_layer_fwd<false, true, C>) : launch(k_layer_fwd<false, false, C>);
+        };
+        if (one) FNO_CHECK(cells(std::integral_constant<int, kCellsOne>{}));
+        else if (f->Z % 2 == 0) FNO_CHECK(cells(std::integral_constant<int, kCellsPair>{}));
+        else FNO_CHECK(cells(std::integral_constant<int, kCellsApart>{}));
     }
     if (!out) return PFGB_OK;   // training: the projection backward recomputes it
     const float *vl = train ? f->vs[f->L] : (f->L % 2 == 0 ? f->va : f->vb);
