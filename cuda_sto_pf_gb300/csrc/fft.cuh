@@ -321,6 +321,14 @@ __device__ __forceinline__ void fft_lines(const cplx_t<T> *buf, const cplx_t<T> 
     fft_lines_at<T, DIR>(t, &p);
 }
 
+// inputs of the direct sums that a point of a line goes through
+static inline int pfgb_direct_inputs(const AxisPlan &p) {
+    int d = 0;
+    for (int s = 0; s < p.nst; ++s)
+        if (p.st[s].kind == 2) d += p.st[s].R;
+    return d;
+}
+
 // threads of a block whose tile has L lines: one trip of every stage where 256
 // threads hold it, else equal trips (a second trip of a few butterflies would
 // leave the block's other warps waiting).  The last stage has one butterfly per
@@ -336,6 +344,7 @@ static inline int pfgb_line_threads(const AxisPlan &p, int L) {
             items = (long long)L * p.n;
             per = PFGB_DIRECT_SUMS;
             least = std::max(least, (p.n + per - 1) / per);
+            t = std::max(t, (int)std::min<long long>(items, PFGB_LINE_THREADS));   // fewer sums one after the other
         } else if (s == p.nst - 1) least = std::max(least, nb);
         const long long trips = (items + PFGB_LINE_THREADS * per - 1) / (PFGB_LINE_THREADS * per);
         t = std::max(t, (int)((items + trips * per - 1) / (trips * per)));

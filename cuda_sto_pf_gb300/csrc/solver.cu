@@ -241,15 +241,29 @@ static TileDiv tile_div(int tk, int nin, int nout) {
     t.out.init((unsigned)(tk * std::max(nout, 1)));
     return t;
 }
+// A direct stage's time is its sums, not the tile's traffic, and it differs by
+// whole blocks from SM to SM: from 32 inputs a point on its passes take many small
+// blocks of a few lines, and single columns where even those leave SMs empty.
+// FP64 transforms, with the rule above / this one: 401x64x64 7.7 / 4.1 ms, 64x379x64
+// 5.1 / 3.2, 128x40x751 20.4 / 17.0; FP32 dynamics 1021x8x16 134 / 82 ms.  Below 32
+// inputs the traffic counts: 68x119x51 FP32 dynamics 0.55 / 0.68 of the former engine's.
+constexpr int kDirectInputs = 32, kDirectBlocks = 912, kDirectLines = 2;
 template <typename T2>
-static int axis_tile(int n, int arrays, int slabs, int ncol) {
-    const int least = std::min(ncol, 32 / (int)sizeof(T2) > 1 ? 32 / (int)sizeof(T2) : 1);
+static int axis_tile(const AxisPlan &pl, int arrays, int slabs, int ncol) {
+    const int n = pl.n;
+    const bool direct = pfgb_direct_inputs(pl) >= kDirectInputs;
+    const int sector = direct ? (kDirectLines + arrays - 1) / arrays : 32 / (int)sizeof(T2);
+    const int least = std::min(ncol, sector > 1 ? sector : 1);
     int tk = std::min(ncol, 64);
     while (tk > least && axis_tile_bytes<T2>(n, arrays, tk) > kSmemBudget) --tk;
     while (tk > 1 && axis_tile_bytes<T2>(n, arrays, tk) > kSmemWide) --tk;
     int nblk = (ncol + tk - 1) / tk;
-    if ((long long)slabs * nblk < 304)
-        nblk = std::max(nblk, std::min((304 + slabs - 1) / slabs, (ncol + least - 1) / least));
+    auto at_least = [&](int blocks, int columns) {
+        if ((long long)slabs * nblk < blocks)
+            nblk = std::max(nblk, std::min((blocks + slabs - 1) / slabs, (ncol + columns - 1) / columns));
+    };
+    at_least(direct ? kDirectBlocks : 304, least);
+    if (direct) at_least(152, 1);
     return (ncol + nblk - 1) / nblk;
 }
 
@@ -591,7 +605,7 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
     }
     constexpr int NW = axis_tile_arrays<NIN, NOUT, Op>();
     const int slabs = (axis == 1 ? c->g.Nx : c->g.kept_rows()) * (Op::kInplace ? NIN : 1);
-    int TK = axis_tile<T2>(n, NW, slabs, c->g.NzK);
+    int TK = axis_tile<T2>(pl, NW, slabs, c->g.NzK);
     if (c->p.fft_autotune & 1) TK = tuned_tk<T, NIN, NOUT, DIN, DOUT, Op>(c, axis, pl, op, TK, tag);
     const size_t smem = axis_tile_bytes<T2>(n, NW, TK);
     auto kern = k_axis_pass<T, NIN, NOUT, DIN, DOUT, Op>;
@@ -708,7 +722,9 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     int R = 64;
     while (R > 2 && bytes(R) > kSmemBudget) R >>= 1;
     const long long rows = (long long)c->g.Nx * c->g.Ny;
-    while (R > 4 && (rows + R - 1) / R < 304) R >>= 1;   // two blocks for every SM
+    // two blocks for every SM; six, and down to two rows, where direct sums are the time (axis_tile)
+    const bool direct = pfgb_direct_inputs(c->plz) >= kDirectInputs;
+    while (R > (direct ? 2 : 4) && (rows + R - 1) / R < (direct ? kDirectBlocks : 304)) R >>= 1;
     while (R > 2 && R / 2 >= rows) R >>= 1;
     if (c->p.fft_autotune & 2) R = tuned_r<T, NFI, NFO>(c, R, &zpass_bytes<T, NFI, NFO>, tag);
     const size_t smem = bytes(R);
@@ -2426,7 +2442,7 @@ template <typename TE>
 static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int mode = 0) {
     using T2 = cplx_t<TE>;
     const int n = c->plx.n;
-    const int TK = axis_tile<T2>(n, 6, c->g.kept_rows(), c->g.NzK);
+    const int TK = axis_tile<T2>(c->plx, 6, c->g.kept_rows(), c->g.NzK);
     const size_t smem = axis_tile_bytes<T2>(n, 6, TK);
     const TileDiv ft = tile_div(TK, 6, 6);
     GreenArgs<TE> A;
