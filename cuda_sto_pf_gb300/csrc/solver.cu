@@ -2786,15 +2786,18 @@ static pfgb_status sync_read(pfgb_ctx *c, int first, int count) {
     return PFGB_OK;
 }
 
-// the kept modes (Grid3) one by one: a warp's lanes walk the columns of one
-// (i, kept j) row, the warps of the grid (blockDim = 32 x 8) the rows
+// the kept modes (Grid3) one by one: a warp's lanes walk the columns of one (i,
+// kept j) row, or of several where the columns are fewer than the lanes; the
+// block (32 x 8) and the grid walk the rows
 template <typename F>
 __device__ __forceinline__ void for_kept(const Grid3 &g, F &&f) {
     const int nj = g.kept_rows();
-    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < g.Nx * nj; r += gridDim.x * blockDim.y) {
+    const int lg = g.NzK >= 32 ? 5 : 32 - __clz(g.NzK - 1);   // lanes of a row: 1 << lg
+    const int t = threadIdx.y * 32 + threadIdx.x, rows = 256 >> lg;
+    for (int r = blockIdx.x * rows + (t >> lg); r < g.Nx * nj; r += gridDim.x * rows) {
         const int i = r / nj, j = g.kept_row(r - i * nj);
         const long long o = ((long long)i * g.Ny + j) * g.NzC;
-        for (int k = threadIdx.x; k < g.NzK; k += 32) f(o + k);
+        for (int k = t & ((1 << lg) - 1); k < g.NzK; k += 1 << lg) f(o + k);
     }
 }
 
