@@ -134,6 +134,18 @@ __device__ __forceinline__ void fs_add_square_diff(fsum &s, float p, float q) {
     if (d.lo == 0.f) fs_add_square(s, d.hi);
     else s.x += ((double)p - (double)q) * ((double)p - (double)q);
 }
+// s += a d for a difference d = df_two_sum(p, -q), if it is in the range that the
+// exact products have
+__device__ __forceinline__ bool fs_add_product(fsum &s, float a, dfl d) {
+    const float u = fabsf(a), v = fabsf(d.hi);
+    if (!((u > 0x1p-46f && u < 0x1p48f) || u == 0.f) || !((v > 0x1p-46f && v < 0x1p48f) || v == 0.f)) return false;
+    const dfl p = df_two_prod(a, d.hi), r = df_two_prod(a, d.lo);
+    fs_add_in_range(s, p.hi);
+    fs_add_low(s, p.lo);
+    fs_add_low(s, r.hi);
+    s.l += r.lo;
+    return true;
+}
 __device__ __forceinline__ void fs_merge(fsum &s, const fsum &b) {
     fs_add_in_range(s, b.h);
     fs_add_low(s, b.m);

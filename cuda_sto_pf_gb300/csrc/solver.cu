@@ -3876,11 +3876,33 @@ struct AccMinE {
     }
 };
 
-// (in FP64 per cell; 163 us at 96^3, bound by the FP64 pipe)
+// The same of FP32 fields: the sums of floats and squares on the FP32 pipe, with
+// more bits than FP64 sums (fsum), of a cell's terms in FP64 those that are no such
+// sums.  (All in FP64, 73 instructions of a pipe of 1/64 of the rate: 156 us at
+// 96^3; so, with a quarter of the blocks to reduce, 72 us.)
+struct AccMinEf {
+    static constexpr bool kActive = true;
+    fsum mh, gx, gy, gz, dw;
+    double gel, gelh, chem;
+    __device__ static AccMinEf identity() { return {fs_zero(), fs_zero(), fs_zero(), fs_zero(), fs_zero(), 0, 0, 0}; }
+    __device__ static AccMinEf combine(AccMinEf a, const AccMinEf &b) {
+        fs_merge(a.mh, b.mh); fs_merge(a.gx, b.gx); fs_merge(a.gy, b.gy); fs_merge(a.gz, b.gz); fs_merge(a.dw, b.dw);
+        a.gel += b.gel; a.gelh += b.gelh; a.chem += b.chem;
+        return a;
+    }
+    __device__ static AccMinEf shfl_down(const AccMinEf &a, int o) {
+        const unsigned all = 0xffffffffu;
+        return {fs_shfl_down(a.mh, o), fs_shfl_down(a.gx, o), fs_shfl_down(a.gy, o), fs_shfl_down(a.gz, o),
+                fs_shfl_down(a.dw, o), __shfl_down_sync(all, a.gel, o), __shfl_down_sync(all, a.gelh, o),
+                __shfl_down_sync(all, a.chem, o)};
+    }
+};
 template <typename T, typename TE>
 __global__ void __launch_bounds__(256)
 k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *phi, double g0, int chem, AccMinE *part) {
-    AccMinE a = AccMinE::identity();
+    constexpr bool F64 = sizeof(T) == 8;
+    using Acc = std::conditional_t<F64, AccMinE, AccMinEf>;
+    Acc a = Acc::identity();
     const int Nx = d.g.Nx, Ny = d.g.Ny, Nz = d.g.Nz;
     const double idx2 = 0.5 / cd.dx, idy2 = 0.5 / cd.dy, idz2 = 0.5 / cd.dz;
     for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < d.g.N;
@@ -3891,26 +3913,50 @@ k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *ph
         const int ip = i + 1 == Nx ? 0 : i + 1, im = i == 0 ? Nx - 1 : i - 1;
         const int jp = j + 1 == Ny ? 0 : j + 1, jm = j == 0 ? Ny - 1 : j - 1;
         const int kp = k + 1 == Nz ? 0 : k + 1, km = k == 0 ? Nz - 1 : k - 1;
-        const double gx = (double(phi[((long long)ip * Ny + j) * Nz + k]) - double(phi[((long long)im * Ny + j) * Nz + k])) * idx2;
-        const double gy = (double(phi[((long long)i * Ny + jp) * Nz + k]) - double(phi[((long long)i * Ny + jm) * Nz + k])) * idy2;
-        const double gz = (double(phi[r * Nz + kp]) - double(phi[r * Nz + km])) * idz2;
-        const T p = phi[cell];
-        a.grad += 0.5 * cd.kappa * (gx * gx + gy * gy + gz * gz);
-        a.dw += cd.W * double(pf_g(p));
+        const T px = phi[((long long)ip * Ny + j) * Nz + k], mx = phi[((long long)im * Ny + j) * Nz + k];
+        const T py = phi[((long long)i * Ny + jp) * Nz + k], my = phi[((long long)i * Ny + jm) * Nz + k];
+        const T pz = phi[r * Nz + kp], mz = phi[r * Nz + km], p = phi[cell];
         const T h = pf_h(clamp01(p));
-        a.mh += double(h);
+        if constexpr (F64) {
+            const double gx = (px - mx) * idx2, gy = (py - my) * idy2, gz = (pz - mz) * idz2;
+            a.grad += 0.5 * cd.kappa * (gx * gx + gy * gy + gz * gz);
+            a.dw += cd.W * pf_g(p);
+            a.mh += h;
+        } else {
+            fs_add_square_diff(a.gx, px, mx);
+            fs_add_square_diff(a.gy, py, my);
+            fs_add_square_diff(a.gz, pz, mz);
+            fs_add(a.dw, pf_g(p));
+            fs_add(a.mh, h);
+        }
         // the monitor's composition: sigmoid(Y), capped once clamped
         const T xB = xB_of_Y<T>(c, d.Y[cell] + T(d.Yc));
         const T xm = xB < T(c.xbcap) ? xB : T(c.xbcap);
         if (c.elastic) {
             TE e0[6];
             eigenstrain<T, TE>(c, ec, p, c.gp ? d.eta_old[cell] : T(0), clamp01(xm), c.gp_el != 0, e0);
-            double sd = 0.0;
+            // 1/2 sigma : (eps - e0); shear enters twice
+            TE s[6], e[6];
 #pragma unroll
-            for (int q = 0; q < 6; ++q)
-                sd += (q < 3 ? 1.0 : 2.0) * double(d.sig[q][cell]) * (double(d.eps[q][cell]) - double(e0[q]));
-            a.gel += 0.5 * sd;
-            a.gelh += 0.5 * sd * double(h);
+            for (int q = 0; q < 6; ++q) { s[q] = d.sig[q][cell]; e[q] = d.eps[q][cell]; }
+            double sd = 0.0;
+            bool done = false;
+            if constexpr (!F64) {
+                fsum f = fs_zero();
+                done = true;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    done = fs_add_product(f, q < 3 ? 0.5f * s[q] : s[q], df_two_sum(e[q], -e0[q])) && done;
+                if (done) sd = (double)f.h + ((double)f.m + (double)f.l);
+            }
+            if (!done) {
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    sd += (q < 3 ? 1.0 : 2.0) * double(s[q]) * (double(e[q]) - double(e0[q]));
+                sd *= 0.5;
+            }
+            a.gel += sd;
+            a.gelh += sd * double(h);
         }
         if (chem) {
             const T x = clamp_eps(xm, T(1e-12));
@@ -3921,7 +3967,14 @@ k_min_energy(DevState<T, TE> d, PhysCT<T> c, PhysC cd, ElasC<TE> ec, const T *ph
         }
     }
     block_reduce_acc(a);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
+    if (threadIdx.x == 0) {
+        if constexpr (F64) part[blockIdx.x] = a;
+        else {
+            const double g = idx2 * idx2 * fs_to_double(a.gx) + idy2 * idy2 * fs_to_double(a.gy) +
+                             idz2 * idz2 * fs_to_double(a.gz);
+            part[blockIdx.x] = {fs_to_double(a.mh), 0.5 * cd.kappa * g, cd.W * fs_to_double(a.dw), a.gel, a.gelh, a.chem};
+        }
+    }
 }
 
 // projected KKT residual (:684-708) with the exact multiplier, and |phi - phi^n|^2
@@ -3991,7 +4044,9 @@ k_min_dy(DevState<T, TE> d, PhysCT<T> c, double yc_prev, AccSumMax *part) {
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
 
-static const int kMinBlocks = 1216;   // 8 x 152 SMs
+// blocks of the minimiser's sums: 8 per SM, 2 with FP32 fields, whose sums of three
+// floats cost more to merge than a cell costs to add
+template <typename T> constexpr int kMinBlocks = sizeof(T) == 8 ? 1216 : 304;
 
 // Lap(phi), g_e and the multiplier sums at `phi`; returns -sum h'g / sum h'^2
 template <typename T, typename TE>
@@ -4031,14 +4086,14 @@ static pfgb_status min_step(pfgb_ctx *c, const DevState<T, TE> &d, const T *src,
     return PFGB_OK;
 }
 
-template <typename Acc, typename K, typename... A>
+template <typename T, typename Acc, typename K, typename... A>
 static pfgb_status min_reduce(pfgb_ctx *c, const char *tag, double bytes, int slot, int n, K kern, A... args) {
     {
         ProfScope ps(c, {tag, bytes});
-        kern<<<kMinBlocks, 256, 0, c->stream>>>(args..., (Acc *)c->partials);
+        kern<<<kMinBlocks<T>, 256, 0, c->stream>>>(args..., (Acc *)c->partials);
         PFGB_CUDA_TRY(cudaGetLastError());
     }
-    TRY(reduce_to<Acc>(c, kMinBlocks, slot));
+    TRY(reduce_to<Acc>(c, kMinBlocks<T>, slot));
     TRY(sync_read(c, slot, n));
     return PFGB_OK;
 }
@@ -4071,7 +4126,7 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     thermo_mu_off<double>(c->pc.tc, xref, oA, oB);
     const double muAr = c->pc.tc.GA_s + oA, muBf = c->pc.tc.GB_s + oB;
     const double g0 = (1.0 - xref) * muAr + xref * muBf;
-    TRY((min_reduce<AccMinE>(c, "min_energy", (2.0 * Nf) * sizeof(T) + 12.0 * Nf * sizeof(TE), 42, 6,
+    TRY((min_reduce<T, AccMinE>(c, "min_energy", (2.0 * Nf) * sizeof(T) + 12.0 * Nf * sizeof(TE), 42, 6,
                              k_min_energy<T, TE>, d, pc, c->pc, ec, (const T *)pa, g0, phi_only ? 0 : 1)));
     const double *E = c->hscal + 42;
     double mean_h = E[0] / Nf;
@@ -4112,7 +4167,7 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     // ---- projected KKT residual and rms_dphi at phi^{n+1} ----
     double lk = 0.0;
     TRY((min_gradient<T, TE>(c, d, pb, &lk)));
-    TRY((min_reduce<AccSum2>(c, "min_resid", 4.0 * Nf * sizeof(T), 44, 2, k_min_resid<T, TE>, d, (const T *)pb,
+    TRY((min_reduce<T, AccSum2>(c, "min_resid", 4.0 * Nf * sizeof(T), 44, 2, k_min_resid<T, TE>, d, (const T *)pb,
                              (const T *)pa, P.kappa_phi, lk)));
     const double rms_res = std::sqrt(c->hscal[44] / Nf);
     const double rms_dphi = std::sqrt(c->hscal[45] / Nf) / P.dt;
@@ -4136,7 +4191,7 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
         TRY((min_step<T, TE>(c, d, cur, oth, l)));
         std::swap(cur, oth);
     }
-    TRY((min_reduce<AccSum2>(c, "min_hsums", Nf * sizeof(T), 46, 2, k_min_hsums<T>, (const T *)cur, N)));
+    TRY((min_reduce<T, AccSum2>(c, "min_hsums", Nf * sizeof(T), 46, 2, k_min_hsums<T>, (const T *)cur, N)));
     mean_h = c->hscal[46] / Nf;
 
     // ---- first-order projection of <h> onto V0 ----
@@ -4147,10 +4202,10 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
             const double lc = mhp2 > 1e-30 ? vol_err / mhp2 : 0.0;
             {
                 ProfScope ps(c, {"min_project", 2.0 * Nf * sizeof(T)});
-                k_min_project<T><<<kMinBlocks, 256, 0, c->stream>>>(cur, N, lc);
+                k_min_project<T><<<1216, 256, 0, c->stream>>>(cur, N, lc);
                 PFGB_CUDA_TRY(cudaGetLastError());
             }
-            TRY((min_reduce<AccSum2>(c, "min_hsums", Nf * sizeof(T), 46, 2, k_min_hsums<T>, (const T *)cur, N)));
+            TRY((min_reduce<T, AccSum2>(c, "min_hsums", Nf * sizeof(T), 46, 2, k_min_hsums<T>, (const T *)cur, N)));
             mean_h = c->hscal[46] / Nf;
         }
     }
@@ -4161,7 +4216,7 @@ pfgb_status minimize_once(pfgb_ctx *c, pfgb_min_stats *ms) {
     // minimize, main_cuda.cu:32425-32440, 25262)
     double rms_dY = NAN, xmax = 0.0;
     if (!phi_only) {
-        TRY((min_reduce<AccSumMax>(c, "min_dy", 2.0 * Nf * sizeof(T), 48, 2, k_min_dy<T, TE>, d, phys_as<T>(c->pc),
+        TRY((min_reduce<T, AccSumMax>(c, "min_dy", 2.0 * Nf * sizeof(T), 48, 2, k_min_dy<T, TE>, d, phys_as<T>(c->pc),
                                    c->Yc_prev)));
         rms_dY = std::sqrt(c->hscal[48] / Nf) / P.dt;
         xmax = c->hscal[49];

@@ -4,6 +4,7 @@ range."""
 import ctypes
 import math
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -13,11 +14,13 @@ pytestmark = pytest.mark.gpu
 # one block; its threads' sums are merged as the solver's block reductions do
 SRC = r"""
 #include "dfloat.cuh"
-template <int KIND> __global__ void k_sum(const float *v, const float *q, int n, double *out) {
+template <int KIND> __global__ void k_sum(const float *v, const float *q, const float *w, int n, double *out) {
     __shared__ fsum red[32];
     fsum s = fs_zero();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        if (KIND == 2) fs_add_square_diff(s, v[i], q[i]);
+        if (KIND == 3) {
+            if (!fs_add_product(s, w[i], df_two_sum(v[i], -q[i]))) s.x += (double)w[i] * ((double)v[i] - (double)q[i]);
+        } else if (KIND == 2) fs_add_square_diff(s, v[i], q[i]);
         else KIND ? fs_add_square(s, v[i]) : fs_add(s, v[i]);
     }
     for (int o = 16; o > 0; o >>= 1) fs_merge(s, fs_shfl_down(s, o));
@@ -28,10 +31,11 @@ template <int KIND> __global__ void k_sum(const float *v, const float *q, int n,
         out[0] = fs_to_double(s);
     }
 }
-extern "C" int run(int kind, const float *v, const float *q, int n, double *out) {
-    if (kind == 2) k_sum<2><<<1, 256>>>(v, q, n, out);
-    else if (kind) k_sum<1><<<1, 256>>>(v, q, n, out);
-    else k_sum<0><<<1, 256>>>(v, q, n, out);
+extern "C" int run(int kind, const float *v, const float *q, const float *w, int n, double *out) {
+    if (kind == 3) k_sum<3><<<1, 256>>>(v, q, w, n, out);
+    else if (kind == 2) k_sum<2><<<1, 256>>>(v, q, w, n, out);
+    else if (kind) k_sum<1><<<1, 256>>>(v, q, w, n, out);
+    else k_sum<0><<<1, 256>>>(v, q, w, n, out);
     return (int)cudaDeviceSynchronize();
 }
 """
@@ -47,13 +51,14 @@ def lib(tmp_path_factory):
     return ctypes.CDLL(str(d / "fs.so"))
 
 
-def _sum(lib, v, square, q=None):
+def _sum(lib, v, square, q=None, w=None):
     import torch
-    d, e = [torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).cuda() for x in (v, v if q is None else q)]
+    d = [torch.from_numpy(np.ascontiguousarray(v if x is None else x, dtype=np.float32)).cuda() for x in (v, q, w)]
     out = torch.zeros(1, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
-    p = [ctypes.c_void_p(x.data_ptr()) for x in (d, e, out)]
-    assert lib.run(2 if q is not None else int(square), p[0], p[1], v.size, p[2]) == 0
+    p = [ctypes.c_void_p(x.data_ptr()) for x in (*d, out)]
+    kind = 3 if w is not None else 2 if q is not None else int(square)
+    assert lib.run(kind, p[0], p[1], p[2], v.size, p[3]) == 0
     return out.item()
 
 
@@ -100,3 +105,19 @@ def test_squared_differences(lib, step):
     t = ((p.astype(np.float64) - q.astype(np.float64)) ** 2).tolist()
     want = math.fsum(t)
     assert abs(_sum(lib, p, True, q) - want) <= 2.0 ** -53 * (math.ceil(p.size / 256) + 19) * want
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-3, 1e-11, 1e-30, 1e20])
+def test_products_with_differences(lib, scale):
+    """a (p - q), exact in the sum over the range of its products; two roundings to
+    float64 a term beyond it."""
+    rng = np.random.default_rng(9)
+    n = 4099
+    a = (rng.uniform(-1.0, 1.0, n) * 10.0 ** rng.uniform(-3, 3, n)).astype(np.float32)
+    p = (scale * rng.uniform(-1.0, 1.0, n)).astype(np.float32)
+    q = (scale * rng.uniform(-1.0, 1.0, n) * 10.0 ** rng.uniform(-6, 0, n)).astype(np.float32)
+    t = [Fraction(float(x)) * (Fraction(float(y)) - Fraction(float(z))) for x, y, z in zip(a, p, q)]
+    mag = float(sum(map(abs, t)))
+    err = float(abs(Fraction(_sum(lib, p, False, q, a)) - sum(t)))
+    roundings = 5 if 1e-9 < scale < 1e9 else math.ceil(n / 256) + 19
+    assert err <= 2.0 ** -53 * roundings * mag
