@@ -96,17 +96,22 @@ __device__ __forceinline__ void st8(uint32_t taddr, const float *v) {
                  "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
                  : "memory");
 }
-__device__ __forceinline__ void ld8(uint32_t taddr, float *v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
+// eight columns from each of two addresses.  The loads' registers may not be read,
+// and so not be moved either, before the wait: all are one statement.
+__device__ __forceinline__ void ld8x2(uint32_t ta, uint32_t tb, float *v, float *w) {
+    uint32_t r[8], q[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(q[0]), "=&r"(q[1]), "=&r"(q[2]), "=&r"(q[3]), "=&r"(q[4]), "=&r"(q[5]), "=&r"(q[6]), "=&r"(q[7])
+        : "r"(ta), "r"(tb)
+        : "memory");
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 8; ++i) { v[i] = __uint_as_float(r[i]); w[i] = __uint_as_float(q[i]); }
 }
 __device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
     asm volatile(
@@ -248,9 +253,7 @@ __device__ __forceinline__ void stage_c(float2 *buf, Ctx &c) {
             float dr[8], di[8];
 #pragma unroll
             for (int g = 0; g < 5; ++g) {
-                ld8(c.tmem + lane_base + COL_DRE + 8 * g, dr);
-                ld8(c.tmem + lane_base + COL_DIM + 8 * g, di);
-                wait_ld();
+                ld8x2(c.tmem + lane_base + COL_DRE + 8 * g, c.tmem + lane_base + COL_DIM + 8 * g, dr, di);
                 if (mine && ok) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
