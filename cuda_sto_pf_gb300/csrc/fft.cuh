@@ -164,24 +164,33 @@ template <int DIR, typename T2> __device__ __forceinline__ T2 rot_mi(T2 a) {
     return DIR < 0 ? mk2<T2>(a.y, -a.x) : mk2<T2>(-a.y, a.x);
 }
 
-// complex sums in FP32: one packed instruction for both parts, rounded as two
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return f2x::un(f2x::add(f2x::pk(a), f2x::pk(b))); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return f2x::un(f2x::sub(f2x::pk(a), f2x::pk(b))); }
+// Sums within the butterflies; in FP32 one packed instruction for both parts,
+// rounded as two.  Only for operands that are no products: the compiler cannot
+// fuse a product into these, as it does into cadd and csub, and its own rounding
+// would be one more.  pmad is k a + b, rounded once, for FP32's that are.  (With every
+// sum packed the error of FP32 transforms with radices 3 to 9 was up to 7% larger.)
+template <typename T2> __device__ __forceinline__ T2 padd(T2 a, T2 b) { return cadd(a, b); }
+template <typename T2> __device__ __forceinline__ T2 psub(T2 a, T2 b) { return csub(a, b); }
+__device__ __forceinline__ float2 padd(float2 a, float2 b) { return f2x::un(f2x::add(f2x::pk(a), f2x::pk(b))); }
+__device__ __forceinline__ float2 psub(float2 a, float2 b) { return f2x::un(f2x::sub(f2x::pk(a), f2x::pk(b))); }
+__device__ __forceinline__ float2 pmad(float2 a, float k, float2 b) {
+    return f2x::un(f2x::fma(f2x::pk(a), f2x::both(k), f2x::pk(b)));
+}
 
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly2(cplx_t<T> *v) {
     auto a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
+    v[0] = padd(a, b);
+    v[1] = psub(a, b);
 }
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly4(cplx_t<T> *v) {
-    auto t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-    auto t2 = cadd(v[1], v[3]), t3 = rot_mi<DIR>(csub(v[1], v[3]));
-    v[0] = cadd(t0, t2);
-    v[2] = csub(t0, t2);
-    v[1] = cadd(t1, t3);
-    v[3] = csub(t1, t3);
+    auto t0 = padd(v[0], v[2]), t1 = psub(v[0], v[2]);
+    auto t2 = padd(v[1], v[3]), t3 = rot_mi<DIR>(psub(v[1], v[3]));
+    v[0] = padd(t0, t2);
+    v[2] = psub(t0, t2);
+    v[1] = padd(t1, t3);
+    v[3] = psub(t1, t3);
 }
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly8(cplx_t<T> *v) {
@@ -192,26 +201,32 @@ __device__ __forceinline__ void bfly8(cplx_t<T> *v) {
     bfly4<T, DIR>(o);
     const T r = T(0.70710678118654752440084436210485);
     // W8^1 = r(1 -+ i), W8^2 = -+i, W8^3 = r(-1 -+ i)
-    T2 o1 = DIR < 0 ? mk2<T2>(r * (o[1].x + o[1].y), r * (o[1].y - o[1].x))
-                    : mk2<T2>(r * (o[1].x - o[1].y), r * (o[1].y + o[1].x));
-    T2 o2 = rot_mi<DIR>(o[2]);
-    T2 o3 = DIR < 0 ? mk2<T2>(r * (o[3].y - o[3].x), -r * (o[3].x + o[3].y))
-                    : mk2<T2>(-r * (o[3].x + o[3].y), r * (o[3].x - o[3].y));
-    v[0] = cadd(e[0], o[0]); v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);   v[5] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);   v[6] = csub(e[2], o2);
-    v[3] = cadd(e[3], o3);   v[7] = csub(e[3], o3);
+    const T2 o2 = rot_mi<DIR>(o[2]), r1 = rot_mi<DIR>(o[1]), r3 = rot_mi<DIR>(o[3]);
+    const T2 o1 = padd(o[1], r1), o3 = psub(r3, o[3]);
+    v[0] = padd(e[0], o[0]); v[4] = psub(e[0], o[0]);
+    v[2] = padd(e[2], o2);   v[6] = psub(e[2], o2);
+    if constexpr (sizeof(T) == 4) {
+        v[1] = pmad(o1, r, e[1]); v[5] = pmad(o1, -r, e[1]);
+        v[3] = pmad(o3, r, e[3]); v[7] = pmad(o3, -r, e[3]);
+    } else {
+        v[1] = cadd(e[1], cscale(o1, r)); v[5] = csub(e[1], cscale(o1, r));
+        v[3] = cadd(e[3], cscale(o3, r)); v[7] = csub(e[3], cscale(o3, r));
+    }
 }
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly3(cplx_t<T> *v) {
     using T2 = cplx_t<T>;
     const T s3 = T(0.86602540378443864676372317075294);
-    T2 a = v[0], s = cadd(v[1], v[2]), d = csub(v[1], v[2]);
-    T2 m = mk2<T2>(a.x - T(0.5) * s.x, a.y - T(0.5) * s.y);
-    T2 r = rot_mi<DIR>(cscale(d, s3));
-    v[0] = cadd(a, s);
-    v[1] = cadd(m, r);
-    v[2] = csub(m, r);
+    T2 a = v[0], s = padd(v[1], v[2]), d = psub(v[1], v[2]);
+    const T2 m = mk2<T2>(a.x - T(0.5) * s.x, a.y - T(0.5) * s.y), r = rot_mi<DIR>(d);
+    v[0] = padd(a, s);
+    if constexpr (sizeof(T) == 4) {
+        v[1] = pmad(r, s3, m);
+        v[2] = pmad(r, -s3, m);
+    } else {
+        v[1] = cadd(m, cscale(r, s3));
+        v[2] = csub(m, cscale(r, s3));
+    }
 }
 template <typename T, int DIR>
 __device__ __forceinline__ void bfly5(cplx_t<T> *v) {
@@ -221,17 +236,27 @@ __device__ __forceinline__ void bfly5(cplx_t<T> *v) {
     const T s1 = T(0.95105651629515357211643933337938);
     const T s2 = T(0.58778525229247312916870595463907);
     T2 x0 = v[0];
-    T2 a1 = cadd(v[1], v[4]), b1 = csub(v[1], v[4]);
-    T2 a2 = cadd(v[2], v[3]), b2 = csub(v[2], v[3]);
-    T2 p1 = mk2<T2>(x0.x + c1 * a1.x + c2 * a2.x, x0.y + c1 * a1.y + c2 * a2.y);
-    T2 p2 = mk2<T2>(x0.x + c2 * a1.x + c1 * a2.x, x0.y + c2 * a1.y + c1 * a2.y);
-    T2 q1 = rot_mi<DIR>(mk2<T2>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y));
-    T2 q2 = rot_mi<DIR>(mk2<T2>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y));
-    v[0] = mk2<T2>(x0.x + a1.x + a2.x, x0.y + a1.y + a2.y);
-    v[1] = cadd(p1, q1);
-    v[4] = csub(p1, q1);
-    v[2] = cadd(p2, q2);
-    v[3] = csub(p2, q2);
+    T2 a1 = padd(v[1], v[4]), b1 = psub(v[1], v[4]);
+    T2 a2 = padd(v[2], v[3]), b2 = psub(v[2], v[3]);
+    if constexpr (sizeof(T) == 4) {
+        const T2 p1 = pmad(a2, c2, pmad(a1, c1, x0)), p2 = pmad(a2, c1, pmad(a1, c2, x0));
+        const T2 r1 = rot_mi<DIR>(b1), r2 = rot_mi<DIR>(b2);
+        v[0] = padd(padd(x0, a1), a2);
+        v[1] = pmad(r1, s1, pmad(r2, s2, p1));
+        v[4] = pmad(r1, -s1, pmad(r2, -s2, p1));
+        v[2] = pmad(r1, s2, pmad(r2, -s1, p2));
+        v[3] = pmad(r1, -s2, pmad(r2, s1, p2));
+    } else {
+        T2 p1 = mk2<T2>(x0.x + c1 * a1.x + c2 * a2.x, x0.y + c1 * a1.y + c2 * a2.y);
+        T2 p2 = mk2<T2>(x0.x + c2 * a1.x + c1 * a2.x, x0.y + c2 * a1.y + c1 * a2.y);
+        T2 q1 = rot_mi<DIR>(mk2<T2>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y));
+        T2 q2 = rot_mi<DIR>(mk2<T2>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y));
+        v[0] = mk2<T2>(x0.x + a1.x + a2.x, x0.y + a1.y + a2.y);
+        v[1] = cadd(p1, q1);
+        v[4] = csub(p1, q1);
+        v[2] = cadd(p2, q2);
+        v[3] = csub(p2, q2);
+    }
 }
 
 // Asynchronous global->shared element copy (cp.async, sm_80+): all of a
@@ -266,14 +291,20 @@ __device__ __forceinline__ void bfly6(cplx_t<T> *v) {
     T2 e[3] = {v[0], v[2], v[4]}, o[3] = {v[1], v[3], v[5]};
     bfly3<T, DIR>(e);
     bfly3<T, DIR>(o);
-    const T h = T(0.5), s3 = T(0.86602540378443864676372317075294);
     // W6^1 = (1/2, -+ s3), W6^2 = (-1/2, -+ s3)
-    const T sg = DIR < 0 ? -s3 : s3;
-    T2 o1 = mk2<T2>(h * o[1].x - sg * o[1].y, h * o[1].y + sg * o[1].x);
-    T2 o2 = mk2<T2>(-h * o[2].x - sg * o[2].y, -h * o[2].y + sg * o[2].x);
-    v[0] = cadd(e[0], o[0]); v[3] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);   v[4] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);   v[5] = csub(e[2], o2);
+    const T h = T(0.5), s3 = T(0.86602540378443864676372317075294);
+    v[0] = padd(e[0], o[0]); v[3] = psub(e[0], o[0]);
+    if constexpr (sizeof(T) == 4) {
+        const T2 r1 = rot_mi<DIR>(o[1]), r2 = rot_mi<DIR>(o[2]);
+        v[1] = pmad(o[1], h, pmad(r1, s3, e[1]));    v[4] = pmad(o[1], -h, pmad(r1, -s3, e[1]));
+        v[2] = pmad(o[2], -h, pmad(r2, s3, e[2]));   v[5] = pmad(o[2], h, pmad(r2, -s3, e[2]));
+    } else {
+        const T sg = DIR < 0 ? -s3 : s3;
+        T2 o1 = mk2<T2>(h * o[1].x - sg * o[1].y, h * o[1].y + sg * o[1].x);
+        T2 o2 = mk2<T2>(-h * o[2].x - sg * o[2].y, -h * o[2].y + sg * o[2].x);
+        v[1] = cadd(e[1], o1);   v[4] = csub(e[1], o1);
+        v[2] = cadd(e[2], o2);   v[5] = csub(e[2], o2);
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -49,9 +49,9 @@ __device__ __forceinline__ void bfly_odd(cplx_t<T> *v) {
     T2 a[H], b[H], s = v[0];
 #pragma unroll
     for (int j = 1; j <= H; ++j) {
-        a[j - 1] = cadd(v[j], v[R - j]);
-        b[j - 1] = csub(v[j], v[R - j]);
-        s = cadd(s, a[j - 1]);
+        a[j - 1] = padd(v[j], v[R - j]);
+        b[j - 1] = psub(v[j], v[R - j]);
+        s = padd(s, a[j - 1]);
     }
     const T2 v0 = v[0];
     v[0] = s;
@@ -65,8 +65,8 @@ __device__ __forceinline__ void bfly_odd(cplx_t<T> *v) {
             d = mk2<T2>(d.x + b[j - 1].x * si, d.y + b[j - 1].y * si);
         }
         const T2 e = rot_mi<DIR>(d);   // DIR i d
-        v[k] = cadd(c, e);
-        v[R - k] = csub(c, e);
+        v[k] = padd(c, e);
+        v[R - k] = psub(c, e);
     }
 }
 
@@ -82,15 +82,28 @@ __device__ __forceinline__ void bfly_pq(cplx_t<T> *v) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) w[p][q] = v[p + P * q];
         bfly<T, DIR, Q>(w[p]);
-#pragma unroll
-        for (int q = 1; q < Q; ++q)
-            if (p > 0) {
-                const T co = T(root_c<P * Q>(p * q)), si = T(root_s<P * Q>(p * q));
-                const T sg = DIR < 0 ? -si : si;
-                const T2 x = w[p][q];
-                w[p][q] = mk2<T2>(x.x * co - x.y * sg, x.x * sg + x.y * co);
-            }
     }
+    if constexpr (P == 2 && sizeof(T) == 4) {   // the twiddles' products fused into the last sums
+        v[0] = padd(w[0][0], w[1][0]);
+        v[Q] = psub(w[0][0], w[1][0]);
+#pragma unroll
+        for (int q = 1; q < Q; ++q) {
+            const T co = T(root_c<P * Q>(q)), si = T(root_s<P * Q>(q));
+            const T2 x = w[1][q], r = rot_mi<DIR>(x);
+            v[q] = pmad(x, co, pmad(r, si, w[0][q]));
+            v[q + Q] = pmad(x, -co, pmad(r, -si, w[0][q]));
+        }
+        return;
+    }
+#pragma unroll
+    for (int p = 1; p < P; ++p)
+#pragma unroll
+        for (int q = 1; q < Q; ++q) {
+            const T co = T(root_c<P * Q>(p * q)), si = T(root_s<P * Q>(p * q));
+            const T sg = DIR < 0 ? -si : si;
+            const T2 x = w[p][q];
+            w[p][q] = mk2<T2>(x.x * co - x.y * sg, x.x * sg + x.y * co);
+        }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         T2 u[P];
@@ -332,10 +345,10 @@ __device__ __noinline__ void stage_rader41(LineTile tl, int nb) {
         for (int q = 0; q < 5; ++q) v[q] = lds2(sb + inoff[q], T(0));
         const T2 x0 = lds2(sb, T(0));
         // X_0 = x_0 + sum over the 40 permuted inputs
-        T2 s = cadd(cadd(cadd(v[0], v[1]), cadd(v[2], v[3])), v[4]);
-        s = cadd(s, shfl_x(s, 1, gmask));
-        s = cadd(s, shfl_x(s, 2, gmask));
-        s = cadd(s, shfl_x(s, 4, gmask));
+        T2 s = padd(padd(padd(v[0], v[1]), padd(v[2], v[3])), v[4]);
+        s = padd(s, shfl_x(s, 1, gmask));
+        s = padd(s, shfl_x(s, 2, gmask));
+        s = padd(s, shfl_x(s, 4, gmask));
         // forward FFT40 of a: in-lane DFT5, twiddle, cross-lane DFT8 (DIF)
         bfly5<T, -1>(v);
 #pragma unroll
@@ -354,13 +367,13 @@ __device__ __noinline__ void stage_rader41(LineTile tl, int nb) {
             // w b; lower: a + (w b), upper: a - (w b)
             T2 sv = v[q];                                  // span 1: w = 1
             u = shfl_x(sv, 1, gmask);
-            v[q] = (t & 1) ? csub(u, sv) : cadd(v[q], u);
+            v[q] = (t & 1) ? psub(u, sv) : padd(v[q], u);
             sv = (t & 2) ? cmul(v[q], c2) : v[q];
             u = shfl_x(sv, 2, gmask);
-            v[q] = (t & 2) ? csub(u, sv) : cadd(v[q], u);
+            v[q] = (t & 2) ? psub(u, sv) : padd(v[q], u);
             sv = (t & 4) ? cmul(v[q], c4) : v[q];
             u = shfl_x(sv, 4, gmask);
-            v[q] = (t & 4) ? csub(u, sv) : cadd(v[q], u);
+            v[q] = (t & 4) ? psub(u, sv) : padd(v[q], u);
         }
 #pragma unroll
         for (int q = 1; q < 5; ++q) v[q] = cmulconj(v[q], W[q]);
@@ -370,8 +383,8 @@ __device__ __noinline__ void stage_rader41(LineTile tl, int nb) {
 #pragma unroll
         for (int q = 0; q < 5; ++q)
             sts2(sb + (uint32_t)(oidx[q] * nb * tl.PS),
-                 twmul<DIR>(cadd(x0, v[q]), lds2(tl.tw + oidx[q] * j * (int)sizeof(T2), T(0))));
-        if (t == 0) sts2(sb, cadd(x0, s));
+                 twmul<DIR>(padd(x0, v[q]), lds2(tl.tw + oidx[q] * j * (int)sizeof(T2), T(0))));
+        if (t == 0) sts2(sb, padd(x0, s));
     }
 }
 
