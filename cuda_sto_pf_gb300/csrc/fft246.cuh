@@ -208,9 +208,10 @@ constexpr int Y_NL = 42;          // columns per block of the elastic y pass
 // ---------------------------------------------------------------------------
 // y-axis transform of six spectra in place.  Block (bx, i, s): spectrum s,
 // columns kz = 42 bx .. 42 bx + 41 of x-plane i: 336-byte row segments, and
-// two blocks cover the 82 kept columns of a 246-point z axis.  121 us per pass
-// at 246^3 (21 columns in four blocks per SM: 127 us; three spectra of 16
-// columns in one block, 14 of every 96 lines empty: 133 us).
+// two blocks cover the 82 kept columns of a 246-point z axis.  103 to 108 us per
+// pass at 246^3; 121 us before the packed butterflies, when 21 columns in four
+// blocks per SM took 127 us and three spectra of 16 columns in one block, 14 of
+// every 96 lines empty, 133 us.
 // ---------------------------------------------------------------------------
 template <int DIR>
 __global__ void __launch_bounds__(f246::Eng<f246::Y_NL>::THREADS, f246::Eng<f246::Y_NL>::BLOCKS)
