@@ -272,8 +272,9 @@ __device__ __forceinline__ void dependent_begin() {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
 }
-template <typename T = float, typename... P, typename... A>
-static cudaError_t pfgb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+template <typename... P, typename... A>
+static cudaError_t pfgb_launch_as(bool dependent, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t stream, A &&...args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -283,10 +284,23 @@ static cudaError_t pfgb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = at;
-    cfg.numAttrs = kDependent<T> ? 1 : 0;
+    cfg.numAttrs = dependent ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
     if (e != cudaSuccess) cudaGetLastError();   // reported here, not by the thread's next call
     return e;
+}
+template <typename T = float, typename... P, typename... A>
+static cudaError_t pfgb_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    return pfgb_launch_as(kDependent<T>, kern, grid, block, smem, stream, static_cast<A &&>(args)...);
+}
+// A pass of few blocks with much work each (points of a block's tile) is launched
+// plainly too: early blocks would share the SMs that become free first while others
+// stay empty (FP32 dynamics 1021x8x16, 30 blocks of 1.2 ms in the Green pass: 93 ms
+// with all passes dependent, 46 ms of kernels).  Below that many points a block is
+// shorter than the launch it would wait for.
+constexpr long long kFewBlocks = 152, kHeavyTile = 2048;
+template <typename T> static bool pass_dependent(dim3 grid, long long points) {
+    return kDependent<T> && ((long long)grid.x * grid.y * grid.z > kFewBlocks || points < kHeavyTile);
 }
 
 // ---------------------------------------------------------------------------

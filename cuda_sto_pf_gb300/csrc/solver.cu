@@ -245,7 +245,8 @@ static TileDiv tile_div(int tk, int nin, int nout) {
 // whole blocks from SM to SM: from 32 inputs a point on its passes take many small
 // blocks of a few lines, and single columns where even those leave SMs empty.
 // FP64 transforms, with the rule above / this one: 401x64x64 7.7 / 4.1 ms, 64x379x64
-// 5.1 / 3.2, 128x40x751 20.4 / 17.0; FP32 dynamics 1021x8x16 134 / 82 ms.  Below 32
+// 5.1 / 3.2, 128x40x751 20.4 / 17.0; FP32 dynamics 1021x8x16 134 / 45 ms (with plain
+// launches, pass_dependent).  Below 32
 // inputs the traffic counts: 68x119x51 FP32 dynamics 0.55 / 0.68 of the former engine's.
 constexpr int kDirectInputs = 32, kDirectBlocks = 912, kDirectLines = 2;
 template <typename T2>
@@ -263,7 +264,10 @@ static int axis_tile(const AxisPlan &pl, int arrays, int slabs, int ncol) {
             nblk = std::max(nblk, std::min((blocks + slabs - 1) / slabs, (ncol + columns - 1) / columns));
     };
     at_least(direct ? kDirectBlocks : 304, least);
-    if (direct) at_least(152, 1);
+    // single columns where even those leave SMs empty, of direct passes and long lines
+    // (x_green at 1024x8x16 83 -> 53 us, 512x8x16 41 -> 29; short ones are latency)
+    const int cols = (ncol + nblk - 1) / nblk;
+    if (direct || (sizeof(T2) == 8 && (long long)n * arrays * cols >= 8192)) at_least(152, 1);
     return (ncol + nblk - 1) / nblk;
 }
 
@@ -598,8 +602,8 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
             PFGB_CUDA_TRY(allow_smem(kern, smem));
             dim3 grid((c->g.NzK + TCW - 1) / TCW, axis == 1 ? c->g.Nx : c->g.kept_rows());
             ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-            PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, smem, c->stream, c->g, axis,
-                                      (const float2 *)twp<T>(c, axis == 1 ? 1 : 0), io, op, c->skip));
+            PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<T>(grid, E::NL * n), kern, grid, E::THREADS, smem, c->stream, c->g,
+                                         axis, (const float2 *)twp<T>(c, axis == 1 ? 1 : 0), io, op, c->skip));
             return PFGB_OK;
         }
     }
@@ -613,8 +617,9 @@ static pfgb_status launch_axis(pfgb_ctx *c, int axis, AxisIO<T, NIN, NOUT> io, O
     dim3 grid((c->g.NzK + TK - 1) / TK, axis == 1 ? c->g.Nx : c->g.kept_rows(), Op::kInplace ? NIN : 1);
     const TileDiv ft = tile_div(TK, Op::kInplace ? 1 : NIN, Op::kInplace ? 1 : NOUT);
     ProfScope ps(c, {tag, axis_bytes<T2>(c, axis, NIN, NOUT, DIN)});
-    PFGB_CUDA_TRY(pfgb_launch<T>(kern, grid, pfgb_line_threads(pl, NW * TK), smem, c->stream, c->g, axis, pl,
-                              twp<T>(c, axis == 1 ? 1 : 0), ft, io, op, c->skip));
+    PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<T>(grid, (long long)NW * TK * n), kern, grid,
+                                 pfgb_line_threads(pl, NW * TK), smem, c->stream, c->g, axis, pl,
+                                 twp<T>(c, axis == 1 ? 1 : 0), ft, io, op, c->skip));
     return PFGB_OK;
 }
 
@@ -712,8 +717,8 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
             const long long rows = (long long)c->g.Nx * c->g.Ny;
             const int nb = (int)((rows + R - 1) / R);
             ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-            PFGB_CUDA_TRY(pfgb_launch(kern, nb, E::THREADS, smem, c->stream, c->g, (const float2 *)twp<T>(c, 2), op,
-                                      c->skip));
+            PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<T>(nb, E::NL * n), kern, nb, E::THREADS, smem, c->stream, c->g,
+                                         (const float2 *)twp<T>(c, 2), op, c->skip));
             if (nblocks) *nblocks = nb;
             return PFGB_OK;
         }
@@ -732,8 +737,9 @@ static pfgb_status launch_z(pfgb_ctx *c, Op op, const char *tag, double extra_by
     PFGB_CUDA_TRY(allow_smem(kern, smem));
     const int nb = (int)((rows + R - 1) / R);
     ProfScope ps(c, {tag, (double)(NFI + NFO) * c->g.cols() * sizeof(T2) + extra_bytes});
-    PFGB_CUDA_TRY(pfgb_launch<T>(kern, nb, pfgb_line_threads(c->plz, zpass_lines<NFI, NFO>(R)), smem, c->stream, c->g,
-                              c->plz, twp<T>(c, 2), R, op, zdiv<NFI, NFO>(c->g, R), c->skip));
+    const int lines = zpass_lines<NFI, NFO>(R);
+    PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<T>(nb, (long long)lines * n), kern, nb, pfgb_line_threads(c->plz, lines),
+                                 smem, c->stream, c->g, c->plz, twp<T>(c, 2), R, op, zdiv<NFI, NFO>(c->g, R), c->skip));
     if (nblocks) *nblocks = nb;
     return PFGB_OK;
 }
@@ -2464,17 +2470,19 @@ static pfgb_status launch_green(pfgb_ctx *c, bool eigen, int resid, int mode = 0
     A.res = resid_args(c);
     A.mode = mode;
     dim3 grid((c->g.NzK + TK - 1) / TK, c->g.kept_rows());
+    const bool dep = pass_dependent<TE>(grid, 6LL * TK * n);
+    const int nt = pfgb_line_threads(c->plx, 6 * TK);
     // reads 6 source spectra (+3 old u for the residual), writes 3 u + 6 strain spectra
     ProfScope ps(c, {eigen ? "x_green_eigen" : "x_green_hij",
                      (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(T2)});
     if (eigen) {
         auto kern = k_x_green<TE, true>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        PFGB_CUDA_TRY(pfgb_launch<TE>(kern, grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream, A, c->plx, ft));
+        PFGB_CUDA_TRY(pfgb_launch_as(dep, kern, grid, nt, smem, c->stream, A, c->plx, ft));
     } else {
         auto kern = k_x_green<TE, false>;
         PFGB_CUDA_TRY(allow_smem(kern, smem));
-        PFGB_CUDA_TRY(pfgb_launch<TE>(kern, grid, pfgb_line_threads(c->plx, 6 * TK), smem, c->stream, A, c->plx, ft));
+        PFGB_CUDA_TRY(pfgb_launch_as(dep, kern, grid, nt, smem, c->stream, A, c->plx, ft));
     }
     PFGB_CUDA_TRY(cudaGetLastError());
     return PFGB_OK;
@@ -2697,7 +2705,8 @@ static pfgb_status launch_y246(pfgb_ctx *c, const char *tag) {
     for (int i = 0; i < 6; ++i) { io.in[i] = (const float2 *)c->E[i]; io.out[i] = (float2 *)c->E[i]; }
     dim3 grid((c->g.NzK + E::NL - 1) / E::NL, c->g.Nx, 6);
     ProfScope ps(c, {tag, axis_bytes<float2>(c, 1, 6, 6, DIR)});
-    PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, smem, c->stream, c->g, (const float2 *)c->tw[1][1], io, c->skip));
+    PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<float>(grid, E::NL * f246::N), kern, grid, E::THREADS, smem, c->stream,
+                                 c->g, (const float2 *)c->tw[1][1], io, c->skip));
     return PFGB_OK;
 }
 
@@ -2728,7 +2737,7 @@ static pfgb_status launch_green246(pfgb_ctx *c, bool eigen, int resid, int mode 
                      (double)(6 + 3 + 6 + green_extra(c, mode, resid)) * c->g.kept() * sizeof(float2)});
     auto go = [&](auto kern, size_t sm) -> pfgb_status {
         PFGB_CUDA_TRY(allow_smem(kern, sm));
-        PFGB_CUDA_TRY(pfgb_launch(kern, grid, E::THREADS, sm, c->stream, A));
+        PFGB_CUDA_TRY(pfgb_launch_as(pass_dependent<float>(grid, E::NL * f246::N), kern, grid, E::THREADS, sm, c->stream, A));
         return PFGB_OK;
     };
     if (c->tc_x)   // the 41-point stages on the tensor cores
